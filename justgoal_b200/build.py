@@ -38,7 +38,7 @@ def build(force: bool = False, verbose: bool = False, out: str = None) -> str:
     cmd = [_nvcc(), "-std=c++17", "-O3", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
            "-shared", "-Xcompiler", "-fPIC", "-I", os.path.join(HERE, "..", "include"),
            "-o", out or LIB] + [os.path.join(CSRC, s) for s in SOURCES]
-    extra = os.environ.get("B200MOE_NVCC_FLAGS")      # e.g. -DB200MOE_ENABLE_ABLATE for timing experiments
+    extra = os.environ.get("B200MOE_NVCC_FLAGS")      # e.g. -DB200MOE_ENABLE_KLOG for the per-K-block log
     if extra:
         cmd[1:1] = extra.split()
     if verbose:

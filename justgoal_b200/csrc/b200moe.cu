@@ -35,7 +35,6 @@ struct b200moe_ctx {
     int prof_slots;            // 0 = profiling off
     long long prof_calls;      // forwards recorded since profiling was enabled
     cudaEvent_t* prof_events;  // [prof_slots][PROF_POINTS]
-    int ablate;                // B200MOE_ABLATE environment variable at create (timing experiments; 0 in normal use)
     unsigned long long wait_limit_ns;   // limit of the waits on a PEER (barrier flags); b200moe_set_wait_limit_ns
     int pair_grid[2];          // CTAs of the SM-pair kernels (GEMM1, GEMM2): 2 x clusters that can be resident; 0 = unusable
     int token_tile;            // b200moe_set_token_tile: 0 = chosen from the token count, else 16 / 32 / 64 / 128
@@ -472,7 +471,6 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     }
     g1.sk_count = reinterpret_cast<int*>(ws + L.sk_count);
     g1.sk_partial = reinterpret_cast<float*>(ws + L.sk_partial);
-    g1.ablate = h->ablate & 0xFF;
     g1.trace = reinterpret_cast<long long*>(ws + L.trace);
     g1.klog = g1.trace + (size_t)2 * h->num_sms * TRACE_SLOTS;
     if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
@@ -490,7 +488,6 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g2.evict_first_weights = evf && ntok < 128;
     g2.sk_count = reinterpret_cast<int*>(ws + L.sk_count) + 4 * h->num_sms + 4;
     g2.sk_partial = g1.sk_partial;
-    g2.ablate = (h->ablate >> 8) & 0xFF;
     g2.trace = g1.trace + (size_t)h->num_sms * TRACE_SLOTS;
     g2.klog = g1.klog + 8 * KLOG_N;
     // Optional (b200moe_set_fused_combine): the operator's own forward with narrow token tiles lets the GEMM2 unit that
@@ -598,12 +595,6 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
         delete h;
         return rc_p;
     }
-#ifdef B200MOE_ENABLE_ABLATE
-    const char* ab = getenv("B200MOE_ABLATE");
-    h->ablate = ab ? atoi(ab) : 0;
-#else
-    h->ablate = 0;      // the timing switches exist only in builds made for timing experiments
-#endif
     *out = h;
     return 0;
 }

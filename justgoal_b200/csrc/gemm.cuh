@@ -100,9 +100,6 @@ struct GemmParams {
     int* tok_count;
     const int32_t* row_token; const int32_t* pair_row; const int32_t* c_topk;
     int c_stride, top_k, T, c_local_offset;
-    int ablate;           // timing experiments only, builds with -DB200MOE_ENABLE_ABLATE (results are wrong when
-                          // non-zero): 1 = issue no MMA, 2 = narrow-tile promotion skips tcgen05.ld/FMA, 4 = producer
-                          // skips the token-side loads, 8 = the MMA warp consumes the stages alone
 };
 
 template <int NTOK, bool G1>
@@ -314,11 +311,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 8) + 15) & ~uintptr_t(15));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#ifdef B200MOE_ENABLE_ABLATE
-    const int kAblate = p.ablate;      // timing experiments (build with -DB200MOE_ENABLE_ABLATE)
-#else
-    constexpr int kAblate = 0;         // the ablation branches compile away in the product build
-#endif
     const long long t_entry = clock64();
     long long* const trace = p.trace ? p.trace + (size_t)blockIdx.x * TRACE_SLOTS : nullptr;
     auto stamp = [&](int slot) { if (trace) trace[slot] = clock64() - t_entry; };
@@ -520,7 +512,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
-                    mbar_arrive_expect_tx(full, (kAblate & 4) ? C::NA * C::A_BYTES : C::TX_BYTES);
+                    mbar_arrive_expect_tx(full, C::TX_BYTES);
                     if (p.evict_first_weights) {
                         tma_load_2d_hint(st, &tm_w, kb * 128, wrow, full, pol);
                         tma_load_2d_hint(st + C::A_BYTES, &tm_w, kb * 128, wrow + p.gate_offset, full, pol);
@@ -539,7 +531,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     for (int i = 0; i < 32; ++i) reinterpret_cast<int4*>(s_g4)[i] = __ldg(src + i);
                 }
                 auto load_tokens = [&](int s_, int kb) {
-                    if (kAblate & 4) return;
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
                     if (g4) {
@@ -600,15 +591,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             WorkItem wi;
             while (ok && wq_fetch(n_item++, wi, ok, false)) {
                 const int gb = wi.gb, ge = wi.ge;
-                if (kAblate & 8) {      // timing experiment: consume stages directly, no MMA, no TMEM hand-off
-                    const int kb_end = min(p.KB, ge * C::KPB);
-                    for (int kb = gb * C::KPB; kb < kb_end && ok; ++kb) {
-                        if (!mbar_wait(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL)) { ok = false; break; }
-                        for (int i = 0; i < C::EMPTY_COUNT; ++i) mbar_arrive(bar_empty + 8 * stage);
-                        if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-                    }
-                    continue;
-                }
                 for (int grp = gb; grp < ge && ok; ++grp) {
                     if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
                     const int nj = min(C::KPB, p.KB - grp * C::KPB);
@@ -625,8 +607,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             if (C::TOK_ON_M) umma_f8(dd, tdesc, wdesc, idesc, accum);
                             else umma_f8(dd, wdesc, tdesc, idesc, accum);
                         };
-                        if (kAblate & 1) {
-                        } else if (C::TOK_ON_M) {
+                        if (C::TOK_ON_M) {
                             // The two weight tiles of a stage are adjacent in shared memory (256 rows of 128 B)
                             // and so are their accumulators in TMEM: ONE N = 256 MMA per 32-byte K step covers
                             // both.  (An N = 128 MMA reads 8 KB of operands per 64 tensor-pipe cycles, all the
@@ -734,7 +715,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         int n_item = 0;
         WorkItem wi;
         while (ok && wq_fetch(n_item++, wi, ok, true)) {
-            if (kAblate & 8) continue;          // timing experiment: the MMA warp consumes the stages alone
             const int u = wi.u, gb = wi.gb, ge = wi.ge;
             Unit un;
             if (!decode_unit(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
@@ -779,7 +759,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if (C::TOK_ON_M) stokn = __ldcg(tsp + (size_t)min(kb0 + 1, p.KB - 1) * (G4 ? p.ts_stride : p.rows_cap));
                 const int st0 = stage;
                 float scr[C::EARLY_SCALES ? C::KPB : 1][C::EARLY_SCALES ? C::NC : 1];
-                if (C::EARLY_SCALES && !(kAblate & 2)) {
+                if (C::EARLY_SCALES) {
 #pragma unroll
                     for (int j = 0; j < C::KPB; ++j) {
                         if (j < nj) {
@@ -865,14 +845,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                 }
                 float part[2][C::CH];
-                if (!C::TOK_ON_M && !(kAblate & 2)) tmem_ld_chunk<C::CH>(tbuf, part[0]);
+                if (!C::TOK_ON_M) tmem_ld_chunk<C::CH>(tbuf, part[0]);
 #pragma unroll
                 for (int k = 0; k < NK; ++k) {
                     const int sp = k % C::NSPLIT;
                     const int a = (k / C::NSPLIT) % C::NACCUM;
                     const int ch = (k / (C::NSPLIT * C::NACCUM)) % NCH;
                     const int j = k / (C::NSPLIT * C::NACCUM * NCH);
-                    if (j < nj && !(kAblate & 2)) {
+                    if (j < nj) {
                         tmem_wait_ld();
                         if (k + 1 < NK) {
                             const int sp1 = (k + 1) % C::NSPLIT;
@@ -925,7 +905,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 }
                 if (!C::TOK_ON_M && lane == 0) {
                     mbar_arrive(bar_tempty + 8 * ab);
-                    if (C::SCALES_IN_STAGE && (!C::EARLY_SCALES || (kAblate & 2))) {
+                    if (C::SCALES_IN_STAGE && !C::EARLY_SCALES) {
                         for (int j = 0; j < nj; ++j) {
                             int sj = st0 + j; if (sj >= C::STAGES) sj -= C::STAGES;
                             mbar_arrive(bar_empty + 8 * sj);
