@@ -310,7 +310,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
     int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 8) + 15) & ~uintptr_t(15));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform for the compiler too
     const long long t_entry = clock64();
     long long* const trace = p.trace ? p.trace + (size_t)blockIdx.x * TRACE_SLOTS : nullptr;
     auto stamp = [&](int slot) { if (trace) trace[slot] = clock64() - t_entry; };
@@ -395,16 +395,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     const int sched_U0 = sched_q * (int)gridDim.x;                 // first chunked unit
     int* const claim = p.sk_count + 4 * (int)gridDim.x;
 
-    // Consumer side of the work queue: item n sits in slot n % WQ.  WARP: every lane of the calling warp waits and
-    // reads, lane 0 then tells the producer that the warp has its copy; otherwise the caller is a single thread.
-    // false = list ended or a wait gave up.
-    auto wq_fetch = [&](int n, WorkItem& w, bool& ok, bool whole_warp) -> bool {
+    // Consumer side of the work queue: item n sits in slot n % WQ.  Every lane of the calling warp waits and reads,
+    // lane 0 then tells the producer that the warp has its copy.  false = list ended or a wait gave up.
+    auto wq_fetch = [&](int n, WorkItem& w, bool& ok) -> bool {
         const int slot = n % C::WQ;
         if (!mbar_wait(bar_wqfull + 8 * slot, (uint32_t)(n / C::WQ) & 1u, p.status, ERR_WAIT_GROUP)) { ok = false; return false; }
         const volatile int* q = s_wq + slot * 8;
         w.u = q[0]; w.gb = q[1]; w.ge = q[2]; w.kind = q[3]; w.ut = q[4]; w.slot = q[5]; w.nwait = q[6];
-        if (whole_warp) __syncwarp();
-        if (!whole_warp || lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
         return w.u >= 0;
     };
 
@@ -414,8 +413,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::CTRL_REGS));
     }
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        // ------------------------------------------------------------ TMA producer: the whole warp runs the loop, one
+        // elected lane issues (see elect_one)
+        {
             const uint64_t pol = policy_evict_first();
             // Chunk size of the left-over units: about two chunks per CTA in total, never below CHUNK_GROUPS groups.  A few
             // left-over units are cut finely so that every CTA gets a piece; many are cut into two or three chunks each
@@ -426,8 +426,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     const int per_unit = (2 * (int)gridDim.x + (total_units - sched_U0) - 1) / (total_units - sched_U0);
                     chunk_groups = max(chunk_groups, (NG + per_unit - 1) / per_unit);
                 }
-                s_flag[4] = chunk_groups;
-                s_flag[5] = (NG + chunk_groups - 1) / chunk_groups;           // chunks per chunked unit
+                if (lane == 0) {
+                    s_flag[4] = chunk_groups;
+                    s_flag[5] = (NG + chunk_groups - 1) / chunk_groups;       // chunks per chunked unit
+                }
+                __syncwarp();
             }
             // (kept in shared memory between the rare claims rather than in registers for the whole loop)
             volatile int* const s_sched = s_flag + 4;
@@ -441,9 +444,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             auto publish = [&](const WorkItem& w) -> bool {
                 const int slot = n_item % C::WQ;
                 if (!mbar_wait(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
-                volatile int* q = s_wq + slot * 8;
-                q[0] = w.u; q[1] = w.gb; q[2] = w.ge; q[3] = w.kind; q[4] = w.ut; q[5] = w.slot; q[6] = w.nwait;
-                mbar_arrive(bar_wqfull + 8 * slot);          // release: the item is visible to whoever sees the phase flip
+                if (lane == 0) {
+                    volatile int* q = s_wq + slot * 8;
+                    q[0] = w.u; q[1] = w.gb; q[2] = w.ge; q[3] = w.kind; q[4] = w.ut; q[5] = w.slot; q[6] = w.nwait;
+                    mbar_arrive(bar_wqfull + 8 * slot);      // release: the item is visible to whoever sees the phase flip
+                }
+                __syncwarp();
                 ++n_item;
                 return true;
             };
@@ -487,7 +493,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     wi.u = n_whole * (int)gridDim.x + (int)blockIdx.x; wi.gb = 0; wi.ge = NG;
                     ++n_whole;
                 } else {
-                    const int c = (!C::STATIC_TAIL && total_chunks > 0) ? atomicAdd(claim, 1) : total_chunks;
+                    int c = total_chunks;
+                    if (!C::STATIC_TAIL && total_chunks > 0) {
+                        if (lane == 0) c = atomicAdd(claim, 1);
+                        c = __shfl_sync(0xFFFFFFFFu, c, 0);
+                    }
                     if (c >= total_chunks) { wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break; }
                     const int chunk_groups = s_sched[0], CPU_ = s_sched[1];
                     wi.ut = c / CPU_;
@@ -505,9 +515,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const int u = wi.u, gb = wi.gb, ge = wi.ge;
                 Unit un;
                 if (!decode_unit(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) {
-                    atomicCAS(p.status, 0, ERR_BAD_SCHEDULE); ok = false; break;
+                    if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
+                    ok = false; break;
                 }
-                const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows;
+                // from here on the coordinates are warp-uniform in the compiler's eyes as well
+                un.row0 = __shfl_sync(0xFFFFFFFFu, un.row0, 0);
+                const int wrow = __shfl_sync(0xFFFFFFFFu, un.e * p.rows_per_expert + un.mt * p.unit_rows, 0);
                 const int kb_end = min(p.KB, ge * C::KPB);
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
@@ -528,7 +541,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     // row index outside the tensor reads zeros)
                     const int4* src = reinterpret_cast<const int4*>(p.g4_row_token + un.row0);
 #pragma unroll 1
-                    for (int i = 0; i < 32; ++i) reinterpret_cast<int4*>(s_g4)[i] = __ldg(src + i);
+                    for (int i = lane; i < 32; i += 32) reinterpret_cast<int4*>(s_g4)[i] = __ldg(src + i);
+                    __syncwarp();
                 }
                 auto load_tokens = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
@@ -551,25 +565,35 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the front end still
                     // permutes and gathers, then the wait for it, then the token side of the same stages
                     const int npre = min(C::STAGES, kb_end - kb_first);
-                    for (int i = 0; i < npre; ++i) load_weights(i, kb_first + i);
-                    stamp(TR_TMA_FIRST); issued = true;
+                    for (int i = 0; i < npre; ++i) {
+                        if (elect_one()) load_weights(i, kb_first + i);
+                        __syncwarp();
+                    }
+                    if (lane == 0) stamp(TR_TMA_FIRST);
+                    issued = true;
                     pdl_wait();
                     waited = true;
-                    for (int i = 0; i < npre; ++i) { load_tokens(i, kb_first + i); klog_put(0, nk++); }
+                    for (int i = 0; i < npre; ++i) {
+                        if (elect_one()) load_tokens(i, kb_first + i);
+                        __syncwarp();
+                        if (lane == 0) klog_put(0, nk);
+                        ++nk;
+                    }
                     kb_first += npre;
                     stage = npre;
                     if (stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
                 for (int kb = kb_first; kb < kb_end; ++kb) {
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
-                    load_weights(stage, kb);
-                    load_tokens(stage, kb);
-                    if (!issued) { stamp(TR_TMA_FIRST); issued = true; }
-                    klog_put(0, nk++);
+                    if (elect_one()) { load_weights(stage, kb); load_tokens(stage, kb); }
+                    __syncwarp();
+                    if (!issued) { if (lane == 0) stamp(TR_TMA_FIRST); issued = true; }
+                    if (lane == 0) klog_put(0, nk);
+                    ++nk;
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
-            stamp(TR_TMA_LAST);
+            if (lane == 0) stamp(TR_TMA_LAST);
             if (!ok) {
                 // gave up: end the list for the other roles (if the queue still moves), then give copies that are
                 // still in flight time to land before the CTA's shared memory goes away
@@ -580,8 +604,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // ------------------------------------------------------------ MMA issuer (whole warp, one elected lane issues)
+        {
             constexpr uint32_t idesc = make_idesc_f8(128, NTOK);
             int stage = 0; uint32_t phase = 0;
             int ab = 0; uint32_t aphase = 0;
@@ -589,16 +613,17 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int nk = 0;
             int n_item = 0;
             WorkItem wi;
-            while (ok && wq_fetch(n_item++, wi, ok, false)) {
+            while (ok && wq_fetch(n_item++, wi, ok)) {
                 const int gb = wi.gb, ge = wi.ge;
                 for (int grp = gb; grp < ge && ok; ++grp) {
                     if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
                     const int nj = min(C::KPB, p.KB - grp * C::KPB);
                     for (int j = 0; j < nj; ++j) {
-                        klog_put(6, nk);
+                        if (lane == 0) klog_put(6, nk);
                         if (!mbar_wait(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL)) { ok = false; break; }
-                        if (!seen) { stamp(TR_MMA_FIRST); seen = true; }
-                        klog_put(1, nk++);
+                        if (!seen) { if (lane == 0) stamp(TR_MMA_FIRST); seen = true; }
+                        if (lane == 0) klog_put(1, nk);
+                        ++nk;
                         tc_fence_after();
                         const uint32_t st = smem_base + stage * C::STAGE_BYTES;
                         const uint32_t d = tmem_base + ab * C::BUFCOLS + j * C::CPB;
@@ -607,6 +632,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             if (C::TOK_ON_M) umma_f8(dd, tdesc, wdesc, idesc, accum);
                             else umma_f8(dd, wdesc, tdesc, idesc, accum);
                         };
+                        if (elect_one()) {
                         if (C::TOK_ON_M) {
                             // The two weight tiles of a stage are adjacent in shared memory (256 rows of 128 B)
                             // and so are their accumulators in TMEM: ONE N = 256 MMA per 32-byte K step covers
@@ -650,14 +676,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             }
                         }
                         umma_commit(bar_empty + 8 * stage);
+                        if (j + 1 == nj) umma_commit(bar_tfull + 8 * ab);
+                        }
+                        __syncwarp();
                         if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                     }
                     if (!ok) break;
-                    umma_commit(bar_tfull + 8 * ab);
                     if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
                 }
             }
-            stamp(TR_MMA_LAST);
+            if (lane == 0) stamp(TR_MMA_LAST);
         }
         __syncwarp();
     } else if (!G1 && p.fuse_out) {
@@ -714,7 +742,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 
         int n_item = 0;
         WorkItem wi;
-        while (ok && wq_fetch(n_item++, wi, ok, true)) {
+        while (ok && wq_fetch(n_item++, wi, ok)) {
             const int u = wi.u, gb = wi.gb, ge = wi.ge;
             Unit un;
             if (!decode_unit(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
