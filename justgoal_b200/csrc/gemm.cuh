@@ -178,8 +178,11 @@ struct GemmCfg {
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
     static constexpr int TABLE_INTS = 3 * (MAX_LOCAL + 1);
     static constexpr int RED_BYTES = NPW * NC * 4;
+    static constexpr int TSD = 8;                          // tokens-on-M: slots of the token-scale ring (see the scale warps)
+    static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
+    static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
     static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * 32 /*work queue*/ +
-                                      TABLE_INTS * 4 + RED_BYTES + 32 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/;
+                                      TABLE_INTS * 4 + RED_BYTES + 32 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
     static_assert(NTOK % 16 == 0 && NTOK >= 16 && NTOK <= 128, "token tile");
     static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "tmem");
     static_assert(STAGES >= KPB + 1, "a group must fit the stage ring with room to prefetch");
@@ -309,6 +312,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_flag = reinterpret_cast<int*>(s_red + C::NPW * C::NC);   // 8 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
     int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 8) + 15) & ~uintptr_t(15));
+    float2* s_sx = reinterpret_cast<float2*>(s_g4 + 128);          // tokens-on-M: [NACC][128] products of token and weight scale
+    float* s_ts = reinterpret_cast<float*>(s_sx + C::NACC * 128);  // ... and [TSD][128] token scales on their way
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform for the compiler too
     const long long t_entry = clock64();
@@ -333,10 +338,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, C::EMPTY_COUNT); }
-        for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1); mbar_init(bar_tempty + 8 * b, C::NPW); }
+        for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1 + C::NHELP); mbar_init(bar_tempty + 8 * b, C::NPW); }
         for (int g = 0; g < 4; ++g) mbar_init(bar_red + 8 * g, 4);
         mbar_init(bar_all, C::NPW);
-        for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + C::NPW); }
+        for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + C::NHELP + C::NPW); }
         mbar_fence_init();
         tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_b0);
         if (!G1) tma_prefetch_desc(&tm_b1);
@@ -521,7 +526,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 // from here on the coordinates are warp-uniform in the compiler's eyes as well
                 un.row0 = __shfl_sync(0xFFFFFFFFu, un.row0, 0);
                 const int wrow = __shfl_sync(0xFFFFFFFFu, un.e * p.rows_per_expert + un.mt * p.unit_rows, 0);
-                const int kb_end = min(p.KB, ge * C::KPB);
+                const int kb_end = __shfl_sync(0xFFFFFFFFu, min(p.KB, ge * C::KPB), 0);
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
@@ -560,7 +565,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (C::SCALES_IN_STAGE)
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
-                int kb_first = gb * C::KPB;
+                int kb_first = __shfl_sync(0xFFFFFFFFu, gb * C::KPB, 0);
                 if (G1 && !waited) {
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the front end still
                     // permutes and gathers, then the wait for it, then the token side of the same stages
@@ -614,8 +619,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int n_item = 0;
             WorkItem wi;
             while (ok && wq_fetch(n_item++, wi, ok)) {
-                const int gb = wi.gb, ge = wi.ge;
-                for (int grp = gb; grp < ge && ok; ++grp) {
+                const int gb = __shfl_sync(0xFFFFFFFFu, wi.gb, 0), ge = __shfl_sync(0xFFFFFFFFu, wi.ge, 0);      // uniform for the compiler
+                for (int grp = gb; grp < ge; ++grp) {
                     if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
                     const int nj = min(C::KPB, p.KB - grp * C::KPB);
                     for (int j = 0; j < nj; ++j) {
@@ -688,6 +693,75 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if (lane == 0) stamp(TR_MMA_LAST);
         }
         __syncwarp();
+    } else if constexpr (C::TOK_ON_M) {
+        // ------------------------------------------------------------ scale warps (2 and 3), tokens on M: for every K block
+        // the products token scale x weight scale of both weight tiles, one float2 per token row, into the buffer that
+        // belongs to the block's accumulator.  They count in on the same barrier as the MMA commit, so the promotion
+        // warps - the busiest role: ~600 cycles of TMEM loads and FMAs per 128 x 256 block with two warps per scheduler
+        // and nothing to hide a wait behind - have one wait and one shared-memory load per block instead of three
+        // global loads (their latency under load is longer than a block) and the products.
+        // Token scales travel through a ring of asynchronous copies TSD - 1 blocks ahead (a thread reads back only what it
+        // copied itself); the weight scales of 64 K blocks sit in the lanes and are handed out by shuffles.
+        const int h = threadIdx.x - 64;                // this thread: rows h and h + 64
+        const uint32_t ring = smem_u32(s_ts + h);
+        int ab = 0; uint32_t aphase = 0;
+        bool ok = true;
+        int n_item = 0;
+        WorkItem wi;
+        while (ok && wq_fetch(n_item++, wi, ok)) {
+            const int gb = wi.gb, ge = wi.ge;
+            Unit un;
+            if (!decode_unit(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
+            // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
+            const int srow0 = un.mt * (p.unit_rows >> 7);
+            const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
+            const float* ws0 = p.w_scale + ((size_t)un.e * p.scale_rows + srow0) * p.KB;
+            const float* ws1 = p.w_scale + ((size_t)un.e * p.scale_rows + srow1) * p.KB;
+            const float* ts[2];
+            const int ts_stride = G4 ? p.ts_stride : p.rows_cap;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                ts[r] = p.b_scale + (size_t)un.row0 + h + 64 * r;
+                if (G4) {
+                    const int tok = __ldg(p.g4_row_token + un.row0 + h + 64 * r);
+                    ts[r] = p.g4_scale + (tok >= 0 && tok < p.g4_T ? (size_t)tok * (unsigned)p.g4_tok_stride : 0);   // any finite scale for a row of zeros
+                }
+            }
+            auto ts_fetch = [&](int kb) {
+                if (kb < ge) {                          // nothing past the piece's end: no copy is left in flight for the next piece
+                    const uint32_t dst = ring + (uint32_t)((kb % C::TSD) * 128 * 4);
+                    cp_async4(dst, ts[0] + (size_t)kb * ts_stride);
+                    cp_async4(dst + 64 * 4, ts[1] + (size_t)kb * ts_stride);
+                }
+                cp_async_commit();
+            };
+            float wl[2][2];                             // [weight tile][K blocks 0-31 / 32-63 of the window]
+            auto ws_window = [&](int kb) {
+                const int k0 = min((kb & ~63) + lane, p.KB - 1), k1 = min((kb & ~63) + 32 + lane, p.KB - 1);
+                wl[0][0] = __ldg(ws0 + k0); wl[0][1] = __ldg(ws0 + k1);
+                wl[1][0] = __ldg(ws1 + k0); wl[1][1] = __ldg(ws1 + k1);
+            };
+#pragma unroll
+            for (int i = 0; i < C::TSD - 1; ++i) ts_fetch(gb + i);
+            ws_window(gb);
+            for (int kb = gb; kb < ge; ++kb) {
+                if ((kb & 63) == 0 && kb > gb) ws_window(kb);
+                const bool hi = (kb & 32) != 0;
+                const float sw0 = __shfl_sync(0xFFFFFFFFu, hi ? wl[0][1] : wl[0][0], kb & 31);
+                const float sw1 = __shfl_sync(0xFFFFFFFFu, hi ? wl[1][1] : wl[1][0], kb & 31);
+                cp_async_wait<C::TSD - 2>();
+                const float* slot = s_ts + (kb % C::TSD) * 128 + h;
+                const float t0 = slot[0], t1 = slot[64];
+                ts_fetch(kb + C::TSD - 1);              // into the slot read one block ago
+                if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+                s_sx[ab * 128 + h] = make_float2(t0 * sw0, t0 * sw1);
+                s_sx[ab * 128 + h + 64] = make_float2(t1 * sw0, t1 * sw1);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_tfull + 8 * ab);
+                if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
+            }
+        }
+        cp_async_wait<0>();
     } else if (!G1 && p.fuse_out) {
         // ------------------------------------------------------------ warps 2-3, fused combine: zero rows of the
         // tokens that have no pair on this rank (nobody else writes them)
@@ -750,28 +824,73 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             for (int a = 0; a < C::NACCUM; ++a)
 #pragma unroll
                 for (int i = 0; i < C::NC; ++i) acc[a][i] = 0.f;
-            // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
-            const int srow0 = un.mt * (p.unit_rows >> 7);
-            const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
-            const float* ws0 = p.w_scale + ((size_t)un.e * p.scale_rows + srow0) * p.KB;
-            const float* ws1 = p.w_scale + ((size_t)un.e * p.scale_rows + srow1) * p.KB;
-
-            // weight scales of a group are fetched one group ahead, so their global-load latency
-            // never sits between the TMEM hand-off and the first FMA
+            // narrow tiles: the weight scales of a group are fetched one group ahead (the token scales travel in the
+            // stage), so their global-load latency never sits between the TMEM hand-off and the first FMA
+            const float* ws0 = nullptr; const float* ws1 = nullptr;
             float swn[C::KPB][C::NACCUM];
+            if (!C::TOK_ON_M) {
+                // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
+                const int srow0 = un.mt * (p.unit_rows >> 7);
+                const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
+                ws0 = p.w_scale + ((size_t)un.e * p.scale_rows + srow0) * p.KB;
+                ws1 = p.w_scale + ((size_t)un.e * p.scale_rows + srow1) * p.KB;
 #pragma unroll
-            for (int j = 0; j < C::KPB; ++j) {
-                const int kb = min(gb * C::KPB + j, p.KB - 1);
-                swn[j][0] = __ldg(ws0 + kb);
-                swn[j][1] = __ldg(ws1 + kb);
+                for (int j = 0; j < C::KPB; ++j) {
+                    const int kb = min(gb * C::KPB + j, p.KB - 1);
+                    swn[j][0] = __ldg(ws0 + kb);
+                    swn[j][1] = __ldg(ws1 + kb);
+                }
             }
-            // tokens-on-M: this thread's token scale, also one K block ahead (KPB == 1 there)
-            const float* tsp = p.b_scale + (size_t)un.row0 + m;
-            if (G4) {
-                const int tok = __ldg(p.g4_row_token + un.row0 + m);
-                tsp = p.g4_scale + (tok >= 0 && tok < p.g4_T ? (size_t)tok * (unsigned)p.g4_tok_stride : 0);   // any finite scale for a row of zeros
-            }
-            float stokn = C::TOK_ON_M ? __ldcg(tsp + (size_t)min(gb * C::KPB, p.KB - 1) * (G4 ? p.ts_stride : p.rows_cap)) : 0.f;
+            if constexpr (C::TOK_ON_M) {
+                // Tokens on M: this thread's row is one token, so a K block folds with ONE scalar per weight tile.  The
+                // block is read as four 32-column chunks, two tcgen05.ld in flight per wait (a wait covers every
+                // outstanding load).  The loop is rotated: the next block's first two chunks are requested while the
+                // last two of this block are folded, so the hand-off wait, the scale load and the TMEM latency of a
+                // block's start hide behind those FMAs; the buffer goes back as soon as its last load has completed.
+                constexpr int QC = 32, QPA = C::NC / QC, NQ = C::NACCUM * QPA;
+                static_assert(C::NC % QC == 0 && NQ == 4 && C::KPB == 1, "tokens-on-M chunking");
+                float stg[2][QC];
+                float2 sx2;
+                uint32_t tbuf;
+                auto qload = [&](int q) { tmem_ld_chunk<QC>(tbuf + (q / QPA) * NTOK + (q % QPA) * QC, stg[q & 1]); };
+                auto qfold = [&](int q, float sx) {
+                    const float2 s2 = make_float2(sx, sx);
+                    float* ac = &acc[q / QPA][(q % QPA) * QC];
+                    const float* v = stg[q & 1];
+#pragma unroll
+                    for (int i = 0; i < QC; i += 2) {
+                        const float2 r0 = __ffma2_rn(make_float2(v[i], v[i + 1]), s2, make_float2(ac[i], ac[i + 1]));
+                        ac[i] = r0.x; ac[i + 1] = r0.y;
+                    }
+                };
+                auto acquire = [&]() -> bool {
+                    if (!mbar_wait(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) return false;
+                    tc_fence_after();
+                    sx2 = s_sx[ab * 128 + m];              // written by the scale warps before they counted in
+                    tbuf = tmem_base + tlane + ab * C::BUFCOLS + c0;
+                    return true;
+                };
+                if (!acquire()) { ok = false; break; }
+                if (ptid == 0 && !seen) { stamp(TR_PROMO_FIRST); seen = true; }
+                qload(0); qload(1);
+#pragma unroll 1
+                for (int n = ge - gb; n > 0; --n) {
+                    if (ptid == 0) klog_put(2, ng);
+                    tmem_wait_ld();
+                    qfold(0, sx2.x); qload(2);
+                    qfold(1, sx2.x); qload(3);
+                    tmem_wait_ld();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
+                    if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
+                    const float s_hi = sx2.y;
+                    if (n > 1 && !acquire()) { ok = false; break; }
+                    qfold(2, s_hi); if (n > 1) qload(0);
+                    qfold(3, s_hi); if (n > 1) qload(1);
+                    if (ptid == 0) klog_put(3, ng++);
+                }
+            } else
             for (int grp = gb; grp < ge; ++grp) {
                 const int kb0 = grp * C::KPB;
                 const int nj = min(C::KPB, p.KB - kb0);
@@ -783,8 +902,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     swn[j][0] = __ldg(ws0 + kb);
                     swn[j][1] = __ldg(ws1 + kb);
                 }
-                const float stok_cur = stokn;
-                if (C::TOK_ON_M) stokn = __ldcg(tsp + (size_t)min(kb0 + 1, p.KB - 1) * (G4 ? p.ts_stride : p.rows_cap));
                 const int st0 = stage;
                 float scr[C::EARLY_SCALES ? C::KPB : 1][C::EARLY_SCALES ? C::NC : 1];
                 if (C::EARLY_SCALES) {
@@ -820,60 +937,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 // flattened chunk list (K block, column chunk, accumulator, partial); the tcgen05.ld of
                 // chunk k+1 is in flight while chunk k is folded into the accumulators
                 constexpr int NCH = C::NC / C::CH;
-                constexpr int NK = C::TOK_ON_M ? 0 : C::KPB * NCH * C::NACCUM * C::NSPLIT;
-                if constexpr (C::TOK_ON_M) {
-                    // Tokens on M: this thread's row is one token, so a K block folds with ONE scalar per
-                    // weight tile.  The block is read as 32-column chunks, two tcgen05.ld in flight per
-                    // wait (a wait covers every outstanding load, so depth comes from issuing in pairs).
-                    constexpr int QC = 32, QPA = C::NC / QC, NQ = C::NACCUM * QPA;
-                    static_assert(C::NC % QC == 0 && NQ % 2 == 0, "tokens-on-M chunking");
-                    float stg[2][QC];
-                    auto qaddr = [&](int q) { return tbuf + (q / QPA) * NTOK + (q % QPA) * QC; };
-                    auto qfold = [&](int q, const float* v) {
-                        const int a = q / QPA;
-                        const float sx = stok_cur * sw[0][a];
-                        const float2 s2 = make_float2(sx, sx);
-                        float* ac = &acc[a][(q % QPA) * QC];
-#pragma unroll
-                        for (int i = 0; i < QC; i += 2) {
-                            const float2 r0 = __ffma2_rn(make_float2(v[i], v[i + 1]), s2, make_float2(ac[i], ac[i + 1]));
-                            ac[i] = r0.x; ac[i + 1] = r0.y;
-                        }
-                    };
-                    // the buffer goes back to the MMA warp as soon as its last tcgen05.ld has
-                    // completed; the FMAs of the last chunks run after the release
-                    auto release = [&]() {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
-                    };
-                    {
-                        // Scheduling fence.  `never` is 0, but ptxas cannot know: with the fold inside a real branch it
-                        // does not pull the fold's TMEM loads and FMAs up across the hand-off wait above, and the
-                        // kernel measures 3 % faster (prefill GEMM1 414 against 466 us with stage events, results
-                        // bit-identical; a plain compiler barrier does not have the effect).  Re-measure when the
-                        // fold changes: `python bench.py --workload prefill` with and without the branch.
-                        int never;
-                        asm volatile("mov.u32 %0, 0;" : "=r"(never));
-                        if (never) {
-                            release();
-                        } else {
-                        tmem_ld_chunk<QC>(qaddr(0), stg[0]);
-                        tmem_ld_chunk<QC>(qaddr(1), stg[1]);
-#pragma unroll
-                        for (int q = 0; q < NQ; q += 2) {
-                            tmem_wait_ld();
-                            if (q + 2 >= NQ) release();
-                            qfold(q, stg[0]);
-                            if (q + 2 < NQ) tmem_ld_chunk<QC>(qaddr(q + 2), stg[0]);
-                            qfold(q + 1, stg[1]);
-                            if (q + 3 < NQ) tmem_ld_chunk<QC>(qaddr(q + 3), stg[1]);
-                        }
-                        }
-                    }
-                }
+                constexpr int NK = C::KPB * NCH * C::NACCUM * C::NSPLIT;
                 float part[2][C::CH];
-                if (!C::TOK_ON_M) tmem_ld_chunk<C::CH>(tbuf, part[0]);
+                tmem_ld_chunk<C::CH>(tbuf, part[0]);
 #pragma unroll
                 for (int k = 0; k < NK; ++k) {
                     const int sp = k % C::NSPLIT;
@@ -927,11 +993,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 }
                 if (!ok) break;
                 // all tcgen05.ld of this buffer have completed (the last wait above) and all scale reads are done
-                if (!C::TOK_ON_M) {
-                    tc_fence_before();
-                    __syncwarp();
-                }
-                if (!C::TOK_ON_M && lane == 0) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
                     mbar_arrive(bar_tempty + 8 * ab);
                     if (C::SCALES_IN_STAGE && !C::EARLY_SCALES) {
                         for (int j = 0; j < nj; ++j) {

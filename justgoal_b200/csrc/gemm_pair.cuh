@@ -144,7 +144,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     int* s_tiles = s_cnt + (MAX_LOCAL + 1);
     float* s_red = reinterpret_cast<float*>(s_tiles + (MAX_LOCAL + 1));
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform for the compiler too
     const uint32_t crank = cluster_rank();
 #ifdef B200MOE_PAIR_TRACE
     // timing build only: cycles one thread of every role spends in each of its waits, summed over the kernel
@@ -214,27 +214,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::CTRL_REGS));
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        // ------------------------------------------------------------ TMA producer (both CTAs; whole warp, one elected lane issues)
+        {
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             PT_DECL(w_empty = 0);
             for (int ui = 0; ui < my_units && ok; ++ui) {
                 PairUnit un;
                 if (!decode_pair_unit(cidx + ui * ncl, p.n_mtiles, p.num_local, s_pp, s_row0, s_cnt, (int)crank, un)) {
-                    atomicCAS(p.status, 0, ERR_BAD_SCHEDULE); break;
+                    if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
+                    break;
                 }
-                const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows + (int)crank * p.gate_offset;
+                un.row0 = __shfl_sync(0xFFFFFFFFu, un.row0, 0);
+                const int wrow = __shfl_sync(0xFFFFFFFFu, un.e * p.rows_per_expert + un.mt * p.unit_rows + (int)crank * p.gate_offset, 0);
                 for (int kb = 0; kb < p.KB; ++kb) {
                     { PT_T0();
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
                     PT_ADD(w_empty); }
+                    if (elect_one()) {
                     const uint32_t st = smem_base + stage * C::STAGE_BYTES;
                     const uint32_t full0 = cluster_map(bar_full + 8 * stage, 0);      // the leader's barrier
                     if (crank == 0) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * C::STAGE_BYTES);
                     tma_load_2d_pair(st, &tm_b0, kb * 128, un.row0, full0);
                     if (!G1) tma_load_2d_pair(st + C::A_BYTES, &tm_b1, kb * 128, un.row0, full0);
                     tma_load_2d_pair(st + C::B_OFF, &tm_w, kb * 128, wrow, full0);
+                    }
+                    __syncwarp();
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
@@ -252,7 +257,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (leader CTA, for the pair)
-        if (lane == 0 && crank == 0) {
+        if (crank == 0) {
             constexpr uint32_t idesc = make_idesc_f8(256, 256);     // M = 256 over the pair, N = both weight tiles
             int stage = 0; uint32_t phase = 0;
             int ab = 0; uint32_t aphase = 0;
@@ -267,6 +272,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                     if (!mbar_wait(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL)) { ok = false; break; }
                     PT_ADD(w_full); }
                     tc_fence_after();
+                    if (elect_one()) {
                     const uint32_t st = smem_base + stage * C::STAGE_BYTES;
                     const uint32_t d = tmem_base + ab * 256;
                     const uint64_t a0 = make_smem_desc(st);
@@ -280,6 +286,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                     }
                     umma_commit_pair(bar_empty + 8 * stage);
                     umma_commit_pair(bar_tfull + 8 * ab);
+                    }
+                    __syncwarp();
                     if (++ab == C::NBUF) { ab = 0; aphase ^= 1; }
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
