@@ -92,6 +92,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
     }
 }
 
+// Two barriers by a converged warp: both are tried before either answer is looked at (one round trip when both phases
+// have completed), and the answers are voted on, so the control flow after it stays uniform for the compiler.
+__device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a, int code_a, uint32_t bar_b, uint32_t parity_b,
+                                               int code_b, int* status) {
+    const bool a = mbar_try_wait(bar_a, parity_a), b = mbar_try_wait(bar_b, parity_b);
+    if (__all_sync(0xFFFFFFFFu, a && b)) return true;
+    const bool ok = mbar_wait(bar_a, parity_a, status, code_a) && mbar_wait(bar_b, parity_b, status, code_b);
+    return __all_sync(0xFFFFFFFFu, ok);
+}
+
 // The wrappers below are one PTX instruction each; their bodies are fixed by the ISA (operand order, state spaces,
 // qualifiers), so any sm_100a code base that wraps the same instructions reads alike.
 // ---------------------------------------------------------------- TMA (non-multicast only)
