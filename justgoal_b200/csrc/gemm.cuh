@@ -218,6 +218,17 @@ __device__ __forceinline__ bool decode_unit(int u, int n_mtiles, int num_local, 
     return o.mt < n_mtiles && o.nvalid > 0;
 }
 
+// The same by a converged warp; the result is uniform for the compiler (see mbar_wait_warp).
+__device__ __forceinline__ bool decode_unit_warp(int u, int n_mtiles, int num_local, int ntok, const int* s_tiles,
+                                                 const int* s_row0, const int* s_cnt, Unit& o) {
+    Unit d = {0, 0, 0, 0, 0};
+    const bool ok = decode_unit(u, n_mtiles, num_local, ntok, s_tiles, s_row0, s_cnt, d);
+    const unsigned FULL = 0xFFFFFFFFu;
+    o.e = __shfl_sync(FULL, d.e, 0); o.mt = __shfl_sync(FULL, d.mt, 0); o.tt = __shfl_sync(FULL, d.tt, 0);
+    o.row0 = __shfl_sync(FULL, d.row0, 0); o.nvalid = __shfl_sync(FULL, d.nvalid, 0);
+    return __all_sync(FULL, ok);
+}
+
 // One piece of work: unit u, K groups [gb, ge).  kind WK_WHOLE: the whole unit.  WK_PART: a piece of split unit ut
 // that does not end the unit - its partial sum goes to slot `slot`.  WK_FINISH: the piece that ends split unit ut -
 // it waits for `nwait` other pieces, adds the slots slot .. slot + nwait - 1 in that order and runs the epilogue.
@@ -404,12 +415,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     // lane 0 then tells the producer that the warp has its copy.  false = list ended or a wait gave up.
     auto wq_fetch = [&](int n, WorkItem& w, bool& ok) -> bool {
         const int slot = n % C::WQ;
-        if (!mbar_wait(bar_wqfull + 8 * slot, (uint32_t)(n / C::WQ) & 1u, p.status, ERR_WAIT_GROUP)) { ok = false; return false; }
+        if (!mbar_wait_warp(bar_wqfull + 8 * slot, (uint32_t)(n / C::WQ) & 1u, p.status, ERR_WAIT_GROUP)) { ok = false; return false; }
         const volatile int* q = s_wq + slot * 8;
-        w.u = q[0]; w.gb = q[1]; w.ge = q[2]; w.kind = q[3]; w.ut = q[4]; w.slot = q[5]; w.nwait = q[6];
-        __syncwarp();
+        auto word = [&](int i) { return __shfl_sync(0xFFFFFFFFu, (int)q[i], 0); };       // uniform for the compiler
+        w.u = word(0); w.gb = word(1); w.ge = word(2); w.kind = word(3); w.ut = word(4); w.slot = word(5); w.nwait = word(6);
         if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
-        w.u = __shfl_sync(0xFFFFFFFFu, w.u, 0);                // uniform for the compiler
         return w.u >= 0;
     };
 
@@ -449,7 +459,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int n_item = 0, n_whole = 0;
             auto publish = [&](const WorkItem& w) -> bool {
                 const int slot = n_item % C::WQ;
-                if (!mbar_wait(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
+                if (!mbar_wait_warp(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
                 if (lane == 0) {
                     volatile int* q = s_wq + slot * 8;
                     q[0] = w.u; q[1] = w.gb; q[2] = w.ge; q[3] = w.kind; q[4] = w.ut; q[5] = w.slot; q[6] = w.nwait;
@@ -520,14 +530,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if (!publish(wi)) { ok = false; break; }
                 const int u = wi.u, gb = wi.gb, ge = wi.ge;
                 Unit un;
-                if (!decode_unit(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) {
+                if (!decode_unit_warp(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) {
                     if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
                     ok = false; break;
                 }
-                // from here on the coordinates are warp-uniform in the compiler's eyes as well
-                un.row0 = __shfl_sync(0xFFFFFFFFu, un.row0, 0);
-                const int wrow = __shfl_sync(0xFFFFFFFFu, un.e * p.rows_per_expert + un.mt * p.unit_rows, 0);
-                const int kb_end = __shfl_sync(0xFFFFFFFFu, min(p.KB, ge * C::KPB), 0);
+                const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows;
+                const int kb_end = min(p.KB, ge * C::KPB);
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
@@ -566,7 +574,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (C::SCALES_IN_STAGE)
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
-                int kb_first = __shfl_sync(0xFFFFFFFFu, gb * C::KPB, 0);
+                int kb_first = gb * C::KPB;
                 if (G1 && !waited) {
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the front end still
                     // permutes and gathers, then the wait for it, then the token side of the same stages
@@ -590,7 +598,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
                 for (int kb = kb_first; kb < kb_end; ++kb) {
-                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
                     if (elect_one()) { load_weights(stage, kb); load_tokens(stage, kb); }
                     __syncwarp();
                     if (!issued) { if (lane == 0) stamp(TR_TMA_FIRST); issued = true; }
@@ -620,7 +628,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int n_item = 0;
             WorkItem wi;
             while (ok && wq_fetch(n_item++, wi, ok)) {
-                const int gb = __shfl_sync(0xFFFFFFFFu, wi.gb, 0), ge = __shfl_sync(0xFFFFFFFFu, wi.ge, 0);      // uniform for the compiler
+                const int gb = wi.gb, ge = wi.ge;
                 for (int grp = gb; grp < ge; ++grp) {
                     const int nj = min(C::KPB, p.KB - grp * C::KPB);
                     for (int j = 0; j < nj; ++j) {
@@ -629,7 +637,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         // queue is only two or three MMAs deep, two waits in a row leave it idle
                         if (!(j == 0 ? mbar_wait_both(bar_tempty + 8 * ab, aphase ^ 1, ERR_WAIT_TMEM_EMPTY,
                                                       bar_full + 8 * stage, phase, ERR_WAIT_SMEM_FULL, p.status)
-                                     : __all_sync(0xFFFFFFFFu, mbar_wait(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL)))) { ok = false; break; }
+                                     : mbar_wait_warp(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL))) { ok = false; break; }
                         if (!seen) { if (lane == 0) stamp(TR_MMA_FIRST); seen = true; }
                         if (lane == 0) klog_put(1, nk);
                         ++nk;
@@ -715,7 +723,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
             Unit un;
-            if (!decode_unit(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
+            if (!decode_unit_warp(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
             // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
             const int srow0 = un.mt * (p.unit_rows >> 7);
             const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
@@ -757,7 +765,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const float* slot = s_ts + (kb % C::TSD) * 128 + h;
                 const float t0 = slot[0], t1 = slot[64];
                 ts_fetch(kb + C::TSD - 1);              // into the slot read one block ago
-                if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+                if (!mbar_wait_warp(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
                 s_sx[ab * 128 + h] = make_float2(t0 * sw0, t0 * sw1);
                 s_sx[ab * 128 + h + 64] = make_float2(t1 * sw0, t1 * sw1);
                 __syncwarp();
@@ -804,7 +812,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         auto group_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(my_red);
-            const bool r = mbar_wait(my_red, rphase, p.status, ERR_WAIT_GROUP);
+            const bool r = mbar_wait_warp(my_red, rphase, p.status, ERR_WAIT_GROUP);
             rphase ^= 1;
             return r;
         };
@@ -813,7 +821,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         auto all_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_all);
-            const bool r = mbar_wait(bar_all, allphase, p.status, ERR_WAIT_GROUP);
+            const bool r = mbar_wait_warp(bar_all, allphase, p.status, ERR_WAIT_GROUP);
             allphase ^= 1;
             return r;
         };
@@ -823,7 +831,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int u = wi.u, gb = wi.gb, ge = wi.ge;
             Unit un;
-            if (!decode_unit(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
+            if (!decode_unit_warp(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
 #pragma unroll
             for (int a = 0; a < C::NACCUM; ++a)
 #pragma unroll
@@ -868,7 +876,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                 };
                 auto acquire = [&]() -> bool {
-                    if (!mbar_wait(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) return false;
+                    if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) return false;
                     tc_fence_after();
                     sx2 = s_sx[ab * 128 + m];              // written by the scale warps before they counted in
                     tbuf = tmem_base + tlane + ab * C::BUFCOLS + c0;
@@ -914,7 +922,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         if (j < nj) {
                             int sj = st0 + j; if (sj >= C::STAGES) sj -= C::STAGES;
                             const uint32_t ph = (st0 + j >= C::STAGES) ? (phase ^ 1) : phase;
-                            if (!mbar_wait(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
+                            if (!mbar_wait_warp(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
                             const float* scp = reinterpret_cast<const float*>(smem + sj * C::STAGE_BYTES + C::SC_OFF) + c0;
 #pragma unroll
                             for (int i = 0; i < C::NC; i += 4) {
@@ -932,7 +940,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         }
                     }
                 }
-                if (!mbar_wait(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+                if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
                 if (ptid == 0 && !seen) { stamp(TR_PROMO_FIRST); seen = true; }
                 if (ptid == 0) klog_put(2, ng);
                 tc_fence_after();
@@ -977,7 +985,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             if (C::SCALES_IN_STAGE && ch == 0 && a == 0 && sp == 0) {
                                 // token scales of this K block arrived with the stage's transaction barrier
                                 const uint32_t ph = (st0 + j >= C::STAGES) ? (phase ^ 1) : phase;
-                                if (!mbar_wait(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
+                                if (!mbar_wait_warp(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
                             }
                             {
                                 const float* scp = reinterpret_cast<const float*>(smem + sj * C::STAGE_BYTES + C::SC_OFF) + c0 + ch * C::CH;
