@@ -984,11 +984,19 @@ int b200moe_quantize_1x128(const void* x_bf16, int T, int H, void* q_e4m3, float
     if (!x_bf16 || !q_e4m3 || !scale) return B200MOE_E_BADARG;
     if ((reinterpret_cast<uintptr_t>(x_bf16) & 15) || (reinterpret_cast<uintptr_t>(q_e4m3) & 7)) return B200MOE_E_BADARG;
     const int sms = b200moe_num_sms();
-    const long long groups = (long long)T * (H >> 7);
-    long long grid = (groups + 15) / 16;                   // 16 groups (half warps) per CTA
-    if (grid > (long long)sms * 16) grid = (long long)sms * 16;
-    quantize_1x128_kernel<<<(int)(grid < 1 ? 1 : grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x_bf16), T, H, static_cast<uint8_t*>(q_e4m3), scale);
+    // Block of a CTA: eight tokens (a full sector of scales) as long as that leaves a few CTAs per SM, then fewer; the
+    // groups of a row in equal parts of at most QUANT_GROUPS, cut further while the grid does not fill the chip.
+    const int groups = H >> 7;
+    int tpc = QUANT_TOKENS, parts = (groups + QUANT_GROUPS - 1) / QUANT_GROUPS;
+    auto ctas = [&](int tp, int pa) { return (long long)((T + tp - 1) / tp) * pa; };
+    while (ctas(tpc, parts) < 4ll * sms && parts * 32 < groups) parts *= 2;
+    while (ctas(tpc, parts) < 2ll * sms && tpc > 1) tpc /= 2;
+    const int gpc = (groups + parts - 1) / parts;
+    const dim3 grid((T + tpc - 1) / tpc, (groups + gpc - 1) / gpc);
+    const bool wide = !((reinterpret_cast<uintptr_t>(x_bf16) & 31) || (reinterpret_cast<uintptr_t>(q_e4m3) & 15));
+    auto* kern = wide ? quantize_1x128_kernel<true> : quantize_1x128_kernel<false>;
+    kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x_bf16), T, H, tpc, gpc, static_cast<uint8_t*>(q_e4m3), scale);
     CU_TRY(cudaGetLastError());
     return 0;
 }

@@ -225,6 +225,13 @@ __device__ __forceinline__ void st_global_v8(void* ptr, uint32_t a, uint32_t b, 
                  ::"l"(ptr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
 }
 
+// 256-bit global load of read-once data (sm_100), 32-byte aligned
+__device__ __forceinline__ void ld_global_v8(const void* ptr, uint32_t* v) {
+    asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(ptr) : "memory");
+}
+
 // e4m3 helpers
 __device__ __forceinline__ uint16_t f32x2_to_e4m3x2(float lo, float hi) {
     uint16_t r;

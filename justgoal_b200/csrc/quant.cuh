@@ -6,43 +6,111 @@
 // from its harness (goal_full_shape/fable-5.1/moe_fp8_fwd/<def>/moe_host.cu:100-103) and has no such
 // kernel; the arithmetic is the one its input contract states (1x128 groups, amax / 448).
 //
-// HBM-bound byte work: 2 bytes read and 1 byte written per element.  16 lanes own one group of 128
-// columns (8 bf16 = one 16-byte load per lane), so a warp covers 256 contiguous columns per step.
+// HBM-bound byte work: 2 bytes read and 1 byte written per element, as long as the instructions stay few: 8 lanes own one
+// group of 128 columns (16 bf16 = one 32-byte load per lane, so the group's scale, its reciprocal and the maximum's
+// shuffles are shared by 16 elements), two groups' loads in flight per lane, the maximum over packed bf16 pairs.  A CTA owns a block of tokens x groups, so that it can
+// walk the block without divisions and keep the scales in shared memory until a K block's run of tokens leaves as one
+// store (one 4-byte store per group into the [H/128, T] layout touched a sector each).
+//
+// The divisions.  Eight IEEE divisions per lane and 128 columns made the kernel instruction-bound (4096 x 7168: 30.8 us,
+// 2.9 TB/s).  With y = fl(1/s) a quotient needs three operations (Markstein, "IA-64 and Elementary Functions", ch. 8):
+// q0 = fl(x y), e = fl(x - q0 s), q = fl(q0 + e y).  q0 is off by at most two units in the last place, e carries a relative
+// error of 2^-25, so q rounds a value within 2^-22 units of x/s and can only differ from fl(x/s) where x/s lies that close
+// to the middle between two floats.  For the e4m3 byte to differ, one of the two must be a tie M of the e4m3 grid as well,
+// x/s = (M + half a unit)(1 + 2^-46): with x an 8-bit and s a 24-bit integer times a power of two this asks for
+// r n = c, n the odd part of M, 2^24 > c 2^(25 - bits(n)) >= 2^23, |r| <= 8, which only n = c = r = 1 solves - a scale whose
+// mantissa is all ones, and the quotient of an 8-bit number by 448 never is.  (The test runs all pairs of mantissas.)
+// Scales below 2^-90 or above 2^126, where e or y would lose bits to the exponent range, take the dividing path.
 #pragma once
 #include <cuda_bf16.h>
 #include "common.cuh"
 
 namespace b200moe {
 
-__global__ void __launch_bounds__(256) quantize_1x128_kernel(const __nv_bfloat16* __restrict__ x, int T, int H,
+// Four quotients v / s of one lane, rounded to e4m3 (one byte each); y = fl(1 / s)
+__device__ __forceinline__ uint32_t quantize4(const float2 v0, const float2 v1, float s, float y) {
+    const float2 ns = make_float2(-s, -s), yy = make_float2(y, y);
+    const float2 p0 = __fmul2_rn(v0, yy), p1 = __fmul2_rn(v1, yy);
+    const float2 q0 = __ffma2_rn(__ffma2_rn(p0, ns, v0), yy, p0), q1 = __ffma2_rn(__ffma2_rn(p1, ns, v1), yy, p1);
+    return (uint32_t)f32x2_to_e4m3x2(q0.x, q0.y) | ((uint32_t)f32x2_to_e4m3x2(q1.x, q1.y) << 16);
+}
+
+constexpr int QUANT_TOKENS = 8;         // most tokens of a CTA: a sector of scales
+constexpr int QUANT_GROUPS = 64;        // most groups (128 columns) of a CTA
+
+// CTA (x, y): tokens [x * tpc, ...), groups [y * gpc, ...).  WIDE: x is 32-byte and q 16-byte aligned (torch tensors are);
+// otherwise two 16-byte loads and two 8-byte stores take their place.
+template <bool WIDE>
+__global__ void __launch_bounds__(256) quantize_1x128_kernel(const __nv_bfloat16* __restrict__ x, int T, int H, int tpc, int gpc,
                                                              uint8_t* __restrict__ q, float* __restrict__ scale) {
+    __shared__ float s_scale[QUANT_GROUPS][QUANT_TOKENS];
     const int groups = H >> 7;
-    const int lane16 = threadIdx.x & 15;
-    const int half_warps = (gridDim.x * blockDim.x) >> 4;
-    const long long total = (long long)T * groups;
-    for (long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4; g < total; g += half_warps) {
-        const int t = (int)(g / groups), kb = (int)(g - (long long)t * groups);
-        const size_t off = (size_t)t * H + (size_t)kb * 128 + lane16 * 8;
-        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(x + off));
-        const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-        float v[8];
-        float amax = 0.f;
+    const int t0 = blockIdx.x * tpc, k0 = blockIdx.y * gpc;
+    const int nt = min(tpc, T - t0), nk = min(gpc, groups - k0);
+    const int sub = threadIdx.x & 7;      // lane inside the group
+    constexpr int GP = 32;                // groups a CTA works on at a time
+    constexpr int U = 2;                  // ... and per lane in flight
+    const int total = nt * nk;
+    int t = 0, k = threadIdx.x >> 3;      // this lane's next group inside the block
+    while (k >= nk) { k -= nk; ++t; }
+    // the trip count is the same for all lanes (the shuffles below stay inside a group, but name the warp)
+    for (int i0 = 0; i0 < total; i0 += U * GP) {
+        alignas(16) uint32_t raw[U][8];
+        int tt[U], kk[U];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __bfloat1622float2(h2[i]);
-            v[2 * i] = f.x; v[2 * i + 1] = f.y;
-            amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+        for (int u = 0; u < U; ++u) {
+            tt[u] = t; kk[u] = k;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) raw[u][i] = 0u;
+            const __nv_bfloat16* src = x + (size_t)(t0 + t) * H + (size_t)(k0 + k) * 128 + sub * 16;
+            if (t < nt) {
+                if (WIDE) {
+                    ld_global_v8(src, raw[u]);
+                } else {
+                    *reinterpret_cast<uint4*>(&raw[u][0]) = __ldcs(reinterpret_cast<const uint4*>(src));
+                    *reinterpret_cast<uint4*>(&raw[u][4]) = __ldcs(reinterpret_cast<const uint4*>(src) + 1);
+                }
+            }
+            k += GP;
+            while (k >= nk) { k -= nk; ++t; }
         }
 #pragma unroll
-        for (int o = 8; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-        const float s = amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f;
-        uint2 out;
-        out.x = (uint32_t)f32x2_to_e4m3x2(__fdiv_rn(v[0], s), __fdiv_rn(v[1], s)) |
-                ((uint32_t)f32x2_to_e4m3x2(__fdiv_rn(v[2], s), __fdiv_rn(v[3], s)) << 16);
-        out.y = (uint32_t)f32x2_to_e4m3x2(__fdiv_rn(v[4], s), __fdiv_rn(v[5], s)) |
-                ((uint32_t)f32x2_to_e4m3x2(__fdiv_rn(v[6], s), __fdiv_rn(v[7], s)) << 16);
-        *reinterpret_cast<uint2*>(q + off) = out;
-        if (lane16 == 0) scale[(size_t)kb * T + t] = s;
+        for (int u = 0; u < U; ++u) {
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(raw[u]);
+            __nv_bfloat162 m = __habs2(h2[0]);
+#pragma unroll
+            for (int i = 1; i < 8; ++i) m = __hmax2(m, __habs2(h2[i]));
+            float amax = fmaxf(__low2float(m), __high2float(m));
+#pragma unroll
+            for (int o = 4; o; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+            if (tt[u] >= nt) continue;
+            const float s = amax > 0.f ? __fdiv_rn(amax, 448.0f) : 1.0f;
+            const float y = __fdiv_rn(1.0f, s);
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = quantize4(__bfloat1622float2(h2[2 * j]), __bfloat1622float2(h2[2 * j + 1]), s, y);
+            if (!(s >= 0x1p-90f && y >= 0x1p-126f)) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float2 f0 = __bfloat1622float2(h2[2 * j]), f1 = __bfloat1622float2(h2[2 * j + 1]);
+                    w[j] = (uint32_t)f32x2_to_e4m3x2(__fdiv_rn(f0.x, s), __fdiv_rn(f0.y, s)) |
+                           ((uint32_t)f32x2_to_e4m3x2(__fdiv_rn(f1.x, s), __fdiv_rn(f1.y, s)) << 16);
+                }
+            }
+            uint8_t* dst = q + (size_t)(t0 + tt[u]) * H + (size_t)(k0 + kk[u]) * 128 + sub * 16;
+            if (WIDE) {
+                *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+            } else {
+                reinterpret_cast<uint2*>(dst)[0] = make_uint2(w[0], w[1]);
+                reinterpret_cast<uint2*>(dst)[1] = make_uint2(w[2], w[3]);
+            }
+            if (sub == 0) s_scale[kk[u]][tt[u]] = s;
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < nk * QUANT_TOKENS; i += 256) {
+        const int kb = i / QUANT_TOKENS, tl = i % QUANT_TOKENS;
+        if (tl < nt) scale[(size_t)(k0 + kb) * T + t0 + tl] = s_scale[kb][tl];
     }
 }
 

@@ -32,6 +32,46 @@ def test_quantiser_bit_exact(T, H):
     assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
 
 
+@pytest.mark.parametrize("spread", [1.0, 2.0 ** -88, 2.0 ** -120, 2.0 ** 119])
+def test_quantiser_every_pair_of_mantissas(spread):
+    """The kernel's quotients are corrected products, not divisions: every pair of bf16 mantissas (group maximum, element)
+    at every exponent gap that still reaches the e4m3 grid gives the byte of the IEEE division; tiny and huge scales too."""
+    from justgoal_b200 import quantize_1x128
+    m = 1.0 + torch.arange(128, dtype=torch.float64) / 128
+    gaps = 2.0 ** -torch.arange(0, 20, dtype=torch.float64)
+    x = (m[None, None, :] * gaps[None, :, None] * 0.5).repeat(128, 1, 1)         # [maximum, gap, element], elements below the maximum
+    x = (x * spread).to(torch.bfloat16).clone()
+    x[:, :, ::3] *= -1
+    tail = x[:, :, 127].clone()
+    x[:, :, 127] = (m * spread).to(torch.bfloat16)[:, None]             # the group's maximum
+    x[:, :, 64] = tail                                                  # (element 64 gives way to the one the maximum displaced)
+    x = x.reshape(128 * 20, 128)
+    x = torch.cat([x, x.flip(0)], dim=1).contiguous()
+    q_ref, s_ref = I.quantize_rows_1x128(x)
+    q, s = quantize_1x128(x.cuda())
+    assert torch.equal(s.cpu().view(torch.int32), s_ref.view(torch.int32))
+    assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
+
+
+@pytest.mark.parametrize("T,H,off", [(1, 128, 0), (9, 256, 8), (31, 4352, 8), (600, 8320, 0), (4739, 128, 16)])
+def test_quantiser_blocks_and_alignment(T, H, off):
+    """Ragged token blocks, rows cut over several CTAs, and activations that are only 16-byte aligned."""
+    from justgoal_b200 import _lib, quantize_1x128
+    import ctypes as C
+    x = _case(T, H, seed=T)
+    buf = torch.zeros(T * H + 16, dtype=torch.bfloat16, device="cuda")
+    view = buf[off:off + T * H].view(T, H)
+    view.copy_(x)
+    q_ref, s_ref = I.quantize_rows_1x128(x)
+    q, s = quantize_1x128(view)
+    assert torch.equal(s.cpu().view(torch.int32), s_ref.view(torch.int32))
+    assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
+    qb = torch.zeros(T * H + 8, dtype=torch.uint8, device="cuda")       # output that is only 8-byte aligned
+    rc = _lib.lib.b200moe_quantize_1x128(C.c_void_p(view.data_ptr()), T, H, C.c_void_p(qb.data_ptr() + 8), C.c_void_p(s.data_ptr()), None)
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(qb[8:].cpu().view(T, H), q_ref.view(torch.uint8))
+
+
 def test_quantiser_feeds_the_operator():
     """bf16 activations -> quantiser kernel -> layer: same output as with host-quantised inputs."""
     from justgoal_b200 import MoELayer, quantize_1x128
