@@ -96,6 +96,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
 // loop around it carries (stage, buffer, phase) stays in uniform registers, which TMA, tcgen05.mma and tcgen05.ld take
 // their operands from.  (A 128-K block of four MMAs: 606 cycles of the issuing loop without, 513 with.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int code) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;      // the usual case costs one try and one vote
     return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, status, code));
 }
 // Two barriers by a converged warp: both are tried before either answer is looked at (one round trip when both phases

@@ -174,14 +174,14 @@ struct GemmCfg {
     // chunks measured 30 % slower there: every CTA finishes units it has to collect six partial sums for, late in
     // the kernel).  Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
     static constexpr bool STATIC_TAIL = G1 && NTOK <= 32;
-    static constexpr int WQ = 4;                           // depth of the in-CTA work queue
+    static constexpr int WQ = 4, WQ_INTS = 12;             // depth of the in-CTA work queue, words of an entry (WorkItem)
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
     static constexpr int TABLE_INTS = 3 * (MAX_LOCAL + 1);
     static constexpr int RED_BYTES = NPW * NC * 4;
     static constexpr int TSD = 8;                          // tokens-on-M: slots of the token-scale ring (see the scale warps)
     static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
     static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
-    static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * 32 /*work queue*/ +
+    static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * WQ_INTS * 4 /*work queue*/ +
                                       TABLE_INTS * 4 + RED_BYTES + 32 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
     static_assert(NTOK % 16 == 0 && NTOK >= 16 && NTOK <= 128, "token tile");
     static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "tmem");
@@ -234,7 +234,7 @@ __device__ __forceinline__ bool decode_unit_warp(int u, int n_mtiles, int num_lo
 // it waits for `nwait` other pieces, adds the slots slot .. slot + nwait - 1 in that order and runs the epilogue.
 // u < 0 ends the list.
 enum : int { WK_WHOLE = 0, WK_PART = 1, WK_FINISH = 2 };
-struct WorkItem { int u, gb, ge, kind, ut, slot, nwait; };
+struct WorkItem { int u, gb, ge, kind, ut, slot, nwait; Unit un; };
 
 // CTA that owns flat index x when `total` indices are cut into `parts` equal contiguous ranges (part c starts at
 // c * total / parts)
@@ -315,8 +315,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(tail);     // full[S], empty[S], tfull[NTB], tempty[NTB], red[4], all, wq_full[WQ], wq_empty[WQ]
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tail + C::BAR_BYTES - 8);
-    int* s_wq = reinterpret_cast<int*>(tail + C::BAR_BYTES);          // [WQ][8] work items (WorkItem + padding)
-    int* s_tiles = s_wq + C::WQ * 8;
+    int* s_wq = reinterpret_cast<int*>(tail + C::BAR_BYTES);          // [WQ][WQ_INTS] work items, 16-byte aligned
+    int* s_tiles = s_wq + C::WQ * C::WQ_INTS;
     int* s_row0 = s_tiles + (MAX_LOCAL + 1);
     int* s_cnt = s_row0 + (MAX_LOCAL + 1);
     uint32_t* s_red = reinterpret_cast<uint32_t*>(s_cnt + (MAX_LOCAL + 1));
@@ -416,9 +416,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     auto wq_fetch = [&](int n, WorkItem& w, bool& ok) -> bool {
         const int slot = n % C::WQ;
         if (!mbar_wait_warp(bar_wqfull + 8 * slot, (uint32_t)(n / C::WQ) & 1u, p.status, ERR_WAIT_GROUP)) { ok = false; return false; }
-        const volatile int* q = s_wq + slot * 8;
-        auto word = [&](int i) { return __shfl_sync(0xFFFFFFFFu, (int)q[i], 0); };       // uniform for the compiler
-        w.u = word(0); w.gb = word(1); w.ge = word(2); w.kind = word(3); w.ut = word(4); w.slot = word(5); w.nwait = word(6);
+        // (the wait above and the arrival below are compiler barriers: plain loads)
+        const int4* q = reinterpret_cast<const int4*>(s_wq + slot * C::WQ_INTS);
+        const int4 q0 = q[0], q1 = q[1], q2 = q[2];
+        auto uni = [](int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); };                  // uniform for the compiler
+        w.u = uni(q0.x); w.gb = uni(q0.y); w.ge = uni(q0.z); w.kind = uni(q0.w);
+        w.ut = uni(q1.x); w.slot = uni(q1.y); w.nwait = uni(q1.z); w.un.e = uni(q1.w);
+        w.un.mt = uni(q2.x); w.un.row0 = uni(q2.y); w.un.nvalid = uni(q2.z); w.un.tt = 0;
+        __syncwarp();
         if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
         return w.u >= 0;
     };
@@ -461,8 +466,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const int slot = n_item % C::WQ;
                 if (!mbar_wait_warp(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
                 if (lane == 0) {
-                    volatile int* q = s_wq + slot * 8;
-                    q[0] = w.u; q[1] = w.gb; q[2] = w.ge; q[3] = w.kind; q[4] = w.ut; q[5] = w.slot; q[6] = w.nwait;
+                    int4* q = reinterpret_cast<int4*>(s_wq + slot * C::WQ_INTS);
+                    q[0] = make_int4(w.u, w.gb, w.ge, w.kind);
+                    q[1] = make_int4(w.ut, w.slot, w.nwait, w.un.e);
+                    q[2] = make_int4(w.un.mt, w.un.row0, w.un.nvalid, 0);
                     mbar_arrive(bar_wqfull + 8 * slot);      // release: the item is visible to whoever sees the phase flip
                 }
                 __syncwarp();
@@ -481,7 +488,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int st_pass = has_tail ? 0 : 3, st_ut = t_lo / NG;
             while (ok) {
                 WorkItem wi;
-                wi.kind = WK_WHOLE; wi.ut = -1; wi.slot = 0; wi.nwait = 0;
+                wi.kind = WK_WHOLE; wi.ut = -1; wi.slot = 0; wi.nwait = 0; wi.un = Unit{0, 0, 0, 0, 0};
                 bool have = false;
                 while (st_pass < 3 && !have) {
                     const int ut_last = (t_hi - 1) / NG;
@@ -527,13 +534,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         wi.nwait = CPU_ - 1;
                     }
                 }
-                if (!publish(wi)) { ok = false; break; }
-                const int u = wi.u, gb = wi.gb, ge = wi.ge;
-                Unit un;
-                if (!decode_unit_warp(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) {
+                if (!decode_unit_warp(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, wi.un)) {
                     if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
                     ok = false; break;
                 }
+                if (!publish(wi)) { ok = false; break; }
+                const int gb = wi.gb, ge = wi.ge;
+                const Unit un = wi.un;
                 const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows;
                 const int kb_end = min(p.KB, ge * C::KPB);
                 auto load_weights = [&](int s_, int kb) {
@@ -611,7 +618,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if (!ok) {
                 // gave up: end the list for the other roles (if the queue still moves), then give copies that are
                 // still in flight time to land before the CTA's shared memory goes away
-                WorkItem end_; end_.u = -1; end_.gb = end_.ge = 0; end_.kind = WK_WHOLE; end_.ut = -1; end_.slot = end_.nwait = 0;
+                WorkItem end_; end_.u = -1; end_.gb = end_.ge = 0; end_.kind = WK_WHOLE; end_.ut = -1; end_.slot = end_.nwait = 0; end_.un = Unit{0, 0, 0, 0, 0};
                 publish(end_);
                 for (int i = 0; i < 64; ++i) __nanosleep(10000);
             }
@@ -722,8 +729,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         WorkItem wi;
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
-            Unit un;
-            if (!decode_unit_warp(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
+            const Unit un = wi.un;
             // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
             const int srow0 = un.mt * (p.unit_rows >> 7);
             const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
@@ -829,9 +835,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         int n_item = 0;
         WorkItem wi;
         while (ok && wq_fetch(n_item++, wi, ok)) {
-            const int u = wi.u, gb = wi.gb, ge = wi.ge;
-            Unit un;
-            if (!decode_unit_warp(u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, un)) break;
+            const int gb = wi.gb, ge = wi.ge;
+            const Unit un = wi.un;
 #pragma unroll
             for (int a = 0; a < C::NACCUM; ++a)
 #pragma unroll
