@@ -28,6 +28,18 @@ using namespace b200moe;
 
 constexpr int PROF_POINTS = 7;   // before route, after route, permute, gather, gemm1, gemm2, combine
 
+// The tensor maps of a forward depend on addresses and sizes only; a caller repeats them from step to step (weights,
+// workspace), and encoding five of them is ~4 us of host time per forward.
+struct MapSet { CUtensorMap w13, w2, a, hi, lo; };
+struct MapKey {
+    const void *w13, *w2, *a, *hi, *lo;
+    int rows_cap, ntok;
+    bool operator==(const MapKey& o) const {
+        return w13 == o.w13 && w2 == o.w2 && a == o.a && hi == o.hi && lo == o.lo && rows_cap == o.rows_cap && ntok == o.ntok;
+    }
+};
+constexpr int MAP_SETS = 8;      // kept per handle, oldest replaced first
+
 struct b200moe_ctx {
     b200moe_config cfg;
     int device;
@@ -42,6 +54,10 @@ struct b200moe_ctx {
     int fuse_combine;          // b200moe_set_fused_combine: GEMM2 epilogue adds a token's rows up (narrow tiles); default off
     int* d_sync;               // device, 64 bytes, zero between calls: the meeting words of the fused front end
                                // (front.cuh).  One forward per handle may be in flight at a time.
+    std::mutex map_mutex;
+    MapKey map_key[MAP_SETS];
+    MapSet map_set[MAP_SETS];
+    int map_count, map_next;   // entries in use, entry to replace next
 };
 
 namespace {
@@ -367,6 +383,28 @@ inline cudaError_t prof_mark(b200moe_ctx* h, int point, cudaStream_t st) {
     return cudaEventRecord(h->prof_events[slot * PROF_POINTS + point], st);
 }
 
+// The tensor maps of a forward, from the handle's small cache or encoded now.
+int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
+    const b200moe_config& c = h->cfg;
+    std::lock_guard<std::mutex> lock(h->map_mutex);
+    for (int i = 0; i < h->map_count; ++i)
+        if (h->map_key[i] == k) { *out = h->map_set[i]; return 0; }
+    MapSet m;
+    int rc;
+    const uint64_t El = (uint64_t)c.num_local_experts, H = (uint64_t)c.hidden, I = (uint64_t)c.intermediate;
+    if ((rc = make_map(&m.w13, k.w13, El * 2 * I, H, 128))) return rc;
+    if ((rc = make_map(&m.w2, k.w2, El * H, I, 128))) return rc;
+    if ((rc = make_map(&m.a, k.a, k.rows_cap, H, k.ntok))) return rc;
+    if ((rc = make_map(&m.hi, k.hi, k.rows_cap, I, k.ntok))) return rc;
+    if ((rc = make_map(&m.lo, k.lo, k.rows_cap, I, k.ntok))) return rc;
+    h->map_key[h->map_next] = k;
+    h->map_set[h->map_next] = m;
+    h->map_next = (h->map_next + 1) % MAP_SETS;
+    if (h->map_count < MAP_SETS) ++h->map_count;
+    *out = m;
+    return 0;
+}
+
 // Everything after routing: permute -> gather -> GEMM1 -> GEMM2 -> combine.
 int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, const void* hidden,
                 const void* hidden_scale, const void* w13, const void* s13, const void* w2, const void* s2, int T,
@@ -392,21 +430,17 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     float* act_scale = reinterpret_cast<float*>(ws + L.act_scale);
     __half* y = reinterpret_cast<__half*>(ws + L.y);
 
-    CUtensorMap m_w13, m_w2, m_a, m_hi, m_lo;
+    MapSet maps;
     int rc;
     const bool pairs = use_pairs(h, ntok);
-    if ((rc = make_map(&m_w13, w13, (uint64_t)El * 2 * I, H, 128))) return rc;
-    if ((rc = make_map(&m_w2, w2, (uint64_t)El * H, I, 128))) return rc;
     // Optional (b200moe_set_tma_gather), 128-token tiles: GEMM1 reads the token rows straight from the caller's
     // activations with four-row TMA gathers through row_token (one-row boxes; rows `pitch` bytes apart when they sit
     // inside packed dispatch rows) - no gather copy.  Same results; measured three times slower (32 gathers per
     // 128-K block from one producer thread: ~100 ns each), so the copy stays the default.
     const bool g4 = ntok == 128 && !pairs && h->tma_gather;
-    if (g4) {
-        if ((rc = make_map(&m_a, hidden, (uint64_t)T, H, 1, wire_pitch > 0 ? (uint64_t)wire_pitch : 0))) return rc;
-    } else if ((rc = make_map(&m_a, a_perm, rows_cap, H, ntok))) return rc;
-    if ((rc = make_map(&m_hi, act_hi, rows_cap, I, ntok))) return rc;
-    if ((rc = make_map(&m_lo, act_lo, rows_cap, I, ntok))) return rc;
+    if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, ntok}, &maps))) return rc;
+    if (g4 && (rc = make_map(&maps.a, hidden, (uint64_t)T, H, 1, wire_pitch > 0 ? (uint64_t)wire_pitch : 0))) return rc;
+    const CUtensorMap &m_w13 = maps.w13, &m_w2 = maps.w2, &m_a = maps.a, &m_hi = maps.hi, &m_lo = maps.lo;
 
     PlanParams pp;
     pp.T = T; pp.top_k = c.top_k; pp.num_local = El; pp.local_offset = local_offset; pp.token_tile = ntok;
@@ -581,6 +615,7 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
     h->wait_limit_ns = WAIT_LIMIT_NS;
     { const char* e = getenv("B200MOE_FUSE_COMBINE"); h->fuse_combine = e ? atoi(e) != 0 : 0; }
     h->token_tile = 0;
+    h->map_count = h->map_next = 0;
     { const char* e = getenv("B200MOE_GATHER4"); h->tma_gather = e ? atoi(e) != 0 : 0; }
     h->d_sync = nullptr;
     if (cudaMalloc(&h->d_sync, 64) != cudaSuccess || cudaMemset(h->d_sync, 0, 64) != cudaSuccess) {

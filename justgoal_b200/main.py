@@ -32,6 +32,12 @@ def _scalar(v, kind):
     return kind(v)
 
 
+# The raw handle of the current stream of a device, without building a torch.cuda.Stream object first (2.5 us of the
+# ~30 us of host time a small forward had); the public call where this torch has no such function.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 class MoELayer:
     """One rank's share of an MoE layer of a fixed shape: a library handle plus workspaces
     cached per token count (the reference caches per (T, device): GF main.py:68-94)."""
@@ -47,6 +53,9 @@ class MoELayer:
         with torch.cuda.device(self.device):
             _lib.check(_lib.lib.b200moe_create(C.byref(cfg), C.byref(self._h)), "b200moe_create")
         self._ws = {}
+        self._ws_last = (-1, None, 0, 0)      # workspace() of the last token count: (T, tensor, address, bytes)
+        self._shapes = (-1, ())               # tensor shapes of a forward over that many tokens
+        self._forward = _lib.lib.b200moe_forward
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -112,6 +121,7 @@ class MoELayer:
         (tuning and tests).  Workspaces are sized per tile, so the cached ones are dropped."""
         _lib.check(_lib.lib.b200moe_set_token_tile(self._h, int(tokens)), "b200moe_set_token_tile")
         self._ws.clear()
+        self._ws_last = (-1, None, 0, 0)
 
     def set_tma_gather(self, on: bool):
         """128-token tiles only: GEMM1 gathers its token rows by TMA instead of reading a gathered copy (same bits;
@@ -139,26 +149,51 @@ class MoELayer:
     def forward(self, routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                 gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                 routed_scaling_factor, output=None):
-        s = self.shape
-        T = int(hidden_states.shape[0])
-        self._check(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
-                    gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, T)
+        T = hidden_states.shape[0]
+        tensors = (routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
+                   gemm2_weights, gemm2_weights_scale)
+        if not self._as_expected(tensors, T):
+            self._check(*tensors, T)               # names the tensor that is off
         if output is None:
-            output = torch.empty(T, s.hidden, dtype=torch.bfloat16, device=hidden_states.device)
-        elif output.shape != (T, s.hidden) or output.dtype != torch.bfloat16 or not output.is_contiguous():
+            output = torch.empty(T, self.shape.hidden, dtype=torch.bfloat16, device=hidden_states.device)
+        elif output.shape != (T, self.shape.hidden) or output.dtype != torch.bfloat16 or not output.is_contiguous():
             raise ValueError("output must be a contiguous bf16 [T, hidden] tensor")
         if T == 0:
             return output
-        ws = self.workspace(T)
-        tensors = [_contig(t) if t is not None else None for t in (
-            routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
-            gemm1_weights_scale, gemm2_weights, gemm2_weights_scale)]
-        stream = torch.cuda.current_stream(hidden_states.device).cuda_stream
-        rc = _lib.lib.b200moe_forward(self._h, *[_ptr(t) for t in tensors], T,
-                                      _scalar(local_expert_offset, int), _scalar(routed_scaling_factor, float),
-                                      _ptr(output), _ptr(ws), ws.numel(), C.c_void_p(stream))
-        _lib.check(rc, "b200moe_forward")
+        last = self._ws_last
+        if last[0] != T:
+            ws = self.workspace(T)
+            last = self._ws_last = (T, ws, ws.data_ptr(), ws.numel())
+        tensors = [t if t is None or t.is_contiguous() else t.contiguous() for t in tensors]
+        if type(local_expert_offset) is not int:
+            local_expert_offset = _scalar(local_expert_offset, int)
+        if type(routed_scaling_factor) is not float:
+            routed_scaling_factor = _scalar(routed_scaling_factor, float)
+        rc = self._forward(self._h, *[None if t is None else t.data_ptr() for t in tensors], T, local_expert_offset,
+                           routed_scaling_factor, output.data_ptr(), last[2], last[3], _raw_stream(hidden_states.get_device()))
+        if rc:
+            _lib.check(rc, "b200moe_forward")
         return output
+
+    def _as_expected(self, tensors, T) -> bool:
+        """Whether a forward's tensors have the shapes, dtypes and place that `_check` asks for, in one expression (the
+        shapes of the last token count are kept: a decode loop repeats it)."""
+        known = self._shapes
+        if known[0] != T:
+            s = self.shape
+            H, I, E, El = s.hidden, s.intermediate, s.num_experts, s.num_local_experts
+            known = self._shapes = (T, tuple(torch.Size(x) for x in (
+                (T, E), (T, H), (H // 128, T), (El, 2 * I, H), (El, 2 * I // 128, H // 128), (El, H, I), (El, H // 128, I // 128),
+                (E,))))
+        n = known[1]
+        lg, bias, hs, hss, w13, s13, w2, s2 = tensors
+        f8, f32 = torch.float8_e4m3fn, torch.float32
+        return (lg.shape == n[0] and hs.shape == n[1] and hss.shape == n[2] and w13.shape == n[3] and s13.shape == n[4]
+                and w2.shape == n[5] and s2.shape == n[6]
+                and lg.dtype is f32 and hs.dtype is f8 and hss.dtype is f32 and w13.dtype is f8 and s13.dtype is f32
+                and w2.dtype is f8 and s2.dtype is f32
+                and lg.is_cuda and hs.is_cuda and hss.is_cuda and w13.is_cuda and s13.is_cuda and w2.is_cuda and s2.is_cuda
+                and (bias is None or (bias.shape == n[7] and bias.dtype is torch.bfloat16 and bias.is_cuda)))
 
     def forward_routed(self, topk_idx, topk_w, hidden_states, hidden_states_scale, gemm1_weights,
                        gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset, output=None,
@@ -300,9 +335,9 @@ def quantize_1x128(x: torch.Tensor):
     T, H = int(x.shape[0]), int(x.shape[1])
     q = torch.empty(T, H, dtype=torch.float8_e4m3fn, device=x.device)
     sc = torch.empty(H // 128, T, dtype=torch.float32, device=x.device)
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    _lib.check(_lib.lib.b200moe_quantize_1x128(_ptr(x), T, H, _ptr(q), _ptr(sc), C.c_void_p(stream)),
-               "b200moe_quantize_1x128")
+    rc = _lib.lib.b200moe_quantize_1x128(x.data_ptr(), T, H, q.data_ptr(), sc.data_ptr(), _raw_stream(x.get_device()))
+    if rc:
+        _lib.check(rc, "b200moe_quantize_1x128")
     return q, sc
 
 
@@ -387,21 +422,29 @@ class HostPipeline:
             st.synchronize()
 
 
-@torch.no_grad()
+def _operator_layer(routing_logits, hidden_states, gemm1_weights) -> MoELayer:
+    """`_layer_for` with the operator's routing, looked up by the tensors' sizes alone."""
+    w = gemm1_weights.shape
+    key = (hidden_states.shape[1], w[1], routing_logits.shape[1], w[0], hidden_states.get_device())
+    layer = _layers.get(key)
+    if layer is None:
+        layer = _layers[key] = _layer_for(routing_logits, hidden_states, gemm1_weights)
+    return layer
+
+
 def run(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
         gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor):
     """DeepSeek-V3 routing (top-8 of 8 groups, 4 groups kept), returns bf16 [T, hidden]."""
-    layer = _layer_for(routing_logits, hidden_states, gemm1_weights)
+    layer = _operator_layer(routing_logits, hidden_states, gemm1_weights)
     return layer.forward(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                          gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                          routed_scaling_factor)
 
 
-@torch.no_grad()
 def run_dps(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights, gemm1_weights_scale,
             gemm2_weights, gemm2_weights_scale, local_expert_offset, routed_scaling_factor, output):
     """Destination-passing twin of `run`: writes into `output` and returns it."""
-    layer = _layer_for(routing_logits, hidden_states, gemm1_weights)
+    layer = _operator_layer(routing_logits, hidden_states, gemm1_weights)
     return layer.forward(routing_logits, routing_bias, hidden_states, hidden_states_scale, gemm1_weights,
                          gemm1_weights_scale, gemm2_weights, gemm2_weights_scale, local_expert_offset,
                          routed_scaling_factor, output=output)
