@@ -33,9 +33,9 @@ constexpr int PROF_POINTS = 7;   // before route, after route, permute, gather, 
 struct MapSet { CUtensorMap w13, w2, a, hi, lo; };
 struct MapKey {
     const void *w13, *w2, *a, *hi, *lo;
-    int rows_cap, ntok;
+    int rows_cap, box_rows;
     bool operator==(const MapKey& o) const {
-        return w13 == o.w13 && w2 == o.w2 && a == o.a && hi == o.hi && lo == o.lo && rows_cap == o.rows_cap && ntok == o.ntok;
+        return w13 == o.w13 && w2 == o.w2 && a == o.a && hi == o.hi && lo == o.lo && rows_cap == o.rows_cap && box_rows == o.box_rows;
     }
 };
 constexpr int MAP_SETS = 8;      // kept per handle, oldest replaced first
@@ -154,6 +154,12 @@ int pick_token_tile(const b200moe_ctx* h, int T) {
     return 128;
 }
 
+// 128-token tiles: do most tiles hold fewer than 128 rows?  Below one tile's worth of expected rows per expert they do,
+// and the kernels that leave empty row quarters out are ahead (gemm.cuh, PART); above it full tiles dominate.
+bool tiles_mostly_part_full(const b200moe_config& c, int T) {
+    return (double)T * c.top_k / c.num_experts < 128.0;
+}
+
 // Partial-sum slots of the chunked units: (fewer than grid units) x (chunks per unit) x (floats per slot), the larger
 // of the two GEMMs (they run one after the other and share the area).
 template <int NTOK>
@@ -212,17 +218,17 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     L->total_bytes = off;
 }
 
-template <int NTOK, bool G1, bool G4 = false>
+template <int NTOK, bool G1, bool G4 = false, bool PART = false>
 cudaError_t set_attr() {
     using C = GemmCfg<NTOK, G1>;
     if (C::REALLOC_REGS) {
         // the kernel's setmaxnreg arithmetic assumes the launch allocation; refuse to run otherwise
         cudaFuncAttributes fa;
-        cudaError_t e = cudaFuncGetAttributes(&fa, gemm_kernel<NTOK, G1, G4>);
+        cudaError_t e = cudaFuncGetAttributes(&fa, gemm_kernel<NTOK, G1, G4, PART>);
         if (e != cudaSuccess) return e;
         if (fa.numRegs != C::LAUNCH_REGS) return (cudaError_t)(-B200MOE_E_BUILD + 100000);   // decoded by CU_TRY_ATTR
     }
-    return cudaFuncSetAttribute(gemm_kernel<NTOK, G1, G4>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    return cudaFuncSetAttribute(gemm_kernel<NTOK, G1, G4, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
 }
 
 template <int NTOK, bool G1>
@@ -237,6 +243,14 @@ cudaError_t launch_gemm_g4(int grid, cudaStream_t st, const CUtensorMap& w, cons
                            const GemmParams& p) {
     return launch_k(PDL_GEMM1, gemm_kernel<128, true, true>, dim3(grid), dim3(GemmCfg<128, true>::NTHREADS),
                     GemmCfg<128, true>::SMEM_BYTES, st, w, b0, b1, p);
+}
+
+// 128-token tiles, most of them part full
+template <bool G1>
+cudaError_t launch_gemm_part(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+                             const GemmParams& p) {
+    return launch_k(G1 ? PDL_GEMM1 : PDL_GEMM2, gemm_kernel<128, G1, false, true>, dim3(grid), dim3(GemmCfg<128, G1>::NTHREADS),
+                    GemmCfg<128, G1>::SMEM_BYTES, st, w, b0, b1, p);
 }
 
 template <bool G1>
@@ -394,9 +408,9 @@ int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
     const uint64_t El = (uint64_t)c.num_local_experts, H = (uint64_t)c.hidden, I = (uint64_t)c.intermediate;
     if ((rc = make_map(&m.w13, k.w13, El * 2 * I, H, 128))) return rc;
     if ((rc = make_map(&m.w2, k.w2, El * H, I, 128))) return rc;
-    if ((rc = make_map(&m.a, k.a, k.rows_cap, H, k.ntok))) return rc;
-    if ((rc = make_map(&m.hi, k.hi, k.rows_cap, I, k.ntok))) return rc;
-    if ((rc = make_map(&m.lo, k.lo, k.rows_cap, I, k.ntok))) return rc;
+    if ((rc = make_map(&m.a, k.a, k.rows_cap, H, k.box_rows))) return rc;
+    if ((rc = make_map(&m.hi, k.hi, k.rows_cap, I, k.box_rows))) return rc;
+    if ((rc = make_map(&m.lo, k.lo, k.rows_cap, I, k.box_rows))) return rc;
     h->map_key[h->map_next] = k;
     h->map_set[h->map_next] = m;
     h->map_next = (h->map_next + 1) % MAP_SETS;
@@ -438,7 +452,8 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     // inside packed dispatch rows) - no gather copy.  Same results; measured three times slower (32 gathers per
     // 128-K block from one producer thread: ~100 ns each), so the copy stays the default.
     const bool g4 = ntok == 128 && !pairs && h->tma_gather;
-    if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, ntok}, &maps))) return rc;
+    const bool part = ntok == 128 && !pairs && !g4 && tiles_mostly_part_full(c, T);
+    if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, part ? GemmCfg<128, true>::PART_ROWS : ntok}, &maps))) return rc;
     if (g4 && (rc = make_map(&maps.a, hidden, (uint64_t)T, H, 1, wire_pitch > 0 ? (uint64_t)wire_pitch : 0))) return rc;
     const CUtensorMap &m_w13 = maps.w13, &m_w2 = maps.w2, &m_a = maps.a, &m_hi = maps.hi, &m_lo = maps.lo;
 
@@ -509,6 +524,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g1.klog = g1.trace + (size_t)2 * h->num_sms * TRACE_SLOTS;
     if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
     else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, g1));
+    else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, g1));
     else CU_TRY(launch_gemm_ntok<true>(ntok, h->num_sms, st, m_w13, m_a, m_a, g1));
     CU_TRY(prof_mark(h, 4, st));
 
@@ -536,6 +552,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
     }
     if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
+    else if (part) CU_TRY(launch_gemm_part<false>(h->num_sms, st, m_w2, m_hi, m_lo, g2));
     else CU_TRY(launch_gemm_ntok<false>(ntok, h->num_sms, st, m_w2, m_hi, m_lo, g2));
     CU_TRY(prof_mark(h, 5, st));
 
@@ -607,6 +624,7 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
     CU_TRY_ATTR((set_attr<32, true>()));  CU_TRY_ATTR((set_attr<32, false>()));
     CU_TRY_ATTR((set_attr<64, true>()));  CU_TRY_ATTR((set_attr<64, false>()));
     CU_TRY_ATTR((set_attr<128, true>())); CU_TRY_ATTR((set_attr<128, false>())); CU_TRY_ATTR((set_attr<128, true, true>()));
+    CU_TRY_ATTR((set_attr<128, true, false, true>())); CU_TRY_ATTR((set_attr<128, false, false, true>()));
 #undef CU_TRY_ATTR
     b200moe_ctx* h = new (std::nothrow) b200moe_ctx;
     if (!h) return B200MOE_E_BADARG;

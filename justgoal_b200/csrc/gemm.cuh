@@ -114,6 +114,9 @@ struct GemmCfg {
     // block ahead; the others get the tile's NTOK scales copied into the stage
     static constexpr bool SCALES_IN_STAGE = NTOK != 128;
     static constexpr int TX_BYTES = NA * A_BYTES + NB * B_BYTES + (SCALES_IN_STAGE ? NTOK * 4 : 0);
+    // 128-token tiles that are mostly part full (kernel parameter PART): the token rows travel in boxes of PART_ROWS, and
+    // only the boxes that hold rows of the unit
+    static constexpr int PART_ROWS = 32;
     static constexpr int EMPTY_COUNT = 1 + (SCALES_IN_STAGE ? (NTOK >= 64 ? 8 : 4) : 0);   // MMA commit (+ promotion warps)
     static constexpr int STAGES_RAW = (208 * 1024) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -304,16 +307,21 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 
 // G4 (GEMM1 with 128-token tiles only): the token rows come straight from the caller's activations by four-row TMA
 // gathers (GemmParams::g4_row_token); a separate instantiation, so the plain kernel's code is unchanged by it.
-template <int NTOK, bool G1, bool G4 = false>
+// PART (128-token tiles): quarters of a token tile (32 rows, one warp's TMEM lanes) that hold no row of the unit are neither
+// loaded nor folded; what the stage holds there only reaches result rows that nobody reads.  Measured at 39 rows per
+// expert (901 tokens): GEMM1 160 -> 148 us, GEMM2 90 -> 86 us.  With full tiles the extra path costs the promotion loop 4 %
+// of its cycles, so the host picks the instance by the expected number of rows per expert (b200moe.cu).
+template <int NTOK, bool G1, bool G4 = false, bool PART = false>
 __global__ void __launch_bounds__(GemmCfg<NTOK, G1>::NTHREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
             const __grid_constant__ CUtensorMap tm_b1, const GemmParams p) {
     using C = GemmCfg<NTOK, G1>;
     static_assert(!G4 || (C::TOK_ON_M && G1), "TMA-gathered token rows: GEMM1 with 128-token tiles");
+    static_assert(!PART || (C::TOK_ON_M && !G4), "part-full tiles: tokens on M");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);     // full[S], empty[S], tfull[NTB], tempty[NTB], red[4], all, wq_full[WQ], wq_empty[WQ]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);     // full[S], empty[S], tfull[NTB], tempty[NTB], red[4], wq_full[WQ], wq_empty[WQ]
     uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tail + C::BAR_BYTES - 8);
     int* s_wq = reinterpret_cast<int*>(tail + C::BAR_BYTES);          // [WQ][WQ_INTS] work items, 16-byte aligned
     int* s_tiles = s_wq + C::WQ * C::WQ_INTS;
@@ -341,17 +349,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     const uint32_t bar_empty = bar_full + 8 * C::STAGES;
     const uint32_t bar_tfull = bar_empty + 8 * C::STAGES;
     const uint32_t bar_tempty = bar_tfull + 8 * C::NTB;
-    const uint32_t bar_red = bar_tempty + 8 * C::NTB;    // one per column group: its 4 warps meet here (bounded)
-    const uint32_t bar_all = bar_red + 8 * 4;             // all promotion warps meet here (tokens-on-M epilogue)
-    const uint32_t bar_wqfull = bar_all + 8;              // work queue: the producer has published item n
+    // warps that meet in the epilogue (bounded): the 4 warps of a column group or, tokens on M, those of a lane quarter
+    const uint32_t bar_red = bar_tempty + 8 * C::NTB;
+    const uint32_t bar_wqfull = bar_red + 8 * 4;            // work queue: the producer has published item n
     const uint32_t bar_wqempty = bar_wqfull + 8 * C::WQ;  // ... and the MMA warp and every promotion warp have read it
-    static_assert(8 * (2 * C::STAGES + 2 * C::NTB + 5 + 2 * C::WQ) <= C::BAR_BYTES - 8, "barrier area");
+    static_assert(8 * (2 * C::STAGES + 2 * C::NTB + 4 + 2 * C::WQ) <= C::BAR_BYTES - 8, "barrier area");
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, C::EMPTY_COUNT); }
         for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1 + C::NHELP); mbar_init(bar_tempty + 8 * b, C::NPW); }
-        for (int g = 0; g < 4; ++g) mbar_init(bar_red + 8 * g, 4);
-        mbar_init(bar_all, C::NPW);
+        for (int g = 0; g < 4; ++g) mbar_init(bar_red + 8 * g, C::TOK_ON_M ? C::NGRP : 4);
         for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + C::NHELP + C::NPW); }
         mbar_fence_init();
         tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_b0);
@@ -543,10 +550,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const Unit un = wi.un;
                 const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows;
                 const int kb_end = min(p.KB, ge * C::KPB);
+                const int boxes = PART ? (un.nvalid + C::PART_ROWS - 1) / C::PART_ROWS : 1;
+                const uint32_t tx = PART ? (uint32_t)(C::NA * C::A_BYTES + C::NB * boxes * C::PART_ROWS * 128) : (uint32_t)C::TX_BYTES;
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
-                    mbar_arrive_expect_tx(full, C::TX_BYTES);
+                    mbar_arrive_expect_tx(full, tx);
                     if (p.evict_first_weights) {
                         tma_load_2d_hint(st, &tm_w, kb * 128, wrow, full, pol);
                         tma_load_2d_hint(st + C::A_BYTES, &tm_w, kb * 128, wrow + p.gate_offset, full, pol);
@@ -576,8 +585,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         }
                         return;
                     }
-                    tma_load_2d(st + C::NA * C::A_BYTES, &tm_b0, kb * 128, un.row0, full);
-                    if (!G1) tma_load_2d(st + C::NA * C::A_BYTES + C::B_BYTES, &tm_b1, kb * 128, un.row0, full);
+                    for (int b = 0; b < boxes; ++b) {
+                        const uint32_t dst = st + C::NA * C::A_BYTES + b * C::PART_ROWS * 128;
+                        tma_load_2d(dst, &tm_b0, kb * 128, un.row0 + b * C::PART_ROWS, full);
+                        if (!G1) tma_load_2d(dst + C::B_BYTES, &tm_b1, kb * 128, un.row0 + b * C::PART_ROWS, full);
+                    }
                     if (C::SCALES_IN_STAGE)
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
@@ -806,15 +818,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         const int m = quarter * 32 + lane;             // weight row inside the tile
         const int ptid = threadIdx.x - 128;
         const uint32_t tlane = (uint32_t)(quarter * 32) << 16;
-        const uint32_t my_red = bar_red + 8 * grp_id;
+        const uint32_t my_red = bar_red + 8 * (C::TOK_ON_M ? quarter : grp_id);
         int stage = 0; uint32_t phase = 0;
         int ab = 0; uint32_t aphase = 0;
-        uint32_t rphase = 0, allphase = 0;
+        uint32_t rphase = 0;
         bool ok = true, seen = false;
         int ng = 0, nu = 0;
         float acc[C::NACCUM][C::NC];
 
-        // the 4 warps of one column group meet (bounded); false = gave up
+        // the warps that share my_red meet (bounded); false = gave up
         auto group_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(my_red);
@@ -823,20 +835,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             return r;
         };
 
-        // all promotion warps meet (bounded); false = gave up
-        auto all_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_all);
-            const bool r = mbar_wait_warp(bar_all, allphase, p.status, ERR_WAIT_GROUP);
-            allphase ^= 1;
-            return r;
-        };
-
         int n_item = 0;
         WorkItem wi;
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
             const Unit un = wi.un;
+            if (PART && quarter * 32 >= un.nvalid) {
+                // no row of the unit in this warp's lanes: only hand the buffers back and count in (the warp it meets in
+                // the epilogue has no row either)
+                for (int n = ge - gb; n > 0; --n) {
+                    if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+                    if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
+                    if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
+                }
+                if (wi.kind == WK_PART && lane == 0)
+                    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.sk_count + wi.ut * 4) : "memory");
+                continue;
+            }
 #pragma unroll
             for (int a = 0; a < C::NACCUM; ++a)
 #pragma unroll
@@ -1110,12 +1125,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     acc[0][i] = v;
                     amax = fmaxf(amax, fabsf(v));
                 }
-                float* redf = reinterpret_cast<float*>(s_red);            // [NGRP][128]
+                // [2][NGRP][128], used in turn: a warp is at most one meeting ahead of the one it meets
+                static_assert(!C::TOK_ON_M || 2 * C::NGRP * 128 * 4 <= C::RED_BYTES, "row maxima");
+                float* redf = reinterpret_cast<float*>(s_red) + rphase * (C::NGRP * 128);
                 redf[grp_id * 128 + m] = amax;
-                if (!all_sync()) { ok = false; break; }
+                if (!group_sync()) { ok = false; break; }
 #pragma unroll
                 for (int g2 = 0; g2 < C::NGRP; ++g2) amax = fmaxf(amax, redf[g2 * 128 + m]);
-                if (!all_sync()) { ok = false; break; }                   // redf is reused by the next unit
                 const float scale = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
                 const float inv = amax > 0.f ? 448.0f / amax : 0.f;
                 if (m < un.nvalid) {
