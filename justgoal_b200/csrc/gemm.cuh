@@ -180,7 +180,7 @@ struct GemmCfg {
     static constexpr int WQ = 4, WQ_INTS = 12;             // depth of the in-CTA work queue, words of an entry (WorkItem)
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
     static constexpr int TABLE_INTS = 3 * (MAX_LOCAL + 1);
-    static constexpr int RED_BYTES = NPW * NC * 4;
+    static constexpr int RED_BYTES = 2 * (TOK_ON_M ? NGRP * 128 : NPW * NC) * 4;      // maxima, two halves used in turn
     static constexpr int TSD = 8;                          // tokens-on-M: slots of the token-scale ring (see the scale warps)
     static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
     static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
@@ -328,7 +328,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_row0 = s_tiles + (MAX_LOCAL + 1);
     int* s_cnt = s_row0 + (MAX_LOCAL + 1);
     uint32_t* s_red = reinterpret_cast<uint32_t*>(s_cnt + (MAX_LOCAL + 1));
-    int* s_flag = reinterpret_cast<int*>(s_red + C::NPW * C::NC);   // 8 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing
+    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 8 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
     int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 8) + 15) & ~uintptr_t(15));
     float2* s_sx = reinterpret_cast<float2*>(s_g4 + 128);          // tokens-on-M: [NACC][128] products of token and weight scale
@@ -698,17 +698,24 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             const uint64_t a0 = make_smem_desc(st);
                             const uint64_t a1 = make_smem_desc(st + C::A_BYTES);
                             const uint64_t bh = make_smem_desc(st + 2 * C::A_BYTES);
-                            const uint64_t bl = make_smem_desc(st + 2 * C::A_BYTES + C::B_BYTES);
-                            // tile t, operand half o (hi, lo): partial accumulator o when NSPLIT == 2, else both into one
+                            if constexpr (C::NSPLIT == 2) {
+                                // hi and lo token tiles are adjacent in the stage and their partial accumulators adjacent in
+                                // TMEM: ONE N = 2 NTOK MMA per weight tile and K step covers both (an MMA this narrow costs
+                                // its weight-operand read, ~60 cycles, whatever N is: 16 of them per block took 950 cycles)
+                                constexpr uint32_t idesc2 = make_idesc_f8(128, 2 * NTOK);
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                mm(d, a0 + 2 * k, bh + 2 * k, k > 0);
-                                mm(d + C::NSPLIT * NTOK, a1 + 2 * k, bh + 2 * k, k > 0);
-                            }
+                                for (int k = 0; k < 4; ++k) {
+                                    umma_f8(d, a0 + 2 * k, bh + 2 * k, idesc2, k > 0);
+                                    umma_f8(d + 2 * NTOK, a1 + 2 * k, bh + 2 * k, idesc2, k > 0);
+                                }
+                            } else {
+                                // hi and lo accumulate on top of each other
+                                const uint64_t bl = make_smem_desc(st + 2 * C::A_BYTES + C::B_BYTES);
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                mm(d + (C::NSPLIT - 1) * NTOK, a0 + 2 * k, bl + 2 * k, C::NSPLIT == 1 || k > 0);
-                                mm(d + (2 * C::NSPLIT - 1) * NTOK, a1 + 2 * k, bl + 2 * k, C::NSPLIT == 1 || k > 0);
+                                for (int k = 0; k < 8; ++k) {
+                                    mm(d, a0 + 2 * (k & 3), (k < 4 ? bh : bl) + 2 * (k & 3), k > 0);
+                                    mm(d + NTOK, a1 + 2 * (k & 3), (k < 4 ? bh : bl) + 2 * (k & 3), k > 0);
+                                }
                             }
                         }
                         umma_commit(bar_empty + 8 * stage);
@@ -822,6 +829,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         int stage = 0; uint32_t phase = 0;
         int ab = 0; uint32_t aphase = 0;
         uint32_t rphase = 0;
+        int rbuf = 0;                                  // half of s_red the next epilogue uses
         bool ok = true, seen = false;
         int ng = 0, nu = 0;
         float acc[C::NACCUM][C::NC];
@@ -1126,8 +1134,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     amax = fmaxf(amax, fabsf(v));
                 }
                 // [2][NGRP][128], used in turn: a warp is at most one meeting ahead of the one it meets
-                static_assert(!C::TOK_ON_M || 2 * C::NGRP * 128 * 4 <= C::RED_BYTES, "row maxima");
-                float* redf = reinterpret_cast<float*>(s_red) + rphase * (C::NGRP * 128);
+                                float* redf = reinterpret_cast<float*>(s_red) + rbuf * (C::NGRP * 128);
+                rbuf ^= 1;
                 redf[grp_id * 128 + m] = amax;
                 if (!group_sync()) { ok = false; break; }
 #pragma unroll
@@ -1171,45 +1179,55 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                 }
             } else if (G1) {
-                // SwiGLU, then amax over the 128 rows of the tile for every token column
-                uint32_t* red = s_red + pw * C::NC;
+                // SwiGLU, then amax over the 128 rows of the tile for every token column.  A column's scale and reciprocal
+                // are computed by one lane of every warp (lane i: column i) and handed out by shuffles; four columns'
+                // bytes are transposed inside lane quads so that a store carries four weight rows of one token.  (Per
+                // column and thread a division and two byte stores, with one warp per scheduler to hide nothing behind:
+                // 6000 cycles for 16 columns at the end of every unit.)
+                uint32_t* red = s_red + rbuf * (C::NPW * C::NC);
+                rbuf ^= 1;
+                uint32_t colmax = 0;
 #pragma unroll
                 for (int i = 0; i < C::NC; ++i) {
                     const float v = silu_f(acc[1][i]) * acc[0][i];
                     acc[0][i] = v;
                     const uint32_t wm = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fabsf(v)));
-                    if (lane == 0) red[i] = wm;
+                    if (lane == i) colmax = wm;
                 }
+                if (lane < C::NC) red[pw * C::NC + lane] = colmax;
                 if (!group_sync()) { ok = false; break; }
-                const uint32_t* rg = s_red + grp_id * 4 * C::NC;
-                const size_t col = (size_t)un.mt * 128 + m;
+                float inv = 0.f;
+                if (lane < C::NC) {
+                    const uint32_t* rg = red + grp_id * 4 * C::NC + lane;
+                    const float amax = __uint_as_float(max(max(rg[0], rg[C::NC]), max(rg[2 * C::NC], rg[3 * C::NC])));
+                    inv = amax > 0.f ? 448.0f / amax : 0.f;
+                    if (quarter == 0 && c0 + lane < un.nvalid)
+                        p.act_scale[(size_t)un.mt * p.rows_cap + un.row0 + c0 + lane] = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
+                }
+                const size_t out0 = (size_t)(un.row0 + c0 + (lane & 3)) * p.I + (size_t)un.mt * 128 + quarter * 32 + (lane & ~3);
+                // 4 x 4 byte transpose inside a lane quad: in, byte j = column i + j of this lane's weight row; out, byte j =
+                // weight row (lane & ~3) + j of column i + (lane & 3)
+                auto quad_transpose = [&](uint32_t x) -> uint32_t {
+                    const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, 1);
+                    const uint32_t r = __byte_perm(x, y, (lane & 1) ? 0x3715 : 0x6240);
+                    const uint32_t z = __shfl_xor_sync(0xFFFFFFFFu, r, 2);
+                    return __byte_perm(r, z, (lane & 2) ? 0x3276 : 0x5410);
+                };
 #pragma unroll
-                for (int i = 0; i < C::NC; i += 2) {
-                    float sc2[2], inv2[2];
+                for (int i = 0; i < C::NC; i += 4) {
+                    float q[4];
 #pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const uint32_t a4 = max(max(rg[i + j], rg[C::NC + i + j]), max(rg[2 * C::NC + i + j], rg[3 * C::NC + i + j]));
-                        const float amax = __uint_as_float(a4);
-                        sc2[j] = amax > 0.f ? amax * (1.0f / 448.0f) : 1.0f;
-                        inv2[j] = amax > 0.f ? 448.0f / amax : 0.f;
-                    }
-                    const float q0 = acc[0][i] * inv2[0], q1 = acc[0][i + 1] * inv2[1];
-                    const uint16_t hi = f32x2_to_e4m3x2(q0, q1);
-                    const float2 hf = e4m3x2_to_f32x2(hi);
-                    const uint16_t lo = f32x2_to_e4m3x2(q0 - hf.x, q1 - hf.y);
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        const int c = c0 + i + j;
-                        if (c < un.nvalid) {
-                            const size_t row = (size_t)(un.row0 + c);
-                            p.act_hi[row * p.I + col] = (uint8_t)(j ? (hi >> 8) : (hi & 0xFF));
-                            p.act_lo[row * p.I + col] = (uint8_t)(j ? (lo >> 8) : (lo & 0xFF));
-                            if (quarter == 0 && lane == ((i + j) & 31))
-                                p.act_scale[(size_t)un.mt * p.rows_cap + row] = sc2[j];
-                        }
+                    for (int j = 0; j < 4; ++j) q[j] = acc[0][i + j] * __shfl_sync(0xFFFFFFFFu, inv, i + j);
+                    const uint16_t h01 = f32x2_to_e4m3x2(q[0], q[1]), h23 = f32x2_to_e4m3x2(q[2], q[3]);
+                    const float2 f01 = e4m3x2_to_f32x2(h01), f23 = e4m3x2_to_f32x2(h23);
+                    const uint16_t l01 = f32x2_to_e4m3x2(q[0] - f01.x, q[1] - f01.y), l23 = f32x2_to_e4m3x2(q[2] - f23.x, q[3] - f23.y);
+                    const uint32_t hi = quad_transpose((uint32_t)h01 | ((uint32_t)h23 << 16));
+                    const uint32_t lo = quad_transpose((uint32_t)l01 | ((uint32_t)l23 << 16));
+                    if (c0 + i + (lane & 3) < un.nvalid) {
+                        *reinterpret_cast<uint32_t*>(p.act_hi + out0 + (size_t)i * p.I) = hi;
+                        *reinterpret_cast<uint32_t*>(p.act_lo + out0 + (size_t)i * p.I) = lo;
                     }
                 }
-                if (!group_sync()) { ok = false; break; }          // s_red is reused by the next unit
             } else {
                 const int col0 = un.mt * p.unit_rows + m;
                 const bool second = col0 + p.gate_offset < p.valid_rows;
