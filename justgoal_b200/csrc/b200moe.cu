@@ -218,17 +218,17 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     L->total_bytes = off;
 }
 
-template <int NTOK, bool G1, bool G4 = false, bool PART = false>
+template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
 cudaError_t set_attr() {
     using C = GemmCfg<NTOK, G1>;
     if (C::REALLOC_REGS) {
         // the kernel's setmaxnreg arithmetic assumes the launch allocation; refuse to run otherwise
         cudaFuncAttributes fa;
-        cudaError_t e = cudaFuncGetAttributes(&fa, gemm_kernel<NTOK, G1, G4, PART>);
+        cudaError_t e = cudaFuncGetAttributes(&fa, gemm_kernel<NTOK, G1, G4, PART, FUSE>);
         if (e != cudaSuccess) return e;
         if (fa.numRegs != C::LAUNCH_REGS) return (cudaError_t)(-B200MOE_E_BUILD + 100000);   // decoded by CU_TRY_ATTR
     }
-    return cudaFuncSetAttribute(gemm_kernel<NTOK, G1, G4, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    return cudaFuncSetAttribute(gemm_kernel<NTOK, G1, G4, PART, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
 }
 
 template <int NTOK, bool G1>
@@ -243,6 +243,22 @@ cudaError_t launch_gemm_g4(int grid, cudaStream_t st, const CUtensorMap& w, cons
                            const GemmParams& p) {
     return launch_k(PDL_GEMM1, gemm_kernel<128, true, true>, dim3(grid), dim3(GemmCfg<128, true>::NTHREADS),
                     GemmCfg<128, true>::SMEM_BYTES, st, w, b0, b1, p);
+}
+
+// GEMM2 with the combine in its epilogue
+template <int NTOK>
+cudaError_t launch_gemm_fused_ntok(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+                                   const GemmParams& p) {
+    return launch_k(PDL_GEMM2, gemm_kernel<NTOK, false, false, false, true>, dim3(grid), dim3(GemmCfg<NTOK, false>::NTHREADS),
+                    GemmCfg<NTOK, false>::SMEM_BYTES, st, w, b0, b1, p);
+}
+cudaError_t launch_gemm_fused(int ntok, int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+                              const GemmParams& p) {
+    switch (ntok) {
+        case 16: return launch_gemm_fused_ntok<16>(grid, st, w, b0, b1, p);
+        case 32: return launch_gemm_fused_ntok<32>(grid, st, w, b0, b1, p);
+        default: return launch_gemm_fused_ntok<64>(grid, st, w, b0, b1, p);
+    }
 }
 
 // 128-token tiles, most of them part full
@@ -536,6 +552,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g2.w_scale = static_cast<const float*>(s2); g2.b_scale = act_scale; g2.rows_cap = rows_cap;
     g2.row_w = row_w; g2.y = y; g2.H = H; g2.I = I; g2.ts_stride = rows_cap;
     g2.evict_first_weights = evf && ntok < 128;
+    g2.tables_done = pairs ? 0 : 1;
     g2.sk_count = reinterpret_cast<int*>(ws + L.sk_count) + 4 * h->num_sms + 4;
     g2.sk_partial = g1.sk_partial;
     g2.trace = g1.trace + (size_t)h->num_sms * TRACE_SLOTS;
@@ -552,6 +569,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
     }
     if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
+    else if (fuse) CU_TRY(launch_gemm_fused(ntok, h->num_sms, st, m_w2, m_hi, m_lo, g2));
     else if (part) CU_TRY(launch_gemm_part<false>(h->num_sms, st, m_w2, m_hi, m_lo, g2));
     else CU_TRY(launch_gemm_ntok<false>(ntok, h->num_sms, st, m_w2, m_hi, m_lo, g2));
     CU_TRY(prof_mark(h, 5, st));
@@ -624,6 +642,8 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
     CU_TRY_ATTR((set_attr<32, true>()));  CU_TRY_ATTR((set_attr<32, false>()));
     CU_TRY_ATTR((set_attr<64, true>()));  CU_TRY_ATTR((set_attr<64, false>()));
     CU_TRY_ATTR((set_attr<128, true>())); CU_TRY_ATTR((set_attr<128, false>())); CU_TRY_ATTR((set_attr<128, true, true>()));
+    CU_TRY_ATTR((set_attr<16, false, false, false, true>())); CU_TRY_ATTR((set_attr<32, false, false, false, true>()));
+    CU_TRY_ATTR((set_attr<64, false, false, false, true>()));
     CU_TRY_ATTR((set_attr<128, true, false, true>())); CU_TRY_ATTR((set_attr<128, false, false, true>()));
 #undef CU_TRY_ATTR
     b200moe_ctx* h = new (std::nothrow) b200moe_ctx;

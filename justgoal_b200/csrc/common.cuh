@@ -77,36 +77,52 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// Keeps the compiler from drawing conclusions about a flag at the place where the paths that set it meet.  Without it
+// the code that follows a wait is duplicated for "the first try succeeded" and "a later one did", and again for every wait
+// after that: the GEMM kernels grew to two and a half times their size, and their epilogues no longer stayed in the
+// instruction cache (20-30 k cycles for the first one of a launch, from L2 under full load, instead of 4 k).
+__device__ __forceinline__ bool merged(bool flag) {
+    uint32_t f = flag;
+    asm volatile("" : "+r"(f));
+    return f != 0;
+}
 // Bounded wait.  Returns false (after recording `code` in *status, first error wins) when
 // the phase did not complete within WAIT_LIMIT_NS; the caller then leaves its loop and
 // falls through to the kernel's common teardown.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = globaltimer_ns();
-    for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 0x3FFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
-            atomicCAS(status, 0, code);
-            return false;
+    bool ok = mbar_try_wait(bar, parity);
+    if (!ok) {
+        const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
+        for (uint32_t it = 1;; ++it) {
+            ok = mbar_try_wait(bar, parity);
+            if (ok || ((it & 0x3FFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS)) break;
         }
+        if (!ok) atomicCAS(status, 0, code);
     }
+    return merged(ok);
 }
 
 // The same by a converged warp, with a vote on the answer: the branch on it is then uniform for the compiler, and what the
 // loop around it carries (stage, buffer, phase) stays in uniform registers, which TMA, tcgen05.mma and tcgen05.ld take
 // their operands from.  (A 128-K block of four MMAs: 606 cycles of the issuing loop without, 513 with.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int code) {
-    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;      // the usual case costs one try and one vote
-    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, status, code));
+    bool ok = __all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity));      // the usual case costs one try and one vote
+    if (!ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, status, code));
+    return merged(ok);
 }
 // Two barriers by a converged warp: both are tried before either answer is looked at (one round trip when both phases
 // have completed), and the answers are voted on, so the control flow after it stays uniform for the compiler.
 __device__ __forceinline__ bool mbar_wait_both(uint32_t bar_a, uint32_t parity_a, int code_a, uint32_t bar_b, uint32_t parity_b,
                                                int code_b, int* status) {
     const bool a = mbar_try_wait(bar_a, parity_a), b = mbar_try_wait(bar_b, parity_b);
-    if (__all_sync(0xFFFFFFFFu, a && b)) return true;
-    const bool ok = mbar_wait(bar_a, parity_a, status, code_a) && mbar_wait(bar_b, parity_b, status, code_b);
-    return __all_sync(0xFFFFFFFFu, ok);
+    bool ok = __all_sync(0xFFFFFFFFu, a && b);
+    if (!ok) {
+        ok = mbar_wait(bar_a, parity_a, status, code_a);
+        ok = mbar_wait(bar_b, parity_b, status, code_b) && ok;
+        ok = __all_sync(0xFFFFFFFFu, ok);
+    }
+    return merged(ok);
 }
 
 // The wrappers below are one PTX instruction each; their bodies are fixed by the ISA (operand order, state spaces,

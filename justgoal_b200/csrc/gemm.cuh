@@ -22,22 +22,24 @@
 // a weight tile shared by several token tiles comes from HBM once).  The remaining U mod grid units are cut
 // along K into CHUNKS of a few K blocks, and the CTAs CLAIM those chunks one at a time from a counter in global
 // memory: SMs do not stream at the same rate under full load, and a CTA that finishes early simply takes more
-// chunks (with equal static shares the finish times of the CTAs spread by 7-10 % of the kernel).  A chunked
-// unit is finished by the CTA that runs its LAST chunk: every other chunk stores its fp32 partial to its own slot
-// and counts itself in with a release; the finisher waits (bounded) for that count, adds the slots in CHUNK order
-// (a fixed order: results are bit-identical from run to run) and runs the epilogue.  Chunks are claimed in order, so
-// the finisher only ever waits for chunks that were claimed before its own - no cycle of waiting CTAs can form.
+// chunks (with equal static shares the finish times of the CTAs spread by 7-10 % of the kernel).  Every chunk stores
+// its fp32 partial to its own slot and counts itself in; whoever arrives last adds the slots in a fixed order (results
+// are bit-identical from run to run) and runs the epilogue, so nobody waits.  GEMM1 with narrow tiles cuts the remaining
+// units into equal ranges instead (STATIC_TAIL): the piece that ends a unit waits (bounded) for pieces that their CTAs
+// ran before everything else, so no cycle of waiting CTAs can form.
 // Inside a CTA the producer claims the work and hands it to the MMA and promotion warps through a small queue
 // in shared memory.
 //
 // Small token counts (GemmParams::routed): GEMM1 follows a front-end kernel that routes, permutes and gathers in one
 // launch.  GEMM1's CTAs are resident while it runs; when it announces the routing result they build the expert tables
 // themselves and the producer streams the first weight tiles before the front end has completed - only the token
-// side of those stages waits for it.  Optionally (GemmParams::fuse_out) GEMM2's epilogue also does the combine.
+// side of those stages waits for it.  GEMM2 does the same with the tables the front end left (GemmParams::tables_done), as
+// soon as its CTA has an SM: the first weights travel under the tail of GEMM1 (T=64: 132 -> 130 us, T=7: 72 -> 70 us).
+// Optionally (FUSE) GEMM2's epilogue also does the combine.
 //
-// Warp roles: warp 0 = TMA producer (one lane), warp 1 = MMA issuer (one lane) + TMEM owner,
-// warps 2-3 idle (they complete the first warpgroup so register re-allocation is legal; with the fused combine
-// they write the zero rows of tokens that have no pair on this rank),
+// Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (whole warps, one elected lane issues),
+// warps 2-3: scale products for 128-token tiles, otherwise idle (they complete the first warpgroup so register
+// re-allocation is legal; with the fused combine they write the zero rows of tokens that have no pair on this rank),
 // warps 4.. = promotion/epilogue (4 or 8 warps; warp % 4 selects the TMEM lane quarter).
 // Every wait is bounded (common.cuh); no TMA load uses cluster multicast.
 #pragma once
@@ -68,9 +70,9 @@ struct GemmParams {
     const float* row_w; __half* y; int H;                         // GEMM2 output: y[row, h] = O[row, h] as fp16 (the routing
                                                                   // weight is applied by the combine, in fp32)
     int evict_first_weights;
-    int* sk_count;        // [4 * gridDim.x + 4] zero at launch: [4 * ut] promotion warps of chunked unit ut that have stored
-                          // their partial sums, [4 * gridDim.x] the chunk claim counter
-    float* sk_partial;    // [gridDim.x * chunks per unit] slots of SLOT_FLOATS floats: slot (ut, chunk)
+    int* sk_count;        // [4 * gridDim.x + 4] zero at launch: [4 * ut ...] arrivals of split unit ut (claimed chunks: one byte
+                          // per group of warps that arrives together), [4 * gridDim.x] the chunk claim counter
+    float* sk_partial;    // [gridDim.x * chunks per unit] slots of SLOT_FLOATS floats
     long long* klog;      // [4][KLOG_N]: CTA 0's clock at its first KLOG_N K blocks: TMA issue, data seen by the
                           // MMA warp, group seen by the promotion warps, group folded (hand-back)
     long long* trace;     // [gridDim.x][TRACE_SLOTS]: slot 0 = %globaltimer at entry, others = SM clocks since entry
@@ -79,6 +81,7 @@ struct GemmParams {
     // histogram and scan as the front end) and the producer streams the first weight tiles while the front end still
     // permutes and gathers; the token rows are loaded after the front end has completed.
     const int* routed;
+    int tables_done;              // GEMM2: the expert tables are complete before this kernel can start (see the kernel's prologue)
     const int32_t* topk_idx;      // [n_pairs] global expert ids (pair_stride == top_k on this path)
     int n_pairs, local_offset;
     // GEMM1 with 128-token tiles reading the token rows straight from the caller's activations (no gather copy), else
@@ -91,8 +94,8 @@ struct GemmParams {
     int g4_T;
     int ts_stride;        // tokens-on-M tiles: floats between a row's token scales of consecutive K blocks (rows_cap for the
                           // gathered copy, the caller's K-block stride when g4_row_token is set); K blocks * ts_stride < 2^31
-    // GEMM2 with the combine fused into its epilogue (narrow token tiles of the operator's own forward), else
-    // fuse_out == null.  tok_count[t * n_mtiles + mt] (zero at launch) counts the units that have stored the columns
+    // GEMM2 with the combine fused into its epilogue (FUSE: narrow token tiles of the operator's own forward).
+    // tok_count[t * n_mtiles + mt] (zero at launch) counts the warps (four per row) that have stored the columns
     // [256 mt, 256 mt + 256) of one of token t's rows; the warp that brings it to the number of the token's local
     // pairs adds those rows up (permute.cuh, combine_token_slab) and writes the bf16 output.  Tokens without a local
     // pair get their zero row from the otherwise idle warps 2-3.
@@ -172,10 +175,12 @@ struct GemmCfg {
     // 32 chunks instead of 8)
     static constexpr int CHUNK_BLOCKS = NTOK / 8;
     static constexpr int CHUNK_GROUPS = (CHUNK_BLOCKS / KPB) < 1 ? 1 : (CHUNK_BLOCKS / KPB);
+    static constexpr int CHUNKS_PER_CTA = 2;               // measured: 4 and 6 cost 2-10 us more at every decode size
     // GEMM1 with narrow tiles has few, long units (decode: 256 units of 3.7 MB for 148 CTAs): there the units left
-    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA, processed first (claimed
-    // chunks measured 30 % slower there: every CTA finishes units it has to collect six partial sums for, late in
-    // the kernel).  Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
+    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA, processed first.  A range touches at
+    // most two units, so a CTA stores at most one partial sum and the piece that ends a unit waits for pieces that other
+    // CTAs ran first (claimed chunks measured 5-15 us slower: every one of them costs a partial sum, late in the kernel).
+    // Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
     static constexpr bool STATIC_TAIL = G1 && NTOK <= 32;
     static constexpr int WQ = 4, WQ_INTS = 12;             // depth of the in-CTA work queue, words of an entry (WorkItem)
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
@@ -185,7 +190,7 @@ struct GemmCfg {
     static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
     static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
     static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * WQ_INTS * 4 /*work queue*/ +
-                                      TABLE_INTS * 4 + RED_BYTES + 32 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
+                                      TABLE_INTS * 4 + RED_BYTES + 48 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
     static_assert(NTOK % 16 == 0 && NTOK >= 16 && NTOK <= 128, "token tile");
     static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "tmem");
     static_assert(STAGES >= KPB + 1, "a group must fit the stage ring with room to prefetch");
@@ -201,43 +206,32 @@ enum : int { TR_ENTRY = 0, TR_PROLOGUE = 1, TR_TMA_FIRST = 2, TR_TMA_LAST = 3, T
 
 struct Unit { int e, mt, tt, row0, nvalid; };
 
-__device__ __forceinline__ bool decode_unit(int u, int n_mtiles, int num_local, int ntok, const int* s_tiles,
-                                            const int* s_row0, const int* s_cnt, Unit& o) {
-    const int q = u / n_mtiles;
-    int lo = 0, hi = num_local;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (s_tiles[mid] <= q) lo = mid; else hi = mid - 1;
-    }
-    if (lo >= num_local) return false;
-    const int ntt = s_tiles[lo + 1] - s_tiles[lo];
-    if (ntt <= 0) return false;
-    const int ul = u - s_tiles[lo] * n_mtiles;
-    o.e = lo;
-    o.mt = ul / ntt;
-    o.tt = ul - o.mt * ntt;
-    o.row0 = s_row0[lo] + o.tt * ntok;
-    o.nvalid = min(ntok, s_cnt[lo] - o.tt * ntok);
-    return o.mt < n_mtiles && o.nvalid > 0;
-}
-
-// The same by a converged warp; the result is uniform for the compiler (see mbar_wait_warp).
+// Unit number -> expert, weight tile, token tile, by a converged warp; the result is the same in all lanes and uniform for
+// the compiler (see mbar_wait_warp).  The expert is the last one whose first unit is not beyond u: two rounds of one
+// comparison per lane (a binary search was eight dependent shared-memory reads, ~500 cycles of every piece of work).
 __device__ __forceinline__ bool decode_unit_warp(int u, int n_mtiles, int num_local, int ntok, const int* s_tiles,
-                                                 const int* s_row0, const int* s_cnt, Unit& o) {
-    Unit d = {0, 0, 0, 0, 0};
-    const bool ok = decode_unit(u, n_mtiles, num_local, ntok, s_tiles, s_row0, s_cnt, d);
+                                                 const int* s_row0, const int* s_cnt, int lane, Unit& o) {
     const unsigned FULL = 0xFFFFFFFFu;
-    o.e = __shfl_sync(FULL, d.e, 0); o.mt = __shfl_sync(FULL, d.mt, 0); o.tt = __shfl_sync(FULL, d.tt, 0);
-    o.row0 = __shfl_sync(FULL, d.row0, 0); o.nvalid = __shfl_sync(FULL, d.nvalid, 0);
-    return __all_sync(FULL, ok);
+    const int per = (num_local + 31) >> 5;
+    const int i1 = lane * per;
+    const int base = (__popc(__ballot_sync(FULL, i1 < num_local && s_tiles[i1] * n_mtiles <= u)) - 1) * per;
+    const int i2 = base + lane;
+    const int e = base + __popc(__ballot_sync(FULL, lane < per && i2 < num_local && s_tiles[i2] * n_mtiles <= u)) - 1;
+    if (u < 0 || e < 0) return false;
+    const int t0 = s_tiles[e], ntt = s_tiles[e + 1] - t0;
+    const int ul = u - t0 * n_mtiles;
+    int mt = ul, tt = 0;
+    if (ntt > 1) { mt = ul / ntt; tt = ul - mt * ntt; }
+    auto uni = [&](int v) { return __shfl_sync(FULL, v, 0); };
+    o.e = uni(e); o.mt = uni(mt); o.tt = uni(tt);
+    o.row0 = uni(s_row0[e] + tt * ntok); o.nvalid = uni(min(ntok, s_cnt[e] - tt * ntok));
+    return __all_sync(FULL, ntt > 0 && o.mt < n_mtiles && o.nvalid > 0);
 }
 
-// One piece of work: unit u, K groups [gb, ge).  kind WK_WHOLE: the whole unit.  WK_PART: a piece of split unit ut
-// that does not end the unit - its partial sum goes to slot `slot`.  WK_FINISH: the piece that ends split unit ut -
-// it waits for `nwait` other pieces, adds the slots slot .. slot + nwait - 1 in that order and runs the epilogue.
-// u < 0 ends the list.
-enum : int { WK_WHOLE = 0, WK_PART = 1, WK_FINISH = 2 };
-struct WorkItem { int u, gb, ge, kind, ut, slot, nwait; Unit un; };
+// One piece of work: unit u, K groups [gb, ge).  pieces == 1: the whole unit; otherwise piece number `piece` of the split
+// unit number `ut`, whose partial sums live in the slots from `slot` on.  u < 0 ends the list.
+struct WorkItem { int u, gb, ge, ut, piece, pieces, slot; Unit un; };
+constexpr int MAX_PIECES = 128;      // arrivals of a split unit are counted in bytes
 
 // CTA that owns flat index x when `total` indices are cut into `parts` equal contiguous ranges (part c starts at
 // c * total / parts)
@@ -311,12 +305,15 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 // loaded nor folded; what the stage holds there only reaches result rows that nobody reads.  Measured at 39 rows per
 // expert (901 tokens): GEMM1 160 -> 148 us, GEMM2 90 -> 86 us.  With full tiles the extra path costs the promotion loop 4 %
 // of its cycles, so the host picks the instance by the expected number of rows per expert (b200moe.cu).
-template <int NTOK, bool G1, bool G4 = false, bool PART = false>
+// FUSE (GEMM2, narrow tiles): with the combine in the epilogue (GemmParams::fuse_out); an instance of its own, so the plain
+// kernel stays small.
+template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
 __global__ void __launch_bounds__(GemmCfg<NTOK, G1>::NTHREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
             const __grid_constant__ CUtensorMap tm_b1, const GemmParams p) {
     using C = GemmCfg<NTOK, G1>;
     static_assert(!G4 || (C::TOK_ON_M && G1), "TMA-gathered token rows: GEMM1 with 128-token tiles");
+    static_assert(!FUSE || (!G1 && !C::TOK_ON_M), "fused combine: GEMM2, narrow tiles");
     static_assert(!PART || (C::TOK_ON_M && !G4), "part-full tiles: tokens on M");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -328,9 +325,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_row0 = s_tiles + (MAX_LOCAL + 1);
     int* s_cnt = s_row0 + (MAX_LOCAL + 1);
     uint32_t* s_red = reinterpret_cast<uint32_t*>(s_cnt + (MAX_LOCAL + 1));
-    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 8 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing
+    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 12 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last)
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
-    int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 8) + 15) & ~uintptr_t(15));
+    int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 12) + 15) & ~uintptr_t(15));
     float2* s_sx = reinterpret_cast<float2*>(s_g4 + 128);          // tokens-on-M: [NACC][128] products of token and weight scale
     float* s_ts = reinterpret_cast<float*>(s_sx + C::NACC * 128);  // ... and [TSD][128] token scales on their way
 
@@ -365,57 +362,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         if (!G1) tma_prefetch_desc(&tm_b1);
     }
     if (warp == 1) { tmem_alloc(smem_u32(s_tmem), C::TMEM_COLS); tmem_relinquish(); }
-    // everything above touches only this CTA's shared memory and TMEM; the tables below are
-    // written by the kernels before this one
-    bool early = false;             // tables built here, before the previous kernel has completed
-    if (G1 && p.routed) {
-        if (threadIdx.x == 0) {
-            int seen = 0;
-            const unsigned long long t0 = globaltimer_ns();
-            for (uint32_t it = 1;; ++it) {
-                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.routed) : "memory");
-                if (seen) break;
-                if ((it & 0xFFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) break;     // fall back to the tables
-            }
-            *s_flag = seen;
-        }
-        for (int i = threadIdx.x; i <= p.num_local; i += blockDim.x) s_cnt[i] = 0;
-        __syncthreads();
-        early = *s_flag != 0;
-    }
-    if (early) {
-        for (int i = threadIdx.x; i < p.n_pairs; i += blockDim.x) {
-            const int le = __ldcg(p.topk_idx + i) - p.local_offset;
-            if (le >= 0 && le < p.num_local) atomicAdd(&s_cnt[le], 1);
-        }
-        __syncthreads();
-        if (warp == 0) scan_counts(s_cnt, p.num_local, NTOK, s_row0, s_tiles, nullptr, lane);
-    } else {
-        pdl_wait();
-        for (int i = threadIdx.x; i <= p.num_local; i += blockDim.x) {
-            s_tiles[i] = p.tile_prefix[i];
-            s_row0[i] = p.expert_row0[i];
-            s_cnt[i] = i < p.num_local ? p.counts[i] : 0;
-        }
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // early schedule: the producer (lane 0 of warp 0, the only lane of that warp that works) waits after its first
-    // weight loads; the other warps wait here, before anything that reads the token rows.  The condition is uniform
-    // over a warp on purpose: lanes of one warp that wait would hold the producer lane at their reconvergence point.
-    if (early && warp != 0) pdl_wait();
-    pdl_launch();
     const uint32_t tmem_base = *s_tmem;
     const uint32_t smem_base = smem_u32(smem);
-    if (threadIdx.x == 0) stamp(TR_PROLOGUE);
 
     // Schedule (see the head of this file): q whole units per CTA, then chunks of the remaining units claimed
     // from a global counter.
     const int NG = (p.KB + C::KPB - 1) / C::KPB;
-    const int total_units = s_tiles[p.num_local] * p.n_mtiles;
-    const int sched_q = total_units / (int)gridDim.x;              // whole units per CTA
-    const int sched_U0 = sched_q * (int)gridDim.x;                 // first chunked unit
     int* const claim = p.sk_count + 4 * (int)gridDim.x;
 
     // Consumer side of the work queue: item n sits in slot n % WQ.  Every lane of the calling warp waits and reads,
@@ -427,8 +382,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         const int4* q = reinterpret_cast<const int4*>(s_wq + slot * C::WQ_INTS);
         const int4 q0 = q[0], q1 = q[1], q2 = q[2];
         auto uni = [](int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); };                  // uniform for the compiler
-        w.u = uni(q0.x); w.gb = uni(q0.y); w.ge = uni(q0.z); w.kind = uni(q0.w);
-        w.ut = uni(q1.x); w.slot = uni(q1.y); w.nwait = uni(q1.z); w.un.e = uni(q1.w);
+        w.u = uni(q0.x); w.gb = uni(q0.y); w.ge = uni(q0.z); w.ut = uni(q0.w);
+        w.piece = uni(q1.x); w.pieces = uni(q1.y); w.slot = uni(q1.z); w.un.e = uni(q1.w);
         w.un.mt = uni(q2.x); w.un.row0 = uni(q2.y); w.un.nvalid = uni(q2.z); w.un.tt = 0;
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
@@ -440,29 +395,67 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     if (C::REALLOC_REGS) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::CTRL_REGS));
     }
+    // Expert tables, by the control warps (the others get decoded work items).  They are written by the kernels before this
+    // one; three forms:
+    //   GEMM1 after the fused front end (p.routed): built here from the routing result, while the front end still runs;
+    //   GEMM2 (p.tables_done): written by a kernel that had completed before any CTA of the kernel before this one let
+    //     this kernel start - read past L1, without a wait;
+    //   otherwise: read after the wait for the kernel before this one.
+    // In the first two forms the producer streams weights before that wait.
+    const int ctid = threadIdx.x;
+    auto ctrl_sync = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+    bool early = false;             // the producer has not waited for the previous kernel yet
+    if (G1 && p.routed) {
+        if (ctid == 0) {
+            int seen = 0;
+            const unsigned long long t0 = globaltimer_ns();
+            for (uint32_t it = 1;; ++it) {
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.routed) : "memory");
+                if (seen) break;
+                if ((it & 0xFFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) break;     // fall back to the tables
+            }
+            *s_flag = seen;
+        }
+        for (int i = ctid; i <= p.num_local; i += 128) s_cnt[i] = 0;
+        ctrl_sync();
+        early = *s_flag != 0;
+    }
+    if (early) {
+        for (int i0 = ctid; i0 < p.n_pairs; i0 += 128 * 8) {
+            int id[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) id[j] = i0 + 128 * j < p.n_pairs ? __ldcg(p.topk_idx + i0 + 128 * j) - p.local_offset : -1;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (id[j] >= 0 && id[j] < p.num_local) atomicAdd(&s_cnt[id[j]], 1);
+        }
+        ctrl_sync();
+        if (warp == 0) scan_counts(s_cnt, p.num_local, NTOK, s_row0, s_tiles, nullptr, lane);
+    } else {
+        early = !G1 && p.tables_done;
+        if (!early) pdl_wait();
+        for (int i = ctid; i <= p.num_local; i += 128) {
+            s_tiles[i] = __ldcg(p.tile_prefix + i);
+            s_row0[i] = __ldcg(p.expert_row0 + i);
+            s_cnt[i] = i < p.num_local ? __ldcg(p.counts + i) : 0;
+        }
+    }
+    ctrl_sync();
+    // The producer (warp 0) waits after its first weight loads.  Nobody lets the next kernel start before having waited
+    // for the previous one: the next kernel may rely on everything before this one (tables_done).
+    if (warp != 0) {
+        if (early) pdl_wait();
+        pdl_launch();
+    }
+    if (threadIdx.x == 0) stamp(TR_PROLOGUE);
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer: the whole warp runs the loop, one
         // elected lane issues (see elect_one)
         {
             const uint64_t pol = policy_evict_first();
-            // Chunk size of the left-over units: about two chunks per CTA in total, never below CHUNK_GROUPS groups.  A few
-            // left-over units are cut finely so that every CTA gets a piece; many are cut into two or three chunks each
-            // (every chunk but a unit's last costs a partial-sum slot written and read, and its finisher a wait).
-            {
-                int chunk_groups = C::CHUNK_GROUPS;
-                if (total_units > sched_U0) {
-                    const int per_unit = (2 * (int)gridDim.x + (total_units - sched_U0) - 1) / (total_units - sched_U0);
-                    chunk_groups = max(chunk_groups, (NG + per_unit - 1) / per_unit);
-                }
-                if (lane == 0) {
-                    s_flag[4] = chunk_groups;
-                    s_flag[5] = (NG + chunk_groups - 1) / chunk_groups;       // chunks per chunked unit
-                }
-                __syncwarp();
-            }
-            // (kept in shared memory between the rare claims rather than in registers for the whole loop)
-            volatile int* const s_sched = s_flag + 4;
-            const int total_chunks = (total_units - sched_U0) * s_sched[1];
+            const int total_units = s_tiles[p.num_local] * p.n_mtiles;
+            const int sched_q = total_units / (int)gridDim.x;              // whole units per CTA
+            const int sched_U0 = sched_q * (int)gridDim.x;                 // first chunked unit
             int stage = 0; uint32_t phase = 0;
             bool ok = true, issued = false;
             bool waited = !early;               // early schedule: has this thread waited for the previous kernel yet
@@ -474,8 +467,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if (!mbar_wait_warp(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
                 if (lane == 0) {
                     int4* q = reinterpret_cast<int4*>(s_wq + slot * C::WQ_INTS);
-                    q[0] = make_int4(w.u, w.gb, w.ge, w.kind);
-                    q[1] = make_int4(w.ut, w.slot, w.nwait, w.un.e);
+                    q[0] = make_int4(w.u, w.gb, w.ge, w.ut);
+                    q[1] = make_int4(w.piece, w.pieces, w.slot, w.un.e);
                     q[2] = make_int4(w.un.mt, w.un.row0, w.un.nvalid, 0);
                     mbar_arrive(bar_wqfull + 8 * slot);      // release: the item is visible to whoever sees the phase flip
                 }
@@ -483,65 +476,79 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 ++n_item;
                 return true;
             };
-            // static tail: this CTA's range [t_lo, t_hi) of the flat (left-over unit, K group) space, as per-unit pieces;
-            // pieces that do not end their unit come first, then the one that does (it waits for pieces other CTAs
-            // run first, so no chain of waiting CTAs can form), then whole units
-            const int tail_units = total_units - sched_U0;
-            const int flat = tail_units * NG;
-            const int parts = flat < (int)gridDim.x ? (flat > 0 ? flat : 1) : (int)gridDim.x;
-            const bool has_tail = C::STATIC_TAIL && flat > 0 && (int)blockIdx.x < parts;
-            const int t_lo = has_tail ? range_start((int)blockIdx.x, flat, parts) : 0;
-            const int t_hi = has_tail ? range_start((int)blockIdx.x + 1, flat, parts) : 0;
-            int st_pass = has_tail ? 0 : 3, st_ut = t_lo / NG;
+            // Left-over units: `pieces` chunks of chunk_groups groups each, claimed one at a time.  How many per CTA: enough
+            // that the CTAs' finish times even out, few enough that the partial sums stay small traffic - every chunk leaves
+            // 1 KB * NTOK.  (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
+            volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, [1] pieces
+            bool sized = false;
+            auto size_chunks = [&]() {
+                const int tail_units = total_units - sched_U0;
+                int chunk_groups = C::CHUNK_GROUPS;
+                if (tail_units > 0) {
+                    const int per_unit = (C::CHUNKS_PER_CTA * (int)gridDim.x + tail_units - 1) / tail_units;
+                    chunk_groups = max(chunk_groups, (NG + per_unit - 1) / per_unit);
+                }
+                chunk_groups = max(chunk_groups, (NG + MAX_PIECES - 1) / MAX_PIECES);
+                if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = (NG + chunk_groups - 1) / chunk_groups; }
+                __syncwarp();
+                sized = true;
+            };
+            // A claim is an atomic round trip (~1 us under load): it is sent while the piece before it is still being loaded.
+            // Without whole units the first chunk is the CTA's own number, so that the start does not wait for one.
+            int ahead = (int)blockIdx.x;                                   // lane 0's is the one that counts
+            bool have_ahead = sched_q == 0;
+            const int claim0 = sched_q == 0 ? (int)gridDim.x : 0;
+            auto claim_ahead = [&]() {
+                if (!have_ahead && lane == 0) ahead = claim0 + atomicAdd(claim, 1);
+                have_ahead = true;
+            };
+            // Static tail: this CTA's range [t_lo, t_hi) of the flat (left-over unit, K group) space: the end of one unit
+            // and perhaps the start of the next.  What others wait for comes first, then the whole units, then the piece
+            // that ends a unit and waits itself (T=257: 214 -> 209 us against running it before the whole units).
+            int t_lo = 0, t_hi = 0, t_unit = 0;
+            const int flat = (total_units - sched_U0) * NG;
+            const int parts = min(flat, (int)gridDim.x);
+            if (C::STATIC_TAIL && (int)blockIdx.x < parts) {
+                t_lo = range_start((int)blockIdx.x, flat, parts); t_hi = range_start((int)blockIdx.x + 1, flat, parts);
+                t_unit = t_lo / NG;
+            }
             while (ok) {
                 WorkItem wi;
-                wi.kind = WK_WHOLE; wi.ut = -1; wi.slot = 0; wi.nwait = 0; wi.un = Unit{0, 0, 0, 0, 0};
-                bool have = false;
-                while (st_pass < 3 && !have) {
-                    const int ut_last = (t_hi - 1) / NG;
-                    while (st_ut <= ut_last && !have) {
-                        const int ut = st_ut++;
-                        const int u_lo = ut * NG;
-                        const int gb = max(t_lo, u_lo) - u_lo, ge = min(t_hi, u_lo + NG) - u_lo;
-                        const int kind = (gb == 0 && ge == NG) ? WK_WHOLE : (ge == NG ? WK_FINISH : WK_PART);
-                        const int want = st_pass == 0 ? WK_PART : (st_pass == 1 ? WK_FINISH : WK_WHOLE);
-                        if (kind != want) continue;
-                        wi.u = sched_U0 + ut; wi.gb = gb; wi.ge = ge; wi.kind = kind; wi.ut = ut;
-                        if (kind == WK_PART) {
-                            wi.slot = (int)blockIdx.x;              // a CTA stores at most one partial: its own slot
-                        } else if (kind == WK_FINISH) {
-                            wi.slot = range_owner(u_lo, flat, parts);          // CTA of the unit's first piece
-                            wi.nwait = (int)blockIdx.x - wi.slot;
-                            if (wi.nwait == 0) wi.kind = WK_WHOLE;             // cannot happen (gb > 0), kept for safety
-                        }
-                        have = true;
+                wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0, 0};
+                const int u_end = (t_unit + 1) * NG;
+                const bool ends_unit = t_lo > t_unit * NG && t_hi == u_end;         // the rest of the range is such a piece
+                if (C::STATIC_TAIL && t_lo < t_hi && !(ends_unit && n_whole < sched_q)) {
+                    if (t_hi > u_end) {                       // the start of the next unit
+                        wi.ut = t_unit + 1; wi.gb = 0; wi.ge = t_hi - u_end;
+                        t_hi = u_end;
+                    } else {
+                        wi.ut = t_unit; wi.gb = t_lo - t_unit * NG; wi.ge = t_hi - t_unit * NG;
+                        t_lo = t_hi;
                     }
-                    if (!have) { ++st_pass; st_ut = t_lo / NG; }
-                }
-                if (have) {
+                    wi.u = sched_U0 + wi.ut;
+                    if (wi.ge < NG) {                         // does not end its unit: leaves its partial sum in its own slot
+                        wi.slot = (int)blockIdx.x; wi.pieces = 2;
+                    } else if (wi.gb > 0) {
+                        wi.slot = range_owner(wi.ut * NG, flat, parts);        // CTA of the unit's first piece
+                        wi.piece = (int)blockIdx.x - wi.slot; wi.pieces = wi.piece + 1;
+                    }
                 } else if (n_whole < sched_q) {
                     wi.u = n_whole * (int)gridDim.x + (int)blockIdx.x; wi.gb = 0; wi.ge = NG;
                     ++n_whole;
                 } else {
-                    int c = total_chunks;
-                    if (!C::STATIC_TAIL && total_chunks > 0) {
-                        if (lane == 0) c = atomicAdd(claim, 1);
-                        c = __shfl_sync(0xFFFFFFFFu, c, 0);
-                    }
-                    if (c >= total_chunks) { wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break; }
-                    const int chunk_groups = s_sched[0], CPU_ = s_sched[1];
-                    wi.ut = c / CPU_;
-                    const int ci = c - wi.ut * CPU_;
+                    if (C::STATIC_TAIL || total_units == sched_U0) { wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break; }
+                    claim_ahead();
+                    if (!sized) size_chunks();
+                    const int chunk_groups = s_sched[0], pieces = s_sched[1];
+                    const int c = __shfl_sync(0xFFFFFFFFu, ahead, 0);
+                    have_ahead = false;
+                    if (c >= (total_units - sched_U0) * pieces) { wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break; }
+                    wi.ut = c / pieces; wi.piece = c - wi.ut * pieces; wi.pieces = pieces;
+                    wi.slot = wi.ut * pieces;
                     wi.u = sched_U0 + wi.ut;
-                    wi.gb = ci * chunk_groups; wi.ge = min(NG, wi.gb + chunk_groups);
-                    if (CPU_ > 1) {
-                        // chunks are claimed in order: the one that ends the unit is claimed last and finishes it
-                        wi.kind = ci + 1 < CPU_ ? WK_PART : WK_FINISH;
-                        wi.slot = wi.kind == WK_PART ? wi.ut * CPU_ + ci : wi.ut * CPU_;
-                        wi.nwait = CPU_ - 1;
-                    }
+                    wi.gb = wi.piece * chunk_groups; wi.ge = min(NG, wi.gb + chunk_groups);
                 }
-                if (!decode_unit_warp(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, wi.un)) {
+                if (!decode_unit_warp(wi.u, p.n_mtiles, p.num_local, NTOK, s_tiles, s_row0, s_cnt, lane, wi.un)) {
                     if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
                     ok = false; break;
                 }
@@ -594,9 +601,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
                 int kb_first = gb * C::KPB;
-                if (G1 && !waited) {
-                    // early schedule, first item: the (empty) stage ring takes weight tiles while the front end still
-                    // permutes and gathers, then the wait for it, then the token side of the same stages
+                if (!waited) {
+                    // early schedule, first item: the (empty) stage ring takes weight tiles while the kernel before this one
+                    // still runs, then the wait for it, then the token side of the same stages
                     const int npre = min(C::STAGES, kb_end - kb_first);
                     for (int i = 0; i < npre; ++i) {
                         if (elect_one()) load_weights(i, kb_first + i);
@@ -624,13 +631,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (lane == 0) klog_put(0, nk);
                     ++nk;
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+                    if (!C::STATIC_TAIL && kb + 3 == kb_end && n_whole == sched_q && total_units > sched_U0) claim_ahead();
                 }
             }
             if (lane == 0) stamp(TR_TMA_LAST);
             if (!ok) {
                 // gave up: end the list for the other roles (if the queue still moves), then give copies that are
                 // still in flight time to land before the CTA's shared memory goes away
-                WorkItem end_; end_.u = -1; end_.gb = end_.ge = 0; end_.kind = WK_WHOLE; end_.ut = -1; end_.slot = end_.nwait = 0; end_.un = Unit{0, 0, 0, 0, 0};
+                WorkItem end_; end_.u = -1; end_.gb = end_.ge = end_.ut = end_.piece = end_.slot = 0; end_.pieces = 1; end_.un = Unit{0, 0, 0, 0, 0};
                 publish(end_);
                 for (int i = 0; i < 64; ++i) __nanosleep(10000);
             }
@@ -799,7 +807,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             }
         }
         cp_async_wait<0>();
-    } else if (!G1 && p.fuse_out) {
+    } else if (FUSE) {
         // ------------------------------------------------------------ warps 2-3, fused combine: zero rows of the
         // tokens that have no pair on this rank (nobody else writes them)
         for (int t = (int)blockIdx.x * 2 + (warp - 2); t < p.T; t += (int)gridDim.x * 2) {
@@ -825,6 +833,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         const int m = quarter * 32 + lane;             // weight row inside the tile
         const int ptid = threadIdx.x - 128;
         const uint32_t tlane = (uint32_t)(quarter * 32) << 16;
+        volatile int* const s_last = s_flag + 8;
         const uint32_t my_red = bar_red + 8 * (C::TOK_ON_M ? quarter : grp_id);
         int stage = 0; uint32_t phase = 0;
         int ab = 0; uint32_t aphase = 0;
@@ -845,19 +854,19 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 
         int n_item = 0;
         WorkItem wi;
+        pdl_wait();
+        pdl_launch();
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
             const Unit un = wi.un;
             if (PART && quarter * 32 >= un.nvalid) {
-                // no row of the unit in this warp's lanes: only hand the buffers back and count in (the warp it meets in
-                // the epilogue has no row either)
+                // no row of the unit in this warp's lanes: only hand the buffers back (the warp it meets in the epilogue has
+                // no row either, here and in the CTAs that run other pieces of the unit)
                 for (int n = ge - gb; n > 0; --n) {
                     if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
                     if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
                     if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
                 }
-                if (wi.kind == WK_PART && lane == 0)
-                    asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.sk_count + wi.ut * 4) : "memory");
                 continue;
             }
 #pragma unroll
@@ -1052,28 +1061,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if (!ok) break;
             if (ptid == 0) stamp(TR_PROMO_LAST);
 
-            if (wi.kind != WK_WHOLE) {
-                // ---- piece of a split unit.  The unit is finished by the CTA that runs the piece that ends it.  Every
-                // other piece only stores its partial sums and counts its warps in with a release - no meeting of
-                // the warps, no answer to wait for.
-                int* const arrived = p.sk_count + wi.ut * 4;
-                if (wi.kind == WK_PART) {
-                    float* slot = p.sk_partial + (size_t)wi.slot * C::SLOT_FLOATS;
+            if (wi.pieces > 1) {
+                float* const slots = p.sk_partial + (size_t)wi.slot * C::SLOT_FLOATS + ptid;
+                auto store_partial = [&]() {
+                    float* slot = slots + (size_t)wi.piece * C::SLOT_FLOATS;
 #pragma unroll
                     for (int a = 0; a < C::NACCUM; ++a)
 #pragma unroll
-                        for (int i = 0; i < C::NC; ++i) __stcg(slot + (size_t)(a * C::NC + i) * C::NPT + ptid, acc[a][i]);
-                    __syncwarp();        // orders the lanes' stores before lane 0's release below
-                    if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrived) : "memory");
-                    if (ptid == 0) stamp(TR_PARTIAL);
-                    continue;
-                }
-                // the piece that ends the unit: wait (bounded) until the warps of all other pieces have counted in, then
-                // add their partial sums in K order on top of this piece's own - a fixed order, whoever was quick or slow
-                const int n_other = wi.nwait;
-                const float* const slots = p.sk_partial + (size_t)wi.slot * C::SLOT_FLOATS;
-                {
-                    const int want = n_other * C::NPW;
+                        for (int i = 0; i < C::NC; ++i) __stcg(slot + (size_t)(a * C::NC + i) * C::NPT, acc[a][i]);
+                };
+                int* const arrived = p.sk_count + 4 * wi.ut;
+                if constexpr (C::STATIC_TAIL) {
+                    // ---- piece of a split unit, static ranges: the piece that ends the unit finishes it.  The others store
+                    // their partial sums and count their warps in with a release - no meeting of the warps, no answer to
+                    // wait for; the finisher waits (bounded) for that count.
+                    if (wi.ge < NG) {
+                        store_partial();
+                        __syncwarp();        // orders the lanes' stores before lane 0's release below
+                        if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrived) : "memory");
+                        if (ptid == 0) stamp(TR_PARTIAL);
+                        continue;
+                    }
+                    const int want = (wi.pieces - 1) * C::NPW;
                     bool here = true;
                     if (lane == 0) {
                         const unsigned long long t0 = globaltimer_ns();
@@ -1088,10 +1097,46 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                     here = __shfl_sync(0xFFFFFFFFu, here, 0);
                     if (!here) { ok = false; break; }
+                } else {
+                    // ---- piece of a split unit, claimed chunks: every piece stores its partial sums; the warps that arrive
+                    // last (a warp of GEMM2 by itself; those that meet in the epilogue, my_red, together in GEMM1) add all
+                    // pieces in a fixed order - the last one in K, then the others from the first on - and run the epilogue.
+                    // Nobody waits for another CTA.  (Waiting in the CTA that runs the last piece chained the waits: partial
+                    // sums are stored only after the piece before them in the same CTA, which may be waiting itself.
+                    // T=257, GEMM2: 81 -> 74 us.)
+                    const int fld = G1 ? (C::TOK_ON_M ? quarter : grp_id) : pw;
+                    store_partial();
+                    __threadfence();
+                    __syncwarp();
+                    if (ptid == 0) stamp(TR_PARTIAL);
+                    int seen_pieces = 0;
+                    auto count_in = [&]() {
+                        seen_pieces = (int)((unsigned)atomicAdd(arrived + (fld >> 2), 1 << (8 * (fld & 3))) >> (8 * (fld & 3))) & 0xFF;
+                    };
+                    if (G1) {
+                        if (!group_sync()) { ok = false; break; }
+                        const bool leader = C::TOK_ON_M ? grp_id == 0 : quarter == 0;
+                        if (leader && lane == 0) { count_in(); s_last[fld] = seen_pieces; }
+                        if (!group_sync()) { ok = false; break; }
+                        seen_pieces = s_last[fld];
+                    } else {
+                        if (lane == 0) count_in();
+                        seen_pieces = __shfl_sync(0xFFFFFFFFu, seen_pieces, 0);
+                    }
+                    if (seen_pieces != wi.pieces - 1) continue;
+                    __threadfence();
                 }
-                auto slot_of = [&](int c) -> const float* { return slots + (size_t)c * C::SLOT_FLOATS + ptid; };
+                auto slot_of = [&](int c) -> const float* { return slots + (size_t)c * C::SLOT_FLOATS; };
+                if (!C::STATIC_TAIL && wi.piece != wi.pieces - 1) {
+                    const float* src = slot_of(wi.pieces - 1);
+#pragma unroll
+                    for (int a = 0; a < C::NACCUM; ++a)
+#pragma unroll
+                        for (int i = 0; i < C::NC; ++i) acc[a][i] = __ldcg(src + (size_t)(a * C::NC + i) * C::NPT);
+                }
+                const int n_other = wi.pieces - 1;
                 if constexpr (C::NACCUM * C::NC <= 32) {
-                    // narrow tiles: the next chunk's slot is in flight while this one is added (same fixed order)
+                    // narrow tiles: the next piece's slot is in flight while this one is added (same fixed order)
                     float nxt[C::NACCUM * C::NC];
                     const float* src = slot_of(0);
 #pragma unroll
@@ -1240,14 +1285,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         if (second) p.y[row * p.H + col0 + p.gate_offset] = __float2half_rn(acc[1][i]);
                     }
                 }
-                if (p.fuse_out) {
-                    // Fused combine.  The four warps of this column group have now stored all 256 columns of the
-                    // group's NC rows: fence, meet, then count the unit in for every row's token (the group's rows
-                    // are dealt over its warps and lanes, one atomic per row, all in flight together).
+                if (FUSE) {
+                    // Fused combine.  This warp has stored its 64 of the 256 columns of the column group's NC rows: fence,
+                    // then count it in for every row's token (lane i: row i, all atomics in flight together); four warps
+                    // deliver a row.
                     __threadfence();
-                    if (!group_sync()) { ok = false; break; }
-                    const int c = c0 + quarter + 4 * lane;
-                    const bool mine = lane < C::NC / 4 && c < un.nvalid;
+                    __syncwarp();
+                    const int c = c0 + lane;
+                    const bool mine = lane < C::NC && c < un.nvalid;
                     int t = -1;
                     bool last = false;
                     if (mine) {
@@ -1257,10 +1302,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             const int le = __ldg(p.c_topk + (size_t)t * p.c_stride + k) - p.c_local_offset;
                             need += le >= 0 && le < p.num_local;
                         }
-                        last = atomicAdd(p.tok_count + (size_t)t * p.n_mtiles + un.mt, 1) == need - 1;
+                        last = atomicAdd(p.tok_count + (size_t)t * p.n_mtiles + un.mt, 1) == 4 * need - 1;
                     }
                     unsigned todo = __ballot_sync(0xFFFFFFFFu, last);
-                    if (todo) __threadfence();          // the other units' rows, counted in before this one, are visible
+                    if (todo) __threadfence();          // the other warps' rows, counted in before this one, are visible
                     while (todo) {
                         const int srcl = __ffs(todo) - 1;
                         todo &= todo - 1;
