@@ -90,11 +90,11 @@ int pdl_mask() {
     return v;
 }
 
-// Measured: with thousands of tokens the early-resident dependents slow the front kernels down
-// (2.17 ms against 1.93 ms at T=4096), with a few dozen tokens the overlap saves ~9 us per forward.
-// So the forward turns the attribute on only for small token counts (a shape-only decision).
+// With thousands of tokens the early-resident dependents slow the front kernels and GEMM1 down (8192 tokens, 256 experts:
+// 5.60 -> 5.85 ms), so only GEMM2 and the combine overlap there (14107 tokens: 1.025 -> 1.005 ms); up to 2048 tokens all
+// launches do (901 tokens: 288 -> 278 us, 2048 tokens of the 4096-wide shape: 150 -> 132 us).  A shape-only decision.
 thread_local int g_call_pdl = 0;
-inline void set_call_pdl(int num_tokens) { g_call_pdl = num_tokens <= 512 ? pdl_mask() : 0; }
+inline void set_call_pdl(int num_tokens) { g_call_pdl = num_tokens <= 2048 ? pdl_mask() : pdl_mask() & (PDL_GEMM2 | PDL_COMBINE); }
 
 template <typename... KArgs, typename... Args>
 cudaError_t launch_k(int site, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
@@ -579,20 +579,23 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         if (h->prof_slots) ++h->prof_calls;
         return 0;
     }
-    const int cgrid_x = T < h->num_sms * 8 ? T : h->num_sms * 8;
-    const dim3 cgrid(cgrid_x, T <= 256 ? 4 : 1);        // few tokens: four CTAs share a token's columns
+    // tokens a combine CTA takes at a time: as many as leave every SM its eight CTAs
+    int batch = 1;
+    while (batch < COMBINE_BATCH && T >= h->num_sms * 8 * batch * 2) batch *= 2;
+    const int cgrid_need = (T + batch - 1) / batch;
+    const dim3 cgrid(cgrid_need < h->num_sms * 8 ? cgrid_need : h->num_sms * 8, T <= 256 ? 4 : 1);   // few tokens: four CTAs share a token's columns
     SlotOut so;
     memset(&so, 0, sizeof(so));            // cap == 0: rows go to `out`
     if (slot_out) so = *slot_out;
     if (out_kind == OUT_BF16)
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_BF16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
     else if (out_kind == OUT_F16)
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
     else
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F32>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
     CU_TRY(prof_mark(h, 6, st));
     if (h->prof_slots) ++h->prof_calls;
     return 0;

@@ -187,7 +187,8 @@ __global__ void __launch_bounds__(PERMUTE_THREADS) permute_kernel(const PlanPara
 }
 
 // Expert-sorted copy of the fp8 activations and of their scales: a_perm[row] = hidden[token],
-// a_scale_perm[kb][row] = hidden_scale[kb][token].  One warp per row, grid-stride.
+// a_scale_perm[kb][row] = hidden_scale[kb][token].  One warp per row, grid-stride.  Bound by the writes: 65536 rows of 7168
+// bytes take 150-160 us, 3.1-3.3 TB/s written, whether rows, tokens or 16-row blocks are dealt out (all three measured).
 // Source forms: the operator's layouts (row pitch H, scales K-block major in hscale[kb][token]) or - hscale ==
 // nullptr - packed dispatch rows read in place (row pitch `src_pitch` bytes, the token's H/128 scales right
 // behind its H fp8 bytes).
@@ -328,33 +329,37 @@ __device__ __forceinline__ void combine_token_slab(const __half* y, const int32_
     if (h < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + h) = pack8_bf16(acc);
 }
 
+// A CTA takes `batch` (1..8) tokens at a time: warp w looks up token w's rows and weights (a chain of dependent loads, ~2 us
+// under load), then all warps stream the rows of the batch without meeting again.  With one token at a time and eight
+// CTAs per SM the chains alone were the kernel's time (14107 tokens: 100 us for 340 MB); few tokens keep batch = 1 and
+// share a token's columns over gridDim.y CTAs instead.
+constexpr int COMBINE_BATCH = 8;
 template <int OUT>
 __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__ y, const int32_t* __restrict__ topk_idx,
                                                       const int32_t* __restrict__ pair_row, const float* __restrict__ row_w,
                                                       void* __restrict__ out, int T, int H, int top_k, int pair_stride,
-                                                      int local_offset, int num_local, const SlotOut slots) {
-    __shared__ int s_rows[8];
-    __shared__ float s_w[8];
-    __shared__ int s_n;
+                                                      int local_offset, int num_local, int batch, const SlotOut slots) {
+    __shared__ int s_rows[2][COMBINE_BATCH][8];
+    __shared__ float s_w[2][COMBINE_BATCH][8];
+    __shared__ int s_n[2][COMBINE_BATCH];          // rows of the token, -1: nothing to write
     pdl_wait();
     pdl_launch();
     // gridDim.y CTAs share a token's columns (few tokens: more CTAs in flight, shorter latency chain per CTA)
     const int h_per = ((H / 8 + gridDim.y - 1) / gridDim.y) * 8;
     const int h_lo = blockIdx.y * h_per, h_hi = min(H, h_lo + h_per);
-    for (int t = blockIdx.x; t < T; t += gridDim.x) {
-        uint16_t* out_row = reinterpret_cast<uint16_t*>(out) + (size_t)t * H;      // 2-byte kinds
-        if (OUT == OUT_F16 && slots.cap > 0) {
-            if (topk_idx[(size_t)t * pair_stride] < 0) continue;    // same for the whole CTA
-            const int r = t / slots.cap;
-            out_row = static_cast<uint16_t*>(slots.back.p[r]) + ((size_t)slots.my_rank * slots.cap + (t - r * slots.cap)) * H;
-        }
-        __syncthreads();
-        if (threadIdx.x < 32) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int buf = 0;
+    for (int t0 = blockIdx.x * batch; t0 < T; t0 += gridDim.x * batch, buf ^= 1) {
+        // (two buffers: a warp is at most one meeting ahead of the others, which still read the other one)
+        if (warp < batch) {
             // lanes 0..top_k-1 fetch their pair in parallel; rows are ranked by row index (= expert order)
-            const int lane = threadIdx.x;
+            const int t = t0 + warp;
             int r = 0x7FFFFFFF;
-            if (lane < top_k) {
-                const int le = topk_idx[(size_t)t * pair_stride + lane] - local_offset;
+            bool present = t < T;
+            if (t < T && lane < top_k) {
+                const int id = topk_idx[(size_t)t * pair_stride + lane];
+                const int le = id - local_offset;
+                if (OUT == OUT_F16 && slots.cap > 0 && lane == 0 && id < 0) present = false;
                 if (le >= 0 && le < num_local) r = pair_row[(size_t)t * top_k + lane];
             }
             int rank = 0;
@@ -363,31 +368,40 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
                 rank += (rj < r) || (rj == r && j < lane);
             }
             const unsigned have = __ballot_sync(0xFFFFFFFFu, r != 0x7FFFFFFF);
-            if (r != 0x7FFFFFFF) { s_rows[rank] = r; s_w[rank] = __ldg(row_w + r); }
-            if (lane == 0) s_n = __popc(have);
+            if (r != 0x7FFFFFFF) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldg(row_w + r); }
+            if (lane == 0) s_n[buf][warp] = present ? __popc(have) : -1;
         }
         __syncthreads();
-        const int n = s_n;
-        for (int h = h_lo + threadIdx.x * 8; h < h_hi; h += blockDim.x * 8) {
-            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            // four rows' loads in flight at a time (the rows are independent; the sum order stays j = 0, 1, ...)
-            for (int j0 = 0; j0 < n; j0 += 4) {
-                uint4 v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (j0 + u < n) v[u] = *reinterpret_cast<const uint4*>(y + (size_t)s_rows[j0 + u] * H + h);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (j0 + u < n) fma8_f16(acc, v[u], s_w[j0 + u]);
+        const int nt = min(batch, T - t0);
+        for (int b = 0; b < nt; ++b) {
+            const int t = t0 + b, n = s_n[buf][b];
+            if (n < 0) continue;
+            uint16_t* out_row = reinterpret_cast<uint16_t*>(out) + (size_t)t * H;      // 2-byte kinds
+            if (OUT == OUT_F16 && slots.cap > 0) {
+                const int r = t / slots.cap;
+                out_row = static_cast<uint16_t*>(slots.back.p[r]) + ((size_t)slots.my_rank * slots.cap + (t - r * slots.cap)) * H;
             }
-            if (OUT == OUT_BF16) {
-                *reinterpret_cast<uint4*>(out_row + h) = pack8_bf16(acc);
-            } else if (OUT == OUT_F16) {
-                *reinterpret_cast<uint4*>(out_row + h) = pack8_f16(acc);
-            } else {
-                float* o = reinterpret_cast<float*>(out) + (size_t)t * H + h;
-                *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                *reinterpret_cast<float4*>(o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+            for (int h = h_lo + threadIdx.x * 8; h < h_hi; h += blockDim.x * 8) {
+                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                // four rows' loads in flight at a time (the rows are independent; the sum order stays j = 0, 1, ...)
+                for (int j0 = 0; j0 < n; j0 += 4) {
+                    uint4 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (j0 + u < n) v[u] = __ldcs(reinterpret_cast<const uint4*>(y + (size_t)s_rows[buf][b][j0 + u] * H + h));
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (j0 + u < n) fma8_f16(acc, v[u], s_w[buf][b][j0 + u]);
+                }
+                if (OUT == OUT_BF16) {
+                    *reinterpret_cast<uint4*>(out_row + h) = pack8_bf16(acc);
+                } else if (OUT == OUT_F16) {
+                    *reinterpret_cast<uint4*>(out_row + h) = pack8_f16(acc);
+                } else {
+                    float* o = reinterpret_cast<float*>(out) + (size_t)t * H + h;
+                    *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                    *reinterpret_cast<float4*>(o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+                }
             }
         }
     }
