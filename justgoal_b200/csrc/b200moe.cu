@@ -29,13 +29,13 @@ using namespace b200moe;
 constexpr int PROF_POINTS = 7;   // before route, after route, permute, gather, gemm1, gemm2, combine
 
 // The tensor maps of a forward depend on addresses and sizes only; a caller repeats them from step to step (weights,
-// workspace), and encoding five of them is ~4 us of host time per forward.
-struct MapSet { CUtensorMap w13, w2, a, hi, lo; };
+// workspace), and encoding them is ~5 us of host time per forward.
+struct MapSet { CUtensorMap w13, w2, a, hi, lo, a_box, hi_box, lo_box; };      // *_box: boxes of a part-full 128-token tile
 struct MapKey {
     const void *w13, *w2, *a, *hi, *lo;
-    int rows_cap, box_rows;
+    int rows_cap, ntok;
     bool operator==(const MapKey& o) const {
-        return w13 == o.w13 && w2 == o.w2 && a == o.a && hi == o.hi && lo == o.lo && rows_cap == o.rows_cap && box_rows == o.box_rows;
+        return w13 == o.w13 && w2 == o.w2 && a == o.a && hi == o.hi && lo == o.lo && rows_cap == o.rows_cap && ntok == o.ntok;
     }
 };
 constexpr int MAP_SETS = 8;      // kept per handle, oldest replaced first
@@ -232,51 +232,51 @@ cudaError_t set_attr() {
 }
 
 template <int NTOK, bool G1>
-cudaError_t launch_gemm(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+cudaError_t launch_gemm(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1,
                         const GemmParams& p) {
     return launch_k(G1 ? PDL_GEMM1 : PDL_GEMM2, gemm_kernel<NTOK, G1>, dim3(grid), dim3(GemmCfg<NTOK, G1>::NTHREADS),
-                    GemmCfg<NTOK, G1>::SMEM_BYTES, st, w, b0, b1, p);
+                    GemmCfg<NTOK, G1>::SMEM_BYTES, st, w, b0, b1, s0, s1, p);
 }
 
 // GEMM1 over 128-token tiles with TMA-gathered token rows
-cudaError_t launch_gemm_g4(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+cudaError_t launch_gemm_g4(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1,
                            const GemmParams& p) {
     return launch_k(PDL_GEMM1, gemm_kernel<128, true, true>, dim3(grid), dim3(GemmCfg<128, true>::NTHREADS),
-                    GemmCfg<128, true>::SMEM_BYTES, st, w, b0, b1, p);
+                    GemmCfg<128, true>::SMEM_BYTES, st, w, b0, b1, s0, s1, p);
 }
 
 // GEMM2 with the combine in its epilogue
 template <int NTOK>
-cudaError_t launch_gemm_fused_ntok(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+cudaError_t launch_gemm_fused_ntok(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1,
                                    const GemmParams& p) {
     return launch_k(PDL_GEMM2, gemm_kernel<NTOK, false, false, false, true>, dim3(grid), dim3(GemmCfg<NTOK, false>::NTHREADS),
-                    GemmCfg<NTOK, false>::SMEM_BYTES, st, w, b0, b1, p);
+                    GemmCfg<NTOK, false>::SMEM_BYTES, st, w, b0, b1, s0, s1, p);
 }
-cudaError_t launch_gemm_fused(int ntok, int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+cudaError_t launch_gemm_fused(int ntok, int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1,
                               const GemmParams& p) {
     switch (ntok) {
-        case 16: return launch_gemm_fused_ntok<16>(grid, st, w, b0, b1, p);
-        case 32: return launch_gemm_fused_ntok<32>(grid, st, w, b0, b1, p);
-        default: return launch_gemm_fused_ntok<64>(grid, st, w, b0, b1, p);
+        case 16: return launch_gemm_fused_ntok<16>(grid, st, w, b0, b1, s0, s1, p);
+        case 32: return launch_gemm_fused_ntok<32>(grid, st, w, b0, b1, s0, s1, p);
+        default: return launch_gemm_fused_ntok<64>(grid, st, w, b0, b1, s0, s1, p);
     }
 }
 
 // 128-token tiles, most of them part full
 template <bool G1>
-cudaError_t launch_gemm_part(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1,
+cudaError_t launch_gemm_part(int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0, const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1,
                              const GemmParams& p) {
     return launch_k(G1 ? PDL_GEMM1 : PDL_GEMM2, gemm_kernel<128, G1, false, true>, dim3(grid), dim3(GemmCfg<128, G1>::NTHREADS),
-                    GemmCfg<128, G1>::SMEM_BYTES, st, w, b0, b1, p);
+                    GemmCfg<128, G1>::SMEM_BYTES, st, w, b0, b1, s0, s1, p);
 }
 
 template <bool G1>
 cudaError_t launch_gemm_ntok(int ntok, int grid, cudaStream_t st, const CUtensorMap& w, const CUtensorMap& b0,
-                             const CUtensorMap& b1, const GemmParams& p) {
+                             const CUtensorMap& b1, const CUtensorMap& s0, const CUtensorMap& s1, const GemmParams& p) {
     switch (ntok) {
-        case 16: return launch_gemm<16, G1>(grid, st, w, b0, b1, p);
-        case 32: return launch_gemm<32, G1>(grid, st, w, b0, b1, p);
-        case 64: return launch_gemm<64, G1>(grid, st, w, b0, b1, p);
-        default: return launch_gemm<128, G1>(grid, st, w, b0, b1, p);
+        case 16: return launch_gemm<16, G1>(grid, st, w, b0, b1, s0, s1, p);
+        case 32: return launch_gemm<32, G1>(grid, st, w, b0, b1, s0, s1, p);
+        case 64: return launch_gemm<64, G1>(grid, st, w, b0, b1, s0, s1, p);
+        default: return launch_gemm<128, G1>(grid, st, w, b0, b1, s0, s1, p);
     }
 }
 
@@ -424,9 +424,13 @@ int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
     const uint64_t El = (uint64_t)c.num_local_experts, H = (uint64_t)c.hidden, I = (uint64_t)c.intermediate;
     if ((rc = make_map(&m.w13, k.w13, El * 2 * I, H, 128))) return rc;
     if ((rc = make_map(&m.w2, k.w2, El * H, I, 128))) return rc;
-    if ((rc = make_map(&m.a, k.a, k.rows_cap, H, k.box_rows))) return rc;
-    if ((rc = make_map(&m.hi, k.hi, k.rows_cap, I, k.box_rows))) return rc;
-    if ((rc = make_map(&m.lo, k.lo, k.rows_cap, I, k.box_rows))) return rc;
+    if ((rc = make_map(&m.a, k.a, k.rows_cap, H, k.ntok))) return rc;
+    if ((rc = make_map(&m.hi, k.hi, k.rows_cap, I, k.ntok))) return rc;
+    if ((rc = make_map(&m.lo, k.lo, k.rows_cap, I, k.ntok))) return rc;
+    const uint32_t box = k.ntok == 128 ? GemmCfg<128, true>::BOX_ROWS : (uint32_t)k.ntok;
+    if ((rc = make_map(&m.a_box, k.a, k.rows_cap, H, box))) return rc;
+    if ((rc = make_map(&m.hi_box, k.hi, k.rows_cap, I, box))) return rc;
+    if ((rc = make_map(&m.lo_box, k.lo, k.rows_cap, I, box))) return rc;
     h->map_key[h->map_next] = k;
     h->map_set[h->map_next] = m;
     h->map_next = (h->map_next + 1) % MAP_SETS;
@@ -469,7 +473,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     // 128-K block from one producer thread: ~100 ns each), so the copy stays the default.
     const bool g4 = ntok == 128 && !pairs && h->tma_gather;
     const bool part = ntok == 128 && !pairs && !g4 && tiles_mostly_part_full(c, T);
-    if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, part ? GemmCfg<128, true>::PART_ROWS : ntok}, &maps))) return rc;
+    if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, ntok}, &maps))) return rc;
     if (g4 && (rc = make_map(&maps.a, hidden, (uint64_t)T, H, 1, wire_pitch > 0 ? (uint64_t)wire_pitch : 0))) return rc;
     const CUtensorMap &m_w13 = maps.w13, &m_w2 = maps.w2, &m_a = maps.a, &m_hi = maps.hi, &m_lo = maps.lo;
 
@@ -539,9 +543,9 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g1.trace = reinterpret_cast<long long*>(ws + L.trace);
     g1.klog = g1.trace + (size_t)2 * h->num_sms * TRACE_SLOTS;
     if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
-    else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, g1));
-    else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, g1));
-    else CU_TRY(launch_gemm_ntok<true>(ntok, h->num_sms, st, m_w13, m_a, m_a, g1));
+    else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, m_a, m_a, g1));
+    else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
+    else CU_TRY(launch_gemm_ntok<true>(ntok, h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
     CU_TRY(prof_mark(h, 4, st));
 
     GemmParams g2;
@@ -569,9 +573,9 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
     }
     if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
-    else if (fuse) CU_TRY(launch_gemm_fused(ntok, h->num_sms, st, m_w2, m_hi, m_lo, g2));
-    else if (part) CU_TRY(launch_gemm_part<false>(h->num_sms, st, m_w2, m_hi, m_lo, g2));
-    else CU_TRY(launch_gemm_ntok<false>(ntok, h->num_sms, st, m_w2, m_hi, m_lo, g2));
+    else if (fuse) CU_TRY(launch_gemm_fused(ntok, h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
+    else if (part) CU_TRY(launch_gemm_part<false>(h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
+    else CU_TRY(launch_gemm_ntok<false>(ntok, h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
     CU_TRY(prof_mark(h, 5, st));
 
     if (fuse) {

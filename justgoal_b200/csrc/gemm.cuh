@@ -117,9 +117,12 @@ struct GemmCfg {
     // block ahead; the others get the tile's NTOK scales copied into the stage
     static constexpr bool SCALES_IN_STAGE = NTOK != 128;
     static constexpr int TX_BYTES = NA * A_BYTES + NB * B_BYTES + (SCALES_IN_STAGE ? NTOK * 4 : 0);
-    // 128-token tiles that are mostly part full (kernel parameter PART): the token rows travel in boxes of PART_ROWS, and
-    // only the boxes that hold rows of the unit
-    static constexpr int PART_ROWS = 32;
+    // 128-token tiles: the rows of a part-full tile travel in boxes of BOX_ROWS, and only the boxes that hold rows of the unit.
+    // What the stage held in the others is overwritten with zeros once: zero operands cost the tensor pipe less energy, and
+    // the large forwards run into the power limit (8192 tokens, 256 experts: 5.9 -> 5.6 ms at more cycles; 4201 routed
+    // tokens: 738 -> 720 us).
+    static constexpr bool BOXED = NTOK == 128;
+    static constexpr int BOX_ROWS = BOXED ? 32 : NTOK;
     static constexpr int EMPTY_COUNT = 1 + (SCALES_IN_STAGE ? (NTOK >= 64 ? 8 : 4) : 0);   // MMA commit (+ promotion warps)
     static constexpr int STAGES_RAW = (208 * 1024) / STAGE_BYTES;
     static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
@@ -159,8 +162,8 @@ struct GemmCfg {
     // register count ptxas actually chose, by the host before the first launch).
     static constexpr bool REALLOC_REGS = NPW >= 8;
     static constexpr int LAUNCH_REGS = (65536 / NTHREADS) / 8 * 8;          // what __launch_bounds__(NTHREADS, 1) yields
-    static constexpr int CTRL_REGS = 40;      // measured: 24/240, 40/232, 56/224 and 72/216 run within 1 % of each other
-    static constexpr int PROMO_REGS = 232;
+    static constexpr int CTRL_REGS = 56;      // 40/232 spills in the producer (T=8192: 5.95 against 5.60 ms)
+    static constexpr int PROMO_REGS = 224;
     static_assert(!REALLOC_REGS || 128 * CTRL_REGS + NPT * PROMO_REGS <= NTHREADS * LAUNCH_REGS,
                   "setmaxnreg.inc would wait forever: the control warps do not release enough registers");
     static_assert(!REALLOC_REGS || (CTRL_REGS <= LAUNCH_REGS && PROMO_REGS >= LAUNCH_REGS), "setmaxnreg direction");
@@ -190,7 +193,7 @@ struct GemmCfg {
     static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
     static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
     static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * WQ_INTS * 4 /*work queue*/ +
-                                      TABLE_INTS * 4 + RED_BYTES + 48 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
+                                      TABLE_INTS * 4 + RED_BYTES + 80 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
     static_assert(NTOK % 16 == 0 && NTOK >= 16 && NTOK <= 128, "token tile");
     static_assert(TMEM_COLS >= 32 && TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "tmem");
     static_assert(STAGES >= KPB + 1, "a group must fit the stage ring with room to prefetch");
@@ -301,8 +304,8 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 
 // G4 (GEMM1 with 128-token tiles only): the token rows come straight from the caller's activations by four-row TMA
 // gathers (GemmParams::g4_row_token); a separate instantiation, so the plain kernel's code is unchanged by it.
-// PART (128-token tiles): quarters of a token tile (32 rows, one warp's TMEM lanes) that hold no row of the unit are neither
-// loaded nor folded; what the stage holds there only reaches result rows that nobody reads.  Measured at 39 rows per
+// PART (128-token tiles): quarters of a token tile (32 rows, one warp's TMEM lanes) that hold no row of the unit are not
+// folded.  Measured at 39 rows per
 // expert (901 tokens): GEMM1 160 -> 148 us, GEMM2 90 -> 86 us.  With full tiles the extra path costs the promotion loop 4 %
 // of its cycles, so the host picks the instance by the expected number of rows per expert (b200moe.cu).
 // FUSE (GEMM2, narrow tiles): with the combine in the epilogue (GemmParams::fuse_out); an instance of its own, so the plain
@@ -310,7 +313,8 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
 __global__ void __launch_bounds__(GemmCfg<NTOK, G1>::NTHREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
-            const __grid_constant__ CUtensorMap tm_b1, const GemmParams p) {
+            const __grid_constant__ CUtensorMap tm_b1, const __grid_constant__ CUtensorMap tm_s0,
+            const __grid_constant__ CUtensorMap tm_s1, const GemmParams p) {
     using C = GemmCfg<NTOK, G1>;
     static_assert(!G4 || (C::TOK_ON_M && G1), "TMA-gathered token rows: GEMM1 with 128-token tiles");
     static_assert(!FUSE || (!G1 && !C::TOK_ON_M), "fused combine: GEMM2, narrow tiles");
@@ -325,9 +329,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_row0 = s_tiles + (MAX_LOCAL + 1);
     int* s_cnt = s_row0 + (MAX_LOCAL + 1);
     uint32_t* s_red = reinterpret_cast<uint32_t*>(s_cnt + (MAX_LOCAL + 1));
-    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 12 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last)
+    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 20 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last), [12..] s_filled
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
-    int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 12) + 15) & ~uintptr_t(15));
+    int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 20) + 15) & ~uintptr_t(15));
     float2* s_sx = reinterpret_cast<float2*>(s_g4 + 128);          // tokens-on-M: [NACC][128] products of token and weight scale
     float* s_ts = reinterpret_cast<float*>(s_sx + C::NACC * 128);  // ... and [TSD][128] token scales on their way
 
@@ -462,6 +466,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int nk = 0;
             // the producer decides what this CTA does next and publishes it to the other roles
             int n_item = 0, n_whole = 0;
+            constexpr bool BOXED = C::BOXED && !G4;
+            volatile int* const s_filled = s_flag + 12;  // 128-token tiles: boxes of each stage whose rows are not zero
+            if (BOXED && lane < C::STAGES) s_filled[lane] = 128 / C::BOX_ROWS;
+            __syncwarp();
             auto publish = [&](const WorkItem& w) -> bool {
                 const int slot = n_item % C::WQ;
                 if (!mbar_wait_warp(bar_wqempty + 8 * slot, ((uint32_t)(n_item / C::WQ) & 1u) ^ 1u, p.status, ERR_WAIT_GROUP)) return false;
@@ -557,8 +565,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const Unit un = wi.un;
                 const int wrow = un.e * p.rows_per_expert + un.mt * p.unit_rows;
                 const int kb_end = min(p.KB, ge * C::KPB);
-                const int boxes = PART ? (un.nvalid + C::PART_ROWS - 1) / C::PART_ROWS : 1;
-                const uint32_t tx = PART ? (uint32_t)(C::NA * C::A_BYTES + C::NB * boxes * C::PART_ROWS * 128) : (uint32_t)C::TX_BYTES;
+                const int boxes = BOXED ? (un.nvalid + C::BOX_ROWS - 1) / C::BOX_ROWS : 1;
+                const uint32_t tx = BOXED ? (uint32_t)(C::NA * C::A_BYTES + C::NB * boxes * C::BOX_ROWS * 128) : (uint32_t)C::TX_BYTES;
+                // zeros into the boxes of stage s_ that this unit leaves out and an earlier one filled; the stage is empty
+                auto clear_dead_rows = [&](int s_) {
+                    const int was = s_filled[s_];
+                    if (was > boxes) {
+                        uint8_t* st = smem + s_ * C::STAGE_BYTES + C::NA * C::A_BYTES;
+                        for (int o = boxes * C::BOX_ROWS * 128 + lane * 16; o < was * C::BOX_ROWS * 128; o += 512) {
+                            *reinterpret_cast<uint4*>(st + o) = make_uint4(0u, 0u, 0u, 0u);
+                            if (!G1) *reinterpret_cast<uint4*>(st + C::B_BYTES + o) = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // the MMAs read through the async proxy
+                    }
+                    __syncwarp();
+                    if (lane == 0) s_filled[s_] = boxes;
+                };
                 auto load_weights = [&](int s_, int kb) {
                     const uint32_t st = smem_base + s_ * C::STAGE_BYTES;
                     const uint32_t full = bar_full + 8 * s_;
@@ -592,20 +614,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         }
                         return;
                     }
-                    for (int b = 0; b < boxes; ++b) {
-                        const uint32_t dst = st + C::NA * C::A_BYTES + b * C::PART_ROWS * 128;
-                        tma_load_2d(dst, &tm_b0, kb * 128, un.row0 + b * C::PART_ROWS, full);
-                        if (!G1) tma_load_2d(dst + C::B_BYTES, &tm_b1, kb * 128, un.row0 + b * C::PART_ROWS, full);
+                    const uint32_t dst = st + C::NA * C::A_BYTES;
+                    if (!BOXED || boxes == 128 / C::BOX_ROWS) {
+                        tma_load_2d(dst, &tm_b0, kb * 128, un.row0, full);
+                        if (!G1) tma_load_2d(dst + C::B_BYTES, &tm_b1, kb * 128, un.row0, full);
+                    } else if constexpr (BOXED) {
+                        for (int b = 0; b < boxes; ++b) {
+                            tma_load_2d(dst + b * C::BOX_ROWS * 128, &tm_s0, kb * 128, un.row0 + b * C::BOX_ROWS, full);
+                            if (!G1) tma_load_2d(dst + C::B_BYTES + b * C::BOX_ROWS * 128, &tm_s1, kb * 128, un.row0 + b * C::BOX_ROWS, full);
+                        }
                     }
                     if (C::SCALES_IN_STAGE)
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
                 int kb_first = gb * C::KPB;
+                const int kb_clear = kb_first + C::STAGES;                                  // the first turn of the stage ring
                 if (!waited) {
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the kernel before this one
                     // still runs, then the wait for it, then the token side of the same stages
                     const int npre = min(C::STAGES, kb_end - kb_first);
                     for (int i = 0; i < npre; ++i) {
+                        if (BOXED) clear_dead_rows(i);
                         if (elect_one()) load_weights(i, kb_first + i);
                         __syncwarp();
                     }
@@ -625,6 +654,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 }
                 for (int kb = kb_first; kb < kb_end; ++kb) {
                     if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
+                    if (BOXED && kb < kb_clear) clear_dead_rows(stage);
                     if (elect_one()) { load_weights(stage, kb); load_tokens(stage, kb); }
                     __syncwarp();
                     if (!issued) { if (lane == 0) stamp(TR_TMA_FIRST); issued = true; }
