@@ -154,6 +154,50 @@ def test_fused_combine_equals_the_combine_kernel_bit_for_bit(shape_name, T, tile
     assert torch.equal(out.view(torch.int16), out2.view(torch.int16))
 
 
+@pytest.mark.parametrize("counts", [(1, 31, 32, 33, 96, 97, 128, 129), (127, 160, 161, 255, 256, 257, 16, 64)])
+def test_part_full_128_token_tiles(counts):
+    """128-token tiles at every edge of their 32-row quarters, through the instance for mostly part-full tiles (few tokens)
+    and the one for full tiles (the same tokens among many without a local expert): the oracle's result, and the same
+    bits from both.  The workspace is poisoned: quarters that are left out must not matter."""
+    from justgoal_b200 import MoELayer
+    shape = I.TINY_DS
+    few, many = max(counts), 1100                        # below / above 128 expected rows per expert
+    assert few * shape.top_k / shape.num_experts < 128 <= many * shape.top_k / shape.num_experts
+    d = I.make_inputs(shape, many, seed=17)
+    idx = torch.full((many, shape.top_k), shape.num_experts - 1, dtype=torch.int32)       # not on this rank
+    for k, n in enumerate(counts):
+        idx[:n, k] = 2 * k
+    w = torch.rand(many, shape.top_k, generator=torch.Generator().manual_seed(3)) + 0.1
+    want, _, _ = O.run_experts(d["hidden_states"][:few], d["hidden_states_scale"][:, :few].contiguous(), d["gemm1_weights"],
+                               d["gemm1_weights_scale"], d["gemm2_weights"], d["gemm2_weights_scale"], w[:few], idx[:few].long(),
+                               0, shape.num_experts)
+    dc = util.to_cuda(d)
+    layer = MoELayer(shape)
+    layer.set_token_tile(128)
+    outs = []
+    for T in (few, many):
+        layer.workspace(T).fill_(0xFF)
+        out = layer.forward_routed(idx[:T].cuda(), w[:T].cuda(), dc["hidden_states"][:T], dc["hidden_states_scale"][:, :T].contiguous(),
+                                   dc["gemm1_weights"], dc["gemm1_weights_scale"], dc["gemm2_weights"], dc["gemm2_weights_scale"],
+                                   0, out_dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        assert layer.status(T) == 0
+        outs.append(out.clone())
+    rep = O.compare_output(outs[0], want.to(torch.bfloat16), util.ATOL, util.RTOL)
+    assert rep["finite"] and rep["fail_frac"] == 0.0, rep
+    assert torch.equal(outs[0].view(torch.int16), outs[1][:few].view(torch.int16))
+    assert bool((outs[1][few:].float() == 0).all())
+
+
+@pytest.mark.parametrize("T", [2369, 9473])
+def test_combine_batches(T):
+    """Token counts from which a combine CTA takes two / eight tokens at a time, with a ragged last batch."""
+    shape = I.TINY_RENORM
+    d = I.make_inputs(shape, T, seed=T)
+    layer, out = _forward(shape, d)
+    _check_output(shape, d, out)
+
+
 def test_tma_gathered_token_rows_give_the_same_bits():
     """Optional form of GEMM1 for 128-token tiles: the token rows come from hidden_states by four-row TMA gathers
     through the token-of-row table instead of from a gathered copy (no gather launch).  Ragged last tiles, padding
