@@ -491,9 +491,11 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         fp.hidden = static_cast<const uint8_t*>(hidden); fp.hscale = static_cast<const float*>(hidden_scale);
         fp.a_perm = a_perm; fp.a_scale_perm = a_scale; fp.H = H;
         fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = route_in_front ? (int)(L.expert_row0 / 16) : 0;
-        // enough warps to route 128 tokens at once and to copy a few dozen rows in one pass, few enough that GEMM1 can
-        // start on most SMs while this kernel runs (16 and 64 CTAs both measured slower at 64 tokens)
-        const int fgrid = h->num_sms < 32 ? h->num_sms : 32;
+        // enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that GEMM1 can start on most
+        // SMs while this kernel runs.  64 against 32 CTAs: 64 tokens 130.1 -> 129.6 us, 128 tokens 149.5 -> 148.3 us, but
+        // one token +0.3 us, 7 tokens +0.6 us (the meeting takes longer); 96 CTAs: 128 tokens 148.9 us.
+        const int want = T <= 32 ? 32 : 64;
+        const int fgrid = h->num_sms < want ? h->num_sms : want;
         if (route_in_front) CU_TRY(launch_front_route(c, fgrid, fp, *route_in_front, st));
         else CU_TRY(launch_k(PDL_PERMUTE, front_small_kernel, dim3(fgrid), dim3(FRONT_THREADS), 0, st, fp));
         CU_TRY(prof_mark(h, 2, st));

@@ -61,3 +61,28 @@ def test_other_routing_methods_of_the_family(shape):
     the softmax tolerance, with a bias and without."""
     _check(shape, 1500, seed=9, rsf=1.5)
     _check(shape, 33, seed=10, rsf=1.0, bias_none=True)
+
+
+@pytest.mark.parametrize("E", [32, 64, 128, 256, 512])
+def test_selection_order_with_ties_and_any_alignment(E):
+    """1 to 16 experts per lane, five distinct logits per row: selections come in descending order with the lower expert
+    first among equals (a stable sort's order), and inputs that start on any element give the same bits."""
+    from justgoal_b200 import MoELayer
+    shape = dataclasses.replace(I.QWEN3_MOE, num_experts=E, num_local_experts=32, routing_mode=I.ROUTING_RENORMALIZE)
+    T = 37
+    g = torch.Generator().manual_seed(E)
+    logits = torch.randint(-2, 3, (T, E), generator=g).float()
+    bias = torch.randint(-1, 2, (E,), generator=g).to(torch.bfloat16)
+    layer = MoELayer(shape)
+    want = torch.sort(logits + bias.float(), dim=1, descending=True, stable=True).indices[:, :shape.top_k]
+    first = None
+    for off in range(4):
+        flat = torch.zeros(T * E + off).cuda()
+        flat[off:] = logits.flatten().cuda()
+        fb = torch.zeros(E + off, dtype=torch.bfloat16).cuda()
+        fb[off:] = bias.cuda()
+        idx, w = layer.route(flat[off:].view(T, E), fb[off:], 1.0)
+        torch.cuda.synchronize()
+        assert torch.equal(idx.cpu().long(), want)
+        first = w.clone() if first is None else first
+        assert torch.equal(w, first)
