@@ -490,7 +490,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         fp.plan = pp;
         fp.hidden = static_cast<const uint8_t*>(hidden); fp.hscale = static_cast<const float*>(hidden_scale);
         fp.a_perm = a_perm; fp.a_scale_perm = a_scale; fp.H = H;
-        fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = route_in_front ? (int)(L.expert_row0 / 16) : 0;
+        fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = (int)(L.expert_row0 / 16);
         // enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that GEMM1 can start on most
         // SMs while this kernel runs.  64 against 32 CTAs: 64 tokens 130.1 -> 129.6 us, 128 tokens 149.5 -> 148.3 us, but
         // one token +0.3 us, 7 tokens +0.6 us (the meeting takes longer); 96 CTAs: 128 tokens 148.9 us.
@@ -536,7 +536,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
             g1.g4_scale = static_cast<const float*>(hidden_scale); g1.g4_tok_stride = 1; g1.ts_stride = T;
         }
     }
-    if (route_in_front && !pairs && wire_pitch == 0) {
+    if (fused_front && !pairs && wire_pitch == 0) {
         // the fused front end announces the routing result; GEMM1 schedules itself from it (gemm.cuh)
         g1.routed = status + ST_ROUTED; g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
     }
@@ -763,7 +763,9 @@ int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches
 
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
-    // count, [permute + gather | both in one launch for small T; no gather when GEMM1 gathers by TMA], gemm1, gemm2, combine
+    // count, [permute + gather | both in one launch for small T; no gather when GEMM1 gathers by TMA], gemm1, gemm2, combine.
+    // For small T the figure lies between the two forms it stands for: the slot form launches six kernels, forward_routed
+    // four (its front end needs no count).
     const bool g4 = pick_token_tile(h, num_tokens) == 128 && !use_pairs(h, 128) && h->tma_gather;
     *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 5 : 6) - (g4 ? 1 : 0);
     return 0;
@@ -833,17 +835,23 @@ int b200moe_forward_routed(b200moe_handle h, const int32_t* topk_idx, const floa
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     set_call_pdl(T);
-    CU_TRY(cudaMemsetAsync(ws, 0, L.expert_row0, st));
+    // Small token counts: one front-end launch instead of memset + count + permute + gather, each of which costs a launch
+    // latency in front of GEMM1 (32 of 256 experts: 8 tokens 100.3 -> 92.8 us, 24: 126.6 -> 117.8, 64: 159.6 -> 153.1, 128: 194.1
+    // -> 187.5; 128 of 256 experts, 128 tokens 600.7 -> 589.3 us).  The line is the front end's capacity.
+    const bool fused = T <= FRONT_MAX_T;
+    if (!fused) CU_TRY(cudaMemsetAsync(ws, 0, L.expert_row0, st));
     CU_TRY(prof_mark(h, 0, st));
-    const int n = T * c.top_k;
-    int grid = (n + 255) / 256;
-    if (grid > h->num_sms * 4) grid = h->num_sms * 4;
-    count_kernel<<<grid, 256, 0, st>>>(topk_idx, n, c.top_k, c.top_k, local_offset, c.num_local_experts,
-                                       reinterpret_cast<int*>(ws + L.slices));
-    CU_TRY(cudaGetLastError());
+    if (!fused) {
+        const int n = T * c.top_k;
+        int grid = (n + 255) / 256;
+        if (grid > h->num_sms * 4) grid = h->num_sms * 4;
+        count_kernel<<<grid, 256, 0, st>>>(topk_idx, n, c.top_k, c.top_k, local_offset, c.num_local_experts,
+                                           reinterpret_cast<int*>(ws + L.slices));
+        CU_TRY(cudaGetLastError());
+    }
     CU_TRY(prof_mark(h, 1, st));
     return run_experts(h, topk_idx, topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
-                       output_kind, ws, L, st);
+                       output_kind, ws, L, st, fused);
 }
 
 int b200moe_ep_row_bytes(b200moe_handle h, int* bytes) {

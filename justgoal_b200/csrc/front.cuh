@@ -30,7 +30,7 @@ struct FrontParams {
     uint8_t* a_perm;              // [rows_cap, H]
     float* a_scale_perm;          // [H/128, rows_cap]
     int H;
-    // front_route_kernel only.  `sync` is two words owned by the handle, zero between calls: [0] CTAs that have
+    // `sync` (front_route_kernel only) is two words owned by the handle, zero between calls: [0] CTAs that have
     // arrived at the meeting, [1] CTAs that have left it (the last one to leave clears both).  `head` is the part of
     // the workspace that must be zero before the GEMMs run (status, split-unit counters), in 16-byte units: CTA 0
     // clears it, so the forward needs no memset in front of the kernel.
@@ -152,9 +152,21 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
 }
 
 
-// Front end for tokens that were routed by an earlier kernel.
+// Front end for tokens that were routed elsewhere (the expert-parallel receive side): no meeting, every CTA has the
+// routing from the start.  CTA 0 clears the head of the workspace, announces the routing and only then lets GEMM1 start, which
+// finds the word set and streams weights while the rows are copied.  An error word set by another CTA before the clear is not
+// lost: all CTAs derive the same tables, CTA 0 sets it again.
+// Against count + permute + gather behind a memset: see the rule in b200moe_forward_routed.
 __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const FrontParams fp) {
     pdl_wait();
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < fp.head_vec; i += FRONT_THREADS) fp.head[i] = make_uint4(0u, 0u, 0u, 0u);
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0)
+            asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(fp.plan.status + ST_ROUTED), "r"(1) : "memory");
+        __syncthreads();
+    }
     pdl_launch();
     front_body<false>(fp);
 }

@@ -268,6 +268,43 @@ def test_forward_routed_bf16_and_fp16_are_the_rounded_fp32_result():
     assert torch.equal(h16.view(torch.int16), f32.to(torch.float16).view(torch.int16))
 
 
+def test_forward_routed_around_its_front_ends_boundary():
+    """Routed calls of 1 to 129 tokens (128 is the last size of the one-launch front end, 32 / 33 its grid sizes), queued
+    without a host wait on a poisoned workspace, some ids -1 as on the expert-parallel receive side: each gives the bits of
+    the forward that routes itself, apart from the dropped pairs, which the oracle checks."""
+    from justgoal_b200 import MoELayer
+    shape, sizes = I.TINY_DS, (1, 128, 33, 129, 32, 127)
+    d = I.make_inputs(shape, 129, seed=64)
+    dc = util.to_cuda(d)
+    off = int(d["local_expert_offset"])
+    wts = ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")
+    layer = MoELayer(shape)
+    idx, w = layer.route(dc["routing_logits"], dc["routing_bias"], dc["routed_scaling_factor"])
+    drop = idx.clone()
+    drop[:, 3] = -1
+    for T in sizes:
+        layer.workspace(T).fill_(0xFF)
+    hs = [(dc["hidden_states"][:T], dc["hidden_states_scale"][:, :T].contiguous()) for T in sizes]
+    got = {}
+    for k in range(2):
+        for T, (x, sc) in zip(sizes, hs):
+            for name, ids in (("all", idx), ("drop", drop)):
+                out = layer.forward_routed(ids[:T].contiguous(), w[:T].contiguous(), x, sc, *[dc[n] for n in wts], off,
+                                           out_dtype=torch.bfloat16).clone()
+                if k:
+                    assert torch.equal(out.view(torch.int16), got[T, name].view(torch.int16))
+                got[T, name] = out
+    for T, (x, sc) in zip(sizes, hs):
+        assert layer.status(T) == 0
+        own = layer.forward(dc["routing_logits"][:T], dc["routing_bias"], x, sc, *[dc[n] for n in wts], off,
+                            dc["routed_scaling_factor"])
+        assert torch.equal(own.view(torch.int16), got[T, "all"].view(torch.int16))
+        want, _, _ = O.run_experts(d["hidden_states"][:T], d["hidden_states_scale"][:, :T].contiguous(), *[d[n] for n in wts],
+                                   w[:T].cpu(), drop[:T].cpu().long(), off, shape.num_experts)
+        rep = O.compare_output(got[T, "drop"], want.to(torch.bfloat16), util.ATOL, util.RTOL)
+        assert rep["finite"] and rep["fail_frac"] == 0.0, (T, rep)
+
+
 def test_ep_pack_unpack_round_trip():
     """b200moe_ep_pack / _unpack: the wire row is [fp8 row | scales | ids | weights] padded to 16 bytes;
     unpacking returns the operator's layouts (scales K-block major) for exactly the packed tokens."""
