@@ -53,6 +53,28 @@ def test_quantiser_every_pair_of_mantissas(spread):
     assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
 
 
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -88, 2.0 ** -120, 2.0 ** 119])
+def test_quantiser_keeps_the_sign_of_zeros_and_of_underflow(scale):
+    """-0 becomes the byte 0x80 and +0 the byte 0x00, in a group of zeros, in an ordinary group and where the division is
+    taken instead of the product; elements far below the e4m3 grid round to the zero of their own sign."""
+    from justgoal_b200 import quantize_1x128
+    x = torch.zeros(9, 384)
+    x[:, 0:128:2] = -0.0                                            # zeros of both signs alone: scale 1
+    x[:, 128:256] = torch.randn(9, 128, generator=torch.Generator().manual_seed(6)) * scale
+    x[:, 130:250:7], x[:, 131:250:7] = -0.0, 0.0
+    x[:, 256:384] = torch.tensor([1.0, -1.0]).repeat(64) * scale * 2.0 ** -torch.arange(14, 23).float()[:, None]
+    x[:, 256] = scale                                               # the group's maximum; the others reach the grid's end
+    x = x.to(torch.bfloat16)
+    q_ref, s_ref = I.quantize_rows_1x128(x)
+    want = q_ref.view(torch.uint8)
+    zeros = x.float() == 0
+    negative = torch.signbit(x.float())
+    assert bool((want[zeros & negative] == 0x80).all()) and bool((want[zeros & ~negative] == 0).all())
+    q, s = quantize_1x128(x.cuda())
+    assert torch.equal(s.cpu().view(torch.int32), s_ref.view(torch.int32))
+    assert torch.equal(q.cpu().view(torch.uint8), want)
+
+
 @pytest.mark.parametrize("T,H,off", [(1, 128, 0), (9, 256, 8), (31, 4352, 8), (600, 8320, 0), (4739, 128, 16)])
 def test_quantiser_blocks_and_alignment(T, H, off):
     """Ragged token blocks, rows cut over several CTAs, and activations that are only 16-byte aligned."""
