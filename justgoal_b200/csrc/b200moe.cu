@@ -536,8 +536,9 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
             g1.g4_scale = static_cast<const float*>(hidden_scale); g1.g4_tok_stride = 1; g1.ts_stride = T;
         }
     }
-    if (fused_front && !pairs && wire_pitch == 0) {
-        // the fused front end announces the routing result; GEMM1 schedules itself from it (gemm.cuh)
+    if (fused_front && !pairs && wire_pitch == 0 && !g4) {
+        // the fused front end announces the routing result; GEMM1 schedules itself from it (gemm.cuh).  Not with gathered
+        // rows: the producer reads row_token for its first loads, which the front end writes after the announcement.
         g1.routed = status + ST_ROUTED; g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
     }
     g1.sk_count = reinterpret_cast<int*>(ws + L.sk_count);

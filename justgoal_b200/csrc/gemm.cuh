@@ -409,7 +409,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     const int ctid = threadIdx.x;
     auto ctrl_sync = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     bool early = false;             // the producer has not waited for the previous kernel yet
-    if (G1 && p.routed) {
+    if (G1 && !G4 && p.routed) {
         if (ctid == 0) {
             int seen = 0;
             const unsigned long long t0 = globaltimer_ns();

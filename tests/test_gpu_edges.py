@@ -218,6 +218,37 @@ def test_tma_gathered_token_rows_give_the_same_bits():
     _check_output(shape, d, out2)
 
 
+@pytest.mark.parametrize("T", [73, 128, 129])
+def test_tma_gathered_token_rows_behind_the_small_front_ends(T):
+    """The TMA gather with few tokens (73 is the first count with 128-token tiles here, 128 the last with a one-launch front
+    end): GEMM1's producer reads the token-of-row table, so it may not start on the announced routing alone.  Both entry
+    points, queued back to back with another call's table still in the workspace, give the bits of the gathered copy."""
+    from justgoal_b200 import MoELayer
+    shape = I.TINY_DS
+    sets = [util.to_cuda(I.make_inputs(shape, T, seed=92 + k)) for k in range(2)]
+    layer = MoELayer(shape)
+    assert int(layer.layout(T).token_tile) == 128
+    wts = ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")
+    routed = [layer.route(d["routing_logits"], d["routing_bias"], d["routed_scaling_factor"]) for d in sets]
+
+    def both(k):
+        d = sets[k]
+        a = layer.forward(*util.op_args(d)).clone()
+        b = layer.forward_routed(*routed[k], d["hidden_states"], d["hidden_states_scale"], *[d[n] for n in wts],
+                                 int(d["local_expert_offset"]), out_dtype=torch.bfloat16).clone()
+        return a, b
+
+    want = [both(k) for k in range(2)]
+    layer.set_tma_gather(True)
+    layer.workspace(T).fill_(0xFF)
+    got = [both(n % 2) for n in range(8)]
+    torch.cuda.synchronize()
+    assert layer.status(T) == 0
+    for n, (a, b) in enumerate(got):
+        assert torch.equal(a.view(torch.int16), want[n % 2][0].view(torch.int16)), n
+        assert torch.equal(b.view(torch.int16), want[n % 2][1].view(torch.int16)), n
+
+
 def test_workspace_reuse_across_sizes():
     """One layer object, shrinking and growing token counts back to back (workspace buckets, stale
     tables from the larger call must not leak into the smaller one)."""
