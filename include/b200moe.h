@@ -68,7 +68,8 @@ typedef struct b200moe_ws_layout {
     size_t tile_prefix;   /* int32[E_local+1] exclusive prefix of token tiles              */
     size_t topk_idx;      /* int32[T, top_k] global expert ids                             */
     size_t topk_w;        /* float[T, top_k]                                               */
-    size_t pair_row;      /* int32[T, top_k] row of a local pair (undefined if not local)  */
+    size_t pair_row;      /* int32[T, top_k] row of a local pair (undefined if not local;
+                             2^31 - 1 in a call that was refused for want of rows)         */
     size_t row_token;     /* int32[rows_cap] token of a row, -1 for padding                */
     size_t row_w;         /* float[rows_cap] routing weight of a row                       */
     size_t a_perm;        /* uint8[rows_cap, H] expert-sorted fp8 activations              */
@@ -138,8 +139,10 @@ int b200moe_route(b200moe_handle h, const void* routing_logits, const void* rout
 
 /* Entry points that take topk_idx from the caller (b200moe_forward_routed, _forward_routed_slots,
  * _permute_noalloc) expect the ids of one token's row to be DISTINCT (ids < 0 or outside the local
- * range are ignored): the row buffers hold min(top_k, E_local) rows per token.  A row that repeats a
- * local expert is refused on the device: error word 5, rows beyond the capacity are not written. */
+ * range are ignored): the row buffers hold min(top_k, E_local) rows per token.  A call whose ids need more rows
+ * than that (an expert repeated inside a token's row, top_k > E_local) is refused on the device as a whole: error
+ * word 5, output rows of zeros, nothing stored beyond the buffers.  _permute_noalloc has no error word: there
+ * expert_row0[E_local] > rows_capacity says so, and rows beyond the capacity are not written. */
 
 /* The expert part alone, for tokens that were routed elsewhere (expert-parallel receive
  * side): like b200moe_forward but takes topk_idx/topk_w instead of logits, and writes the

@@ -77,13 +77,15 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
     __syncthreads();
 
     // ---- scan
-    if (warp == 0) scan_counts(s_cnt, El, pp.token_tile, s_row0, s_tiles, publish ? pp.status : nullptr, lane);
+    if (warp == 0) scan_counts(s_cnt, El, pp.token_tile, pp.rows_cap, s_row0, s_tiles, publish ? pp.status : nullptr, lane);
     // pairs of the same expert in the warps before this one (independent byte loads, no second scan phase)
     int before = 0;
     if (local)
         for (int w2 = 0; w2 < warp; ++w2) before += s_wcnt[w2][le];
     __syncthreads();
-    const int total_rows = min(min(s_row0[El], FRONT_MAX_ROWS), pp.rows_cap);
+    // more rows than the caller's capacity (see scan_counts): refuse, place and copy nothing
+    const bool fits = s_row0[El] <= pp.rows_cap;
+    const int total_rows = fits ? s_row0[El] : 0;
     if (publish) {
         for (int i = tid; i <= El; i += blockDim.x) {
             pp.expert_row0[i] = s_row0[i];
@@ -97,11 +99,11 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
     // ---- stable permutation: an expert's pairs take its rows in pair order
     if (local) {
         const int r = s_row0[le] + before + rank;
-        if (r < FRONT_MAX_ROWS && r < pp.rows_cap) {
+        if (fits) {
             s_row_token[r] = tok;
             if (publish) { pp.pair_row[tid] = r; pp.row_w[r] = wgt; }
-        } else {                    // more rows than the caller's capacity: refuse, write nothing
-            atomicCAS(pp.status + ST_ERR, 0, ERR_BAD_SCHEDULE);
+        } else if (publish) {
+            pp.pair_row[tid] = NO_ROW;
         }
     }
     __syncthreads();
@@ -154,8 +156,7 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
 
 // Front end for tokens that were routed elsewhere (the expert-parallel receive side): no meeting, every CTA has the
 // routing from the start.  CTA 0 clears the head of the workspace, announces the routing and only then lets GEMM1 start, which
-// finds the word set and streams weights while the rows are copied.  An error word set by another CTA before the clear is not
-// lost: all CTAs derive the same tables, CTA 0 sets it again.
+// finds the word set and streams weights while the rows are copied.
 // Against count + permute + gather behind a memset: see the rule in b200moe_forward_routed.
 __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const FrontParams fp) {
     pdl_wait();

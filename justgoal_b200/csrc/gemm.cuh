@@ -434,7 +434,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if (id[j] >= 0 && id[j] < p.num_local) atomicAdd(&s_cnt[id[j]], 1);
         }
         ctrl_sync();
-        if (warp == 0) scan_counts(s_cnt, p.num_local, NTOK, s_row0, s_tiles, nullptr, lane);
+        if (warp == 0) scan_counts(s_cnt, p.num_local, NTOK, p.rows_cap, s_row0, s_tiles, nullptr, lane);
     } else {
         early = !G1 && p.tables_done;
         if (!early) pdl_wait();

@@ -17,6 +17,7 @@ namespace b200moe {
 constexpr int ROW_ALIGN = 16;
 constexpr int MAX_LOCAL = 256;
 static_assert((ROW_ALIGN & (ROW_ALIGN - 1)) == 0, "row alignment is a power of two");
+constexpr int NO_ROW = 0x7FFFFFFF;      // pair_row of a local pair that got no row (the call was refused, see scan_counts)
 
 // status word layout (int32[8]) at the head of the workspace
 enum : int { ST_ERR = 0, ST_PAIRS = 1, ST_ROWS = 2, ST_TILES = 3, ST_ACTIVE = 4,
@@ -56,8 +57,12 @@ __global__ void count_kernel(const int32_t* __restrict__ topk_idx, int n, int to
 // [l*per, (l+1)*per).  Fills s_row0[0..n] (first row of each expert, segments padded to
 // ROW_ALIGN) and s_tiles[0..n] (exclusive prefix of token tiles); writes the totals into
 // status[] when it is not null.  Must be called by the 32 lanes of one warp.
-__device__ __forceinline__ void scan_counts(const int* counts, int num_local, int token_tile, int* s_row0, int* s_tiles,
-                                            int* status, int tid) {
+// The row buffers hold min(top_k, num_local) rows per token.  Expert ids from the caller that repeat an expert inside one
+// token's row can need more (top_k > num_local): such a call is refused as a whole - no tiles, no rows to gather, the
+// error word set - so that no kernel after this one gets a unit or a row beyond the buffers.  Whoever places the pairs
+// compares s_row0[num_local] with rows_cap itself.
+__device__ __forceinline__ void scan_counts(const int* counts, int num_local, int token_tile, int rows_cap, int* s_row0,
+                                            int* s_tiles, int* status, int tid) {
     // Runs once per launch, on a cold instruction cache: the loops stay rolled and the token tile (a power of two)
     // divides by a shift, so the code is a few dozen instructions instead of eight unrolled copies with divisions.
     const int per = (num_local + 31) / 32;
@@ -83,22 +88,24 @@ __device__ __forceinline__ void scan_counts(const int* counts, int num_local, in
         pairs += __shfl_xor_sync(0xFFFFFFFFu, pairs, off);
         active += __shfl_xor_sync(0xFFFFFFFFu, active, off);
     }
+    const bool fits = __shfl_sync(0xFFFFFFFFu, rows_in, 31) <= rows_cap;
     int r0 = rows_in - rows, t0 = tiles_in - tiles;       // exclusive prefixes of this lane
 #pragma unroll 1
     for (int k = 0; k < per; ++k) {
         const int i = i0 + k;
         if (i < num_local) {
             const int c = counts[i];
-            s_row0[i] = r0; s_tiles[i] = t0;
+            s_row0[i] = r0; s_tiles[i] = fits ? t0 : 0;
             r0 += (c + ROW_ALIGN - 1) & ~(ROW_ALIGN - 1);
             t0 += (c + token_tile - 1) >> tsh;
         }
     }
     if (tid == 31) {
-        s_row0[num_local] = rows_in; s_tiles[num_local] = tiles_in;
+        s_row0[num_local] = rows_in; s_tiles[num_local] = fits ? tiles_in : 0;
         if (status) {
-            status[ST_PAIRS] = pairs; status[ST_ROWS] = rows_in;
-            status[ST_TILES] = tiles_in; status[ST_ACTIVE] = active;
+            status[ST_PAIRS] = pairs; status[ST_ROWS] = fits ? rows_in : 0;
+            status[ST_TILES] = fits ? tiles_in : 0; status[ST_ACTIVE] = active;
+            if (!fits) atomicCAS(status + ST_ERR, 0, ERR_BAD_SCHEDULE);
         }
     }
 }
@@ -136,7 +143,7 @@ __global__ void __launch_bounds__(PERMUTE_THREADS) permute_kernel(const PlanPara
         if (lane == 0) { s_cnt[e] = tot; s_before[e] = before; }
     }
     __syncthreads();
-    if (warp == 0) scan_counts(s_cnt, El, p.token_tile, s_row0, s_tiles, c == 0 ? p.status : nullptr, lane);
+    if (warp == 0) scan_counts(s_cnt, El, p.token_tile, p.rows_cap, s_row0, s_tiles, c == 0 ? p.status : nullptr, lane);
 
     // this thread's pair: rank among the pairs of the same expert that precede it in the warp
     const int n = p.T * p.top_k;
@@ -175,14 +182,8 @@ __global__ void __launch_bounds__(PERMUTE_THREADS) permute_kernel(const PlanPara
     }
     if (local) {
         const int r = s_row0[le] + s_before[le] + s_wcnt[warp][le] + rank;
-        if (r < p.rows_cap) {
-            p.pair_row[i] = r;
-            p.row_token[r] = tok;
-            p.row_w[r] = p.topk_w[src];
-        } else {
-            // only reachable with expert ids from the caller that repeat an expert inside one token's row
-            atomicCAS(p.status + ST_ERR, 0, ERR_BAD_SCHEDULE);
-        }
+        p.pair_row[i] = s_row0[El] <= p.rows_cap ? r : NO_ROW;
+        if (r < p.rows_cap) { p.row_token[r] = tok; p.row_w[r] = p.topk_w[src]; }
     }
 }
 
@@ -288,26 +289,26 @@ __device__ __forceinline__ void combine_token_slab(const __half* y, const int32_
                                                    const float* row_w, __nv_bfloat16* out, int t, int H, int top_k,
                                                    int pair_stride, int local_offset, int num_local, int h0, int lane) {
     const unsigned FULL = 0xFFFFFFFFu;
-    int r = 0x7FFFFFFF;
+    int r = NO_ROW;
     if (lane < top_k) {
         const int le = __ldcg(topk_idx + (size_t)t * pair_stride + lane) - local_offset;
         if (le >= 0 && le < num_local) r = __ldcg(pair_row + (size_t)t * top_k + lane);
     }
-    const float w = r != 0x7FFFFFFF ? __ldcg(row_w + r) : 0.f;
+    const float w = r != NO_ROW ? __ldcg(row_w + r) : 0.f;
     int rank = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int rj = __shfl_sync(FULL, r, j);
         rank += (rj < r) || (rj == r && j < lane);
     }
-    const int n = __popc(__ballot_sync(FULL, r != 0x7FFFFFFF));
+    const int n = __popc(__ballot_sync(FULL, r != NO_ROW));
     int rs = 0; float ws = 0.f;                // lane j < n: the j-th row in row order and its weight
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
         const int rj = __shfl_sync(FULL, r, j);
         const float wj = __shfl_sync(FULL, w, j);
         const int kj = __shfl_sync(FULL, rank, j);
-        if (rj != 0x7FFFFFFF && kj == lane) { rs = rj; ws = wj; }
+        if (rj != NO_ROW && kj == lane) { rs = rj; ws = wj; }
     }
     const int h = h0 + lane * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
         if (warp < batch) {
             // lanes 0..top_k-1 fetch their pair in parallel; rows are ranked by row index (= expert order)
             const int t = t0 + warp;
-            int r = 0x7FFFFFFF;
+            int r = NO_ROW;
             bool present = t < T;
             if (t < T && lane < top_k) {
                 const int id = topk_idx[(size_t)t * pair_stride + lane];
@@ -367,8 +368,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
                 const int rj = __shfl_sync(0xFFFFFFFFu, r, j);
                 rank += (rj < r) || (rj == r && j < lane);
             }
-            const unsigned have = __ballot_sync(0xFFFFFFFFu, r != 0x7FFFFFFF);
-            if (r != 0x7FFFFFFF) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldg(row_w + r); }
+            const unsigned have = __ballot_sync(0xFFFFFFFFu, r != NO_ROW);
+            if (r != NO_ROW) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldg(row_w + r); }
             if (lane == 0) s_n[buf][warp] = present ? __popc(have) : -1;
         }
         __syncthreads();

@@ -336,6 +336,43 @@ def test_forward_routed_around_its_front_ends_boundary():
         assert rep["finite"] and rep["fail_frac"] == 0.0, (T, rep)
 
 
+@pytest.mark.parametrize("tile", [0, 16, 128])
+@pytest.mark.parametrize("T", [60, 128, 200])
+def test_routed_ids_beyond_the_row_capacity_are_refused_whole(T, tile):
+    """One local expert and top-8 rows that name it eight times: eight rows a token where the buffers hold one.  The call
+    reports error word 5, writes zeros, stores nothing behind the workspace, and the next call on the layer is right.
+    (60 and 128 tokens go through the one-launch front end and GEMM1's own tables, 200 through count and permute.)"""
+    from justgoal_b200 import MoELayer
+    shape = I.TINY_DS.with_local(1)
+    d = I.make_inputs(shape, T, seed=65)
+    dc = util.to_cuda(d)
+    layer = MoELayer(shape)
+    layer.set_token_tile(tile)
+    bucket = 64 if T <= 64 else 128 if T <= 128 else 256
+    used, guard = int(layer.layout(bucket).total_bytes), 1 << 22
+    assert 8 * T > int(layer.layout(T).rows_cap)
+    ws = torch.full((used + guard,), 0xA5, dtype=torch.uint8, device="cuda")
+    layer._ws[bucket] = ws
+    idx = torch.zeros(T, shape.top_k, dtype=torch.int32, device="cuda")
+    w = torch.rand(T, shape.top_k, generator=torch.Generator().manual_seed(4)).cuda() + 0.1
+    wts = [dc[n] for n in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")]
+    for kind in (torch.bfloat16, torch.float32):
+        out = torch.full((T, shape.hidden), 7.0, dtype=kind, device="cuda")
+        layer.forward_routed(idx, w, dc["hidden_states"], dc["hidden_states_scale"], *wts, 0, output=out)
+        torch.cuda.synchronize()
+        assert layer.status(T) == 5
+        assert bool((out == 0).all()) and bool((ws[used:] == 0xA5).all())
+    once = idx.clone()
+    once[:, 1:] = shape.num_experts - 1                  # not on this rank
+    got = layer.forward_routed(once, w, dc["hidden_states"], dc["hidden_states_scale"], *wts, 0, out_dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    assert layer.status(T) == 0
+    want, _, _ = O.run_experts(d["hidden_states"], d["hidden_states_scale"], d["gemm1_weights"], d["gemm1_weights_scale"],
+                               d["gemm2_weights"], d["gemm2_weights_scale"], w.cpu(), once.cpu().long(), 0, shape.num_experts)
+    rep = O.compare_output(got, want.to(torch.bfloat16), util.ATOL, util.RTOL)
+    assert rep["finite"] and rep["fail_frac"] == 0.0, rep
+
+
 def test_ep_pack_unpack_round_trip():
     """b200moe_ep_pack / _unpack: the wire row is [fp8 row | scales | ids | weights] padded to 16 bytes;
     unpacking returns the operator's layouts (scales K-block major) for exactly the packed tokens."""
