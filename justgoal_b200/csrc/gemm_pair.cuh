@@ -16,11 +16,11 @@
 // its 2-SM tile kernel (kda05_reproduction_full_shape/fable-5.1/moe_fp8_fwd/<def>/fable51_moe_v94/
 // kernel.cu:4216-4675).
 //
-// Roles per CTA: warp 0 lane 0 = TMA producer (its token tile + its weight tile; the bytes of
-// both CTAs count on the LEADER's "full" barrier), warp 1 lane 0 of the leader = MMA issuer for the pair,
-// warp 1 of each CTA owns its TMEM, warps 4..11 = promotion / epilogue of the CTA's own token tile.
+// Roles per CTA: warp 0 = TMA producer (its token tile + its weight tile; the bytes of
+// both CTAs count on the LEADER's "full" barrier), warp 1 of the leader = MMA issuer for the pair (whole warps, one
+// elected lane issues), warp 1 of each CTA owns its TMEM, warps 4..11 = promotion / epilogue of the CTA's own token tile.
 // Commits reach both CTAs' barriers; promotion warps of both CTAs release accumulators on the leader.
-// Every software wait is bounded (common.cuh); no load uses cluster multicast; the CTAs of a pair leave
+// Every software wait is bounded and voted on by its warp (common.cuh); no load uses cluster multicast; the CTAs of a pair leave
 // together (cluster barrier) so that nobody signals a barrier of a CTA that is gone.
 #pragma once
 #include "gemm.cuh"
@@ -229,7 +229,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 const int wrow = __shfl_sync(0xFFFFFFFFu, un.e * p.rows_per_expert + un.mt * p.unit_rows + (int)crank * p.gate_offset, 0);
                 for (int kb = 0; kb < p.KB; ++kb) {
                     { PT_T0();
-                    if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
                     PT_ADD(w_empty); }
                     if (elect_one()) {
                     const uint32_t st = smem_base + stage * C::STAGE_BYTES;
@@ -247,7 +247,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             // tail: the commits that release the last stages arrive from the leader asynchronously; stay until every
             // stage this CTA filled has been released, so that none of them can find the CTA gone
             for (int i = 0; i < C::STAGES && ok; ++i) {
-                if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) ok = false;
+                if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) ok = false;
                 if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
             }
             if (!ok) {
@@ -262,14 +262,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
             int stage = 0; uint32_t phase = 0;
             int ab = 0; uint32_t aphase = 0;
             bool ok = true;
-            PT_DECL(w_full = 0, w_tempty = 0);
+            PT_DECL(w_full = 0);
             for (int ui = 0; ui < my_units && ok; ++ui) {
                 for (int kb = 0; kb < p.KB && ok; ++kb) {
                     { PT_T0();
-                    if (!mbar_wait(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
-                    PT_ADD(w_tempty); }
-                    { PT_T0();
-                    if (!mbar_wait(bar_full + 8 * stage, phase, p.status, ERR_WAIT_SMEM_FULL)) { ok = false; break; }
+                    if (!mbar_wait_both(bar_tempty + 8 * ab, aphase ^ 1, ERR_WAIT_TMEM_EMPTY,
+                                        bar_full + 8 * stage, phase, ERR_WAIT_SMEM_FULL, p.status)) { ok = false; break; }
                     PT_ADD(w_full); }
                     tc_fence_after();
                     if (elect_one()) {
@@ -292,7 +290,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
             }
-            PT_PUT(3, w_full); PT_PUT(4, w_tempty); PT_PUT(5, clock64() - t_entry);
+            PT_PUT(3, w_full); PT_PUT(5, clock64() - t_entry);
         }
         __syncwarp();
     }
@@ -315,7 +313,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
         auto all_sync = [&]() -> bool {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_all);
-            const bool r = mbar_wait(bar_all, allphase, p.status, ERR_WAIT_GROUP);
+            const bool r = mbar_wait_warp(bar_all, allphase, p.status, ERR_WAIT_GROUP);
             allphase ^= 1;
             return r;
         };
@@ -342,7 +340,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
                 swn0 = __ldg(ws0 + kn); swn1 = __ldg(ws1 + kn);
                 stokn = __ldcg(tsp + (size_t)kn * p.rows_cap);
                 { PT_T0();
-                if (!mbar_wait(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+                if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
                 PT_ADD(w_tfull); }
                 tc_fence_after();
                 const uint32_t tbuf = tmem_base + tlane + ab * 256 + c0;
