@@ -1126,6 +1126,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         }
                     }
                     here = __shfl_sync(0xFFFFFFFFu, here, 0);
+                    __syncwarp();            // lane 0's acquire orders the other lanes' loads too (a shuffle orders nothing)
                     if (!here) { ok = false; break; }
                 } else {
                     // ---- piece of a split unit, claimed chunks: every piece stores its partial sums; the warps that arrive
@@ -1152,6 +1153,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     } else {
                         if (lane == 0) count_in();
                         seen_pieces = __shfl_sync(0xFFFFFFFFu, seen_pieces, 0);
+                        __syncwarp();        // as above: before the fence of the lanes that read the other pieces
                     }
                     if (seen_pieces != wi.pieces - 1) continue;
                     __threadfence();
@@ -1335,6 +1337,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         last = atomicAdd(p.tok_count + (size_t)t * p.n_mtiles + un.mt, 1) == 4 * need - 1;
                     }
                     unsigned todo = __ballot_sync(0xFFFFFFFFu, last);
+                    __syncwarp();                       // as for the split units: the counting lane before the fence of all
                     if (todo) __threadfence();          // the other warps' rows, counted in before this one, are visible
                     while (todo) {
                         const int srcl = __ffs(todo) - 1;

@@ -1,10 +1,10 @@
-"""CPU: the form of the waits inside the GEMM kernels, read from their sources.
+"""CPU: the form of the waits and hand-outs inside the GEMM kernels, read from their sources.
 
 Every role of these kernels is a whole warp: it waits on an mbarrier and then elects the issuing lane, loads from tensor
 memory or meets (`elect.sync`, `tcgen05.ld.sync.aligned`, `bar.warp.sync`: all name the full warp).  A wait that runs out in
 some lanes only must therefore not let those lanes leave alone - the others would wait for them without a limit.  The voted
 forms (`mbar_wait_warp`, `mbar_wait_both`) give one answer to the warp; `mbar_wait` answers per lane.  Running out of a limit
-inside a kernel cannot be provoked on a GPU from the host, so the rule is held here."""
+inside a kernel, or a warp's lanes apart in time, cannot be provoked from the host, so the rules are held here."""
 import os
 import re
 
@@ -35,3 +35,15 @@ def test_voted_forms_vote():
         assert body.rstrip().endswith("return merged(ok);")
         slow = body[body.rindex("if (!ok)"):]
         assert "__all_sync(0xFFFFFFFFu" in slow
+
+
+def test_what_one_lane_learns_about_other_ctas_orders_the_whole_warp():
+    """One lane acquires (or counts in with an atomic) and hands the answer out by a shuffle or a vote, which order no memory;
+    all lanes then load what other CTAs stored.  A `__syncwarp` has to stand between: static pieces, claimed chunks, fused
+    combine."""
+    code = _code("gemm.cuh")
+    for answer in ("here = __shfl_sync(0xFFFFFFFFu, here, 0);", "seen_pieces = __shfl_sync(0xFFFFFFFFu, seen_pieces, 0);",
+                   "unsigned todo = __ballot_sync(0xFFFFFFFFu, last);"):
+        assert code.count(answer) == 1
+        after = code[code.index(answer) + len(answer):].lstrip()
+        assert after.startswith("__syncwarp();"), answer
