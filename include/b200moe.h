@@ -305,8 +305,10 @@ int b200moe_set_wait_limit_ns(b200moe_handle h, unsigned long long nanoseconds);
 /* Number of this library's kernels one forward over T tokens launches (a count of
  * launches, not of kernels that do useful work). */
 int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches);
-/* The same count for b200moe_forward_routed / b200moe_forward_routed_slots over num_tokens tokens (slots). */
+/* The same count for b200moe_forward_routed over num_tokens tokens, and for b200moe_forward_routed_slots over
+ * num_slots = world * cap slots (at least one). */
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches);
+int b200moe_launches_routed_slots(b200moe_handle h, int num_slots, int* launches);
 
 /* Optional stage timing.  enable(slots > 0) creates slots x 7 CUDA events; every forward then
  * records them around its six kernels (slot = call number modulo slots); enable(0) turns it

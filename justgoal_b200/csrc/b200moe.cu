@@ -160,6 +160,14 @@ bool tiles_mostly_part_full(const b200moe_config& c, int T) {
     return (double)T * c.top_k / c.num_experts < 128.0;
 }
 
+// GEMM1 reads its token rows by TMA gather (b200moe_set_tma_gather); behind a separate permutation there is then no
+// gather launch (the one-launch front ends copy the rows all the same).
+bool use_pairs(const b200moe_ctx* h, int ntok);
+bool gathers_by_tma(const b200moe_ctx* h, int T) {
+    const int ntok = pick_token_tile(h, T);
+    return ntok == 128 && !use_pairs(h, ntok) && h->tma_gather;
+}
+
 // Partial-sum slots of the chunked units: (fewer than grid units) x (chunks per unit) x (floats per slot), the larger
 // of the two GEMMs (they run one after the other and share the area).
 template <int NTOK>
@@ -757,18 +765,21 @@ int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
     // [route, permute, gather | fused route+permute+gather for small T], gemm1, gemm2, [combine unless fused into gemm2]
     const bool fuse = h->fuse_combine && pick_token_tile(h, num_tokens) < 128 && !use_pairs(h, pick_token_tile(h, num_tokens));
-    const bool g4 = pick_token_tile(h, num_tokens) == 128 && !use_pairs(h, 128) && h->tma_gather;
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6) - (fuse ? 1 : 0) - (g4 ? 1 : 0);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (fuse ? 1 : 0);
     return 0;
 }
 
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
-    // count, [permute + gather | both in one launch for small T; no gather when GEMM1 gathers by TMA], gemm1, gemm2, combine.
-    // For small T the figure lies between the two forms it stands for: the slot form launches six kernels, forward_routed
-    // four (its front end needs no count).
-    const bool g4 = pick_token_tile(h, num_tokens) == 128 && !use_pairs(h, 128) && h->tma_gather;
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 5 : 6) - (g4 ? 1 : 0);
+    // [count, permute, gather | all in one launch for small T], gemm1, gemm2, combine
+    *launches = num_tokens == 0 ? 0 : num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0);
+    return 0;
+}
+
+int b200moe_launches_routed_slots(b200moe_handle h, int num_slots, int* launches) {
+    if (!h || !launches || num_slots < 1) return B200MOE_E_BADARG;
+    // count, permute, gather, gemm1, gemm2, combine whatever the number of slots
+    *launches = 6 - (gathers_by_tma(h, num_slots) ? 1 : 0);
     return 0;
 }
 

@@ -309,15 +309,17 @@ class ExpertParallelMoE:
     def launches_per_step(self) -> int:
         """Kernels of this library one step launches on one rank.  Peer-memory form: route, push, barrier, count,
         permute, [gather from the wire slots unless GEMM1 gathers by TMA], GEMM1, GEMM2, combine (stores into the
-        owners' slots), barrier, owner-side sum; collective form: route, pack, unpack, count, permute, [gather],
-        GEMM1, GEMM2, combine, owner-side sum."""
+        owners' slots), barrier, owner-side sum; collective form: route, pack, unpack, [count, permute, gather | one
+        front-end launch up to 128 received rows], GEMM1, GEMM2, combine, owner-side sum - for the rows received in the
+        last step (a rank that received none launches neither the unpacking nor the experts)."""
         layer = getattr(self.backend, "layer", None)
         if layer is None:               # a backend that is not this library (the CPU tests' oracle backend)
             return 0
         if self.peer is not None:       # route, push, barrier | local experts over all slots | barrier, owner-side sum
-            return 5 + layer.launches_routed(self.peer.world * self.peer.cap)
+            return 5 + layer.launches_routed_slots(self.peer.world * self.peer.cap)
         # route, pack, unpack | local experts over the rows received in the last step | owner-side sum
-        return 4 + layer.launches_routed(max(1, getattr(self, "_last_recv", 1)))
+        n = getattr(self, "_last_recv", 1)
+        return (4 if n else 3) + layer.launches_routed(n)
 
     def check_status(self):
         """Raises if a barrier of the peer-memory exchange gave up waiting for a peer since the last check (the

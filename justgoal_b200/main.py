@@ -111,9 +111,15 @@ class MoELayer:
         return dict(zip(self.STAGES, [float(x) for x in ms]))
 
     def launches_routed(self, T: int) -> int:
-        """Kernel launches of forward_routed (or the slot form) over T tokens (slots)."""
+        """Kernel launches of forward_routed over T tokens."""
         n = C.c_int(0)
         _lib.check(_lib.lib.b200moe_launches_routed(self._h, T, C.byref(n)))
+        return n.value
+
+    def launches_routed_slots(self, slots: int) -> int:
+        """Kernel launches of the slot form (local experts over `slots` = world * cap wire slots, read in place)."""
+        n = C.c_int(0)
+        _lib.check(_lib.lib.b200moe_launches_routed_slots(self._h, slots, C.byref(n)))
         return n.value
 
     def set_token_tile(self, tokens: int):

@@ -249,6 +249,56 @@ def test_tma_gathered_token_rows_behind_the_small_front_ends(T):
         assert torch.equal(b.view(torch.int16), want[n % 2][1].view(torch.int16)), n
 
 
+def _kernels_launched(fn):
+    """Kernel nodes of the CUDA graph that captures one call of fn."""
+    import ctypes as C
+    fn()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    cu, graph, n, kind = C.CDLL("libcuda.so.1"), C.c_void_p(g.raw_cuda_graph()), C.c_size_t(0), C.c_int(0)
+    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
+    total = 0
+    for node in nodes:
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        total += kind.value == 0                       # CU_GRAPH_NODE_TYPE_KERNEL
+    return total
+
+
+@pytest.mark.parametrize("tma_gather", [False, True])
+@pytest.mark.parametrize("T", [40, 128, 129])
+def test_launch_counts_are_the_kernels_of_a_captured_call(T, tma_gather):
+    """What launches_per_forward, launches_routed and launches_routed_slots state is what a call launches, on both sides of
+    the one-launch front ends' limit (40 tokens: narrow tiles; 128 and 129: 128-token tiles, where the TMA gather acts)."""
+    from justgoal_b200 import MoELayer
+    from justgoal_b200.ep import PeerExchange
+    shape = I.TINY_DS
+    d = util.to_cuda(I.make_inputs(shape, T, seed=66))
+    off = int(d["local_expert_offset"])
+    wts = {n: d[n] for n in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")}
+    layer = MoELayer(shape)
+    layer.set_tma_gather(tma_gather)
+    args = util.op_args(d)
+    own = layer.launches_per_forward(T)
+    assert own == _kernels_launched(lambda: layer.forward(*args)) == (4 if T <= 128 else 5 if tma_gather else 6)
+    if T == 40:
+        layer.set_fused_combine(True)
+        assert layer.launches_per_forward(T) == _kernels_launched(lambda: layer.forward(*args)) == 3
+        layer.set_fused_combine(False)
+    idx, w = layer.route(d["routing_logits"], d["routing_bias"], d["routed_scaling_factor"])
+    routed = _kernels_launched(lambda: layer.forward_routed(idx, w, d["hidden_states"], d["hidden_states_scale"],
+                                                            *wts.values(), off))
+    assert layer.launches_routed(T) == routed == (4 if T <= 128 else 5 if tma_gather else 6)
+    n = PeerExchange.buffer_bytes(layer, shape, T, 1)
+    px = PeerExchange(layer, shape, T, None, None, local_buffers=[torch.zeros(n, dtype=torch.uint8, device="cuda")], rank=0)
+    px.wire[:, shape.hidden + 4 * (shape.hidden // 128):].view(torch.int32).fill_(-1)          # empty slots
+    slots = _kernels_launched(lambda: px.experts_to_peers(wts, off))
+    assert layer.launches_routed_slots(T) == slots == (5 if tma_gather and T > 72 else 6)
+
+
 def test_workspace_reuse_across_sizes():
     """One layer object, shrinking and growing token counts back to back (workspace buckets, stale
     tables from the larger call must not leak into the smaller one)."""
