@@ -86,9 +86,9 @@ typedef struct b200moe_ws_layout {
                              %globaltimer at entry, slots 1..11 = SM clocks since entry at:
                              prologue done, first/last TMA issue, first/last MMA, first/last
                              promotion, partial published, partials added, epilogue, exit     */
-    size_t tok_count;     /* int32[T][H/256] (narrow token tiles only, else empty): units that have delivered
-                             a row of token t for output columns [256 j, 256 j + 256) - the combine fused
-                             into the GEMM2 epilogue                                          */
+    size_t tok_count;     /* int32[T][ceil(H/256)] (narrow token tiles only, else empty): byte q = rows of token t
+                             delivered for output columns 256 j + {0, 128} + [32 q, 32 q + 32) - the combine
+                             fused into the GEMM2 epilogue                                    */
     size_t rows_cap;      /* number of rows the row-indexed buffers hold                   */
     size_t token_tile;    /* tokens per GEMM tile chosen for this T                        */
     size_t total_bytes;

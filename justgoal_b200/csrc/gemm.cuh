@@ -95,10 +95,10 @@ struct GemmParams {
     int ts_stride;        // tokens-on-M tiles: floats between a row's token scales of consecutive K blocks (rows_cap for the
                           // gathered copy, the caller's K-block stride when g4_row_token is set); K blocks * ts_stride < 2^31
     // GEMM2 with the combine fused into its epilogue (FUSE: narrow token tiles of the operator's own forward).
-    // tok_count[t * n_mtiles + mt] (zero at launch) counts the warps (four per row) that have stored the columns
-    // [256 mt, 256 mt + 256) of one of token t's rows; the warp that brings it to the number of the token's local
-    // pairs adds those rows up (permute.cuh, combine_token_slab) and writes the bf16 output.  Tokens without a local
-    // pair get their zero row from the otherwise idle warps 2-3.
+    // Byte q of tok_count[t * n_mtiles + mt] (zero at launch) counts the rows of token t whose columns of unit mt that belong
+    // to lane quarter q are stored; the warp that brings it to the number of the token's local pairs adds those columns
+    // up (permute.cuh, combine_four_tokens) and writes the bf16 output.  Tokens without a local pair get their zero row
+    // from the otherwise idle warps 2-3.
     __nv_bfloat16* fuse_out;
     int* tok_count;
     const int32_t* row_token; const int32_t* pair_row; const int32_t* c_topk;
@@ -1318,9 +1318,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                 }
                 if (FUSE) {
-                    // Fused combine.  This warp has stored its 64 of the 256 columns of the column group's NC rows: fence,
-                    // then count it in for every row's token (lane i: row i, all atomics in flight together); four warps
-                    // deliver a row.
+                    // Fused combine.  This warp has stored its 64 of the unit's 256 columns (32 of either weight tile) of the
+                    // column group's NC rows: fence, then count them in for every row's token (lane i: row i, all atomics in
+                    // flight together; byte `quarter` of the token's word).  The warp that brings a token's byte to the number
+                    // of its local pairs adds up those 64 columns of its rows, four tokens at a time.  (One warp for all 256
+                    // columns of a token, one token after the other, left up to NC chains of dependent loads to the last of
+                    // the four warps: 200 tokens of a 512-wide shape 66.5 us,
+                    // now 42.7.)
                     __threadfence();
                     __syncwarp();
                     const int c = c0 + lane;
@@ -1334,17 +1338,23 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             const int le = __ldg(p.c_topk + (size_t)t * p.c_stride + k) - p.c_local_offset;
                             need += le >= 0 && le < p.num_local;
                         }
-                        last = atomicAdd(p.tok_count + (size_t)t * p.n_mtiles + un.mt, 1) == 4 * need - 1;
+                        const unsigned was = (unsigned)atomicAdd(p.tok_count + (size_t)t * p.n_mtiles + un.mt, 1 << (8 * quarter));
+                        last = (int)((was >> (8 * quarter)) & 0xFFu) == need - 1;
                     }
                     unsigned todo = __ballot_sync(0xFFFFFFFFu, last);
                     __syncwarp();                       // as for the split units: the counting lane before the fence of all
-                    if (todo) __threadfence();          // the other warps' rows, counted in before this one, are visible
+                    if (todo) __threadfence();          // the other units' rows, counted in before this one, are visible
+                    const int h = un.mt * p.unit_rows + ((lane & 4) ? p.gate_offset : 0) + quarter * 32 + (lane & 3) * 8;
                     while (todo) {
-                        const int srcl = __ffs(todo) - 1;
-                        todo &= todo - 1;
-                        const int tt = __shfl_sync(0xFFFFFFFFu, t, srcl);
-                        combine_token_slab(p.y, p.c_topk, p.pair_row, p.row_w, p.fuse_out, tt, p.H, p.top_k, p.c_stride,
-                                           p.c_local_offset, p.num_local, un.mt * p.unit_rows, lane);
+                        int src = -1;                   // lane that counted the token of this lane's group of eight
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            if ((lane >> 3) == g) src = __ffs(todo) - 1;
+                            todo &= todo - 1;
+                        }
+                        const int tt = __shfl_sync(0xFFFFFFFFu, t, max(src, 0));
+                        combine_four_tokens(p.y, p.c_topk, p.pair_row, p.row_w, p.fuse_out, src < 0 ? -1 : tt, p.H, p.top_k, p.c_stride,
+                                            p.c_local_offset, p.num_local, h, lane);
                     }
                 }
             }

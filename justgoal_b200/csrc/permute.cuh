@@ -281,53 +281,50 @@ __device__ __forceinline__ void add8_f16(float* acc, const uint4& v) {
     }
 }
 
-// The combine of ONE token over 256 output columns by one warp (lane l: columns h0 + 8 l .. + 7): the same sum as
-// combine_kernel below - the token's local rows in row order, weight times row in fp32, one rounding to bf16.  Used
-// by the GEMM2 epilogue that delivers a token's last row (gemm.cuh); the rows were written by other CTAs of the same
+// The combine of up to four tokens by one warp, over the columns whose rows that warp stores in the GEMM2 epilogue (gemm.cuh):
+// eight lanes per token t (-1: none), each with eight columns from h on.  The same sum as combine_kernel below - the token's
+// local rows in row order, weight times row in fp32, one rounding to bf16.  The rows were written by other CTAs of the same
 // launch, so every load goes to L2 (.cg).
-__device__ __forceinline__ void combine_token_slab(const __half* y, const int32_t* topk_idx, const int32_t* pair_row,
-                                                   const float* row_w, __nv_bfloat16* out, int t, int H, int top_k,
-                                                   int pair_stride, int local_offset, int num_local, int h0, int lane) {
+__device__ __forceinline__ void combine_four_tokens(const __half* y, const int32_t* topk_idx, const int32_t* pair_row,
+                                                    const float* row_w, __nv_bfloat16* out, int t, int H, int top_k,
+                                                    int pair_stride, int local_offset, int num_local, int h, int lane) {
     const unsigned FULL = 0xFFFFFFFFu;
+    const int sub = lane & 7;                  // pair of the token while rows are looked up
     int r = NO_ROW;
-    if (lane < top_k) {
-        const int le = __ldcg(topk_idx + (size_t)t * pair_stride + lane) - local_offset;
-        if (le >= 0 && le < num_local) r = __ldcg(pair_row + (size_t)t * top_k + lane);
+    if (t >= 0 && sub < top_k) {
+        const int le = __ldcg(topk_idx + (size_t)t * pair_stride + sub) - local_offset;
+        if (le >= 0 && le < num_local) r = __ldcg(pair_row + (size_t)t * top_k + sub);
     }
     const float w = r != NO_ROW ? __ldcg(row_w + r) : 0.f;
+    const int n = __popc((__ballot_sync(FULL, r != NO_ROW) >> (lane & 24)) & 0xFFu);
     int rank = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const int rj = __shfl_sync(FULL, r, j);
-        rank += (rj < r) || (rj == r && j < lane);
+        const int rj = __shfl_sync(FULL, r, j, 8);
+        rank += (rj < r) || (rj == r && j < sub);
     }
-    const int n = __popc(__ballot_sync(FULL, r != NO_ROW));
-    int rs = 0; float ws = 0.f;                // lane j < n: the j-th row in row order and its weight
+    int rs = NO_ROW; float ws = 0.f;           // lane j < n of the eight: the j-th row in row order and its weight
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const int rj = __shfl_sync(FULL, r, j);
-        const float wj = __shfl_sync(FULL, w, j);
-        const int kj = __shfl_sync(FULL, rank, j);
-        if (rj != NO_ROW && kj == lane) { rs = rj; ws = wj; }
+        const int rj = __shfl_sync(FULL, r, j, 8);
+        const float wj = __shfl_sync(FULL, w, j, 8);
+        if (__shfl_sync(FULL, rank, j, 8) == sub) { rs = rj; ws = wj; }
     }
-    const int h = h0 + lane * 8;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j0 = 0; j0 < n; j0 += 4) {
+    for (int j0 = 0; j0 < 8 && __any_sync(FULL, j0 < n); j0 += 4) {
         uint4 v[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (j0 + u < n) {
-                const int row = __shfl_sync(FULL, rs, j0 + u);
-                if (h < H) v[u] = __ldcg(reinterpret_cast<const uint4*>(y + (size_t)row * H + h));
-            }
+        for (int u = 0; u < 4; ++u) {
+            const int row = __shfl_sync(FULL, rs, j0 + u, 8);
+            if (j0 + u < n && h < H) v[u] = __ldcg(reinterpret_cast<const uint4*>(y + (size_t)row * H + h));
+        }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (j0 + u < n) {
-                const float wu = __shfl_sync(FULL, ws, j0 + u);
-                if (h < H) fma8_f16(acc, v[u], wu);
-            }
+        for (int u = 0; u < 4; ++u) {
+            const float wu = __shfl_sync(FULL, ws, j0 + u, 8);
+            if (j0 + u < n && h < H) fma8_f16(acc, v[u], wu);
+        }
     }
-    if (h < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + h) = pack8_bf16(acc);
+    if (t >= 0 && h < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + h) = pack8_bf16(acc);
 }
 
 // A CTA takes `batch` (1..8) tokens at a time: warp w looks up token w's rows and weights (a chain of dependent loads, ~2 us
