@@ -1092,13 +1092,18 @@ int b200moe_quantize_1x128(const void* x_bf16, int T, int H, void* q_e4m3, float
     int tpc = QUANT_TOKENS, parts = (groups + QUANT_GROUPS - 1) / QUANT_GROUPS;
     auto ctas = [&](int tp, int pa) { return (long long)((T + tp - 1) / tp) * pa; };
     while (ctas(tpc, parts) < 4ll * sms && parts * 32 < groups) parts *= 2;
-    while (ctas(tpc, parts) < 2ll * sms && tpc > 1) tpc /= 2;
     const int gpc = (groups + parts - 1) / parts;
+    // rows of few groups: more tokens, until all threads of a CTA have groups to work on (40000 x 128: eight tokens 25.1 us,
+    // 64 tokens 4.7 us; 40000 x 512: 17.3 us with eight, 12.0 with 16)
+    while (tpc * gpc < QUANT_TURN) tpc *= 2;
+    while (ctas(tpc, parts) < 2ll * sms && tpc > 1) tpc /= 2;
+    int tsh = 0;
+    while (1 << tsh < tpc) ++tsh;
     const dim3 grid((T + tpc - 1) / tpc, (groups + gpc - 1) / gpc);
     const bool wide = !((reinterpret_cast<uintptr_t>(x_bf16) & 31) || (reinterpret_cast<uintptr_t>(q_e4m3) & 15));
     auto* kern = wide ? quantize_1x128_kernel<true> : quantize_1x128_kernel<false>;
-    kern<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x_bf16), T, H, tpc, gpc, static_cast<uint8_t*>(q_e4m3), scale);
+    kern<<<grid, QUANT_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x_bf16), T, H, tsh, gpc, static_cast<uint8_t*>(q_e4m3), scale);
     CU_TRY(cudaGetLastError());
     return 0;
 }

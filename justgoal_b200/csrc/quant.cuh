@@ -22,8 +22,9 @@
 // mantissa is all ones, and the quotient of an 8-bit number by 448 never is.  (The test runs all pairs of mantissas.)
 // Scales below 2^-90 or above 2^126, where e or y would lose bits to the exponent range, take the dividing path.
 // Zeros: e is +0 for x = +-0 (a sum of zeros of opposite sign), so e times the NEGATIVE factor -y is -0, which leaves q0 = +-0
-// its sign; with the residual the other way round, x - q0 s times y, -0 came out as +0.  x enters negated for that, at no
-// measurable cost (4096 x 7168: 20.5 us with either form): a bf16 is unpacked and negated in one integer operation.
+// its sign; with the residual the other way round, x - q0 s times y, -0 came out as +0.  x enters negated for that: a
+// bf16 is unpacked and negated in one integer operation (4096 x 7168: 20.5 us with either form on inputs from memory, 15.9
+// against 16.4 us on inputs that the L2 still holds).
 #pragma once
 #include <cuda_bf16.h>
 #include "common.cuh"
@@ -43,24 +44,30 @@ __device__ __forceinline__ uint32_t quantize4(const float2 n0, const float2 n1, 
     return (uint32_t)f32x2_to_e4m3x2(q0.x, q0.y) | ((uint32_t)f32x2_to_e4m3x2(q1.x, q1.y) << 16);
 }
 
-constexpr int QUANT_TOKENS = 8;         // most tokens of a CTA: a sector of scales
-constexpr int QUANT_GROUPS = 64;        // most groups (128 columns) of a CTA
+constexpr int QUANT_TOKENS = 8;         // tokens of a CTA: a sector of scales (more for rows of few groups, see the host's rule)
+constexpr int QUANT_GROUPS = 64;        // most groups (128 columns) of a token in a CTA
+constexpr int QUANT_THREADS = 256, QUANT_LANES = 8, QUANT_FLIGHT = 2;     // lanes of a group, groups per lane in flight
+constexpr int QUANT_SCALES = QUANT_TOKENS * QUANT_GROUPS;                 // most scales of a CTA
+constexpr int QUANT_TURN = QUANT_THREADS / QUANT_LANES * QUANT_FLIGHT;    // groups a CTA takes at a time
 
-// CTA (x, y): tokens [x * tpc, ...), groups [y * gpc, ...).  WIDE: x is 32-byte and q 16-byte aligned (torch tensors are);
+// CTA (x, y): tokens [x * tpc, ...), groups [y * gpc, ...), tpc = 2^tsh, tpc * gpc <= QUANT_SCALES.  WIDE: x is 32-byte and q 16-byte aligned (torch tensors are);
 // otherwise two 16-byte loads and two 8-byte stores take their place.
 template <bool WIDE>
-__global__ void __launch_bounds__(256) quantize_1x128_kernel(const __nv_bfloat16* __restrict__ x, int T, int H, int tpc, int gpc,
+__global__ void __launch_bounds__(QUANT_THREADS) quantize_1x128_kernel(const __nv_bfloat16* __restrict__ x, int T, int H, int tsh, int gpc,
                                                              uint8_t* __restrict__ q, float* __restrict__ scale) {
-    __shared__ float s_scale[QUANT_GROUPS][QUANT_TOKENS];
+    __shared__ float s_scale[QUANT_SCALES];      // [group][token]
     const int groups = H >> 7;
-    const int t0 = blockIdx.x * tpc, k0 = blockIdx.y * gpc;
-    const int nt = min(tpc, T - t0), nk = min(gpc, groups - k0);
+    const int t0 = blockIdx.x << tsh, k0 = blockIdx.y * gpc;
+    const int nt = min(1 << tsh, T - t0), nk = min(gpc, groups - k0);
     const int sub = threadIdx.x & 7;      // lane inside the group
-    constexpr int GP = 32;                // groups a CTA works on at a time
-    constexpr int U = 2;                  // ... and per lane in flight
+    constexpr int GP = QUANT_THREADS / QUANT_LANES, U = QUANT_FLIGHT;
     const int total = nt * nk;
     int t = 0, k = threadIdx.x >> 3;      // this lane's next group inside the block
-    while (k >= nk) { k -= nk; ++t; }
+    int dt = 0, dk = GP;                  // ... and the way to the one after it
+    if (nk <= GP) {
+        t = k / nk; k -= t * nk;
+        dt = GP / nk; dk = GP - dt * nk;
+    }
     // the trip count is the same for all lanes (the shuffles below stay inside a group, but name the warp)
     for (int i0 = 0; i0 < total; i0 += U * GP) {
         alignas(16) uint32_t raw[U][8];
@@ -79,8 +86,8 @@ __global__ void __launch_bounds__(256) quantize_1x128_kernel(const __nv_bfloat16
                     *reinterpret_cast<uint4*>(&raw[u][4]) = __ldcs(reinterpret_cast<const uint4*>(src) + 1);
                 }
             }
-            k += GP;
-            while (k >= nk) { k -= nk; ++t; }
+            t += dt; k += dk;
+            if (k >= nk) { k -= nk; ++t; }
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -112,13 +119,13 @@ __global__ void __launch_bounds__(256) quantize_1x128_kernel(const __nv_bfloat16
                 reinterpret_cast<uint2*>(dst)[0] = make_uint2(w[0], w[1]);
                 reinterpret_cast<uint2*>(dst)[1] = make_uint2(w[2], w[3]);
             }
-            if (sub == 0) s_scale[kk[u]][tt[u]] = s;
+            if (sub == 0) s_scale[(kk[u] << tsh) + tt[u]] = s;
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nk * QUANT_TOKENS; i += 256) {
-        const int kb = i / QUANT_TOKENS, tl = i % QUANT_TOKENS;
-        if (tl < nt) scale[(size_t)(k0 + kb) * T + t0 + tl] = s_scale[kb][tl];
+    for (int i = threadIdx.x; i < nk << tsh; i += QUANT_THREADS) {
+        const int kb = i >> tsh, tl = i - (kb << tsh);
+        if (tl < nt) scale[(size_t)(k0 + kb) * T + t0 + tl] = s_scale[i];
     }
 }
 

@@ -75,9 +75,11 @@ def test_quantiser_keeps_the_sign_of_zeros_and_of_underflow(scale):
     assert torch.equal(q.cpu().view(torch.uint8), want)
 
 
-@pytest.mark.parametrize("T,H,off", [(1, 128, 0), (9, 256, 8), (31, 4352, 8), (600, 8320, 0), (4739, 128, 16)])
+@pytest.mark.parametrize("T,H,off", [(1, 128, 0), (9, 256, 8), (31, 4352, 8), (600, 8320, 0), (4739, 128, 16), (40003, 128, 0),
+                                     (19001, 384, 8), (9999, 512, 16)])
 def test_quantiser_blocks_and_alignment(T, H, off):
-    """Ragged token blocks, rows cut over several CTAs, and activations that are only 16-byte aligned."""
+    """Ragged token blocks, rows cut over several CTAs, rows of few groups (up to 64 tokens in a CTA), and activations that are
+    only 16-byte aligned."""
     from justgoal_b200 import _lib, quantize_1x128
     import ctypes as C
     x = _case(T, H, seed=T)
