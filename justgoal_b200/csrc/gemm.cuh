@@ -42,6 +42,12 @@
 // re-allocation is legal; with the fused combine they write the zero rows of tokens that have no pair on this rank),
 // warps 4.. = promotion/epilogue (4 or 8 warps; warp % 4 selects the TMEM lane quarter).
 // Every wait is bounded (common.cuh); no TMA load uses cluster multicast.
+//
+// Code size.  A forward runs five or six kernels in turn, and their code together decides whether an SM still holds this
+// kernel's when the next forward comes.  With 90 + 63 KB (GEMM1 + GEMM2, 128-token tiles) it did not: the first epilogue of every
+// launch, 40 KB of straight code, took 12-14 k cycles instead of 4 k (2048 tokens, 16 experts of the 4096-wide shape: 14.5 k).
+// So the roles' loops stay rolled (`unroll 1`: their bodies hold whole waits) and partial sums move four at a time: 80 + 53 KB,
+// 7.8 k cycles there; 300 tokens of a 1024-wide shape 60.6 -> 55.6 us, 901 tokens 255.4 -> 250.6 us.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -72,7 +78,7 @@ struct GemmParams {
     int evict_first_weights;
     int* sk_count;        // [4 * gridDim.x + 4] zero at launch: [4 * ut ...] arrivals of split unit ut (claimed chunks: one byte
                           // per group of warps that arrives together), [4 * gridDim.x] the chunk claim counter
-    float* sk_partial;    // [gridDim.x * chunks per unit] slots of SLOT_FLOATS floats
+    float* sk_partial;    // [gridDim.x * chunks per unit] slots of SLOT_FLOATS floats: [NACCUM * NC / 4][NPT][4]
     long long* klog;      // [4][KLOG_N]: CTA 0's clock at its first KLOG_N K blocks: TMA issue, data seen by the
                           // MMA warp, group seen by the promotion warps, group folded (hand-back)
     long long* trace;     // [gridDim.x][TRACE_SLOTS]: slot 0 = %globaltimer at entry, others = SM clocks since entry
@@ -413,6 +419,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         if (ctid == 0) {
             int seen = 0;
             const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
             for (uint32_t it = 1;; ++it) {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.routed) : "memory");
                 if (seen) break;
@@ -420,11 +427,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             }
             *s_flag = seen;
         }
+#pragma unroll 1
         for (int i = ctid; i <= p.num_local; i += 128) s_cnt[i] = 0;
         ctrl_sync();
         early = *s_flag != 0;
     }
     if (early) {
+#pragma unroll 1
         for (int i0 = ctid; i0 < p.n_pairs; i0 += 128 * 8) {
             int id[8];
 #pragma unroll
@@ -438,6 +447,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     } else {
         early = !G1 && p.tables_done;
         if (!early) pdl_wait();
+#pragma unroll 1
         for (int i = ctid; i <= p.num_local; i += 128) {
             s_tiles[i] = __ldcg(p.tile_prefix + i);
             s_row0[i] = __ldcg(p.expert_row0 + i);
@@ -520,6 +530,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 t_lo = range_start((int)blockIdx.x, flat, parts); t_hi = range_start((int)blockIdx.x + 1, flat, parts);
                 t_unit = t_lo / NG;
             }
+#pragma unroll 1
             while (ok) {
                 WorkItem wi;
                 wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0, 0};
@@ -572,6 +583,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     const int was = s_filled[s_];
                     if (was > boxes) {
                         uint8_t* st = smem + s_ * C::STAGE_BYTES + C::NA * C::A_BYTES;
+#pragma unroll 1
                         for (int o = boxes * C::BOX_ROWS * 128 + lane * 16; o < was * C::BOX_ROWS * 128; o += 512) {
                             *reinterpret_cast<uint4*>(st + o) = make_uint4(0u, 0u, 0u, 0u);
                             if (!G1) *reinterpret_cast<uint4*>(st + C::B_BYTES + o) = make_uint4(0u, 0u, 0u, 0u);
@@ -619,6 +631,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         tma_load_2d(dst, &tm_b0, kb * 128, un.row0, full);
                         if (!G1) tma_load_2d(dst + C::B_BYTES, &tm_b1, kb * 128, un.row0, full);
                     } else if constexpr (BOXED) {
+#pragma unroll 1
                         for (int b = 0; b < boxes; ++b) {
                             tma_load_2d(dst + b * C::BOX_ROWS * 128, &tm_s0, kb * 128, un.row0 + b * C::BOX_ROWS, full);
                             if (!G1) tma_load_2d(dst + C::B_BYTES + b * C::BOX_ROWS * 128, &tm_s1, kb * 128, un.row0 + b * C::BOX_ROWS, full);
@@ -633,6 +646,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the kernel before this one
                     // still runs, then the wait for it, then the token side of the same stages
                     const int npre = min(C::STAGES, kb_end - kb_first);
+#pragma unroll 1
                     for (int i = 0; i < npre; ++i) {
                         if (BOXED) clear_dead_rows(i);
                         if (elect_one()) load_weights(i, kb_first + i);
@@ -642,6 +656,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     issued = true;
                     pdl_wait();
                     waited = true;
+#pragma unroll 1
                     for (int i = 0; i < npre; ++i) {
                         if (elect_one()) load_tokens(i, kb_first + i);
                         __syncwarp();
@@ -652,6 +667,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     stage = npre;
                     if (stage == C::STAGES) { stage = 0; phase ^= 1; }
                 }
+#pragma unroll 1
                 for (int kb = kb_first; kb < kb_end; ++kb) {
                     if (!mbar_wait_warp(bar_empty + 8 * stage, phase ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
                     if (BOXED && kb < kb_clear) clear_dead_rows(stage);
@@ -684,10 +700,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             int nk = 0;
             int n_item = 0;
             WorkItem wi;
+#pragma unroll 1
             while (ok && wq_fetch(n_item++, wi, ok)) {
                 const int gb = wi.gb, ge = wi.ge;
+#pragma unroll 1
                 for (int grp = gb; grp < ge; ++grp) {
                     const int nj = min(C::KPB, p.KB - grp * C::KPB);
+#pragma unroll 1
                     for (int j = 0; j < nj; ++j) {
                         if (lane == 0) klog_put(6, nk);
                         // the group's accumulator buffer (first K block) and the stage, tried together: the tensor pipe's
@@ -784,6 +803,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         bool ok = true;
         int n_item = 0;
         WorkItem wi;
+#pragma unroll 1
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
             const Unit un = wi.un;
@@ -819,6 +839,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #pragma unroll
             for (int i = 0; i < C::TSD - 1; ++i) ts_fetch(gb + i);
             ws_window(gb);
+#pragma unroll 1
             for (int kb = gb; kb < ge; ++kb) {
                 if ((kb & 63) == 0 && kb > gb) ws_window(kb);
                 const bool hi = (kb & 32) != 0;
@@ -840,6 +861,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     } else if (FUSE) {
         // ------------------------------------------------------------ warps 2-3, fused combine: zero rows of the
         // tokens that have no pair on this rank (nobody else writes them)
+#pragma unroll 1
         for (int t = (int)blockIdx.x * 2 + (warp - 2); t < p.T; t += (int)gridDim.x * 2) {
             bool local = false;
             if (lane < p.top_k) {
@@ -848,6 +870,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             }
             if (__any_sync(0xFFFFFFFFu, local)) continue;
             uint4* o = reinterpret_cast<uint4*>(p.fuse_out + (size_t)t * p.H);
+#pragma unroll 1
             for (int i = lane; i < p.H / 8; i += 32) o[i] = make_uint4(0u, 0u, 0u, 0u);
         }
     }
@@ -886,12 +909,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         WorkItem wi;
         pdl_wait();
         pdl_launch();
+#pragma unroll 1
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
             const Unit un = wi.un;
             if (PART && quarter * 32 >= un.nvalid) {
                 // no row of the unit in this warp's lanes: only hand the buffers back (the warp it meets in the epilogue has
                 // no row either, here and in the CTAs that run other pieces of the unit)
+#pragma unroll 1
                 for (int n = ge - gb; n > 0; --n) {
                     if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
                     if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
@@ -970,6 +995,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (ptid == 0) klog_put(3, ng++);
                 }
             } else
+#pragma unroll 1
             for (int grp = gb; grp < ge; ++grp) {
                 const int kb0 = grp * C::KPB;
                 const int nj = min(C::KPB, p.KB - kb0);
@@ -1001,6 +1027,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (!ok) break;
                     __syncwarp();
                     if (lane == 0) {
+#pragma unroll 1
                         for (int j = 0; j < nj; ++j) {
                             int sj = st0 + j; if (sj >= C::STAGES) sj -= C::STAGES;
                             mbar_arrive(bar_empty + 8 * sj);
@@ -1077,6 +1104,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if (lane == 0) {
                     mbar_arrive(bar_tempty + 8 * ab);
                     if (C::SCALES_IN_STAGE && !C::EARLY_SCALES) {
+#pragma unroll 1
                         for (int j = 0; j < nj; ++j) {
                             int sj = st0 + j; if (sj >= C::STAGES) sj -= C::STAGES;
                             mbar_arrive(bar_empty + 8 * sj);
@@ -1092,13 +1120,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if (ptid == 0) stamp(TR_PROMO_LAST);
 
             if (wi.pieces > 1) {
-                float* const slots = p.sk_partial + (size_t)wi.slot * C::SLOT_FLOATS + ptid;
+                // a slot holds four accumulators of a thread together: [NACCUM * NC / 4][NPT] of 16 bytes
+                float4* const slots = reinterpret_cast<float4*>(p.sk_partial + (size_t)wi.slot * C::SLOT_FLOATS) + ptid;
+                constexpr int SLOT_VECS = C::SLOT_FLOATS / 4, ACC_VECS = C::NACCUM * C::NC / 4;
+                auto slot_of = [&](int c) -> float4* { return slots + (size_t)c * SLOT_VECS; };
+                auto acc4 = [&](int k) -> float* { return &acc[4 * k / C::NC][4 * k % C::NC]; };
                 auto store_partial = [&]() {
-                    float* slot = slots + (size_t)wi.piece * C::SLOT_FLOATS;
+                    float4* slot = slot_of(wi.piece);
 #pragma unroll
-                    for (int a = 0; a < C::NACCUM; ++a)
-#pragma unroll
-                        for (int i = 0; i < C::NC; ++i) __stcg(slot + (size_t)(a * C::NC + i) * C::NPT, acc[a][i]);
+                    for (int k = 0; k < ACC_VECS; ++k) __stcg(slot + k * C::NPT, make_float4(acc4(k)[0], acc4(k)[1], acc4(k)[2], acc4(k)[3]));
                 };
                 int* const arrived = p.sk_count + 4 * wi.ut;
                 if constexpr (C::STATIC_TAIL) {
@@ -1116,6 +1146,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     bool here = true;
                     if (lane == 0) {
                         const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
                         for (uint32_t it = 1;; ++it) {
                             int v;
                             asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
@@ -1158,42 +1189,43 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (seen_pieces != wi.pieces - 1) continue;
                     __threadfence();
                 }
-                auto slot_of = [&](int c) -> const float* { return slots + (size_t)c * C::SLOT_FLOATS; };
                 if (!C::STATIC_TAIL && wi.piece != wi.pieces - 1) {
-                    const float* src = slot_of(wi.pieces - 1);
+                    const float4* src = slot_of(wi.pieces - 1);
 #pragma unroll
-                    for (int a = 0; a < C::NACCUM; ++a)
-#pragma unroll
-                        for (int i = 0; i < C::NC; ++i) acc[a][i] = __ldcg(src + (size_t)(a * C::NC + i) * C::NPT);
+                    for (int k = 0; k < ACC_VECS; ++k) {
+                        const float4 v = __ldcg(src + k * C::NPT);
+                        acc4(k)[0] = v.x; acc4(k)[1] = v.y; acc4(k)[2] = v.z; acc4(k)[3] = v.w;
+                    }
                 }
                 const int n_other = wi.pieces - 1;
-                if constexpr (C::NACCUM * C::NC <= 32) {
+                if constexpr (ACC_VECS <= 8) {
                     // narrow tiles: the next piece's slot is in flight while this one is added (same fixed order)
-                    float nxt[C::NACCUM * C::NC];
-                    const float* src = slot_of(0);
+                    float4 nxt[ACC_VECS];
 #pragma unroll
-                    for (int k = 0; k < C::NACCUM * C::NC; ++k) nxt[k] = __ldcg(src + (size_t)k * C::NPT);
+                    for (int k = 0; k < ACC_VECS; ++k) nxt[k] = __ldcg(slot_of(0) + k * C::NPT);
+#pragma unroll 1
                     for (int c = 0; c < n_other; ++c) {
-                        float cur[C::NACCUM * C::NC];
+                        float4 cur[ACC_VECS];
 #pragma unroll
-                        for (int k = 0; k < C::NACCUM * C::NC; ++k) cur[k] = nxt[k];
+                        for (int k = 0; k < ACC_VECS; ++k) cur[k] = nxt[k];
                         if (c + 1 < n_other) {
-                            src = slot_of(c + 1);
 #pragma unroll
-                            for (int k = 0; k < C::NACCUM * C::NC; ++k) nxt[k] = __ldcg(src + (size_t)k * C::NPT);
+                            for (int k = 0; k < ACC_VECS; ++k) nxt[k] = __ldcg(slot_of(c + 1) + k * C::NPT);
                         }
 #pragma unroll
-                        for (int a = 0; a < C::NACCUM; ++a)
-#pragma unroll
-                            for (int i = 0; i < C::NC; ++i) acc[a][i] += cur[a * C::NC + i];
+                        for (int k = 0; k < ACC_VECS; ++k) {
+                            acc4(k)[0] += cur[k].x; acc4(k)[1] += cur[k].y; acc4(k)[2] += cur[k].z; acc4(k)[3] += cur[k].w;
+                        }
                     }
                 } else {
+#pragma unroll 1
                     for (int c = 0; c < n_other; ++c) {
-                        const float* src = slot_of(c);
+                        const float4* src = slot_of(c);
 #pragma unroll
-                        for (int a = 0; a < C::NACCUM; ++a)
-#pragma unroll
-                            for (int i = 0; i < C::NC; ++i) acc[a][i] += __ldcg(src + (size_t)(a * C::NC + i) * C::NPT);
+                        for (int k = 0; k < ACC_VECS; ++k) {
+                            const float4 v = __ldcg(src + k * C::NPT);
+                            acc4(k)[0] += v.x; acc4(k)[1] += v.y; acc4(k)[2] += v.z; acc4(k)[3] += v.w;
+                        }
                     }
                 }
             }
@@ -1334,6 +1366,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (mine) {
                         t = __ldg(p.row_token + un.row0 + c);
                         int need = 0;
+#pragma unroll 1
                         for (int k = 0; k < p.top_k; ++k) {
                             const int le = __ldg(p.c_topk + (size_t)t * p.c_stride + k) - p.c_local_offset;
                             need += le >= 0 && le < p.num_local;
