@@ -641,14 +641,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         bulk_load(st + C::SC_OFF, p.b_scale + (size_t)kb * p.rows_cap + un.row0, NTOK * 4, full);
                 };
                 int kb_first = gb * C::KPB;
-                const int kb_clear = kb_first + C::STAGES;                                  // the first turn of the stage ring
+                // The clearing: in the first turn of the stage ring.  Not for a piece of a few K blocks, which is over before it pays: it
+                // stands in front of the first loads.  (With 4, 5 and 8 K blocks it cost 1-2 us of a 34-55 us forward; pieces of 16
+                // and 56 gain, see BOXED.)
+                const bool clears = BOXED && kb_end - kb_first >= 3 * C::STAGES;
+                const int kb_clear = clears ? kb_first + C::STAGES : kb_first;
+                if (BOXED && !clears && lane < C::STAGES) s_filled[lane] = 128 / C::BOX_ROWS;
+                __syncwarp();
                 if (!waited) {
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the kernel before this one
                     // still runs, then the wait for it, then the token side of the same stages
                     const int npre = min(C::STAGES, kb_end - kb_first);
 #pragma unroll 1
                     for (int i = 0; i < npre; ++i) {
-                        if (BOXED) clear_dead_rows(i);
+                        if (clears) clear_dead_rows(i);
                         if (elect_one()) load_weights(i, kb_first + i);
                         __syncwarp();
                     }

@@ -155,12 +155,15 @@ def test_fused_combine_equals_the_combine_kernel_bit_for_bit(shape_name, T, tile
 
 
 @pytest.mark.parametrize("counts", [(1, 31, 32, 33, 96, 97, 128, 129), (127, 160, 161, 255, 256, 257, 16, 64)])
-def test_part_full_128_token_tiles(counts):
+@pytest.mark.parametrize("hidden,intermediate", [(512, 256), (1536, 1152)])
+def test_part_full_128_token_tiles(counts, hidden, intermediate):
     """128-token tiles at every edge of their 32-row quarters, through the instance for mostly part-full tiles (few tokens)
     and the one for full tiles (the same tokens among many without a local expert): the oracle's result, and the same
-    bits from both.  The workspace is poisoned: quarters that are left out must not matter."""
+    bits from both.  The workspace is poisoned: quarters that are left out must not matter.  (The second size has just the
+    K blocks from which rows that a stage held earlier are cleared, the first one fewer.)"""
+    import dataclasses
     from justgoal_b200 import MoELayer
-    shape = I.TINY_DS
+    shape = dataclasses.replace(I.TINY_DS, hidden=hidden, intermediate=intermediate)
     few, many = max(counts), 1100                        # below / above 128 expected rows per expert
     assert few * shape.top_k / shape.num_experts < 128 <= many * shape.top_k / shape.num_experts
     d = I.make_inputs(shape, many, seed=17)
