@@ -28,8 +28,8 @@ using namespace b200moe;
 
 constexpr int PROF_POINTS = 7;   // before route, after route, permute, gather, gemm1, gemm2, combine
 
-// The tensor maps of a forward depend on addresses and sizes only; a caller repeats them from step to step (weights,
-// workspace), and encoding them is ~5 us of host time per forward.
+// The tensor maps of a forward depend on addresses and sizes only, and a caller repeats them from step to step (weights,
+// workspace).  Encoding one takes 0.1 us of the ~20 us of host time of a small forward.
 struct MapSet { CUtensorMap w13, w2, a, hi, lo, a_box, hi_box, lo_box; };      // *_box: boxes of a part-full 128-token tile
 struct MapKey {
     const void *w13, *w2, *a, *hi, *lo;
@@ -90,9 +90,11 @@ int pdl_mask() {
     return v;
 }
 
-// With thousands of tokens the early-resident dependents slow the front kernels and GEMM1 down (8192 tokens, 256 experts:
-// 5.60 -> 5.85 ms), so only GEMM2 and the combine overlap there (14107 tokens: 1.025 -> 1.005 ms); up to 2048 tokens all
-// launches do (901 tokens: 288 -> 278 us, 2048 tokens of the 4096-wide shape: 150 -> 132 us).  A shape-only decision.
+// With many thousands of tokens the early-resident dependents slow the front kernels and GEMM1 down, so only GEMM2 and the
+// combine overlap there; up to 2048 tokens all launches do.  A shape-only decision.  Overlap of GEMM2 and the combine alone /
+// of all launches, us: 16 experts of the 4096-wide shape 513 tokens 102 / 92, 2048 139 / 131, 4096 191 / 183, 8192 318 / 312; 32 of
+// 256 experts 513 tokens 262 / 253, 2048 350 / 349, 4096 530 / 530, 6000 697 / 717, 12000 1155 / 1188; 128 of 256 experts 2048
+// tokens 1182 / 1198, 6000 2071 / 2179.  (Between 2048 and 4096 tokens a few experts would still gain.)
 thread_local int g_call_pdl = 0;
 inline void set_call_pdl(int num_tokens) { g_call_pdl = num_tokens <= 2048 ? pdl_mask() : pdl_mask() & (PDL_GEMM2 | PDL_COMBINE); }
 
@@ -145,6 +147,10 @@ int num_slices(const b200moe_config& c, int T) {
 // ahead of every narrower one although most of its rows are padding - the step is bound by the weight stream, and
 // the narrow tiles' weights-on-M MMAs are short of shared-memory bandwidth from 64 columns on.  The 64-token tile is
 // never the best choice; it stays available through b200moe_set_token_tile.
+// The estimate is that of a forward that routes itself.  Every token of forward_routed has a local expert, so an expert sees
+// more rows than estimated (DeepSeek-V3 routing, 32 local experts: twice as many), and calls of 150 to 350 tokens run a tile
+// that is up to 11 % slower than the best one there (32 local, tile 16 / 32 / 128: 200 tokens 238 / 228 / 235 us, 288 tokens
+// 287 / 267 / 249; 128 local, 350 tokens 928 / 795 / 751).
 int pick_token_tile(const b200moe_ctx* h, int T) {
     if (h->token_tile) return h->token_tile;
     const b200moe_config& c = h->cfg;
@@ -154,8 +160,11 @@ int pick_token_tile(const b200moe_ctx* h, int T) {
     return 128;
 }
 
-// 128-token tiles: do most tiles hold fewer than 128 rows?  Below one tile's worth of expected rows per expert they do,
-// and the kernels that leave empty row quarters out are ahead (gemm.cuh, PART); above it full tiles dominate.
+// 128-token tiles: do most tiles hold fewer than 128 rows?  Below one tile's worth of expected rows per expert they do, and
+// the kernels that leave empty row quarters out (gemm.cuh, PART) are ahead or level; above it full tiles dominate and the
+// extra path costs a little.  Without / with PART, us, by rows per expert: 16 experts of the 4096-wide shape 32: 93.9 / 92.4, 64:
+// 98.4 / 98.3, 100: 105.0 / 106.3, 128: 132.7 / 133.5, 200: 171 / 173, 400: 271 / 277; 32 of 256 experts 32: 278 / 274, 80: 426 / 398,
+// 128: 533 / 557, 256: 885 / 916, 512: 1502 / 1605.
 bool tiles_mostly_part_full(const b200moe_config& c, int T) {
     return (double)T * c.top_k / c.num_experts < 128.0;
 }
@@ -331,10 +340,9 @@ cudaError_t launch_gemm_pair(int grid, cudaStream_t st, const CUtensorMap& w, co
     return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<G1>, w, b0, b1, p);
 }
 
-// Full token tiles run on SM pairs when B200MOE_PAIR=1.  Off by default: measured on B200, both families run
-// into the 1 kW power cap within milliseconds, and at the clocks the cap leaves (~1.45-1.55 GHz) the pair
-// kernels are 8 % (GEMM1) / 0 % (GEMM2) slower than the single-SM ones although they need fewer cycles per
-// 128-K block at full clock (1008 against 1180).
+// Full token tiles run on SM pairs when B200MOE_PAIR=1.  Off by default: 8192 tokens over 256 experts 7.04 against 5.43 ms,
+// 4096 skewed tokens 992 against 792 us, 2048 tokens of the 4096-wide shape 171 against 132 us.  The pair kernels have neither
+// the scale warps and the rotated promotion loop of gemm.cuh nor its row boxes, and an odd tile of an expert runs as a pair.
 bool use_pairs(const b200moe_ctx* h, int ntok) {
     static int v = -1;
     if (v < 0) { const char* e = getenv("B200MOE_PAIR"); v = e ? atoi(e) : 0; }
@@ -500,8 +508,9 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         fp.a_perm = a_perm; fp.a_scale_perm = a_scale; fp.H = H;
         fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = (int)(L.expert_row0 / 16);
         // enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that GEMM1 can start on most
-        // SMs while this kernel runs.  64 against 32 CTAs: 64 tokens 130.1 -> 129.6 us, 128 tokens 149.5 -> 148.3 us, but
-        // one token +0.3 us, 7 tokens +0.6 us (the meeting takes longer); 96 CTAs: 128 tokens 148.9 us.
+        // SMs while this kernel runs.  32 / 64 CTAs, us: 1 token 18.6 / 18.7 (no local expert), 8 tokens 99.1 / 99.1, 16 tokens
+        // 112.8 / 112.5, 32 tokens 125.0 / 124.3, 33 tokens 124.2 / 123.9, 64 tokens 144.9 / 144.0, 128 tokens 180 / 179; 96 CTAs
+        // gained nothing more.  The line is not sharp: level up to 8 tokens, 0.3 us apart at 16, 0.7 us at 32.
         const int want = T <= 32 ? 32 : 64;
         const int fgrid = h->num_sms < want ? h->num_sms : want;
         if (route_in_front) CU_TRY(launch_front_route(c, fgrid, fp, *route_in_front, st));

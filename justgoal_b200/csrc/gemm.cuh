@@ -92,8 +92,8 @@ struct GemmParams {
     int n_pairs, local_offset;
     // GEMM1 with 128-token tiles reading the token rows straight from the caller's activations (no gather copy), else
     // g4_row_token == null: tm_b0 is then a map over the activations with one-row boxes, a stage's token tile is 32
-    // four-row TMA gathers through row_token, and the promotion threads read their token's block scales from the
-    // caller's scale tensor: scale(token, kb) = g4_scale[token * g4_tok_stride + kb * g4_kb_stride].
+    // four-row TMA gathers through row_token, and the scale warps read their tokens' block scales from the
+    // caller's scale tensor: scale(token, kb) = g4_scale[token * g4_tok_stride + kb * ts_stride].
     const int32_t* g4_row_token;
     const float* g4_scale;
     int g4_tok_stride;    // in floats
@@ -119,14 +119,14 @@ struct GemmCfg {
     static constexpr int B_BYTES = NTOK * 128;
     static constexpr int SC_OFF = NA * A_BYTES + NB * B_BYTES;
     static constexpr int STAGE_BYTES = SC_OFF + 1024;
-    // tokens-on-M tiles read their (per-thread scalar) token scale straight from global memory, one K
-    // block ahead; the others get the tile's NTOK scales copied into the stage
+    // tokens-on-M tiles get their (per-thread scalar) token scales through the scale warps; the others get the tile's
+    // NTOK scales copied into the stage
     static constexpr bool SCALES_IN_STAGE = NTOK != 128;
     static constexpr int TX_BYTES = NA * A_BYTES + NB * B_BYTES + (SCALES_IN_STAGE ? NTOK * 4 : 0);
     // 128-token tiles: the rows of a part-full tile travel in boxes of BOX_ROWS, and only the boxes that hold rows of the unit.
     // What the stage held in the others is overwritten with zeros once: zero operands cost the tensor pipe less energy, and
-    // the large forwards run into the power limit (8192 tokens, 256 experts: 5.9 -> 5.6 ms at more cycles; 4201 routed
-    // tokens: 738 -> 720 us).
+    // the large forwards run into the power limit (8192 tokens, 256 experts: 5.55 -> 5.43 ms at more cycles; 4096 skewed tokens
+    // 801 -> 792 us; 4201 routed tokens 743 -> 736 us).
     static constexpr bool BOXED = NTOK == 128;
     static constexpr int BOX_ROWS = BOXED ? 32 : NTOK;
     static constexpr int EMPTY_COUNT = 1 + (SCALES_IN_STAGE ? (NTOK >= 64 ? 8 : 4) : 0);   // MMA commit (+ promotion warps)
@@ -168,7 +168,7 @@ struct GemmCfg {
     // register count ptxas actually chose, by the host before the first launch).
     static constexpr bool REALLOC_REGS = NPW >= 8;
     static constexpr int LAUNCH_REGS = (65536 / NTHREADS) / 8 * 8;          // what __launch_bounds__(NTHREADS, 1) yields
-    static constexpr int CTRL_REGS = 56;      // 40/232 spills in the producer (T=8192: 5.95 against 5.60 ms)
+    static constexpr int CTRL_REGS = 56;      // 40/232 spills in the control warps (8192 tokens, 256 experts: 5.46 against 5.43 ms)
     static constexpr int PROMO_REGS = 224;
     static_assert(!REALLOC_REGS || 128 * CTRL_REGS + NPT * PROMO_REGS <= NTHREADS * LAUNCH_REGS,
                   "setmaxnreg.inc would wait forever: the control warps do not release enough registers");
@@ -186,9 +186,9 @@ struct GemmCfg {
     static constexpr int CHUNK_GROUPS = (CHUNK_BLOCKS / KPB) < 1 ? 1 : (CHUNK_BLOCKS / KPB);
     static constexpr int CHUNKS_PER_CTA = 2;               // measured: 4 and 6 cost 2-10 us more at every decode size
     // GEMM1 with narrow tiles has few, long units (decode: 256 units of 3.7 MB for 148 CTAs): there the units left
-    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA, processed first.  A range touches at
-    // most two units, so a CTA stores at most one partial sum and the piece that ends a unit waits for pieces that other
-    // CTAs ran first (claimed chunks measured 5-15 us slower: every one of them costs a partial sum, late in the kernel).
+    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA.  A range touches at most two units, so a
+    // CTA stores at most one partial sum, which it makes before anything else; the piece that ends a unit runs after the CTA's
+    // whole units and waits for those other pieces (claimed chunks measured 5-15 us slower: every one of them costs a partial sum, late in the kernel).
     // Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
     static constexpr bool STATIC_TAIL = G1 && NTOK <= 32;
     static constexpr int WQ = 4, WQ_INTS = 12;             // depth of the in-CTA work queue, words of an entry (WorkItem)
@@ -213,7 +213,7 @@ enum : int { TR_ENTRY = 0, TR_PROLOGUE = 1, TR_TMA_FIRST = 2, TR_TMA_LAST = 3, T
              TR_PROMO_FIRST = 6, TR_PROMO_LAST = 7, TR_PARTIAL = 8, TR_REDUCED = 9, TR_EPILOGUE = 10, TR_EXIT = 11,
              TRACE_SLOTS = 16, KLOG_N = 64 };
 
-struct Unit { int e, mt, tt, row0, nvalid; };
+struct Unit { int e, mt, row0, nvalid; };
 
 // Unit number -> expert, weight tile, token tile, by a converged warp; the result is the same in all lanes and uniform for
 // the compiler (see mbar_wait_warp).  The expert is the last one whose first unit is not beyond u: two rounds of one
@@ -232,7 +232,7 @@ __device__ __forceinline__ bool decode_unit_warp(int u, int n_mtiles, int num_lo
     int mt = ul, tt = 0;
     if (ntt > 1) { mt = ul / ntt; tt = ul - mt * ntt; }
     auto uni = [&](int v) { return __shfl_sync(FULL, v, 0); };
-    o.e = uni(e); o.mt = uni(mt); o.tt = uni(tt);
+    o.e = uni(e); o.mt = uni(mt);
     o.row0 = uni(s_row0[e] + tt * ntok); o.nvalid = uni(min(ntok, s_cnt[e] - tt * ntok));
     return __all_sync(FULL, ntt > 0 && o.mt < n_mtiles && o.nvalid > 0);
 }
@@ -311,9 +311,8 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 // G4 (GEMM1 with 128-token tiles only): the token rows come straight from the caller's activations by four-row TMA
 // gathers (GemmParams::g4_row_token); a separate instantiation, so the plain kernel's code is unchanged by it.
 // PART (128-token tiles): quarters of a token tile (32 rows, one warp's TMEM lanes) that hold no row of the unit are not
-// folded.  Measured at 39 rows per
-// expert (901 tokens): GEMM1 160 -> 148 us, GEMM2 90 -> 86 us.  With full tiles the extra path costs the promotion loop 4 %
-// of its cycles, so the host picks the instance by the expected number of rows per expert (b200moe.cu).
+// folded.  With full tiles the extra path costs a few per cent of the promotion loop, so the host picks the instance by the
+// expected number of rows per expert (both sides measured at the rule in b200moe.cu).
 // FUSE (GEMM2, narrow tiles): with the combine in the epilogue (GemmParams::fuse_out); an instance of its own, so the plain
 // kernel stays small.
 template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
@@ -394,7 +393,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         auto uni = [](int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); };                  // uniform for the compiler
         w.u = uni(q0.x); w.gb = uni(q0.y); w.ge = uni(q0.z); w.ut = uni(q0.w);
         w.piece = uni(q1.x); w.pieces = uni(q1.y); w.slot = uni(q1.z); w.un.e = uni(q1.w);
-        w.un.mt = uni(q2.x); w.un.row0 = uni(q2.y); w.un.nvalid = uni(q2.z); w.un.tt = 0;
+        w.un.mt = uni(q2.x); w.un.row0 = uni(q2.y); w.un.nvalid = uni(q2.z);
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
         return w.u >= 0;
@@ -533,7 +532,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #pragma unroll 1
             while (ok) {
                 WorkItem wi;
-                wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0, 0};
+                wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0};
                 const int u_end = (t_unit + 1) * NG;
                 const bool ends_unit = t_lo > t_unit * NG && t_hi == u_end;         // the rest of the range is such a piece
                 if (C::STATIC_TAIL && t_lo < t_hi && !(ends_unit && n_whole < sched_q)) {
@@ -690,7 +689,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if (!ok) {
                 // gave up: end the list for the other roles (if the queue still moves), then give copies that are
                 // still in flight time to land before the CTA's shared memory goes away
-                WorkItem end_; end_.u = -1; end_.gb = end_.ge = end_.ut = end_.piece = end_.slot = 0; end_.pieces = 1; end_.un = Unit{0, 0, 0, 0, 0};
+                WorkItem end_; end_.u = -1; end_.gb = end_.ge = end_.ut = end_.piece = end_.slot = 0; end_.pieces = 1; end_.un = Unit{0, 0, 0, 0};
                 publish(end_);
                 for (int i = 0; i < 64; ++i) __nanosleep(10000);
             }
@@ -1249,7 +1248,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     amax = fmaxf(amax, fabsf(v));
                 }
                 // [2][NGRP][128], used in turn: a warp is at most one meeting ahead of the one it meets
-                                float* redf = reinterpret_cast<float*>(s_red) + rbuf * (C::NGRP * 128);
+                float* redf = reinterpret_cast<float*>(s_red) + rbuf * (C::NGRP * 128);
                 rbuf ^= 1;
                 redf[grp_id * 128 + m] = amax;
                 if (!group_sync()) { ok = false; break; }
