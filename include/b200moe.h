@@ -291,7 +291,7 @@ int b200moe_set_token_tile(b200moe_handle h, int tokens);
  * rows straight from hidden_states (or from the packed dispatch rows) with four-row TMA gathers
  * (`cp.async.bulk.tensor...tile::gather4`, as KF94/kernel.cu:932-941,3014-3056) through the
  * token-of-row table, and the activation gather copy is not launched.  Same results bit for bit;
- * measured three times slower on the GEMM (32 gathers per 128-K block from one producer thread),
+ * measured 2.2 to 2.6 times slower on the GEMM (32 gathers per 128-K block from one producer warp),
  * so the copy stays the default. */
 int b200moe_set_tma_gather(b200moe_handle h, int on);
 

@@ -485,8 +485,8 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     const bool pairs = use_pairs(h, ntok);
     // Optional (b200moe_set_tma_gather), 128-token tiles: GEMM1 reads the token rows straight from the caller's
     // activations with four-row TMA gathers through row_token (one-row boxes; rows `pitch` bytes apart when they sit
-    // inside packed dispatch rows) - no gather copy.  Same results; measured three times slower (32 gathers per
-    // 128-K block from one producer thread: ~100 ns each), so the copy stays the default.
+    // inside packed dispatch rows) - no gather copy.  Same results; GEMM1 measured 2.2 to 2.6 times slower (32 gathers
+    // per 128-K block from one producer warp), so the copy stays the default.
     const bool g4 = ntok == 128 && !pairs && h->tma_gather;
     const bool part = ntok == 128 && !pairs && !g4 && tiles_mostly_part_full(c, T);
     if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, ntok}, &maps))) return rc;
