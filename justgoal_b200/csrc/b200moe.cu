@@ -342,7 +342,7 @@ cudaError_t launch_gemm_pair(int grid, cudaStream_t st, const CUtensorMap& w, co
 
 // Full token tiles run on SM pairs when B200MOE_PAIR=1.  Off by default: 8192 tokens over 256 experts 7.04 against 5.43 ms,
 // 4096 skewed tokens 992 against 792 us, 2048 tokens of the 4096-wide shape 171 against 132 us.  The pair kernels have neither
-// the scale warps and the rotated promotion loop of gemm.cuh nor its row boxes, and an odd tile of an expert runs as a pair.
+// the scale ring and the promotion loop of gemm.cuh nor its row boxes, and an odd tile of an expert runs as a pair.
 bool use_pairs(const b200moe_ctx* h, int ntok) {
     static int v = -1;
     if (v < 0) { const char* e = getenv("B200MOE_PAIR"); v = e ? atoi(e) : 0; }

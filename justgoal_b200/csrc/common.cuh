@@ -77,6 +77,37 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// One look at a barrier; never suspends the thread (try_wait may, for as long as the hardware likes).
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Bounded wait whose answer is data, not control flow: `ok` becomes 0 when the wait gave up, and then every later wait with
+// the same `ok` gives up after its first try.  For loops that cannot afford a vote and a branch per step (40 cycles of a
+// promotion warp's ~450): the caller looks at `ok` once per piece of work, votes there and records the error.
+__device__ __forceinline__ void mbar_wait_flag(uint32_t bar, uint32_t parity, uint32_t& ok) {
+    const unsigned long long limit = ok ? WAIT_LIMIT_NS : 0ull;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u64 t0, t1;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE;\n\t"
+        "mov.u64 t0, %%globaltimer;\n\t"
+        "AGAIN:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra DONE;\n\t"
+        "mov.u64 t1, %%globaltimer;\n\t"
+        "sub.u64 t1, t1, t0;\n\t"
+        "setp.lt.u64 q, t1, %3;\n\t"
+        "@q bra AGAIN;\n\t"
+        "mov.u32 %0, 0;\n\t"
+        "DONE:\n\t}"
+        : "+r"(ok) : "r"(bar), "r"(parity), "l"(limit) : "memory");
+}
 // Keeps the compiler from drawing conclusions about a flag at the place where the paths that set it meet.  Without it
 // the code that follows a wait is duplicated for "the first try succeeded" and "a later one did", and again for every wait
 // after that: the GEMM kernels grew to two and a half times their size, and their epilogues no longer stayed in the
@@ -162,6 +193,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 // Per-thread asynchronous 4-byte copy global -> shared, for values a thread needs several steps later
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+// ... of 16 bytes, both addresses 16-byte aligned
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>

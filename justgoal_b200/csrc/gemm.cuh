@@ -38,7 +38,7 @@
 // Optionally (FUSE) GEMM2's epilogue also does the combine.
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (whole warps, one elected lane issues),
-// warps 2-3: scale products for 128-token tiles, otherwise idle (they complete the first warpgroup so register
+// warps 2-3: scales of 128-token tiles on their way into shared memory, otherwise idle (they complete the first warpgroup so register
 // re-allocation is legal; with the fused combine they write the zero rows of tokens that have no pair on this rank),
 // warps 4.. = promotion/epilogue (4 or 8 warps; warp % 4 selects the TMEM lane quarter).
 // Every wait is bounded (common.cuh); no TMA load uses cluster multicast.
@@ -92,7 +92,7 @@ struct GemmParams {
     int n_pairs, local_offset;
     // GEMM1 with 128-token tiles reading the token rows straight from the caller's activations (no gather copy), else
     // g4_row_token == null: tm_b0 is then a map over the activations with one-row boxes, a stage's token tile is 32
-    // four-row TMA gathers through row_token, and the scale warps read their tokens' block scales from the
+    // four-row TMA gathers through row_token, and the scale warps copy their tokens' block scales from the
     // caller's scale tensor: scale(token, kb) = g4_scale[token * g4_tok_stride + kb * ts_stride].
     const int32_t* g4_row_token;
     const float* g4_scale;
@@ -195,9 +195,10 @@ struct GemmCfg {
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
     static constexpr int TABLE_INTS = 3 * (MAX_LOCAL + 1);
     static constexpr int RED_BYTES = 2 * (TOK_ON_M ? NGRP * 128 : NPW * NC) * 4;      // maxima, two halves used in turn
-    static constexpr int TSD = 8;                          // tokens-on-M: slots of the token-scale ring (see the scale warps)
-    static constexpr int NHELP = TOK_ON_M ? 2 : 0;         // ... and the warps that run it
-    static constexpr int TS_BYTES = TOK_ON_M ? TSD * 128 * 4 + NACC * 128 * 8 : 0;
+    // tokens-on-M: ring of the scales of TSD K blocks, a slot = 128 token scales | 2 weight scales | pad (see the scale warps)
+    static constexpr int TSD = 8, TS_SLOT = 132, TS_AHEAD = 4;
+    static_assert(TS_AHEAD + NACC <= TSD, "a slot is rewritten only when its block has been folded");
+    static constexpr int TS_BYTES = TOK_ON_M ? TSD * TS_SLOT * 4 : 0;
     static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * STAGE_BYTES + BAR_BYTES + WQ * WQ_INTS * 4 /*work queue*/ +
                                       TABLE_INTS * 4 + RED_BYTES + 80 + 16 + 512 /*token ids of the producer's unit, 16-byte aligned*/ + TS_BYTES;
     static_assert(NTOK % 16 == 0 && NTOK >= 16 && NTOK <= 128, "token tile");
@@ -337,8 +338,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 20 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last), [12..] s_filled
     // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
     int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 20) + 15) & ~uintptr_t(15));
-    float2* s_sx = reinterpret_cast<float2*>(s_g4 + 128);          // tokens-on-M: [NACC][128] products of token and weight scale
-    float* s_ts = reinterpret_cast<float*>(s_sx + C::NACC * 128);  // ... and [TSD][128] token scales on their way
+    float* s_ts = reinterpret_cast<float*>(s_g4 + 128);            // tokens-on-M: [TSD][TS_SLOT] scales of a K block
+    constexpr int NHELP = C::TOK_ON_M ? (G4 ? 2 : 1) : 0;          // ... and the warps (2, 3) that fill it
 
     const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform for the compiler too
     const long long t_entry = clock64();
@@ -363,9 +364,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, C::EMPTY_COUNT); }
-        for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1 + C::NHELP); mbar_init(bar_tempty + 8 * b, C::NPW); }
+        for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1 + NHELP); mbar_init(bar_tempty + 8 * b, C::NPW); }
         for (int g = 0; g < 4; ++g) mbar_init(bar_red + 8 * g, C::TOK_ON_M ? C::NGRP : 4);
-        for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + C::NHELP + C::NPW); }
+        for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + NHELP + C::NPW); }
         mbar_fence_init();
         tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_b0);
         if (!G1) tma_prefetch_desc(&tm_b1);
@@ -794,75 +795,63 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         }
         __syncwarp();
     } else if constexpr (C::TOK_ON_M) {
-        // ------------------------------------------------------------ scale warps (2 and 3), tokens on M: for every K block
-        // the products token scale x weight scale of both weight tiles, one float2 per token row, into the buffer that
-        // belongs to the block's accumulator.  They count in on the same barrier as the MMA commit, so the promotion
-        // warps - the busiest role: ~600 cycles of TMEM loads and FMAs per 128 x 256 block with two warps per scheduler
-        // and nothing to hide a wait behind - have one wait and one shared-memory load per block instead of three
-        // global loads (their latency under load is longer than a block) and the products.
-        // Token scales travel through a ring of asynchronous copies TSD - 1 blocks ahead (a thread reads back only what it
-        // copied itself); the weight scales of 64 K blocks sit in the lanes and are handed out by shuffles.
-        const int h = threadIdx.x - 64;                // this thread: rows h and h + 64
-        const uint32_t ring = smem_u32(s_ts + h);
-        int ab = 0; uint32_t aphase = 0;
-        bool ok = true;
-        int n_item = 0;
-        WorkItem wi;
+        // ------------------------------------------------------------ scale warp (2; with gathered rows 2 and 3), tokens on M:
+        // token and weight scales of every K block into the block's slot of the ring, by asynchronous copies TS_AHEAD blocks
+        // ahead.  It counts in on the barrier of the MMAs' commit when the scales of the block AND of the one after it have
+        // landed, so that the promotion warps read a block's scales while they fold the one before: a shared-memory load
+        // beside full-rate MMAs takes ~150 cycles, and nothing in a promotion warp hides that in front of a block's first
+        // FMA (in a loop without TMA fills: 526 cycles per block with the load ahead, 650 with the load in place).
+        if (warp - 2 < NHELP) {
+            const int h = threadIdx.x - 64;            // gathered rows: this thread copies the scales of rows h and h + 64
+            int ab = 0; uint32_t aphase = 0;
+            bool ok = true;
+            int n_item = 0, blk = 0;
+            WorkItem wi;
 #pragma unroll 1
-        while (ok && wq_fetch(n_item++, wi, ok)) {
-            const int gb = wi.gb, ge = wi.ge;
-            const Unit un = wi.un;
-            // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist)
-            const int srow0 = un.mt * (p.unit_rows >> 7);
-            const int srow1 = min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
-            const float* ws0 = p.w_scale + ((size_t)un.e * p.scale_rows + srow0) * p.KB;
-            const float* ws1 = p.w_scale + ((size_t)un.e * p.scale_rows + srow1) * p.KB;
-            const float* ts[2];
-            const int ts_stride = G4 ? p.ts_stride : p.rows_cap;
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                ts[r] = p.b_scale + (size_t)un.row0 + h + 64 * r;
+            while (ok && wq_fetch(n_item++, wi, ok)) {
+                const int gb = wi.gb, ge = wi.ge;
+                const Unit un = wi.un;
+                // weight-scale rows of the unit's two tiles (the second one of GEMM2's last unit may not exist): lanes 0 and 1
+                const int srow0 = un.mt * (p.unit_rows >> 7);
+                const int srow = lane == 0 ? srow0 : min(srow0 + (p.gate_offset >> 7), p.scale_rows - 1);
+                const float* const ws = p.w_scale + ((size_t)un.e * p.scale_rows + srow) * p.KB;
+                const float* ts[2] = {p.b_scale + (size_t)un.row0 + 4 * lane, nullptr};
                 if (G4) {
-                    const int tok = __ldg(p.g4_row_token + un.row0 + h + 64 * r);
-                    ts[r] = p.g4_scale + (tok >= 0 && tok < p.g4_T ? (size_t)tok * (unsigned)p.g4_tok_stride : 0);   // any finite scale for a row of zeros
-                }
-            }
-            auto ts_fetch = [&](int kb) {
-                if (kb < ge) {                          // nothing past the piece's end: no copy is left in flight for the next piece
-                    const uint32_t dst = ring + (uint32_t)((kb % C::TSD) * 128 * 4);
-                    cp_async4(dst, ts[0] + (size_t)kb * ts_stride);
-                    cp_async4(dst + 64 * 4, ts[1] + (size_t)kb * ts_stride);
-                }
-                cp_async_commit();
-            };
-            float wl[2][2];                             // [weight tile][K blocks 0-31 / 32-63 of the window]
-            auto ws_window = [&](int kb) {
-                const int k0 = min((kb & ~63) + lane, p.KB - 1), k1 = min((kb & ~63) + 32 + lane, p.KB - 1);
-                wl[0][0] = __ldg(ws0 + k0); wl[0][1] = __ldg(ws0 + k1);
-                wl[1][0] = __ldg(ws1 + k0); wl[1][1] = __ldg(ws1 + k1);
-            };
 #pragma unroll
-            for (int i = 0; i < C::TSD - 1; ++i) ts_fetch(gb + i);
-            ws_window(gb);
+                    for (int r = 0; r < 2; ++r) {
+                        const int tok = __ldg(p.g4_row_token + un.row0 + h + 64 * r);
+                        ts[r] = p.g4_scale + (tok >= 0 && tok < p.g4_T ? (size_t)tok * (unsigned)p.g4_tok_stride : 0);   // any finite scale for a row of zeros
+                    }
+                }
+                auto fetch = [&](int kb, int b) {
+                    if (kb < ge) {                      // nothing past the piece's end: no copy is left in flight for the next piece
+                        const uint32_t slot = smem_u32(s_ts) + (uint32_t)(b % C::TSD) * (C::TS_SLOT * 4);
+                        if (G4) {
+                            cp_async4(slot + 4 * h, ts[0] + (size_t)kb * p.ts_stride);
+                            cp_async4(slot + 4 * h + 64 * 4, ts[1] + (size_t)kb * p.ts_stride);
+                        } else {
+                            cp_async16(slot + 16 * lane, ts[0] + (size_t)kb * p.rows_cap);      // segments start at multiples of 16 rows
+                        }
+                        if (warp == 2 && lane < 2) cp_async4(slot + 128 * 4 + 4 * lane, ws + kb);
+                    }
+                    cp_async_commit();
+                };
 #pragma unroll 1
-            for (int kb = gb; kb < ge; ++kb) {
-                if ((kb & 63) == 0 && kb > gb) ws_window(kb);
-                const bool hi = (kb & 32) != 0;
-                const float sw0 = __shfl_sync(0xFFFFFFFFu, hi ? wl[0][1] : wl[0][0], kb & 31);
-                const float sw1 = __shfl_sync(0xFFFFFFFFu, hi ? wl[1][1] : wl[1][0], kb & 31);
-                cp_async_wait<C::TSD - 2>();
-                const float* slot = s_ts + (kb % C::TSD) * 128 + h;
-                const float t0 = slot[0], t1 = slot[64];
-                ts_fetch(kb + C::TSD - 1);              // into the slot read one block ago
-                if (!mbar_wait_warp(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
-                s_sx[ab * 128 + h] = make_float2(t0 * sw0, t0 * sw1);
-                s_sx[ab * 128 + h + 64] = make_float2(t1 * sw0, t1 * sw1);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_tfull + 8 * ab);
-                if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
+                for (int i = 0; i < C::TS_AHEAD; ++i) fetch(gb + i, blk + i);
+#pragma unroll 1
+                for (int kb = gb; kb < ge; ++kb) {
+                    cp_async_wait<C::TS_AHEAD - 2>();  // the scales of blocks kb and kb + 1 have landed
+                    __syncwarp();
+                    // the accumulator is free: block blk - NACC has been folded, and nobody reads its slot or one before it
+                    if (!mbar_wait_warp(bar_tempty + 8 * ab, aphase ^ 1, p.status, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+                    if (lane == 0) mbar_arrive(bar_tfull + 8 * ab);
+                    fetch(kb + C::TS_AHEAD, blk + C::TS_AHEAD);
+                    ++blk;
+                    if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
+                }
             }
+            cp_async_wait<0>();
         }
-        cp_async_wait<0>();
     } else if (FUSE) {
         // ------------------------------------------------------------ warps 2-3, fused combine: zero rows of the
         // tokens that have no pair on this rank (nobody else writes them)
@@ -899,6 +888,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         int rbuf = 0;                                  // half of s_red the next epilogue uses
         bool ok = true, seen = false;
         int ng = 0, nu = 0;
+        int blk = 0;                                   // tokens on M: K blocks folded so far
         float acc[C::NACCUM][C::NC];
 
         // the warps that share my_red meet (bounded); false = gave up
@@ -927,6 +917,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
                     if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
                 }
+                blk += ge - gb;
                 continue;
             }
 #pragma unroll
@@ -953,13 +944,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             if constexpr (C::TOK_ON_M) {
                 // Tokens on M: this thread's row is one token, so a K block folds with ONE scalar per weight tile.  The
                 // block is read as four 32-column chunks, two tcgen05.ld in flight per wait (a wait covers every
-                // outstanding load).  The loop is rotated: the next block's first two chunks are requested while the
-                // last two of this block are folded, so the hand-off wait, the scale load and the TMEM latency of a
-                // block's start hide behind those FMAs; the buffer goes back as soon as its last load has completed.
+                // outstanding load).  256 cycles of packed FMAs per block and scheduler; what the loop adds to them are round
+                // trips to shared memory beside full-rate MMAs (~100-150 cycles each), so a block has as few in a row as
+                // possible: its scales were read during the block before, the barrier is looked at between the last two
+                // chunks (the answer is there when they are folded), waits neither vote nor branch, and the buffer goes
+                // back before those two chunks are folded.  GEMM1 of 14107 tokens 925 k -> 815 k cycles against a loop that
+                // waits, votes and reads its scales in place (under the power limit 690 -> 645 us).
                 constexpr int QC = 32, QPA = C::NC / QC, NQ = C::NACCUM * QPA;
                 static_assert(C::NC % QC == 0 && NQ == 4 && C::KPB == 1, "tokens-on-M chunking");
                 float stg[2][QC];
-                float2 sx2;
                 uint32_t tbuf;
                 auto qload = [&](int q) { tmem_ld_chunk<QC>(tbuf + (q / QPA) * NTOK + (q % QPA) * QC, stg[q & 1]); };
                 auto qfold = [&](int q, float sx) {
@@ -972,32 +965,41 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         ac[i] = r0.x; ac[i + 1] = r0.y;
                     }
                 };
-                auto acquire = [&]() -> bool {
-                    if (!mbar_wait_warp(bar_tfull + 8 * ab, aphase, p.status, ERR_WAIT_TMEM_FULL)) return false;
-                    tc_fence_after();
-                    sx2 = s_sx[ab * 128 + m];              // written by the scale warps before they counted in
-                    tbuf = tmem_base + tlane + ab * C::BUFCOLS + c0;
-                    return true;
-                };
-                if (!acquire()) { ok = false; break; }
+                uint32_t landed = 1;
+                bool ready = false;
+                mbar_wait_flag(bar_tfull + 8 * ab, aphase, landed);
+                const float* slot = s_ts + (blk % C::TSD) * C::TS_SLOT;
+                float t = slot[m];
+                float2 w2 = *reinterpret_cast<const float2*>(slot + 128);
                 if (ptid == 0 && !seen) { stamp(TR_PROMO_FIRST); seen = true; }
-                qload(0); qload(1);
 #pragma unroll 1
                 for (int n = ge - gb; n > 0; --n) {
+                    if (!ready) mbar_wait_flag(bar_tfull + 8 * ab, aphase, landed);
                     if (ptid == 0) klog_put(2, ng);
+                    const float2 sx2 = make_float2(t * w2.x, t * w2.y);
+                    tc_fence_after();
+                    tbuf = tmem_base + tlane + ab * C::BUFCOLS + c0;
+                    qload(0); qload(1);
                     tmem_wait_ld();
                     qfold(0, sx2.x); qload(2);
                     qfold(1, sx2.x); qload(3);
+                    ++blk;
+                    slot = s_ts + (blk % C::TSD) * C::TS_SLOT;         // the next block's (behind the last one nobody uses them)
+                    t = slot[m];
+                    w2 = *reinterpret_cast<const float2*>(slot + 128);
                     tmem_wait_ld();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
                     if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
-                    const float s_hi = sx2.y;
-                    if (n > 1 && !acquire()) { ok = false; break; }
-                    qfold(2, s_hi); if (n > 1) qload(0);
-                    qfold(3, s_hi); if (n > 1) qload(1);
+                    qfold(2, sx2.y);
+                    ready = mbar_test(bar_tfull + 8 * ab, aphase);
+                    qfold(3, sx2.y);
                     if (ptid == 0) klog_put(3, ng++);
+                }
+                if (!__all_sync(0xFFFFFFFFu, landed != 0)) {
+                    if (lane == 0) atomicCAS(p.status, 0, ERR_WAIT_TMEM_FULL);
+                    ok = false; break;
                 }
             } else
 #pragma unroll 1

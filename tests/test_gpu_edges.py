@@ -192,6 +192,22 @@ def test_part_full_128_token_tiles(counts, hidden, intermediate):
     assert bool((outs[1][few:].float() == 0).all())
 
 
+@pytest.mark.parametrize("tma_gather", [False, True])
+@pytest.mark.parametrize("hidden,intermediate", [(128, 128), (384, 640), (1152, 1024)])
+def test_scale_ring_of_the_128_token_tiles(hidden, intermediate, tma_gather):
+    """K blocks fewer than the scales travel ahead (1, 3, 5), just as many as the ring holds (8) and one more (9)."""
+    import dataclasses
+    from justgoal_b200 import MoELayer
+    shape = dataclasses.replace(I.TINY_DS, hidden=hidden, intermediate=intermediate)
+    d = I.make_inputs(shape, 300, seed=23)
+    layer = MoELayer(shape)
+    layer.set_token_tile(128)
+    layer.set_tma_gather(tma_gather)
+    layer.workspace(300).fill_(0xFF)
+    _, out = _forward(shape, d, layer)
+    _check_output(shape, d, out)
+
+
 @pytest.mark.parametrize("T", [2369, 9473])
 def test_combine_batches(T):
     """Token counts from which a combine CTA takes two / eight tokens at a time, with a ragged last batch."""
