@@ -19,9 +19,9 @@
 // Schedule: K is cut into GROUPS of KPB 128-K blocks (one TMEM hand-off per group).  The kernel is
 // persistent.  Units are numbered so that the token tiles of one (expert, row tiles) are adjacent.  Every CTA
 // first runs floor(U / grid) WHOLE units, round-robin (CTAs that run at the same time work on adjacent units, so
-// a weight tile shared by several token tiles comes from HBM once).  The remaining U mod grid units are cut
-// along K into CHUNKS of a few K blocks, and the CTAs CLAIM those chunks one at a time from a counter in global
-// memory: SMs do not stream at the same rate under full load, and a CTA that finishes early simply takes more
+// a weight tile shared by several token tiles comes from HBM once).  The remaining U mod grid units stay
+// whole or are cut along K into CHUNKS, whichever is done sooner (size_chunks), and the CTAs CLAIM them one at a time from a counter in
+// global memory: SMs do not stream at the same rate under full load, and a CTA that finishes early simply takes more
 // chunks (with equal static shares the finish times of the CTAs spread by 7-10 % of the kernel).  Every chunk stores
 // its fp32 partial to its own slot and counts itself in; whoever arrives last adds the slots in a fixed order (results
 // are bit-identical from run to run) and runs the epilogue, so nobody waits.  GEMM1 with narrow tiles cuts the remaining
@@ -177,14 +177,10 @@ struct GemmCfg {
     // stage has landed and release the stage at once, instead of holding it until the group is folded
     static constexpr bool EARLY_SCALES = KPB * NC <= 32 && NPW < 16;
     static constexpr int SLOT_FLOATS = NACCUM * NC * NPT;  // = NACCUM * 128 * NTOK
-    // SMALLEST number of K blocks per claimed chunk of a split unit (the producer enlarges the chunks when there are
-    // many left-over units: about two chunks per CTA).  A chunk streams CHUNK_BLOCKS * 32 KB of weights and leaves
-    // 1 KB * NTOK of partial sums: at NTOK / 8 blocks the partial sums are one eighth of the chunk's traffic for every
-    // tile width, and a narrow tile's last few units spread over many CTAs (decode GEMM2: four left-over units become
-    // 32 chunks instead of 8)
+    // SMALLEST number of K blocks per claimed chunk of a split unit: what the partial-sum area is sized for (the producer decides how
+    // many chunks there are).  A chunk streams CHUNK_BLOCKS * 32 KB of weights and leaves 1 KB * NTOK of partial sums.
     static constexpr int CHUNK_BLOCKS = NTOK / 8;
     static constexpr int CHUNK_GROUPS = (CHUNK_BLOCKS / KPB) < 1 ? 1 : (CHUNK_BLOCKS / KPB);
-    static constexpr int CHUNKS_PER_CTA = 2;               // measured: 4 and 6 cost 2-10 us more at every decode size
     // GEMM1 with narrow tiles has few, long units (decode: 256 units of 3.7 MB for 148 CTAs): there the units left
     // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA.  A range touches at most two units, so a
     // CTA stores at most one partial sum, which it makes before anything else; the piece that ends a unit runs after the CTA's
@@ -494,19 +490,32 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 ++n_item;
                 return true;
             };
-            // Left-over units: `pieces` chunks of chunk_groups groups each, claimed one at a time.  How many per CTA: enough
-            // that the CTAs' finish times even out, few enough that the partial sums stay small traffic - every chunk leaves
-            // 1 KB * NTOK.  (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
+            // Left-over units: `pieces` chunks of chunk_groups groups each, claimed one at a time (1: the units stay whole).  Of up to
+            // MOST pieces the number for which the CTA that claims most is done first, by the length of its chunks and by what a
+            // piece costs beside it, in K blocks: storing its partial sums, the meetings, the restart of the pipeline - 14-17 k
+            // cycles measured for a full 128-token tile, hence 12 blocks there, 6 where most of the tile's rows are empty, 8 for narrow
+            // tiles - and one more for every slot that the last piece adds up.  The rule before this one, about two chunks per CTA
+            // whatever a piece costs, made the tail longer than the whole units it cut up.  us, before / now: 32 of 256 experts 4
+            // tokens 59.7 / 53.1, 16: 94.6 / 89.3, 128: 161.9 / 154.5, 257: 197.7 / 191, 901: 278 / 264; 16 experts of the 4096-wide
+            // shape 16: 57.1 / 50.5, 128: 82.7 / 73.3, 2048: 129 / 112; K of 64 blocks in GEMM2 (4 experts, 5120 x 8192) 16: 57.2 / 49,
+            // 400: 150 / 125.  The line is not sharp: 6 / 12 / 18 blocks with 128-token tiles 320 tokens 221 / 227 / 231, 600: 238 / 247 /
+            // 248, 2048: 343 / 338 / 338; 4 / 8 / 12 / 20 blocks with narrow tiles differ by less than 1 us but for the shape of 64 blocks
+            // (64 tokens 89.0 / 87.9 / 88.0 / 88.3) and 4 tokens of a 4096 x 4096 shape (40.0 / 40.0 / 40.0 / 44.4).
+            // (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
             volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, [1] pieces
             bool sized = false;
             auto size_chunks = [&]() {
+                constexpr int PIECE_COST = C::TOK_ON_M ? (PART ? 6 : 12) : 8, MOST = 8;
+                static_assert(MOST <= MAX_PIECES, "arrivals of a split unit");
                 const int tail_units = total_units - sched_U0;
-                int chunk_groups = C::CHUNK_GROUPS;
-                if (tail_units > 0) {
-                    const int per_unit = (C::CHUNKS_PER_CTA * (int)gridDim.x + tail_units - 1) / tail_units;
-                    chunk_groups = max(chunk_groups, (NG + per_unit - 1) / per_unit);
+                const int slots = (int)gridDim.x * ((NG + C::CHUNK_GROUPS - 1) / C::CHUNK_GROUPS);           // what sk_partial holds
+                int best = NG * C::KPB, chunk_groups = NG;
+#pragma unroll 1
+                for (int n = 2; n <= MOST && tail_units * n <= slots; ++n) {
+                    const int len = (NG + n - 1) / n;
+                    const int cost = (tail_units * n + (int)gridDim.x - 1) / (int)gridDim.x * (len * C::KPB + PIECE_COST + n);
+                    if (cost < best) { best = cost; chunk_groups = len; }
                 }
-                chunk_groups = max(chunk_groups, (NG + MAX_PIECES - 1) / MAX_PIECES);
                 if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = (NG + chunk_groups - 1) / chunk_groups; }
                 __syncwarp();
                 sized = true;
@@ -525,7 +534,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             // that ends a unit and waits itself (T=257: 214 -> 209 us against running it before the whole units).
             int t_lo = 0, t_hi = 0, t_unit = 0;
             const int flat = (total_units - sched_U0) * NG;
-            const int parts = min(flat, (int)gridDim.x);
+            // Up to half as many units as CTAs are cut into the same number of pieces each, more into one range per CTA.  (A range
+            // that crosses a unit's end leaves its CTA two pieces.  One range per CTA / equal pieces / equal pieces or whole units
+            // whatever their number, us: 2 tokens 39.8 / 38.9 / 38.9, 16: 89.8 / 88.0 / 88.0, 24: 100.4 / 99.3 / 99.8, 128: 161.4 / 160.4 /
+            // 160.0, 200: 185.1 / 186.1 / 182.2; 16 experts of the 4096-wide shape 64: 66.2 / 63.6 / 63.6; 8 of a 4096 x 4096 shape 128:
+            // 83.5 / 83.7 / 85.7.)
+            const int parts = 2 * (total_units - sched_U0) > (int)gridDim.x || flat == 0
+                                  ? min(flat, (int)gridDim.x)
+                                  : (total_units - sched_U0) * min(NG, (int)gridDim.x / (total_units - sched_U0));
             if (C::STATIC_TAIL && (int)blockIdx.x < parts) {
                 t_lo = range_start((int)blockIdx.x, flat, parts); t_hi = range_start((int)blockIdx.x + 1, flat, parts);
                 t_unit = t_lo / NG;
