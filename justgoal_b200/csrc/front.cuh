@@ -200,12 +200,16 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const Fro
     // arrives there only after its stores (the fence before the arrival orders them).  The next kernel (GEMM1) reads
     // the ST_ROUTED word of the head before this kernel has completed, so CTA 0 lets it start only when the zeros
     // are visible.
-    if (blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < fp.head_vec; i += FRONT_THREADS) fp.head[i] = make_uint4(0u, 0u, 0u, 0u);
+    // Its upper half does that, and alone lets GEMM1 start, while the lower half routes.
+    constexpr int HALF = FRONT_THREADS / 2;
+    if (blockIdx.x != 0) {
+        pdl_launch();
+    } else if (threadIdx.x >= HALF) {
+        for (int i = threadIdx.x - HALF; i < fp.head_vec; i += HALF) fp.head[i] = make_uint4(0u, 0u, 0u, 0u);
         __threadfence();
-        __syncthreads();
+        asm volatile("bar.sync 2, %0;" ::"n"(HALF) : "memory");
+        pdl_launch();
     }
-    pdl_launch();
     for (int t = (int)blockIdx.x + (int)gridDim.x * warp; t < rp.T; t += (int)gridDim.x * (FRONT_THREADS / 32)) {
         int sel_id; float w;
         route_token<VPT, MODE>(rp, t, lane, sel_id, w);
