@@ -613,13 +613,13 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     if (slot_out) so = *slot_out;
     if (out_kind == OUT_BF16)
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_BF16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
     else if (out_kind == OUT_F16)
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
     else
         CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F32>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, so));
+                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
     CU_TRY(prof_mark(h, 6, st));
     if (h->prof_slots) ++h->prof_calls;
     return 0;

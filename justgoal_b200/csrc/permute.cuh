@@ -336,29 +336,29 @@ template <int OUT>
 __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__ y, const int32_t* __restrict__ topk_idx,
                                                       const int32_t* __restrict__ pair_row, const float* __restrict__ row_w,
                                                       void* __restrict__ out, int T, int H, int top_k, int pair_stride,
-                                                      int local_offset, int num_local, int batch, const SlotOut slots) {
+                                                      int local_offset, int num_local, int batch, int tables_done, const SlotOut slots) {
     __shared__ int s_rows[2][COMBINE_BATCH][8];
     __shared__ float s_w[2][COMBINE_BATCH][8];
     __shared__ int s_n[2][COMBINE_BATCH];          // rows of the token, -1: nothing to write
-    pdl_wait();
-    pdl_launch();
     // gridDim.y CTAs share a token's columns (few tokens: more CTAs in flight, shorter latency chain per CTA)
     const int h_per = ((H / 8 + gridDim.y - 1) / gridDim.y) * 8;
     const int h_lo = blockIdx.y * h_per, h_hi = min(H, h_lo + h_per);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int buf = 0;
-    for (int t0 = blockIdx.x * batch; t0 < T; t0 += gridDim.x * batch, buf ^= 1) {
-        // (two buffers: a warp is at most one meeting ahead of the others, which still read the other one)
+    // Rows and weights of the batch from token t0 on.  They were written by a kernel that had completed before any CTA of GEMM2 let
+    // this kernel start (tables_done; not the SM-pair kernels), so the first batch is looked up, past L1, while GEMM2 still
+    // runs: with a few tokens the three dependent loads are a good part of this kernel.
+    auto look_up = [&](int t0) {
         if (warp < batch) {
             // lanes 0..top_k-1 fetch their pair in parallel; rows are ranked by row index (= expert order)
             const int t = t0 + warp;
             int r = NO_ROW;
             bool present = t < T;
             if (t < T && lane < top_k) {
-                const int id = topk_idx[(size_t)t * pair_stride + lane];
+                const int id = __ldcg(topk_idx + (size_t)t * pair_stride + lane);
                 const int le = id - local_offset;
                 if (OUT == OUT_F16 && slots.cap > 0 && lane == 0 && id < 0) present = false;
-                if (le >= 0 && le < num_local) r = pair_row[(size_t)t * top_k + lane];
+                if (le >= 0 && le < num_local) r = __ldcg(pair_row + (size_t)t * top_k + lane);
             }
             int rank = 0;
             for (int j = 0; j < 8; ++j) {
@@ -366,9 +366,17 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
                 rank += (rj < r) || (rj == r && j < lane);
             }
             const unsigned have = __ballot_sync(0xFFFFFFFFu, r != NO_ROW);
-            if (r != NO_ROW) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldg(row_w + r); }
+            if (r != NO_ROW) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldcg(row_w + r); }
             if (lane == 0) s_n[buf][warp] = present ? __popc(have) : -1;
         }
+    };
+    const int t_first = blockIdx.x * batch;
+    if (tables_done) look_up(t_first);
+    pdl_wait();
+    pdl_launch();
+    for (int t0 = t_first; t0 < T; t0 += gridDim.x * batch, buf ^= 1) {
+        // (two buffers: a warp is at most one meeting ahead of the others, which still read the other one)
+        if (!tables_done || t0 != t_first) look_up(t0);
         __syncthreads();
         const int nt = min(batch, T - t0);
         for (int b = 0; b < nt; ++b) {
