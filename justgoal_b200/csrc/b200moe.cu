@@ -558,6 +558,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         // rows: the producer reads row_token for its first loads, which the front end writes after the announcement.
         g1.routed = status + ST_ROUTED; g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
     }
+    g1.tables_done = !fused_front && !pairs && !g4;      // the gather lets GEMM1 start only after the permutation has completed
     g1.sk_count = reinterpret_cast<int*>(ws + L.sk_count);
     g1.sk_partial = reinterpret_cast<float*>(ws + L.sk_partial);
     g1.trace = reinterpret_cast<long long*>(ws + L.trace);

@@ -87,7 +87,7 @@ struct GemmParams {
     // histogram and scan as the front end) and the producer streams the first weight tiles while the front end still
     // permutes and gathers; the token rows are loaded after the front end has completed.
     const int* routed;
-    int tables_done;              // GEMM2: the expert tables are complete before this kernel can start (see the kernel's prologue)
+    int tables_done;              // the expert tables are complete before this kernel can start (see the kernel's prologue)
     const int32_t* topk_idx;      // [n_pairs] global expert ids (pair_stride == top_k on this path)
     int n_pairs, local_offset;
     // GEMM1 with 128-token tiles reading the token rows straight from the caller's activations (no gather copy), else
@@ -404,8 +404,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     // Expert tables, by the control warps (the others get decoded work items).  They are written by the kernels before this
     // one; three forms:
     //   GEMM1 after the fused front end (p.routed): built here from the routing result, while the front end still runs;
-    //   GEMM2 (p.tables_done): written by a kernel that had completed before any CTA of the kernel before this one let
-    //     this kernel start - read past L1, without a wait;
+    //   GEMM2, and GEMM1 behind a gather (p.tables_done): written by a kernel that had completed before any CTA of the kernel
+    //     before this one let this kernel start - read past L1, without a wait;
     //   otherwise: read after the wait for the kernel before this one.
     // In the first two forms the producer streams weights before that wait.
     const int ctid = threadIdx.x;
@@ -441,7 +441,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         ctrl_sync();
         if (warp == 0) scan_counts(s_cnt, p.num_local, NTOK, p.rows_cap, s_row0, s_tiles, nullptr, lane);
     } else {
-        early = !G1 && p.tables_done;
+        early = !G4 && p.tables_done;
         if (!early) pdl_wait();
 #pragma unroll 1
         for (int i = ctid; i <= p.num_local; i += 128) {
