@@ -612,15 +612,14 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     SlotOut so;
     memset(&so, 0, sizeof(so));            // cap == 0: rows go to `out`
     if (slot_out) so = *slot_out;
-    if (out_kind == OUT_BF16)
-        CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_BF16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
-    else if (out_kind == OUT_F16)
-        CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F16>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
-    else
-        CU_TRY(launch_k(PDL_COMBINE, combine_kernel<OUT_F32>, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx,
-                        (const int32_t*)pair_row, (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so));
+    const bool wide = cgrid.y == 1;
+    auto combine = [&](auto kernel) {
+        return launch_k(PDL_COMBINE, kernel, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx, (const int32_t*)pair_row,
+                        (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so);
+    };
+    if (out_kind == OUT_BF16) CU_TRY(wide ? combine(combine_kernel<OUT_BF16, true>) : combine(combine_kernel<OUT_BF16, false>));
+    else if (out_kind == OUT_F16) CU_TRY(wide ? combine(combine_kernel<OUT_F16, true>) : combine(combine_kernel<OUT_F16, false>));
+    else CU_TRY(wide ? combine(combine_kernel<OUT_F32, true>) : combine(combine_kernel<OUT_F32, false>));
     CU_TRY(prof_mark(h, 6, st));
     if (h->prof_slots) ++h->prof_calls;
     return 0;

@@ -331,8 +331,11 @@ __device__ __forceinline__ void combine_four_tokens(const __half* y, const int32
 // under load), then all warps stream the rows of the batch without meeting again.  With one token at a time and eight
 // CTAs per SM the chains alone were the kernel's time (14107 tokens: 100 us for 340 MB); few tokens keep batch = 1 and
 // share a token's columns over gridDim.y CTAs instead.
+// WIDE: a thread takes 16 columns at a time, 32 bytes of every row, instead of 8: twice the bytes in flight where a token has only one or
+// two rows.  8192 tokens over 256 experts 214 -> 190 us, 14107 tokens 116 -> 104 (stage times).  Not where four CTAs share a token's columns:
+// half the threads would be left without any (128 tokens 8.3 -> 10.2 us).
 constexpr int COMBINE_BATCH = 8;
-template <int OUT>
+template <int OUT, bool WIDE>
 __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__ y, const int32_t* __restrict__ topk_idx,
                                                       const int32_t* __restrict__ pair_row, const float* __restrict__ row_w,
                                                       void* __restrict__ out, int T, int H, int top_k, int pair_stride,
@@ -387,26 +390,40 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
                 const int r = t / slots.cap;
                 out_row = static_cast<uint16_t*>(slots.back.p[r]) + ((size_t)slots.my_rank * slots.cap + (t - r * slots.cap)) * H;
             }
-            for (int h = h_lo + threadIdx.x * 8; h < h_hi; h += blockDim.x * 8) {
-                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            // (H is a multiple of 128 and the rows of y start at 256-byte boundaries; the caller's rows are written 16 bytes at a time)
+            constexpr int V = WIDE ? 16 : 8;
+            for (int h = h_lo + threadIdx.x * V; h < h_hi; h += blockDim.x * V) {
+                float acc[V];
+#pragma unroll
+                for (int i = 0; i < V; ++i) acc[i] = 0.f;
                 // four rows' loads in flight at a time (the rows are independent; the sum order stays j = 0, 1, ...)
                 for (int j0 = 0; j0 < n; j0 += 4) {
-                    uint4 v[4];
+                    uint4 v[4][V / 8];
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (j0 + u < n) v[u] = __ldcs(reinterpret_cast<const uint4*>(y + (size_t)s_rows[buf][b][j0 + u] * H + h));
+                        if (j0 + u < n) {
+                            const __half* src = y + (size_t)s_rows[buf][b][j0 + u] * H + h;
+                            if constexpr (WIDE) ld_global_v8(src, reinterpret_cast<uint32_t*>(v[u]));
+                            else v[u][0] = __ldcs(reinterpret_cast<const uint4*>(src));
+                        }
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
-                        if (j0 + u < n) fma8_f16(acc, v[u], s_w[buf][b][j0 + u]);
+                        if (j0 + u < n) {
+#pragma unroll
+                            for (int q = 0; q < V / 8; ++q) fma8_f16(acc + 8 * q, v[u][q], s_w[buf][b][j0 + u]);
+                        }
                 }
-                if (OUT == OUT_BF16) {
-                    *reinterpret_cast<uint4*>(out_row + h) = pack8_bf16(acc);
-                } else if (OUT == OUT_F16) {
-                    *reinterpret_cast<uint4*>(out_row + h) = pack8_f16(acc);
-                } else {
-                    float* o = reinterpret_cast<float*>(out) + (size_t)t * H + h;
-                    *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                    *reinterpret_cast<float4*>(o + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+#pragma unroll
+                for (int q = 0; q < V; q += 8) {
+                    if (OUT == OUT_BF16) {
+                        *reinterpret_cast<uint4*>(out_row + h + q) = pack8_bf16(acc + q);
+                    } else if (OUT == OUT_F16) {
+                        *reinterpret_cast<uint4*>(out_row + h + q) = pack8_f16(acc + q);
+                    } else {
+                        float* o = reinterpret_cast<float*>(out) + (size_t)t * H + h + q;
+                        *reinterpret_cast<float4*>(o) = make_float4(acc[q], acc[q + 1], acc[q + 2], acc[q + 3]);
+                        *reinterpret_cast<float4*>(o + 4) = make_float4(acc[q + 4], acc[q + 5], acc[q + 6], acc[q + 7]);
+                    }
                 }
             }
         }
