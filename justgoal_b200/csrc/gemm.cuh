@@ -34,7 +34,8 @@
 // launch.  GEMM1's CTAs are resident while it runs; when it announces the routing result they build the expert tables
 // themselves and the producer streams the first weight tiles before the front end has completed - only the token
 // side of those stages waits for it.  GEMM2 does the same with the tables the front end left (GemmParams::tables_done), as
-// soon as its CTA has an SM: the first weights travel under the tail of GEMM1 (T=64: 132 -> 130 us, T=7: 72 -> 70 us).
+// soon as its CTA has an SM: the first weights travel under the tail of GEMM1 (T=64: 132 -> 130 us, T=7: 72 -> 70 us).  So does
+// GEMM1 behind a separate gather: its tables come from the permutation before that.
 // Optionally (FUSE) GEMM2's epilogue also does the combine.
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (whole warps, one elected lane issues),
@@ -152,9 +153,8 @@ struct GemmCfg {
     // and a K block took 750 ns instead of 570 ns.
     static constexpr int NTB = NACC;                        // TMEM hand-off barriers per direction
     // promotion warps: 4 (one per TMEM lane quarter) for narrow tiles, 8 (two column groups) from 64 tokens.
-    // With tokens on M the fold of a 128 x 256 fp32 block takes ~630 cycles: two tcgen05.ld round trips of
-    // 2 x 32 columns per thread (128 accumulator registers leave 64 for staging); 16 warps do not fit the
-    // register pool with a deeper staging and measured no gain with the same depth.
+    // With tokens on M a thread folds 2 x 64 columns of a block through 64 staging registers; 16 warps of half the columns do not
+    // fit the register pool with the same staging and were slower with half of it (700 against 526 cycles per block, no fills).
     static constexpr int NPW = NTOK >= 64 ? 8 : 4;
     static constexpr int NGRP = NPW / 4;                   // column groups (a group = 4 warps = all 128 lanes)
     static constexpr int NPT = 32 * NPW;                   // promotion threads
@@ -182,7 +182,7 @@ struct GemmCfg {
     static constexpr int CHUNK_BLOCKS = NTOK / 8;
     static constexpr int CHUNK_GROUPS = (CHUNK_BLOCKS / KPB) < 1 ? 1 : (CHUNK_BLOCKS / KPB);
     // GEMM1 with narrow tiles has few, long units (decode: 256 units of 3.7 MB for 148 CTAs): there the units left
-    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA.  A range touches at most two units, so a
+    // over after the whole rounds are cut into EQUAL contiguous ranges, one per CTA (or, few units, equal pieces of whole units).  A range touches at most two units, so a
     // CTA stores at most one partial sum, which it makes before anything else; the piece that ends a unit runs after the CTA's
     // whole units and waits for those other pieces (claimed chunks measured 5-15 us slower: every one of them costs a partial sum, late in the kernel).
     // Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
