@@ -88,8 +88,10 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait whose answer is data, not control flow: `ok` becomes 0 when the wait gave up, and then every later wait with
-// the same `ok` gives up after its first try.  For loops that cannot afford a vote and a branch per step (40 cycles of a
-// promotion warp's ~450): the caller looks at `ok` once per piece of work, votes there and records the error.
+// the same `ok` gives up after two tries.  For loops that cannot afford a vote and a branch per step (40 cycles of a
+// promotion warp's ~450): the caller looks at `ok` once per piece of work, votes there and records the error.  It answers per
+// lane, and lanes may leave it apart in time: a `__syncwarp` has to stand between it (or mbar_test) and anything that takes the
+// whole warp.
 __device__ __forceinline__ void mbar_wait_flag(uint32_t bar, uint32_t parity, uint32_t& ok) {
     const unsigned long long limit = ok ? WAIT_LIMIT_NS : 0ull;
     asm volatile(

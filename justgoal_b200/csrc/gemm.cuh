@@ -991,6 +991,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #pragma unroll 1
                 for (int n = ge - gb; n > 0; --n) {
                     if (!ready) mbar_wait_flag(bar_tfull + 8 * ab, aphase, landed);
+                    __syncwarp();          // each lane has waited by itself, and the loads below take the whole warp (.aligned)
                     if (ptid == 0) klog_put(2, ng);
                     const float2 sx2 = make_float2(t * w2.x, t * w2.y);
                     tc_fence_after();
@@ -1006,7 +1007,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     tmem_wait_ld();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(bar_tempty + 8 * ab);
+                    if (lane == 0 && landed) mbar_arrive(bar_tempty + 8 * ab);     // never a buffer whose wait gave up
                     if (++ab == C::NACC) { ab = 0; aphase ^= 1; }
                     qfold(2, sx2.y);
                     ready = mbar_test(bar_tfull + 8 * ab, aphase);

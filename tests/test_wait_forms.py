@@ -20,11 +20,48 @@ def _code(name):
     return re.sub(r"//[^\n]*", "", src)
 
 
+VOTED = {"mbar_wait_warp", "mbar_wait_both"}
+
+
+def _waits(code):
+    """Every call that looks at an mbarrier, whatever it is named."""
+    return set(re.findall(r"\b(mbar_\w*(?:wait|test)\w*)\s*\(", code))
+
+
+def _promotion_loop(code):
+    """The tokens-on-M branch of the promotion warps: (before the block loop, the loop, behind it up to the other branch)."""
+    branch = code[code.index("auto qload ="):]
+    branch = branch[:branch.index("} else\n")]
+    head, rest = branch.split("for (int n = ge - gb; n > 0; --n) {")
+    end = rest.index("\n                }\n")
+    return head, rest[:end], rest[end:]
+
+
 @pytest.mark.parametrize("name", ["gemm.cuh", "gemm_pair.cuh"])
 def test_warp_wide_roles_wait_with_a_vote(name):
     code = _code(name)
-    assert re.search(r"\bmbar_wait_warp\s*\(", code)
-    assert not re.search(r"\bmbar_wait\s*\(", code) and not re.search(r"\bmbar_try_wait\s*\(", code)
+    assert "mbar_wait_warp" in _waits(code)
+    if name == "gemm.cuh":
+        for part in _promotion_loop(code):
+            assert code.count(part) == 1
+            code = code.replace(part, "")
+    assert _waits(code) <= VOTED
+    assert "try_wait" not in code and "test_wait" not in code          # no barrier is polled by hand either
+
+
+def test_lanes_that_waited_alone_meet_before_they_load():
+    head, loop, behind = _promotion_loop(_code("gemm.cuh"))
+    for part in (head, loop, behind):
+        assert _waits(part) <= {"mbar_wait_flag", "mbar_test"}
+    assert not re.search(r"\b(break|continue|return)\b", loop) and "qload(0)" not in head.split("};")[-1]
+    before_load = loop[:loop.index("qload(")]
+    assert before_load.rindex("mbar_wait_flag(") < before_load.rindex("__syncwarp();") < before_load.rindex("tc_fence_after();")
+    assert _waits(loop[loop.index("qload("):]) == {"mbar_test"}        # a look; what it says is acted on in front of the meeting
+    assert "mbar_test" not in _waits(before_load)
+    hand_backs = re.findall(r"if \(([^)]*)\) mbar_arrive\(bar_tempty", loop)
+    assert hand_backs == ["lane == 0 && landed"]
+    vote = behind.index("__all_sync(0xFFFFFFFFu, landed != 0)")
+    assert "ok = false; break;" in behind[vote:]
 
 
 def test_voted_forms_vote():
