@@ -604,7 +604,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         if (h->prof_slots) ++h->prof_calls;
         return 0;
     }
-    // tokens a combine CTA takes at a time: as many as leave every SM its eight CTAs
+    // tokens a combine CTA takes at a time: as many as leave eight CTAs per SM in the grid
     int batch = 1;
     while (batch < COMBINE_BATCH && T >= h->num_sms * 8 * batch * 2) batch *= 2;
     const int cgrid_need = (T + batch - 1) / batch;

@@ -328,9 +328,11 @@ __device__ __forceinline__ void combine_four_tokens(const __half* y, const int32
 }
 
 // A CTA takes `batch` (1..8) tokens at a time: warp w looks up token w's rows and weights (a chain of dependent loads, ~2 us
-// under load), then all warps stream the rows of the batch without meeting again.  With one token at a time and eight
-// CTAs per SM the chains alone were the kernel's time (14107 tokens: 100 us for 340 MB); few tokens keep batch = 1 and
-// share a token's columns over gridDim.y CTAs instead.
+// under load), then all warps stream the rows of the batch without meeting again.  With one token at a time
+// the chains alone were the kernel's time (14107 tokens: 100 us for 340 MB); few tokens keep batch = 1 and
+// share a token's columns over gridDim.y CTAs instead.  An SM holds four or five of these CTAs with eight columns a thread (48 to
+// 60 registers) and three with 16 (70); the grid of up to eight per SM evens out what the tokens' numbers of rows make uneven.
+// The look-up stands in the loop once (twice, before and in it: 8 to 9 registers more, and the fp16 form spilled).
 // WIDE: a thread takes 16 columns at a time, 32 bytes of every row, instead of 8: twice the bytes in flight where a token has only one or
 // two rows.  8192 tokens over 256 experts 214 -> 190 us, 14107 tokens 116 -> 104 (stage times).  Not where four CTAs share a token's columns:
 // half the threads would be left without any (128 tokens 8.3 -> 10.2 us).
@@ -348,10 +350,13 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
     const int h_lo = blockIdx.y * h_per, h_hi = min(H, h_lo + h_per);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int buf = 0;
-    // Rows and weights of the batch from token t0 on.  They were written by a kernel that had completed before any CTA of GEMM2 let
-    // this kernel start (tables_done; not the SM-pair kernels), so the first batch is looked up, past L1, while GEMM2 still
-    // runs: with a few tokens the three dependent loads are a good part of this kernel.
-    auto look_up = [&](int t0) {
+    const int t_first = blockIdx.x * batch;
+    if (!tables_done) pdl_wait();
+    for (int t0 = t_first; t0 < T; t0 += gridDim.x * batch, buf ^= 1) {
+        // Rows and weights of the batch.  (Two buffers: a warp is at most one meeting ahead of the others, which still read the
+        // other one.)  They were written by a kernel that had completed before any CTA of GEMM2 let this kernel start
+        // (tables_done; not the SM-pair kernels), so the first batch is looked up, past L1, while GEMM2 still runs: with a
+        // few tokens the three dependent loads are a good part of this kernel.
         if (warp < batch) {
             // lanes 0..top_k-1 fetch their pair in parallel; rows are ranked by row index (= expert order)
             const int t = t0 + warp;
@@ -372,14 +377,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
             if (r != NO_ROW) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldcg(row_w + r); }
             if (lane == 0) s_n[buf][warp] = present ? __popc(have) : -1;
         }
-    };
-    const int t_first = blockIdx.x * batch;
-    if (tables_done) look_up(t_first);
-    pdl_wait();
-    pdl_launch();
-    for (int t0 = t_first; t0 < T; t0 += gridDim.x * batch, buf ^= 1) {
-        // (two buffers: a warp is at most one meeting ahead of the others, which still read the other one)
-        if (!tables_done || t0 != t_first) look_up(t0);
+        if (t0 == t_first) { pdl_wait(); pdl_launch(); }
         __syncthreads();
         const int nt = min(batch, T - t0);
         for (int b = 0; b < nt; ++b) {

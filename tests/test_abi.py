@@ -40,3 +40,12 @@ def test_null_arguments_are_rejected_without_a_device():
     assert _lib.lib.b200moe_create(None, None) == -1
     assert _lib.lib.b200moe_destroy(None) == -1
     assert _lib.lib.b200moe_workspace_bytes(None, 4, None) == -1
+
+
+def test_kernels_do_not_spill(tmp_path, capfd):
+    """Only the optional SM-pair kernels may (their register split leaves the control warps short)."""
+    from justgoal_b200 import build
+    build.build(force=True, verbose=True, out=str(tmp_path / "lib.so"))
+    report = re.findall(r"Function properties for (\S+)\n\s+(\d+) bytes stack frame, (\d+) bytes spill stores", capfd.readouterr().err)
+    assert sum("combine_kernel" in name for name, _, _ in report) >= 6 and sum("gemm_kernel" in name for name, _, _ in report) >= 14
+    assert [name for name, _, spilled in report if int(spilled) and "gemm_pair_kernel" not in name] == []
