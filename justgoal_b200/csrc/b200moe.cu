@@ -612,7 +612,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     SlotOut so;
     memset(&so, 0, sizeof(so));            // cap == 0: rows go to `out`
     if (slot_out) so = *slot_out;
-    const bool wide = cgrid.y == 1;
+    const bool wide = combine_is_wide(T, H);
     auto combine = [&](auto kernel) {
         return launch_k(PDL_COMBINE, kernel, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx, (const int32_t*)pair_row,
                         (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so);

@@ -333,10 +333,23 @@ __device__ __forceinline__ void combine_four_tokens(const __half* y, const int32
 // share a token's columns over gridDim.y CTAs instead.  An SM holds four or five of these CTAs with eight columns a thread (48 to
 // 60 registers) and three with 16 (70); the grid of up to eight per SM evens out what the tokens' numbers of rows make uneven.
 // The look-up stands in the loop once (twice, before and in it: 8 to 9 registers more, and the fp16 form spilled).
-// WIDE: a thread takes 16 columns at a time, 32 bytes of every row, instead of 8: twice the bytes in flight where a token has only one or
-// two rows.  8192 tokens over 256 experts 214 -> 190 us, 14107 tokens 116 -> 104 (stage times).  Not where four CTAs share a token's columns:
-// half the threads would be left without any (128 tokens 8.3 -> 10.2 us).
+// WIDE: a thread takes 16 columns at a time, 32 bytes of every row, instead of 8: twice the bytes in flight per thread, fewer
+// threads and CTAs.  For long calls of wide rows only, see combine_is_wide.
 constexpr int COMBINE_BATCH = 8;
+
+// Where 16 columns a thread are the better form: rows that 256 threads cover in half as many turns as with eight columns (a
+// partly empty turn costs a whole one), and at least two of them; and enough tokens that three CTAs per SM instead of four or five
+// do not matter.  Stage times, us, eight / 16 columns, of 64 experts with 8 rows per token (all local) | with one (8 local):
+// hidden 7168 1000 tokens 25.6 / 30.1 | 12.3 / 12.3, 2000: 49.1 / 53.2 | 17.3 / 19.4, 3000: 73.6 / 73.7 | 20.5 / 22.5, 4000: 98.6 / 93.5
+// | 28.6 / 28.7, 8000: 199 / 173 | 55.6 / 52.6, 14000: 324 / 286 | 85.7 / 81.1; 8192 (4 turns / 2) 2000: 54.0 / 57.4 | 18.3 / 20.5, 4000:
+// 108 / 104 | 30.7 / 32.7, 14000: 360 / 322 | 92.8 / 88.1; 6144 (3 / 2) 4000: 80.0 / 85.8 | 23.6 / 26.6, 14000: 273 / 256 | 71.2 / 74.2; 5120
+// (3 / 2) 4000: 71.7 / 79.7 | 20.6 / 24.5, 14000: 234 / 235 | 63.7 / 67.8; 4096 (2 / 1) 2000: 28.7 / 34.4 | 12.4 / 14.3, 14000: 184 / 171 |
+// 49.1 / 49.2; 2048 (1 / 1) 4000: 28.7 / 40.9 | 14.3 / 15.9; 1024 14000: 49.2 / 83.9 | 19.7 / 24.7.
+__host__ __device__ constexpr bool combine_is_wide(int T, int H) {
+    const int turns8 = (H + 256 * 8 - 1) / (256 * 8), turns16 = (H + 256 * 16 - 1) / (256 * 16);
+    return T >= 4000 && turns16 >= 2 && 2 * turns16 == turns8;
+}
+
 template <int OUT, bool WIDE>
 __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__ y, const int32_t* __restrict__ topk_idx,
                                                       const int32_t* __restrict__ pair_row, const float* __restrict__ row_w,

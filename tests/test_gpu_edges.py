@@ -217,6 +217,66 @@ def test_combine_batches(T):
     _check_output(shape, d, out)
 
 
+def _kernel_names(fn):
+    """Names of the kernel nodes of the CUDA graph that captures one call of fn, in the order of the graph's node list."""
+    import ctypes as C
+
+    class Params(C.Structure):                         # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", C.c_void_p), ("dims", C.c_uint * 7), ("kernel_params", C.c_void_p), ("extra", C.c_void_p),
+                    ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    fn()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        fn()
+    cu, graph, n, kind = C.CDLL("libcuda.so.1"), C.c_void_p(g.raw_cuda_graph()), C.c_size_t(0), C.c_int(0)
+    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
+    names = []
+    for node in nodes:
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value:
+            continue
+        p, name = Params(), C.c_char_p()
+        assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+        if p.func:
+            assert cu.cuFuncGetName(C.byref(name), C.c_void_p(p.func)) == 0
+        else:
+            assert cu.cuKernelGetName(C.byref(name), C.c_void_p(p.kern)) == 0
+        names.append(name.value.decode())
+    return names
+
+
+@pytest.mark.parametrize("T,hidden,wide", [(257, 1024, False), (300, 7168, False), (4000, 2048, False), (4000, 4096, False),
+                                           (4000, 6144, False), (3999, 6272, False), (4000, 6272, True), (9473, 7168, True)])
+def test_columns_of_a_combine_thread(T, hidden, wide):
+    """16 columns a thread only where that is the faster form, on both sides of the rule's lines; the last columns of 6272 are a
+    quarter of a turn.  Every output kind against the oracle, tokens without a local expert among them."""
+    import dataclasses
+    from justgoal_b200 import MoELayer
+    shape = dataclasses.replace(I.TINY_RENORM, hidden=hidden, num_local_experts=2)
+    d = I.make_inputs(shape, T, seed=3)
+    layer = MoELayer(shape)
+    layer.workspace(T).fill_(0xFF)
+    _, out = _forward(shape, d, layer)
+    _check_output(shape, d, out)
+    dc = util.to_cuda(d)
+    idx, w = layer.route(dc["routing_logits"], dc["routing_bias"], dc["routed_scaling_factor"])
+    args = (idx, w, dc["hidden_states"], dc["hidden_states_scale"], dc["gemm1_weights"], dc["gemm1_weights_scale"],
+            dc["gemm2_weights"], dc["gemm2_weights_scale"], int(d["local_expert_offset"]))
+    f32 = layer.forward_routed(*args)
+    assert torch.equal(out.view(torch.int16), f32.to(torch.bfloat16).view(torch.int16))
+    h16 = layer.forward_routed(*args, out_dtype=torch.float16)
+    torch.cuda.synchronize()
+    assert layer.status(T) == 0
+    assert torch.equal(h16.view(torch.int16), f32.to(torch.float16).view(torch.int16))
+    assert bool((out.float() == 0).all(dim=1).any())
+    names = [n for n in _kernel_names(lambda: layer.forward(*util.op_args(dc))) if "combine_kernel" in n]
+    assert len(names) == 1 and ("combine_kernelILi1ELb%dEE" % wide) in names[0], names
+
+
 def test_tma_gathered_token_rows_give_the_same_bits():
     """Optional form of GEMM1 for 128-token tiles: the token rows come from hidden_states by four-row TMA gathers
     through the token-of-row table instead of from a gathered copy (no gather launch).  Ragged last tiles, padding
