@@ -1,6 +1,9 @@
 """Ragged and boundary cases of the CUDA path against the oracle: one token, the first size past the
 fused small-T front end, several permutation slices, every token colliding on the same experts,
 ragged last tiles.  Output tolerance as stated for the operator; integer structures exact."""
+import dataclasses
+import functools
+
 import pytest
 import torch
 
@@ -215,6 +218,93 @@ def test_combine_batches(T):
     d = I.make_inputs(shape, T, seed=T)
     layer, out = _forward(shape, d)
     _check_output(shape, d, out)
+
+
+def _pieces(units, KB, kpb, slots_per_cta, piece_cost, grid):
+    """Pieces of a left-over unit, as gemm.cuh's size_chunks states the rule."""
+    tail, groups = units % grid, -(-KB // kpb)
+    best, length = groups * kpb, groups
+    for n in range(2, 9):
+        if tail * n > grid * slots_per_cta:
+            break
+        size = -(-groups // n)
+        cost = -(-tail * n // grid) * (size * kpb + piece_cost + n)
+        if cost < best:
+            best, length = cost, size
+    return -(-groups // length)
+
+
+@functools.lru_cache(maxsize=1)
+def _wide_intermediate():
+    """32 K blocks in GEMM2: enough for every tile family to cut left-over units."""
+    shape = dataclasses.replace(I.TINY_DS, hidden=1024, intermediate=4096, num_local_experts=8)
+    return shape, I.make_inputs(shape, 1100, seed=29)
+
+
+@pytest.mark.parametrize("tiles", [1, 3, 5, 7, 12, 25])
+@pytest.mark.parametrize("tile,full", [(16, False), (32, False), (64, False), (128, False), (128, True)])
+def test_left_over_units_cut_along_k(tile, full, tiles):
+    """Claimed pieces of GEMM2 in every tile family (both instances of the 128-token tiles), GEMM1's static tails beside them on
+    both sides of half a grid of left-over units, without and with whole units before (32 units of GEMM1 and 4 of GEMM2 per tile; with 12
+    tiles the partial-sum slots end the search for 128-token tiles, with 25 GEMM2's units stay whole).  The oracle's result, the same bits from a second call on a
+    poisoned workspace, and as many pieces as the rule says."""
+    from justgoal_b200 import MoELayer, _lib
+    shape, d = _wide_intermediate()
+    spread = [tiles // 8 + (e < tiles % 8) for e in range(8)]
+    rows = [k * tile - (3 * e + 1) % (tile - 1) if k else 0 for e, k in enumerate(spread)]
+    used = max(rows)
+    T = 1100 if full else used
+    assert (T * shape.top_k / shape.num_experts >= 128) == full
+    idx = torch.full((T, shape.top_k), shape.num_experts - 1, dtype=torch.int32)          # not on this rank
+    for e, n in enumerate(rows):
+        idx[:n, e] = e
+    w = torch.rand(T, shape.top_k, generator=torch.Generator().manual_seed(5)) + 0.1
+    x, sc = d["hidden_states"][:T], d["hidden_states_scale"][:, :T].contiguous()
+    wts = [d[n] for n in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")]
+    want, _, _ = O.run_experts(x[:used], sc[:, :used].contiguous(), *wts, w[:used], idx[:used].long(), 0, shape.num_experts)
+    layer = MoELayer(shape)
+    layer.set_token_tile(tile)
+    args = [t.cuda() for t in (idx, w, x, sc, *wts)]
+    grid, outs = _lib.lib.b200moe_num_sms(), []
+    for _ in range(2):
+        layer.workspace(T).fill_(0xFF)
+        outs.append(layer.forward_routed(*args, 0, out_dtype=torch.bfloat16).clone())
+        torch.cuda.synchronize()
+        assert layer.status(T) == 0
+        arrived = layer.view(T, "sk_count", torch.int32, (2, 4 * grid + 4)).cpu()
+        units = 4 * tiles
+        want_pieces = _pieces(units, 32, 2 if tile == 16 else 1, {16: 16, 32: 8, 64: 4, 128: 2}[tile],
+                              8 if tile < 128 else 12 if full else 6, grid)
+        assert (want_pieces > 1) == (tiles < 25)
+        first = arrived[1, :4 * (units % grid):4]                  # of the first group of warps of every left-over unit
+        assert set((first & 0xFF).tolist()) == {want_pieces if want_pieces > 1 else 0}
+        if tile <= 32:
+            tail = 32 * tiles % grid
+            assert bool((arrived[0, :4 * tail:4] > 0).all())
+    rep = O.compare_output(outs[0][:used], want.to(torch.bfloat16), util.ATOL, util.RTOL)
+    assert rep["finite"] and rep["fail_frac"] == 0.0, rep
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+    assert bool((outs[0][used:].float() == 0).all())
+
+
+@pytest.mark.parametrize("tile,T", [(16, 20), (16, 100), (32, 180), (64, 400)])
+def test_fused_combine_behind_cut_units(tile, T):
+    """The fused combine when GEMM2's units are cut: the warps that add a unit's pieces up deliver its rows."""
+    from justgoal_b200 import MoELayer, _lib
+    shape, d = _wide_intermediate()
+    d = {k: v[:T] if k in ("routing_logits", "hidden_states") else v for k, v in d.items()}
+    d["hidden_states_scale"] = d["hidden_states_scale"][:, :T].contiguous()
+    layer = MoELayer(shape)
+    layer.set_token_tile(tile)
+    _, separate = _forward(shape, d, layer)
+    _check_output(shape, d, separate)
+    layer.set_fused_combine(True)
+    for _ in range(2):
+        layer.workspace(T).fill_(0xFF)
+        _, fused = _forward(shape, d, layer)
+        assert torch.equal(fused.view(torch.int16), separate.view(torch.int16))
+        grid = _lib.lib.b200moe_num_sms()
+        assert int(layer.view(T, "sk_count", torch.int32, (2, 4 * grid + 4))[1, 0]) & 0xFF > 1
 
 
 def _kernel_names(fn):
