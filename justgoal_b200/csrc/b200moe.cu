@@ -90,11 +90,12 @@ int pdl_mask() {
     return v;
 }
 
-// With many thousands of tokens the early-resident dependents slow the front kernels and GEMM1 down, so only GEMM2 and the
-// combine overlap there; up to 2048 tokens all launches do.  A shape-only decision.  Overlap of GEMM2 and the combine alone /
-// of all launches, us: 16 experts of the 4096-wide shape 513 tokens 102 / 92, 2048 139 / 131, 4096 191 / 183, 8192 318 / 312; 32 of
-// 256 experts 513 tokens 262 / 253, 2048 350 / 349, 4096 530 / 530, 6000 697 / 717, 12000 1155 / 1188; 128 of 256 experts 2048
-// tokens 1182 / 1198, 6000 2071 / 2179.  (Between 2048 and 4096 tokens a few experts would still gain.)
+// Up to 2048 tokens all launches overlap, beyond that GEMM2 and the combine only: with GEMM1 behind a gather that it could not
+// stream weights under, early-resident dependents slowed calls of many thousands of tokens down by 2 to 5 %.  A shape-only decision.
+// With the present kernels (GEMM1 streams its first weights there too) that is no longer so, and the line costs 1 to 5 % beyond it.
+// Overlap of GEMM2 and the combine alone / of all launches, us: 16 experts of the 4096-wide shape 513 tokens 102 / 90, 2048
+// 135 / 121, 3000 170 / 162, 4096 204 / 201, 8192 322 / 308; 32 of 256 experts 513 tokens 240 / 222, 2048 314 / 294, 4096 408 / 387, 6000
+// 492 / 478, 12000 768 / 748; 128 of 256 experts 2048 tokens 1330 / 1299, 4000 1704 / 1699, 6000 2324 / 2289.
 thread_local int g_call_pdl = 0;
 inline void set_call_pdl(int num_tokens) { g_call_pdl = num_tokens <= 2048 ? pdl_mask() : pdl_mask() & (PDL_GEMM2 | PDL_COMBINE); }
 
@@ -140,17 +141,22 @@ int num_slices(const b200moe_config& c, int T) {
     return n <= 0 ? 1 : (int)((n + SLICE_PAIRS - 1) / SLICE_PAIRS);
 }
 
-// Measured on the DeepSeek-V3 shape with 32 local experts (microseconds per forward, tile 16 / 32 / 64 / 128):
-// T=64 149/160/202/187, T=192 211/230/244/225, T=256 230/214/244/227, T=320 247/244/245/219, T=512 308/284/292/279,
-// T=1024 482/372/353/301, T=1792 -/-/463/372.  The 16-token tile wins while an expert sees fewer rows than the tile
-// holds; from about nine expected rows per expert the 128-token tile (tokens on M, one N = 256 MMA per K step) is
-// ahead of every narrower one although most of its rows are padding - the step is bound by the weight stream, and
-// the narrow tiles' weights-on-M MMAs are short of shared-memory bandwidth from 64 columns on.  The 64-token tile is
-// never the best choice; it stays available through b200moe_set_token_tile.
+// The 16-token tile wins while an expert sees fewer rows than the tile holds; above that the 128-token tile (tokens on M, one
+// N = 256 MMA per K step) is ahead of every narrower one although most of its rows are padding - the step is bound by the
+// weight stream, and the narrow tiles' weights-on-M MMAs are short of shared-memory bandwidth from 64 columns on.  The 64-token
+// tile is never the best choice; it stays available through b200moe_set_token_tile.
+// us per forward with the present kernels, tile 16 / 32 / 64 / 128, by expected rows per expert (r); one routing per count:
+//   32 of 256 experts       r=4 159/163/198/164, 6 160/176/201/180, 7 172/177/209/181, 8 180/174/211/185, 9 177/170/203/183, 10 188/197/219/194,
+//                           12 201/204/248/207, 16 233/227/253/217, 32 359/307/309/229, 56 500/399/357/278
+//   128 of 256 experts      r=6 665/728/880/632, 7 709/764/913/681, 8 774/753/947/681, 10 863/868/971/701
+//   16 of the 4096-wide     r=4 65/71/82/80, 7 67/72/84/81, 9 69/75/87/86, 10 69/75/88/85, 16 78/77/89/86
+//   8 of a 4096 x 4096      r=4 75/82/102/90, 8 76/83/101/90, 9 78/82/103/91, 12 95/90/107/96, 16 99/90/110/96
+// The lines at 7 and 9 rows were drawn with earlier kernels on the first of these shapes and are a compromise now: the best change
+// from narrow to 128 comes at about 14 rows there, at about 5 with many units (128 experts; the narrow tiles lose 12 to 18 % at 6 to
+// 9) and above 16 with few (where the 128-token tile is 20 % behind at 10).  The number of units should enter; it does not yet.
 // The estimate is that of a forward that routes itself.  Every token of forward_routed has a local expert, so an expert sees
-// more rows than estimated (DeepSeek-V3 routing, 32 local experts: twice as many), and calls of 150 to 350 tokens run a tile
-// that is up to 11 % slower than the best one there (32 local, tile 16 / 32 / 128: 200 tokens 238 / 228 / 235 us, 288 tokens
-// 287 / 267 / 249; 128 local, 350 tokens 928 / 795 / 751).
+// more rows than estimated (DeepSeek-V3 routing, 32 local experts: twice as many), and calls of 150 to 290 tokens run a slower
+// tile than they could (32 local, tile 16 / 32 / 128: 150 tokens 229 / 215 / 212 us, 200: 250 / 245 / 217, 288: 287 / 274 / 222).
 int pick_token_tile(const b200moe_ctx* h, int T) {
     if (h->token_tile) return h->token_tile;
     const b200moe_config& c = h->cfg;
@@ -161,10 +167,12 @@ int pick_token_tile(const b200moe_ctx* h, int T) {
 }
 
 // 128-token tiles: do most tiles hold fewer than 128 rows?  Below one tile's worth of expected rows per expert they do, and
-// the kernels that leave empty row quarters out (gemm.cuh, PART) are ahead or level; above it full tiles dominate and the
-// extra path costs a little.  Without / with PART, us, by rows per expert: 16 experts of the 4096-wide shape 32: 93.9 / 92.4, 64:
-// 98.4 / 98.3, 100: 105.0 / 106.3, 128: 132.7 / 133.5, 200: 171 / 173, 400: 271 / 277; 32 of 256 experts 32: 278 / 274, 80: 426 / 398,
-// 128: 533 / 557, 256: 885 / 916, 512: 1502 / 1605.
+// the kernels that leave empty row quarters out (gemm.cuh, PART) are ahead or level.  Above it full tiles dominate; the extra path
+// cost 2 to 7 % there with the promotion loop before the present one and costs nothing measurable with it.  Without / with PART, us, by
+// rows per expert: 16 experts of the 4096-wide shape 16: 93.6 / 88.5, 32: 94.7 / 91.9, 64: 102.3 / 100.4, 100: 108.9 / 110.0, 128: 123.8 /
+// 124.0, 200: 165.9 / 166.0, 400: 268.5 / 264.1; 32 of 256 experts 32: 254.0 / 251.7, 80: 326.5 / 325.8, 128: 396.7 / 391.4, 256: 589.2 /
+// 588.0, 512: 972.8 / 960.6; 128 of 256 experts 64: 1313 / 1299, 128: 1802 / 1792, 192: 2288 / 2275; 8 of a 4096 x 4096 shape 16: 100.3 /
+// 100.7, 100: 148.8 / 144.6, 200: 202 / 196.  (The two instances also cut left-over units by different costs, see size_chunks.)
 bool tiles_mostly_part_full(const b200moe_config& c, int T) {
     return (double)T * c.top_k / c.num_experts < 128.0;
 }
@@ -340,8 +348,8 @@ cudaError_t launch_gemm_pair(int grid, cudaStream_t st, const CUtensorMap& w, co
     return cudaLaunchKernelEx(&cfg, gemm_pair_kernel<G1>, w, b0, b1, p);
 }
 
-// Full token tiles run on SM pairs when B200MOE_PAIR=1.  Off by default: 8192 tokens over 256 experts 7.04 against 5.43 ms,
-// 4096 skewed tokens 992 against 792 us, 2048 tokens of the 4096-wide shape 171 against 132 us.  The pair kernels have neither
+// Full token tiles run on SM pairs when B200MOE_PAIR=1.  Off by default: 8192 tokens over 256 experts 7.64 against 4.93 ms,
+// 4096 skewed tokens 943 against 635 us, 2048 tokens of the 4096-wide shape 182 against 117 us.  The pair kernels have neither
 // the scale ring and the promotion loop of gemm.cuh nor its row boxes, and an odd tile of an expert runs as a pair.
 bool use_pairs(const b200moe_ctx* h, int ntok) {
     static int v = -1;

@@ -494,7 +494,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             // MOST pieces the number for which the CTA that claims most is done first, by the length of its chunks and by what a
             // piece costs beside it, in K blocks: storing its partial sums, the meetings, the restart of the pipeline - 14-17 k
             // cycles measured for a full 128-token tile, hence 12 blocks there, 6 where most of the tile's rows are empty, 8 for narrow
-            // tiles - and one more for every slot that the last piece adds up.  The rule before this one, about two chunks per CTA
+            // tiles - and one more for every slot that the last piece adds up.  (6 or 12 goes by the instance, not by the tile: a full
+            // tile of a call whose tiles are mostly part full is charged half of what it costs.)  The rule before this one, about two chunks per CTA
             // whatever a piece costs, made the tail longer than the whole units it cut up.  us, before / now: 32 of 256 experts 4
             // tokens 59.7 / 53.1, 16: 94.6 / 89.3, 128: 161.9 / 154.5, 257: 197.7 / 191, 901: 278 / 264; 16 experts of the 4096-wide
             // shape 16: 57.1 / 50.5, 128: 82.7 / 73.3, 2048: 129 / 112; K of 64 blocks in GEMM2 (4 experts, 5120 x 8192) 16: 57.2 / 49,
@@ -963,8 +964,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 // outstanding load).  256 cycles of packed FMAs per block and scheduler; what the loop adds to them are round
                 // trips to shared memory beside full-rate MMAs (~100-150 cycles each), so a block has as few in a row as
                 // possible: its scales were read during the block before, the barrier is looked at between the last two
-                // chunks (the answer is there when they are folded), waits neither vote nor branch, and the buffer goes
-                // back before those two chunks are folded.  GEMM1 of 14107 tokens 925 k -> 815 k cycles against a loop that
+                // chunks (the answer is there when they are folded), waits do not vote (the lanes meet behind them and vote
+                // once per piece), and the buffer goes back before those two chunks are folded.  GEMM1 of 14107 tokens 925 k -> 815 k cycles against a loop that
                 // waits, votes and reads its scales in place (under the power limit 690 -> 645 us).
                 constexpr int QC = 32, QPA = C::NC / QC, NQ = C::NACCUM * QPA;
                 static_assert(C::NC % QC == 0 && NQ == 4 && C::KPB == 1, "tokens-on-M chunking");
