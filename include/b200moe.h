@@ -95,8 +95,8 @@ typedef struct b200moe_ws_layout {
 } b200moe_ws_layout;
 
 /* Create / destroy a layer handle on the CURRENT device.  Does one-time kernel attribute
- * setup and allocates 64 bytes of device memory (two words at which the CTAs of the fused
- * front end meet; no later call allocates).  Replaces the one-time setup block of the reference
+ * setup and allocates 64 bytes of device memory (the counts of the one-launch front ends; no
+ * later call allocates).  Replaces the one-time setup block of the reference
  * launcher (KF94/kernel.cu:5355-5402) and `moe_init` (SF1/kernel.py:40-44).
  * Calls that use one handle must be ordered with respect to each other on the GPU (one stream,
  * or events between streams): b200moe_forward calls for up to 128 tokens share those two words.

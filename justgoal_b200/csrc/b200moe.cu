@@ -52,7 +52,7 @@ struct b200moe_ctx {
     int token_tile;            // b200moe_set_token_tile: 0 = chosen from the token count, else 16 / 32 / 64 / 128
     int tma_gather;            // b200moe_set_tma_gather: GEMM1 (128-token tiles) gathers its token rows by TMA; default off
     int fuse_combine;          // b200moe_set_fused_combine: GEMM2 epilogue adds a token's rows up (narrow tiles); default off
-    int* d_sync;               // device, 64 bytes, zero between calls: the meeting words of the fused front end
+    int* d_sync;               // device, 64 bytes, zero between calls: the counts of the one-launch front ends
                                // (front.cuh).  One forward per handle may be in flight at a time.
     std::mutex map_mutex;
     MapKey map_key[MAP_SETS];
@@ -463,6 +463,19 @@ int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
     return 0;
 }
 
+// CTAs of the one-launch front ends: enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that
+// GEMM1 can start on most SMs while the front end runs.  32 / 64 CTAs, us: 1 token 18.6 / 18.7 (no local expert), 8 tokens 99.1 / 99.1, 16
+// tokens 112.8 / 112.5, 32 tokens 125.0 / 124.3, 33 tokens 124.2 / 123.9, 64 tokens 144.9 / 144.0, 128 tokens 180 / 179; 96 CTAs gained
+// nothing more.  Eight CTAs while about eight rows are to be copied (a routed call's tokens have two of a group's experts each), eight / 32:
+// 32 of 256 experts 2 tokens 38.4 / 39.0, 4: 61.4 / 62.7, 7: 67.6 / 68.8, 12: 83.8 / 82.6, 16: 84.3 / 83.5, routed 8: 79.8 / 76.8; 16 experts of the
+// 4096-wide shape 4: 37.7 / 38.0, 16: 55.6 / 54.9.  Neither line is sharp.
+int front_grid(const b200moe_ctx* h, int T, bool routed) {
+    const b200moe_config& c = h->cfg;
+    const double rows = (double)T * c.top_k * c.num_local_experts / c.num_experts * (routed ? 2 : 1);
+    const int want = rows <= 8.0 ? 8 : T <= 32 ? 32 : 64;
+    return h->num_sms < want ? h->num_sms : want;
+}
+
 // Everything after routing: permute -> gather -> GEMM1 -> GEMM2 -> combine.
 int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, const void* hidden,
                 const void* hidden_scale, const void* w13, const void* s13, const void* w2, const void* s2, int T,
@@ -515,12 +528,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         fp.hidden = static_cast<const uint8_t*>(hidden); fp.hscale = static_cast<const float*>(hidden_scale);
         fp.a_perm = a_perm; fp.a_scale_perm = a_scale; fp.H = H;
         fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = (int)(L.expert_row0 / 16);
-        // enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that GEMM1 can start on most
-        // SMs while this kernel runs.  32 / 64 CTAs, us: 1 token 18.6 / 18.7 (no local expert), 8 tokens 99.1 / 99.1, 16 tokens
-        // 112.8 / 112.5, 32 tokens 125.0 / 124.3, 33 tokens 124.2 / 123.9, 64 tokens 144.9 / 144.0, 128 tokens 180 / 179; 96 CTAs
-        // gained nothing more.  The line is not sharp: level up to 8 tokens, 0.3 us apart at 16, 0.7 us at 32.
-        const int want = T <= 32 ? 32 : 64;
-        const int fgrid = h->num_sms < want ? h->num_sms : want;
+        const int fgrid = front_grid(h, T, !route_in_front);
         if (route_in_front) CU_TRY(launch_front_route(c, fgrid, fp, *route_in_front, st));
         else CU_TRY(launch_k(PDL_PERMUTE, front_small_kernel, dim3(fgrid), dim3(FRONT_THREADS), 0, st, fp));
         CU_TRY(prof_mark(h, 2, st));
@@ -564,7 +572,10 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     if (fused_front && !pairs && wire_pitch == 0 && !g4) {
         // the fused front end announces the routing result; GEMM1 schedules itself from it (gemm.cuh).  Not with gathered
         // rows: the producer reads row_token for its first loads, which the front end writes after the announcement.
-        g1.routed = status + ST_ROUTED; g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
+        if (route_in_front) { g1.routed = h->d_sync; g1.routed_want = front_grid(h, T, !route_in_front); }
+        else { g1.routed = status + ST_ROUTED; g1.routed_want = 1; }
+        g1.copied = h->d_sync + 1; g1.copied_want = front_grid(h, T, !route_in_front);
+        g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
     }
     g1.tables_done = !fused_front && !pairs && !g4;      // the gather lets GEMM1 start only after the permutation has completed
     g1.sk_count = reinterpret_cast<int*>(ws + L.sk_count);
@@ -600,6 +611,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.tok_count = reinterpret_cast<int*>(ws + L.tok_count);
         g2.row_token = row_token; g2.pair_row = pair_row; g2.c_topk = topk_idx; g2.c_stride = pp.pair_stride;
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
+        g2.met = fused_front ? h->d_sync : nullptr;
     }
     if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
     else if (fuse) CU_TRY(launch_gemm_fused(ntok, h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
@@ -620,10 +632,11 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     SlotOut so;
     memset(&so, 0, sizeof(so));            // cap == 0: rows go to `out`
     if (slot_out) so = *slot_out;
+    int* const met = fused_front ? h->d_sync : nullptr;
     const bool wide = combine_is_wide(T, H);
     auto combine = [&](auto kernel) {
         return launch_k(PDL_COMBINE, kernel, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx, (const int32_t*)pair_row,
-                        (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, so);
+                        (const float*)row_w, out, T, H, c.top_k, pp.pair_stride, local_offset, El, batch, pairs ? 0 : 1, met, so);
     };
     if (out_kind == OUT_BF16) CU_TRY(wide ? combine(combine_kernel<OUT_BF16, true>) : combine(combine_kernel<OUT_BF16, false>));
     else if (out_kind == OUT_F16) CU_TRY(wide ? combine(combine_kernel<OUT_F16, true>) : combine(combine_kernel<OUT_F16, false>));
@@ -845,8 +858,10 @@ int b200moe_forward(b200moe_handle h, const void* logits, const void* bias, cons
     if (fused) rp.slices = nullptr;       // the fused front end routes and builds the histogram itself (one launch)
     else CU_TRY(do_route(c, rp, st));
     CU_TRY(prof_mark(h, 1, st));
-    return run_experts(h, rp.topk_idx, rp.topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
-                       OUT_BF16, ws, L, st, fused, nullptr, 0, fused ? &rp : nullptr, true);
+    rc = run_experts(h, rp.topk_idx, rp.topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
+                     OUT_BF16, ws, L, st, fused, nullptr, 0, fused ? &rp : nullptr, true);
+    if (rc && fused) cudaMemsetAsync(h->d_sync, 0, 64, st);       // the kernel that clears the front end's counts may not have been launched
+    return rc;
 }
 
 int b200moe_forward_routed(b200moe_handle h, const int32_t* topk_idx, const float* topk_w, const void* hidden,
@@ -879,8 +894,10 @@ int b200moe_forward_routed(b200moe_handle h, const int32_t* topk_idx, const floa
         CU_TRY(cudaGetLastError());
     }
     CU_TRY(prof_mark(h, 1, st));
-    return run_experts(h, topk_idx, topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
-                       output_kind, ws, L, st, fused);
+    rc = run_experts(h, topk_idx, topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
+                     output_kind, ws, L, st, fused);
+    if (rc && fused) cudaMemsetAsync(h->d_sync, 0, 64, st);       // as in b200moe_forward
+    return rc;
 }
 
 int b200moe_ep_row_bytes(b200moe_handle h, int* bytes) {

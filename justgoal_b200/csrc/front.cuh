@@ -9,8 +9,8 @@
 // among the same-expert pairs of its warp (match.any) plus the counts of the warps before it, which keeps the rows of
 // an expert in token order.  CTA 0 alone writes the tables that later kernels read (counts, row maps); all CTAs
 // derive identical values.  Same results as count_kernel + permute_kernel + gather_kernel (permute.cuh).
-// The next kernel (GEMM1) does not wait for this one to finish before it starts to work: see ST_ROUTED below and
-// GemmParams::routed.  The reference fuses the same stages for small batches
+// The next kernel (GEMM1) does not wait for this one to finish before it starts to work: it watches the two counts of
+// FrontParams::sync (behind front_small_kernel a flag, ST_ROUTED, and the second count), see GemmParams::routed.  The reference fuses the same stages for small batches
 // (kda05_reproduction_full_shape/fable-5.1/moe_fp8_fwd/<def>/fable51_moe_v94/kernel.cu:724-806) and issues its first
 // weight stages during the table build (its MOE_EARLY_W switch, same directory, main.py:50).
 #pragma once
@@ -30,34 +30,38 @@ struct FrontParams {
     uint8_t* a_perm;              // [rows_cap, H]
     float* a_scale_perm;          // [H/128, rows_cap]
     int H;
-    // `sync` (front_route_kernel only) is two words owned by the handle, zero between calls: [0] CTAs that have
-    // arrived at the meeting, [1] CTAs that have left it (the last one to leave clears both).  `head` is the part of
-    // the workspace that must be zero before the GEMMs run (status, split-unit counters), in 16-byte units: CTA 0
+    // `sync` is two words owned by the handle, zero between calls (the last kernel of the forward clears them): [0] CTAs that
+    // have arrived at the meeting (front_route_kernel only), [1] CTAs that have copied their share of the rows.  `head` is the part of the workspace that must be zero before the GEMMs run (status, split-unit counters), in 16-byte units: CTA 0
     // clears it, so the forward needs no memset in front of the kernel.
     int* sync;
     uint4* head;
     int head_vec;
 };
 
-// The body shared by the two entry kernels below.  FRESH: the routing result was written earlier in this same
-// launch by other CTAs (read it past L1).
+struct FrontShared {
+    int cnt[MAX_LOCAL];
+    uint32_t wcnt_words[FRONT_THREADS / 32][MAX_LOCAL / 4];       // bytes: pairs of expert e among the 32 pairs of warp w
+    int row0[MAX_LOCAL + 1], tiles[MAX_LOCAL + 1];
+    int row_token[FRONT_MAX_ROWS];
+};
+__device__ __forceinline__ void front_clear(FrontShared& s) {
+    constexpr int WORDS = MAX_LOCAL + FRONT_THREADS / 32 * (MAX_LOCAL / 4);         // cnt and the bytes behind it
+    static_assert(offsetof(FrontShared, row0) == WORDS * 4, "cleared in one go");
+    for (int i = threadIdx.x; i < WORDS; i += FRONT_THREADS) reinterpret_cast<uint32_t*>(&s)[i] = 0u;
+}
+
+// The body shared by the two entry kernels below, behind front_clear and a barrier.  FRESH: the routing result was written
+// earlier in this same launch by other CTAs (read it past L1).
 template <bool FRESH>
-__device__ __forceinline__ void front_body(const FrontParams& fp) {
-    __shared__ int s_cnt[MAX_LOCAL];
-    __shared__ int s_row0[MAX_LOCAL + 1];
-    __shared__ int s_tiles[MAX_LOCAL + 1];
-    __shared__ int s_row_token[FRONT_MAX_ROWS];
-    __shared__ uint8_t s_wcnt[FRONT_THREADS / 32][MAX_LOCAL];    // pairs of expert e among the 32 pairs of warp w
+__device__ __forceinline__ void front_body(const FrontParams& fp, FrontShared& s) {
+    int* const s_cnt = s.cnt; int* const s_row0 = s.row0; int* const s_tiles = s.tiles; int* const s_row_token = s.row_token;
+    auto s_wcnt = reinterpret_cast<uint8_t(*)[MAX_LOCAL]>(s.wcnt_words);
     static_assert(FRONT_THREADS >= FRONT_MAX_T * 8, "one thread per (token, expert) pair");
     const PlanParams& pp = fp.plan;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int T = pp.T, K = pp.top_k, El = pp.num_local;
     const bool publish = blockIdx.x == 0;
     const int n = T * K;
-
-    for (int i = tid; i < El; i += blockDim.x) s_cnt[i] = 0;
-    for (int i = tid; i < (int)(sizeof(s_wcnt) / 4); i += blockDim.x) reinterpret_cast<uint32_t*>(s_wcnt)[i] = 0u;
-    __syncthreads();
 
     // ---- this thread's pair (pair i = tid, token-major), the histogram of the local experts, and the pair's rank
     // among the pairs of the same expert inside its warp (stable: pair order)
@@ -151,6 +155,9 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
             }
         }
     }
+    // this CTA's rows are there for the GEMM that follows (GemmParams::copied)
+    __syncthreads();
+    if (tid == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(fp.sync + 1) : "memory");
 }
 
 
@@ -159,6 +166,9 @@ __device__ __forceinline__ void front_body(const FrontParams& fp) {
 // finds the word set and streams weights while the rows are copied.
 // Against count + permute + gather behind a memset: see the rule in b200moe_forward_routed.
 __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const FrontParams fp) {
+    __shared__ FrontShared s;
+    front_clear(s);
+    __syncthreads();
     pdl_wait();
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < fp.head_vec; i += FRONT_THREADS) fp.head[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -169,7 +179,7 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const Fro
         __syncthreads();
     }
     pdl_launch();
-    front_body<false>(fp);
+    front_body<false>(fp, s);
 }
 
 // Front end INCLUDING the routing (the operator's own forward for T <= FRONT_MAX_T): one launch, and nothing else on the
@@ -183,6 +193,7 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const Fro
 template <int VPT, int MODE>
 __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const FrontParams fp, const RouteParams rp) {
     __shared__ int s_go;
+    __shared__ FrontShared s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     {
         const size_t gtid = (size_t)blockIdx.x * FRONT_THREADS + threadIdx.x, gth = (size_t)gridDim.x * FRONT_THREADS;
@@ -195,11 +206,11 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const Fro
         pull(fp.hscale, (size_t)(fp.H >> 7) * rp.T * 4);
         if (rp.bias) pull(rp.bias, (size_t)rp.E * 2);
     }
+    front_clear(s);
     pdl_wait();
     // CTA 0 clears the head of the workspace.  Nothing flags an error in it before the meeting below, and CTA 0
-    // arrives there only after its stores (the fence before the arrival orders them).  The next kernel (GEMM1) reads
-    // the ST_ROUTED word of the head before this kernel has completed, so CTA 0 lets it start only when the zeros
-    // are visible.
+    // arrives there only after its stores (its arrival releases them): whoever has seen all arrivals, the next kernel (GEMM1)
+    // included, finds the zeros.
     // Its upper half does that, and alone lets GEMM1 start, while the lower half routes.
     constexpr int HALF = FRONT_THREADS / 2;
     if (blockIdx.x != 0) {
@@ -218,11 +229,18 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const Fro
             rp.topk_w[(size_t)t * rp.top_k + lane] = w;
         }
     }
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+        // The meeting: one count, which GEMM1 watches too.  It builds its schedule from the routing and starts to stream weights
+        // while this kernel still permutes and gathers.  Nobody clears the count before all that watch it are done: the last
+        // kernel of the forward does.  (A call that gave up leaves it dirty; b200moe_status() clears it when it reports the error.)
+        // An earlier form counted those that left as well, so that the last of them could clear both counts, and CTA 0 announced
+        // the routing in a word of its own: two more round trips to L2 in front of GEMM1's first load.  With this one, `copied` and
+        // eight CTAs up to eight tokens, start / now, us: 512-wide shape 1 token 20.6 / 19.1, 40: 22.4 / 21.6; 64 experts of
+        // 1024 x 512 1 token 25.7 / 24.9, 64: 42.8 / 41.5; 32 of 256 experts 1 token 17.1 / 16.5; where the weight stream is long the
+        // ring is full in time either way (64 tokens 131.7 / 131.9).
         int* const meet = fp.sync;
-        atomicAdd(meet, 1);
+        asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(meet) : "memory");
         int go = 1;
         const unsigned long long t0 = globaltimer_ns();
         for (uint32_t it = 1;; ++it) {
@@ -233,19 +251,11 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const Fro
                 atomicCAS(fp.plan.status + ST_ERR, 0, ERR_WAIT_GROUP); go = 0; break;
             }
         }
-        // every CTA that leaves has seen the full count: the last one to leave clears both words for the next call
-        // (a call that gave up leaves them dirty; b200moe_status() clears them when it reports the error)
-        if (go && atomicAdd(meet + 1, 1) == (int)gridDim.x - 1) { meet[0] = 0; meet[1] = 0; }
-        // every CTA fenced its routing results before it arrived and this thread has acquired the full count: whoever
-        // acquires the word below sees the routing of all tokens (GEMM1 builds its schedule from it and starts to
-        // stream weights while this kernel still permutes and gathers)
-        if (go && blockIdx.x == 0)
-            asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(fp.plan.status + ST_ROUTED), "r"(1) : "memory");
         s_go = go;
     }
     __syncthreads();
     if (!s_go) return;
-    front_body<true>(fp);
+    front_body<true>(fp, s);
 }
 
 }  // namespace b200moe

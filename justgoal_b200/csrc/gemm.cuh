@@ -83,11 +83,16 @@ struct GemmParams {
     long long* klog;      // [4][KLOG_N]: CTA 0's clock at its first KLOG_N K blocks: TMA issue, data seen by the
                           // MMA warp, group seen by the promotion warps, group folded (hand-back)
     long long* trace;     // [gridDim.x][TRACE_SLOTS]: slot 0 = %globaltimer at entry, others = SM clocks since entry
-    // GEMM1 after the fused front end (small token counts), else null: the front end sets *routed to 1 when the routing
-    // result of all tokens is visible.  The CTAs then build the expert tables themselves from topk_idx (the same
-    // histogram and scan as the front end) and the producer streams the first weight tiles while the front end still
-    // permutes and gathers; the token rows are loaded after the front end has completed.
+    // GEMM1 after a one-launch front end (small token counts), else null: the routing result of all tokens is visible when
+    // *routed has reached routed_want (the CTAs that have routed their share, or a flag).  The CTAs then build the expert tables
+    // themselves from topk_idx (the same histogram and scan as the front end) and the producer streams the first weight tiles
+    // while the front end still permutes and gathers.  The token rows: with narrow tiles they are there when *copied has reached
+    // copied_want, the CTAs that have copied their share - earlier than the front end's last CTA has left and a waiting kernel
+    // has learned of it -, otherwise after the wait for the front end.
     const int* routed;
+    const int* copied;
+    int routed_want, copied_want;
+    int* met;             // fused combine: the front end's two counts (FrontParams::sync), which the last kernel of a forward clears
     int tables_done;              // the expert tables are complete before this kernel can start (see the kernel's prologue)
     const int32_t* topk_idx;      // [n_pairs] global expert ids (pair_stride == top_k on this path)
     int n_pairs, local_offset;
@@ -418,6 +423,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #pragma unroll 1
             for (uint32_t it = 1;; ++it) {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(p.routed) : "memory");
+                seen = seen >= p.routed_want;
                 if (seen) break;
                 if ((it & 0xFFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) break;     // fall back to the tables
             }
@@ -453,7 +459,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     ctrl_sync();
     // The producer (warp 0) waits after its first weight loads.  Nobody lets the next kernel start before having waited
     // for the previous one: the next kernel may rely on everything before this one (tables_done).
-    if (warp != 0) {
+    // With `copied` only the idle warps 2-3 wait: all that the roles touch but the copied rows was done when the front end let this kernel start.
+    const bool by_count = !C::TOK_ON_M && G1 && early && p.copied;
+    if (by_count ? warp >= 2 : warp != 0) {
         if (early) pdl_wait();
         pdl_launch();
     }
@@ -677,7 +685,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                     if (lane == 0) stamp(TR_TMA_FIRST);
                     issued = true;
-                    pdl_wait();
+                    if (!C::TOK_ON_M && G1 && p.copied) {
+                        const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
+                        for (uint32_t it = 1;; ++it) {
+                            int n = 0;
+                            if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(p.copied) : "memory");
+                            n = __shfl_sync(0xFFFFFFFFu, n, 0);
+                            __syncwarp();
+                            if (merged(n >= p.copied_want)) break;
+                            if ((it & 0xFFu) == 0 && __any_sync(0xFFFFFFFFu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) { ok = false; break; }
+                        }
+                        if (!ok && lane == 0) atomicCAS(p.status, 0, ERR_WAIT_GROUP);
+                        asm volatile("fence.proxy.async.global;" ::: "memory");
+                    } else {
+                        pdl_wait();
+                    }
                     waited = true;
 #pragma unroll 1
                     for (int i = 0; i < npre; ++i) {
@@ -919,8 +942,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 
         int n_item = 0;
         WorkItem wi;
-        pdl_wait();
-        pdl_launch();
+        if (!(!C::TOK_ON_M && G1 && p.copied)) { pdl_wait(); pdl_launch(); }
+        if (FUSE && p.met && blockIdx.x == 0 && ptid < 2) p.met[ptid] = 0;
 #pragma unroll 1
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;

@@ -354,7 +354,7 @@ template <int OUT, bool WIDE>
 __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__ y, const int32_t* __restrict__ topk_idx,
                                                       const int32_t* __restrict__ pair_row, const float* __restrict__ row_w,
                                                       void* __restrict__ out, int T, int H, int top_k, int pair_stride,
-                                                      int local_offset, int num_local, int batch, int tables_done, const SlotOut slots) {
+                                                      int local_offset, int num_local, int batch, int tables_done, int* met, const SlotOut slots) {
     __shared__ int s_rows[2][COMBINE_BATCH][8];
     __shared__ float s_w[2][COMBINE_BATCH][8];
     __shared__ int s_n[2][COMBINE_BATCH];          // rows of the token, -1: nothing to write
@@ -390,7 +390,11 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
             if (r != NO_ROW) { s_rows[buf][warp][rank] = r; s_w[buf][warp][rank] = __ldcg(row_w + r); }
             if (lane == 0) s_n[buf][warp] = present ? __popc(have) : -1;
         }
-        if (t0 == t_first) { pdl_wait(); pdl_launch(); }
+        if (t0 == t_first) {
+            pdl_wait(); pdl_launch();
+            // the front end's counts: all that watch them are done, and the next call counts behind this kernel
+            if (met && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) met[threadIdx.x] = 0;
+        }
         __syncthreads();
         const int nt = min(batch, T - t0);
         for (int b = 0; b < nt; ++b) {

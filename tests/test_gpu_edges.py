@@ -636,3 +636,41 @@ def test_host_pipeline_returns_every_steps_own_result():
         want = layer.forward(s["logits"].cuda(), static[0], s["hidden"].cuda(), s["scale"].cuda(), *static[1:])
         torch.cuda.synchronize()
         assert torch.equal(s["out"].view(torch.int16), want.cpu().view(torch.int16))
+
+
+@pytest.mark.parametrize("tile", [0, 16, 128])
+def test_counts_of_the_one_launch_front_ends(tile):
+    """The front ends' counts belong to the handle and the last kernel of a forward clears them: own and routed calls on both sides
+    of the lines between the grids (8 / 9, 32 / 33 tokens, 128) in turn, queued without a host wait, and the same calls from a
+    graph that is replayed, all give the bits of the first pass."""
+    from justgoal_b200 import MoELayer
+    shape = I.TINY_DS
+    d = util.to_cuda(I.make_inputs(shape, 128, seed=67))
+    off, f = int(d["local_expert_offset"]), d["routed_scaling_factor"]
+    wts = [d[n] for n in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")]
+    layer = MoELayer(shape)
+    layer.set_token_tile(tile)
+    idx, w = layer.route(d["routing_logits"], d["routing_bias"], f)
+    calls = []
+    for T in (8, 128, 9, 1, 33, 32):
+        x, sc = d["hidden_states"][:T], d["hidden_states_scale"][:, :T].contiguous()
+        layer.workspace(T).fill_(0xFF)
+        calls.append(lambda T=T, x=x, sc=sc: layer.forward(d["routing_logits"][:T], d["routing_bias"], x, sc, *wts, off, f))
+        calls.append(lambda T=T, x=x, sc=sc: layer.forward_routed(idx[:T], w[:T], x, sc, *wts, off, out_dtype=torch.bfloat16))
+    want = [c().clone() for c in calls]
+    for own, routed in zip(want[::2], want[1::2]):
+        assert torch.equal(own.view(torch.int16), routed.view(torch.int16))
+    passes = [[c().clone() for c in calls] for _ in range(3)]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        outs = [c() for c in calls]
+    for _ in range(3):
+        for o in outs:
+            o.fill_(7.0)
+        g.replay()
+        passes.append([o.clone() for o in outs])
+    torch.cuda.synchronize()
+    assert [layer.status(T) for T in (1, 8, 9, 32, 33, 128)] == [0] * 6
+    for got in passes:
+        assert all(torch.equal(a.view(torch.int16), b.view(torch.int16)) for a, b in zip(got, want))
