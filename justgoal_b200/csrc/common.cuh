@@ -186,6 +186,13 @@ __device__ __forceinline__ void tma_gather4_2d(uint32_t dst, const CUtensorMap* 
         " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3), "r"(bar) : "memory");
 }
+// A read of shared memory that a barrier hands back behind it: through the shared window, where loads and the arrival that
+// follows them are performed in order.
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t src) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src) : "memory");
+    return v;
+}
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile(

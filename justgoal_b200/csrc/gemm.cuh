@@ -1064,10 +1064,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                             int sj = st0 + j; if (sj >= C::STAGES) sj -= C::STAGES;
                             const uint32_t ph = (st0 + j >= C::STAGES) ? (phase ^ 1) : phase;
                             if (!mbar_wait_warp(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
-                            const float* scp = reinterpret_cast<const float*>(smem + sj * C::STAGE_BYTES + C::SC_OFF) + c0;
+                            // (ld.shared: behind a load through a generic address the stage could be released, and its scales
+                            // overwritten, while the load was still under way - 64-token tiles, a third of 901-token calls)
+                            const uint32_t scp = smem_base + sj * C::STAGE_BYTES + C::SC_OFF + 4 * c0;
 #pragma unroll
                             for (int i = 0; i < C::NC; i += 4) {
-                                const float4 s4 = *reinterpret_cast<const float4*>(scp + i);
+                                const float4 s4 = ld_shared_f4(scp + 4 * i);
                                 scr[j][i] = s4.x; scr[j][i + 1] = s4.y; scr[j][i + 2] = s4.z; scr[j][i + 3] = s4.w;
                             }
                         }
@@ -1130,10 +1132,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                                 if (!mbar_wait_warp(bar_full + 8 * sj, ph, p.status, ERR_WAIT_SMEM_FULL)) ok = false;
                             }
                             {
-                                const float* scp = reinterpret_cast<const float*>(smem + sj * C::STAGE_BYTES + C::SC_OFF) + c0 + ch * C::CH;
+                                const uint32_t scp = smem_base + sj * C::STAGE_BYTES + C::SC_OFF + 4 * (c0 + ch * C::CH);
 #pragma unroll
                                 for (int i = 0; i < C::CH; i += 4) {
-                                    const float4 s4 = *reinterpret_cast<const float4*>(scp + i);
+                                    const float4 s4 = ld_shared_f4(scp + 4 * i);
                                     const float2 m0 = __fmul2_rn(make_float2(s4.x, s4.y), make_float2(swa, swa));
                                     const float2 m1 = __fmul2_rn(make_float2(s4.z, s4.w), make_float2(swa, swa));
                                     float* ac = &acc[a][ch * C::CH + i];

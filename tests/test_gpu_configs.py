@@ -194,3 +194,16 @@ torch.save(outs, sys.argv[1])
         a, b = a.float(), b.float()
         assert bool(((a - b).abs() <= 2.0 ** -7 * torch.maximum(a.abs(), b.abs()) + 1e-4).all())
         assert float((a != b).float().mean()) < 0.05
+
+
+@pytest.mark.parametrize("T,tile", [(901, 16), (901, 32), (901, 64), (901, 128), (64, 0), (3, 0), (4096, 0)])
+def test_forwards_repeat_their_bits(ds_weights, T, tile):
+    """Sixty forwards of every tile family give the bits of the first: a read of a stage's scales that the stage's release does
+    not wait for shows in one call of three (64-token tiles, 901 tokens, when it was there)."""
+    from justgoal_b200 import MoELayer
+    args = util.op_args(_inputs(T, ds_weights, seed=7))
+    layer = MoELayer(I.DEEPSEEK_V3)
+    layer.set_token_tile(tile)
+    first = layer.forward(*args).clone()
+    outs = [torch.equal(first.view(torch.int16), layer.forward(*args).view(torch.int16)) for _ in range(60)]
+    assert layer.status(T) == 0 and all(outs)
