@@ -78,7 +78,9 @@ typedef struct b200moe_ws_layout {
     size_t act_lo;        /* uint8[rows_cap, I] e4m3 of the rounding residual              */
     size_t act_scale;     /* float[I/128, rows_cap]                                        */
     size_t y;             /* fp16[rows_cap, H] expert output per row (before the weight)   */
-    size_t sk_count;      /* int32[2][4*SMs+4] per GEMM: arrival counters of chunked units, chunk claim counter */
+    size_t sk_count;      /* int32[2][4*SMs+4] per GEMM: arrival counters of chunked units, chunk claim counter;
+                             then, with 16- and 32-token tiles, int32 per token tile: warps that have stored
+                             their part of GEMM1's rows (both GEMMs in one launch)             */
     size_t slices;        /* int32[ceil(T*top_k/1024)][E_local] histogram of the local experts per
                              slice of 1024 (token, expert) pairs, token-major                */
     size_t sk_partial;    /* fp32 partial accumulators of the chunked units: slot (unit, chunk) */
@@ -311,7 +313,8 @@ int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches);
 int b200moe_launches_routed_slots(b200moe_handle h, int num_slots, int* launches);
 
 /* Optional stage timing.  enable(slots > 0) creates slots x 7 CUDA events; every forward then
- * records them around its six kernels (slot = call number modulo slots); enable(0) turns it
+ * records them around its six kernels (slot = call number modulo slots; the two GEMMs are two
+ * launches then, with the same bits, also where they are one otherwise); enable(0) turns it
  * off.  read(slot) waits for that call's last event and writes six durations in
  * milliseconds: route (or count), permute, gather, gemm1, gemm2, combine.  Counterpart of
  * the reference's in-kernel time stamps and pybind timing getters

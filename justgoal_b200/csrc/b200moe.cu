@@ -194,6 +194,22 @@ size_t sk_partial_bytes_ntok(const b200moe_config& c, int grid) {
     const size_t b = (size_t)chunks_per_unit(c.intermediate / 128, C2::KPB, C2::CHUNK_GROUPS) * C2::SLOT_FLOATS;
     return (a > b ? a : b) * (size_t)grid * 4;
 }
+// Partial-sum slots per CTA with narrow tiles (those of both GEMMs have the same size)
+int narrow_slots(const b200moe_config& c, int ntok) {
+    const size_t bytes = ntok == 16 ? sk_partial_bytes_ntok<16>(c, 1) / (GemmCfg<16, true>::SLOT_FLOATS * 4)
+                                    : sk_partial_bytes_ntok<32>(c, 1) / (GemmCfg<32, true>::SLOT_FLOATS * 4);
+    return (int)bytes;
+}
+
+// Both GEMMs in one launch?  With narrow tiles and weights that L2 (126 MB) cannot hold, where the call is two streams from HBM
+// (both sides: head of gemm.cuh).  Smaller layers keep the two launches: they are ahead by up to 12 % in one launch as well where
+// they have many units (64 experts of 1024 x 512, 64 tokens 42.1 / 36.4 us; 512-wide 21.5 / 20.3), but the number of launches and of
+// pieces that a small layer makes is what this library has always stated, and the fused combine's bits go with them.
+bool use_both(const b200moe_ctx* h, int ntok) {
+    const b200moe_config& c = h->cfg;
+    return ntok <= 32 && (size_t)c.num_local_experts * 3 * c.hidden * c.intermediate >= ((size_t)128 << 20) && narrow_slots(c, ntok) >= 2;
+}
+
 size_t sk_partial_bytes(const b200moe_config& c, int grid, int ntok) {
     switch (ntok) {
         case 16: return sk_partial_bytes_ntok<16>(c, grid);
@@ -210,6 +226,12 @@ int rows_capacity_for(const b200moe_config& c, int T) {
     return (int)rows;
 }
 
+// Token tiles of a call with narrow tiles, at most: full ones and a part-full one per expert.
+size_t max_narrow_tiles(const b200moe_ctx* h, int T) {
+    const int ntok = pick_token_tile(h, T);
+    return ntok > 32 ? 0 : (size_t)(rows_capacity_for(h->cfg, T) / ntok + h->cfg.num_local_experts);
+}
+
 void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     const b200moe_config& c = h->cfg;
     const size_t A = 256;
@@ -219,7 +241,8 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, A); return o; };
     L->status = take(8 * 4);
     L->counts = take((size_t)El * 4);
-    L->sk_count = take((size_t)2 * (4 * h->num_sms + 4) * 4); // [GEMM1 | GEMM2][4 * grid + 4]; zeroed with the head
+    // [GEMM1 | GEMM2][4 * grid + 4], then a counter per token tile (tile_done); zeroed with the head
+    L->sk_count = take((size_t)2 * (4 * h->num_sms + 4) * 4 + max_narrow_tiles(h, T) * 4);
     L->slices = take((size_t)num_slices(c, T) * El * 4);      // zeroed with the head
     // narrow token tiles: the combine is fused into GEMM2 and counts row deliveries per (token, 256 output columns)
     L->tok_count = take(pick_token_tile(h, T) < 128 ? (size_t)T * ((c.hidden + 255) / 256) * 4 : 0);   // zeroed with the head
@@ -238,6 +261,12 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     L->y = take(rows * c.hidden * 2);
     L->sk_partial = take(sk_partial_bytes(c, h->num_sms, (int)pick_token_tile(h, T)));
     L->trace = take((size_t)2 * h->num_sms * TRACE_SLOTS * 8 + 2 * 8 * KLOG_N * 8);   // [GEMM1 | GEMM2][CTA][slot], then K-block logs
+    // A workspace serves every smaller call, and the counters above exist with narrow tiles only: as much room as the largest
+    // call with them takes.
+    if (pick_token_tile(h, T) == 128) {
+        const int narrow_T = (int)(9ll * c.num_experts / c.top_k);
+        take((size_t)narrow_T * ((c.hidden + 255) / 256) * 4 + ((size_t)rows_capacity_for(c, narrow_T) / 16 + El) * 4 + 512);
+    }
     L->rows_cap = rows;
     L->token_tile = (size_t)pick_token_tile(h, T);
     L->total_bytes = off;
@@ -284,6 +313,21 @@ cudaError_t launch_gemm_fused(int ntok, int grid, cudaStream_t st, const CUtenso
         case 32: return launch_gemm_fused_ntok<32>(grid, st, w, b0, b1, s0, s1, p);
         default: return launch_gemm_fused_ntok<64>(grid, st, w, b0, b1, s0, s1, p);
     }
+}
+
+// Both GEMMs in one launch (parts == 3), or the two parts of that kernel one after the other
+template <int NTOK, bool FUSE>
+cudaError_t launch_gemm_both_form(int parts, int grid, cudaStream_t st, const MapSet& m, const GemmParams& p1, const GemmParams& p2) {
+    return launch_k(parts & 1 ? PDL_GEMM1 : PDL_GEMM2, gemm_both_kernel<NTOK, FUSE>, dim3(grid), dim3(GemmCfg<NTOK, true, true>::NTHREADS),
+                    GemmCfg<NTOK, true, true>::SMEM_BYTES, st, m.w13, m.a, m.w2, m.hi, m.lo, p1, p2, parts);
+}
+cudaError_t launch_gemm_both(int ntok, bool fuse, int parts, int grid, cudaStream_t st, const MapSet& m, const GemmParams& p1, const GemmParams& p2) {
+    if (ntok == 16) return fuse ? launch_gemm_both_form<16, true>(parts, grid, st, m, p1, p2) : launch_gemm_both_form<16, false>(parts, grid, st, m, p1, p2);
+    return fuse ? launch_gemm_both_form<32, true>(parts, grid, st, m, p1, p2) : launch_gemm_both_form<32, false>(parts, grid, st, m, p1, p2);
+}
+template <int NTOK, bool FUSE>
+cudaError_t set_attr_both() {
+    return cudaFuncSetAttribute(gemm_both_kernel<NTOK, FUSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<NTOK, true, true>::SMEM_BYTES);
 }
 
 // 128-token tiles, most of them part full
@@ -582,12 +626,10 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g1.sk_partial = reinterpret_cast<float*>(ws + L.sk_partial);
     g1.trace = reinterpret_cast<long long*>(ws + L.trace);
     g1.klog = g1.trace + (size_t)2 * h->num_sms * TRACE_SLOTS;
-    if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
-    else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, m_a, m_a, g1));
-    else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
-    else CU_TRY(launch_gemm_ntok<true>(ntok, h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
-    CU_TRY(prof_mark(h, 4, st));
-
+    const bool fuse = h->fuse_combine && allow_fuse && ntok < 128 && !pairs && out_kind == OUT_BF16 && !slot_out && wire_pitch == 0;
+    const bool both = use_both(h, ntok);
+    g1.tile_done = g1.sk_count + 2 * (4 * h->num_sms + 4);
+    g1.tile_want = g1.n_mtiles * 4;
     GemmParams g2;
     memset(&g2, 0, sizeof(g2));
     g2.status = status; g2.counts = counts; g2.expert_row0 = row0; g2.tile_prefix = tiles; g2.num_local = El;
@@ -599,13 +641,19 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     g2.tables_done = pairs ? 0 : 1;
     g2.sk_count = reinterpret_cast<int*>(ws + L.sk_count) + 4 * h->num_sms + 4;
     g2.sk_partial = g1.sk_partial;
+    if (both) {        // the area of the larger GEMM's pieces, shared: GEMM2's units may be cut while pieces of GEMM1's still wait
+        const int per_cta = narrow_slots(c, ntok);
+        g1.slots = per_cta / 2 < 3 ? per_cta / 2 : 3; g2.slots = per_cta - g1.slots;
+        g2.sk_partial += (size_t)h->num_sms * g1.slots * (ntok == 16 ? GemmCfg<16, true>::SLOT_FLOATS : GemmCfg<32, true>::SLOT_FLOATS);
+        g1.next_mtiles = g2.n_mtiles; g1.next_KB = g2.KB;
+    }
+    g2.tile_done = g1.tile_done; g2.tile_want = g1.tile_want;
     g2.trace = g1.trace + (size_t)h->num_sms * TRACE_SLOTS;
     g2.klog = g1.klog + 8 * KLOG_N;
     // Optional (b200moe_set_fused_combine): the operator's own forward with narrow token tiles lets the GEMM2 unit that
     // delivers a token's last row add the token's rows up and write the bf16 output - no combine launch.  Same bits
     // as combine_kernel; measured 9 us slower per 64-token step (the fence, the delivery atomics and the row loads
     // sit in the epilogue of every unit, where the separate kernel pays them once), so it is off by default.
-    const bool fuse = h->fuse_combine && allow_fuse && ntok < 128 && !pairs && out_kind == OUT_BF16 && !slot_out && wire_pitch == 0;
     if (fuse) {
         g2.fuse_out = static_cast<__nv_bfloat16*>(out);
         g2.tok_count = reinterpret_cast<int*>(ws + L.tok_count);
@@ -613,7 +661,15 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
         g2.met = fused_front ? h->d_sync : nullptr;
     }
-    if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
+    // (With stage times the two parts of the kernel that does both run as two launches: the same pieces, the same bits.)
+    if (both) { if (h->prof_slots) CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, g2)); }
+    else if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
+    else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, m_a, m_a, g1));
+    else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
+    else CU_TRY(launch_gemm_ntok<true>(ntok, h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
+    CU_TRY(prof_mark(h, 4, st));
+    if (both) CU_TRY(launch_gemm_both(ntok, fuse, h->prof_slots ? 2 : 3, h->num_sms, st, maps, g1, g2));
+    else if (pairs) CU_TRY(launch_gemm_pair<false>(h->pair_grid[1], st, m_w2, m_hi, m_lo, g2));
     else if (fuse) CU_TRY(launch_gemm_fused(ntok, h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
     else if (part) CU_TRY(launch_gemm_part<false>(h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
     else CU_TRY(launch_gemm_ntok<false>(ntok, h->num_sms, st, m_w2, m_hi, m_lo, maps.hi_box, maps.lo_box, g2));
@@ -688,6 +744,7 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
                                if (e_ != cudaSuccess) return (int)e_; } while (0)
     CU_TRY_ATTR((set_attr<16, true>()));  CU_TRY_ATTR((set_attr<16, false>()));
     CU_TRY_ATTR((set_attr<32, true>()));  CU_TRY_ATTR((set_attr<32, false>()));
+    CU_TRY((set_attr_both<16, false>())); CU_TRY((set_attr_both<16, true>())); CU_TRY((set_attr_both<32, false>())); CU_TRY((set_attr_both<32, true>()));
     CU_TRY_ATTR((set_attr<64, true>()));  CU_TRY_ATTR((set_attr<64, false>()));
     CU_TRY_ATTR((set_attr<128, true>())); CU_TRY_ATTR((set_attr<128, false>())); CU_TRY_ATTR((set_attr<128, true, true>()));
     CU_TRY_ATTR((set_attr<16, false, false, false, true>())); CU_TRY_ATTR((set_attr<32, false, false, false, true>()));
@@ -794,22 +851,23 @@ int b200moe_workspace_bytes(b200moe_handle h, int num_tokens, size_t* bytes) {
 int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
     // [route, permute, gather | fused route+permute+gather for small T], gemm1, gemm2, [combine unless fused into gemm2]
-    const bool fuse = h->fuse_combine && pick_token_tile(h, num_tokens) < 128 && !use_pairs(h, pick_token_tile(h, num_tokens));
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (fuse ? 1 : 0);
+    const int ntok = pick_token_tile(h, num_tokens);
+    const bool fuse = h->fuse_combine && ntok < 128 && !use_pairs(h, ntok);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (fuse ? 1 : 0) - (use_both(h, ntok) ? 1 : 0);
     return 0;
 }
 
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
     // [count, permute, gather | all in one launch for small T], gemm1, gemm2, combine
-    *launches = num_tokens == 0 ? 0 : num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (use_both(h, pick_token_tile(h, num_tokens)) ? 1 : 0);
     return 0;
 }
 
 int b200moe_launches_routed_slots(b200moe_handle h, int num_slots, int* launches) {
     if (!h || !launches || num_slots < 1) return B200MOE_E_BADARG;
     // count, permute, gather, gemm1, gemm2, combine whatever the number of slots
-    *launches = 6 - (gathers_by_tma(h, num_slots) ? 1 : 0);
+    *launches = 6 - (gathers_by_tma(h, num_slots) ? 1 : 0) - (use_both(h, pick_token_tile(h, num_slots)) ? 1 : 0);
     return 0;
 }
 

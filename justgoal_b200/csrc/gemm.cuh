@@ -16,7 +16,7 @@
 // unlike them the SwiGLU output keeps a second e4m3 term, because a single e4m3 per element
 // does not meet an absolute/relative tolerance of 1e-2 against the unquantised definition.
 //
-// Schedule: K is cut into GROUPS of KPB 128-K blocks (one TMEM hand-off per group).  The kernel is
+// Schedule (of a kernel that does one GEMM): K is cut into GROUPS of KPB 128-K blocks (one TMEM hand-off per group).  The kernel is
 // persistent.  Units are numbered so that the token tiles of one (expert, row tiles) are adjacent.  Every CTA
 // first runs floor(U / grid) WHOLE units, round-robin (CTAs that run at the same time work on adjacent units, so
 // a weight tile shared by several token tiles comes from HBM once).  The remaining U mod grid units stay
@@ -37,6 +37,18 @@
 // soon as its CTA has an SM: the first weights travel under the tail of GEMM1 (T=64: 132 -> 130 us, T=7: 72 -> 70 us).  So does
 // GEMM1 behind a separate gather: its tables come from the permutation before that.
 // Optionally (FUSE) GEMM2's epilogue also does the combine.
+//
+// Both GEMMs in one launch (gemm_both_kernel, narrow tiles over weights that L2 cannot hold).  Such a call is two weight streams,
+// and between them, with a kernel each, HBM stood idle for 8 to 14 us: the CTAs of GEMM1 end 7 to 15 us apart, a CTA of GEMM2
+// takes 5 us from the end of the one before it to its first load, and all of them wait for GEMM1's last epilogue; the stage ring
+// covers 4 us of that.  In one launch the producer goes on to GEMM2's weights with the next stage of the ring.  Everything is
+// CLAIMED from one counter, in the order GEMM1's whole units, GEMM1's pieces, GEMM2's units and pieces: what a CTA waits for
+// (partial sums, the rows of a token tile) has been claimed before its own item by a CTA that runs, so no cycle of waiting CTAs can form and no CTA
+// has to be resident, whatever other streams run.  GEMM1's left-over units mostly stay whole, because the CTAs without one take up
+// GEMM2's units of the experts that are done.  A token tile's rows are handed over by a counter (tile_done).  us, two launches / one:
+// 32 of 256 experts 12 tokens 90 / 82, 64: 132 / 122, 128: 161 / 150, 200: 190 / 182; 128 of 256 experts 4: 136 / 127, 64: 450 / 440; 16
+// experts of the 4096-wide shape 16: 62.5 / 54.5, 128: 70.5 / 67.5; 4 of 5120 x 8192 30: 117 / 106.  It does not pay with one or two experts and
+// many CTAs to share them (routed, 1 token 32.7 / 34.0), nor with more units than a few per CTA (128 experts, 200 tokens 630 / 635).
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (whole warps, one elected lane issues),
 // warps 2-3: scales of 128-token tiles on their way into shared memory, otherwise idle (they complete the first warpgroup so register
@@ -93,6 +105,12 @@ struct GemmParams {
     const int* copied;
     int routed_want, copied_want;
     int* met;             // fused combine: the front end's two counts (FrontParams::sync), which the last kernel of a forward clears
+    // Both GEMMs in one launch: counter of every token tile, zero at launch; a warp that has stored its part of a GEMM1 unit's
+    // rows counts in, and a unit of GEMM2 may read the tile when tile_want have.
+    int* tile_done;
+    int tile_want;
+    int slots;                    // ... and this GEMM's share of the partial-sum slots, per CTA
+    int next_mtiles, next_KB;     // GEMM1: units of GEMM2 per token tile, and their K blocks
     int tables_done;              // the expert tables are complete before this kernel can start (see the kernel's prologue)
     const int32_t* topk_idx;      // [n_pairs] global expert ids (pair_stride == top_k on this path)
     int n_pairs, local_offset;
@@ -117,13 +135,14 @@ struct GemmParams {
     int c_stride, top_k, T, c_local_offset;
 };
 
-template <int NTOK, bool G1>
+// BOTH: the GEMM is one of two in the same launch (gemm_both_kernel); the stages of both then have the same size.
+template <int NTOK, bool G1, bool BOTH = false>
 struct GemmCfg {
     static constexpr int NA = 2;                          // weight tiles per stage (GEMM1: up + gate rows; GEMM2: two row tiles)
     static constexpr int NB = G1 ? 1 : 2;                 // token tiles per stage
     static constexpr int A_BYTES = 128 * 128;
     static constexpr int B_BYTES = NTOK * 128;
-    static constexpr int SC_OFF = NA * A_BYTES + NB * B_BYTES;
+    static constexpr int SC_OFF = NA * A_BYTES + (BOTH ? 2 : NB) * B_BYTES;
     static constexpr int STAGE_BYTES = SC_OFF + 1024;
     // tokens-on-M tiles get their (per-thread scalar) token scales through the scale warps; the others get the tile's
     // NTOK scales copied into the stage
@@ -191,7 +210,7 @@ struct GemmCfg {
     // CTA stores at most one partial sum, which it makes before anything else; the piece that ends a unit runs after the CTA's
     // whole units and waits for those other pieces (claimed chunks measured 5-15 us slower: every one of them costs a partial sum, late in the kernel).
     // Everywhere else the left-over units are cut into chunks that the CTAs claim as they go.
-    static constexpr bool STATIC_TAIL = G1 && NTOK <= 32;
+    static constexpr bool STATIC_TAIL = G1 && NTOK <= 32 && !BOTH;
     static constexpr int WQ = 4, WQ_INTS = 12;             // depth of the in-CTA work queue, words of an entry (WorkItem)
     static constexpr int BAR_BYTES = 320;                  // mbarriers + TMEM address word
     static constexpr int TABLE_INTS = 3 * (MAX_LOCAL + 1);
@@ -241,7 +260,8 @@ __device__ __forceinline__ bool decode_unit_warp(int u, int n_mtiles, int num_lo
 
 // One piece of work: unit u, K groups [gb, ge).  pieces == 1: the whole unit; otherwise piece number `piece` of the split
 // unit number `ut`, whose partial sums live in the slots from `slot` on.  u < 0 ends the list.
-struct WorkItem { int u, gb, ge, ut, piece, pieces, slot; Unit un; };
+struct WorkItem { int u, gb, ge, ut, piece, pieces, slot; Unit un; int tile; };
+constexpr int GAVE_UP = -2;          // u of the item that ends a list because a wait of the producer ran out
 constexpr int MAX_PIECES = 128;      // arrivals of a split unit are counted in bytes
 
 // CTA that owns flat index x when `total` indices are cut into `parts` equal contiguous ranges (part c starts at
@@ -310,6 +330,82 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
     for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// What the roles of a CTA share, and what a warp carries from GEMM1 to GEMM2 where one launch does both.
+struct GemmCta {
+    uint8_t* smem;
+    uint32_t smem_base, tmem_base;
+    uint32_t bar_full, bar_empty, bar_tfull, bar_tempty, bar_red, bar_wqfull, bar_wqempty;
+    uint32_t* s_tmem;
+    int* s_wq; int* s_tiles; int* s_row0; int* s_cnt; uint32_t* s_red; int* s_flag; int* s_g4; float* s_ts;
+    int warp, lane;
+    long long t_entry;
+    int stage; uint32_t phase;         // ring of stages
+    int ab; uint32_t aphase;           // ring of accumulators
+    uint32_t rphase; int rbuf;         // meetings in the epilogue, half of s_red the next one uses
+    int n_item;                        // work queue
+    int* claim; int claimed, claim_base;      // one launch for both GEMMs: the counter, lane 0's next claim, claims GEMM1 took
+    bool fresh;                        // nothing of this launch has waited for the kernel before it or built the tables yet
+    bool ok;
+};
+
+// Barriers, tensor memory, the carve-up of shared memory.
+template <class C>
+__device__ __forceinline__ void gemm_setup(GemmCta& x, uint8_t* smem_raw) {
+    x.smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* tail = x.smem + C::STAGES * C::STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);     // full[S], empty[S], tfull[NTB], tempty[NTB], red[4], wq_full[WQ], wq_empty[WQ]
+    x.s_tmem = reinterpret_cast<uint32_t*>(tail + C::BAR_BYTES - 8);
+    x.s_wq = reinterpret_cast<int*>(tail + C::BAR_BYTES);          // [WQ][WQ_INTS] work items, 16-byte aligned
+    x.s_tiles = x.s_wq + C::WQ * C::WQ_INTS;
+    x.s_row0 = x.s_tiles + (MAX_LOCAL + 1);
+    x.s_cnt = x.s_row0 + (MAX_LOCAL + 1);
+    x.s_red = reinterpret_cast<uint32_t*>(x.s_cnt + (MAX_LOCAL + 1));
+    x.s_flag = reinterpret_cast<int*>(x.s_red + C::RED_BYTES / 4);   // 20 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last), [12..] s_filled
+    // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
+    x.s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(x.s_flag + 20) + 15) & ~uintptr_t(15));
+    x.s_ts = reinterpret_cast<float*>(x.s_g4 + 128);            // tokens-on-M: [TSD][TS_SLOT] scales of a K block
+    x.warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); x.lane = threadIdx.x & 31;   // uniform for the compiler too
+    x.t_entry = clock64();
+    x.bar_full = smem_u32(bars);
+    x.bar_empty = x.bar_full + 8 * C::STAGES;
+    x.bar_tfull = x.bar_empty + 8 * C::STAGES;
+    x.bar_tempty = x.bar_tfull + 8 * C::NTB;
+    // warps that meet in the epilogue (bounded): the 4 warps of a column group or, tokens on M, those of a lane quarter
+    x.bar_red = x.bar_tempty + 8 * C::NTB;
+    x.bar_wqfull = x.bar_red + 8 * 4;            // work queue: the producer has published item n
+    x.bar_wqempty = x.bar_wqfull + 8 * C::WQ;  // ... and the MMA warp and every promotion warp have read it
+    static_assert(8 * (2 * C::STAGES + 2 * C::NTB + 4 + 2 * C::WQ) <= C::BAR_BYTES - 8, "barrier area");
+    x.stage = 0; x.phase = 0; x.ab = 0; x.aphase = 0; x.rphase = 0; x.rbuf = 0; x.n_item = 0;
+    x.claim = nullptr; x.claimed = 0; x.claim_base = 0; x.fresh = true; x.ok = true;
+}
+template <class C, int NHELP>
+__device__ __forceinline__ void gemm_init(GemmCta& x, const CUtensorMap& m0, const CUtensorMap& m1, const CUtensorMap& m2) {
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < C::STAGES; ++s) { mbar_init(x.bar_full + 8 * s, 1); mbar_init(x.bar_empty + 8 * s, C::EMPTY_COUNT); }
+        for (int b = 0; b < C::NTB; ++b) { mbar_init(x.bar_tfull + 8 * b, 1 + NHELP); mbar_init(x.bar_tempty + 8 * b, C::NPW); }
+        for (int g = 0; g < 4; ++g) mbar_init(x.bar_red + 8 * g, C::TOK_ON_M ? C::NGRP : 4);
+        for (int w = 0; w < C::WQ; ++w) { mbar_init(x.bar_wqfull + 8 * w, 1); mbar_init(x.bar_wqempty + 8 * w, 1 + NHELP + C::NPW); }
+        mbar_fence_init();
+        tma_prefetch_desc(&m0); tma_prefetch_desc(&m1); tma_prefetch_desc(&m2);
+    }
+    if (x.warp == 1) { tmem_alloc(smem_u32(x.s_tmem), C::TMEM_COLS); tmem_relinquish(); }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    x.tmem_base = *x.s_tmem;
+    x.smem_base = smem_u32(x.smem);
+}
+template <class C>
+__device__ __forceinline__ void gemm_teardown(GemmCta& x) {
+    tc_fence_before();
+    __syncthreads();
+    if (x.warp == 1) { tc_fence_after(); tmem_dealloc(*x.s_tmem, C::TMEM_COLS); }
+}
+template <bool TOK_ON_M, bool G4>
+__host__ __device__ constexpr int helper_warps() { return TOK_ON_M ? (G4 ? 2 : 1) : 0; }      // warps (2, 3) that fill the ring of scales
+
+enum : int { SOLE = 0, FIRST = 1, SECOND = 2 };       // a launch's only GEMM; GEMM1, GEMM2 of a launch that does both
+
 // G4 (GEMM1 with 128-token tiles only): the token rows come straight from the caller's activations by four-row TMA
 // gathers (GemmParams::g4_row_token); a separate instantiation, so the plain kernel's code is unchanged by it.
 // PART (128-token tiles): quarters of a token tile (32 rows, one warp's TMEM lanes) that hold no row of the unit are not
@@ -317,33 +413,21 @@ __device__ __forceinline__ void tmem_ld_chunk(uint32_t taddr, float* v) {
 // expected number of rows per expert (both sides measured at the rule in b200moe.cu).
 // FUSE (GEMM2, narrow tiles): with the combine in the epilogue (GemmParams::fuse_out); an instance of its own, so the plain
 // kernel stays small.
-template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
-__global__ void __launch_bounds__(GemmCfg<NTOK, G1>::NTHREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
-            const __grid_constant__ CUtensorMap tm_b1, const __grid_constant__ CUtensorMap tm_s0,
-            const __grid_constant__ CUtensorMap tm_s1, const GemmParams p) {
-    using C = GemmCfg<NTOK, G1>;
+template <int NTOK, bool G1, bool G4, bool PART, bool FUSE, int WHICH>
+__device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, const CUtensorMap& tm_b0, const CUtensorMap& tm_b1,
+                                           const CUtensorMap& tm_s0, const CUtensorMap& tm_s1, const GemmParams& p) {
+    constexpr bool BOTH = WHICH != SOLE;
+    using C = GemmCfg<NTOK, G1, BOTH>;
     static_assert(!G4 || (C::TOK_ON_M && G1), "TMA-gathered token rows: GEMM1 with 128-token tiles");
     static_assert(!FUSE || (!G1 && !C::TOK_ON_M), "fused combine: GEMM2, narrow tiles");
     static_assert(!PART || (C::TOK_ON_M && !G4), "part-full tiles: tokens on M");
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* tail = smem + C::STAGES * C::STAGE_BYTES;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(tail);     // full[S], empty[S], tfull[NTB], tempty[NTB], red[4], wq_full[WQ], wq_empty[WQ]
-    uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tail + C::BAR_BYTES - 8);
-    int* s_wq = reinterpret_cast<int*>(tail + C::BAR_BYTES);          // [WQ][WQ_INTS] work items, 16-byte aligned
-    int* s_tiles = s_wq + C::WQ * C::WQ_INTS;
-    int* s_row0 = s_tiles + (MAX_LOCAL + 1);
-    int* s_cnt = s_row0 + (MAX_LOCAL + 1);
-    uint32_t* s_red = reinterpret_cast<uint32_t*>(s_cnt + (MAX_LOCAL + 1));
-    int* s_flag = reinterpret_cast<int*>(s_red + C::RED_BYTES / 4);   // 20 ints: [0] routing flag seen (early schedule), [4..5] the producer's chunk sizing, [8..11] pieces seen (s_last), [12..] s_filled
-    // [128] token of every row of the producer's unit, 16-byte aligned (read and written as int4)
-    int* s_g4 = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(s_flag + 20) + 15) & ~uintptr_t(15));
-    float* s_ts = reinterpret_cast<float*>(s_g4 + 128);            // tokens-on-M: [TSD][TS_SLOT] scales of a K block
-    constexpr int NHELP = C::TOK_ON_M ? (G4 ? 2 : 1) : 0;          // ... and the warps (2, 3) that fill it
-
-    const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // uniform for the compiler too
-    const long long t_entry = clock64();
+    static_assert(!BOTH || (!C::TOK_ON_M && C::EARLY_SCALES && G1 == (WHICH == FIRST)), "both GEMMs in one launch: narrow tiles");
+    uint8_t* const smem = x.smem;
+    int* const s_wq = x.s_wq; int* const s_tiles = x.s_tiles; int* const s_row0 = x.s_row0; int* const s_cnt = x.s_cnt;
+    uint32_t* const s_red = x.s_red; int* const s_flag = x.s_flag; int* const s_g4 = x.s_g4; float* const s_ts = x.s_ts;
+    constexpr int NHELP = helper_warps<C::TOK_ON_M, G4>();
+    const int warp = x.warp, lane = x.lane;
+    const long long t_entry = x.t_entry;
     long long* const trace = p.trace ? p.trace + (size_t)blockIdx.x * TRACE_SLOTS : nullptr;
     auto stamp = [&](int slot) { if (trace) trace[slot] = clock64() - t_entry; };
 #ifdef B200MOE_ENABLE_KLOG
@@ -352,37 +436,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #else
     auto klog_put = [&](int, int) {};      // the per-K-block log is a build option (-DB200MOE_ENABLE_KLOG)
 #endif
-    if (trace && threadIdx.x == 0) trace[TR_ENTRY] = (long long)globaltimer_ns();
-    const uint32_t bar_full = smem_u32(bars);
-    const uint32_t bar_empty = bar_full + 8 * C::STAGES;
-    const uint32_t bar_tfull = bar_empty + 8 * C::STAGES;
-    const uint32_t bar_tempty = bar_tfull + 8 * C::NTB;
-    // warps that meet in the epilogue (bounded): the 4 warps of a column group or, tokens on M, those of a lane quarter
-    const uint32_t bar_red = bar_tempty + 8 * C::NTB;
-    const uint32_t bar_wqfull = bar_red + 8 * 4;            // work queue: the producer has published item n
-    const uint32_t bar_wqempty = bar_wqfull + 8 * C::WQ;  // ... and the MMA warp and every promotion warp have read it
-    static_assert(8 * (2 * C::STAGES + 2 * C::NTB + 4 + 2 * C::WQ) <= C::BAR_BYTES - 8, "barrier area");
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < C::STAGES; ++s) { mbar_init(bar_full + 8 * s, 1); mbar_init(bar_empty + 8 * s, C::EMPTY_COUNT); }
-        for (int b = 0; b < C::NTB; ++b) { mbar_init(bar_tfull + 8 * b, 1 + NHELP); mbar_init(bar_tempty + 8 * b, C::NPW); }
-        for (int g = 0; g < 4; ++g) mbar_init(bar_red + 8 * g, C::TOK_ON_M ? C::NGRP : 4);
-        for (int w = 0; w < C::WQ; ++w) { mbar_init(bar_wqfull + 8 * w, 1); mbar_init(bar_wqempty + 8 * w, 1 + NHELP + C::NPW); }
-        mbar_fence_init();
-        tma_prefetch_desc(&tm_w); tma_prefetch_desc(&tm_b0);
-        if (!G1) tma_prefetch_desc(&tm_b1);
-    }
-    if (warp == 1) { tmem_alloc(smem_u32(s_tmem), C::TMEM_COLS); tmem_relinquish(); }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *s_tmem;
-    const uint32_t smem_base = smem_u32(smem);
+    const uint32_t bar_full = x.bar_full, bar_empty = x.bar_empty, bar_tfull = x.bar_tfull, bar_tempty = x.bar_tempty;
+    const uint32_t bar_red = x.bar_red, bar_wqfull = x.bar_wqfull, bar_wqempty = x.bar_wqempty;
+    const uint32_t tmem_base = x.tmem_base, smem_base = x.smem_base;
 
     // Schedule (see the head of this file): q whole units per CTA, then chunks of the remaining units claimed
     // from a global counter.
     const int NG = (p.KB + C::KPB - 1) / C::KPB;
-    int* const claim = p.sk_count + 4 * (int)gridDim.x;
+    int* const claim = WHICH == SECOND && !x.fresh ? x.claim : p.sk_count + 4 * (int)gridDim.x;
 
     // Consumer side of the work queue: item n sits in slot n % WQ.  Every lane of the calling warp waits and reads,
     // lane 0 then tells the producer that the warp has its copy.  false = list ended or a wait gave up.
@@ -396,8 +457,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         w.u = uni(q0.x); w.gb = uni(q0.y); w.ge = uni(q0.z); w.ut = uni(q0.w);
         w.piece = uni(q1.x); w.pieces = uni(q1.y); w.slot = uni(q1.z); w.un.e = uni(q1.w);
         w.un.mt = uni(q2.x); w.un.row0 = uni(q2.y); w.un.nvalid = uni(q2.z);
+        if (BOTH && G1) w.tile = uni(q2.w);
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_wqempty + 8 * slot);
+        if (BOTH && w.u == GAVE_UP) ok = false;
         return w.u >= 0;
     };
 
@@ -416,6 +479,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     const int ctid = threadIdx.x;
     auto ctrl_sync = []() { asm volatile("bar.sync 1, 128;" ::: "memory"); };
     bool early = false;             // the producer has not waited for the previous kernel yet
+    if (WHICH != SECOND || x.fresh) {
     if (G1 && !G4 && p.routed) {
         if (ctid == 0) {
             int seen = 0;
@@ -428,6 +492,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 if ((it & 0xFFu) == 0 && globaltimer_ns() - t0 > WAIT_LIMIT_NS) break;     // fall back to the tables
             }
             *s_flag = seen;
+            if (BOTH && seen) x.claimed = atomicAdd(claim, 1);       // cleared before the announcement; the answer travels under the scan
         }
 #pragma unroll 1
         for (int i = ctid; i <= p.num_local; i += 128) s_cnt[i] = 0;
@@ -449,6 +514,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
     } else {
         early = !G4 && p.tables_done;
         if (!early) pdl_wait();
+        if (BOTH && ctid == 0) x.claimed = atomicAdd(claim, 1);
 #pragma unroll 1
         for (int i = ctid; i <= p.num_local; i += 128) {
             s_tiles[i] = __ldcg(p.tile_prefix + i);
@@ -466,6 +532,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         pdl_launch();
     }
     if (threadIdx.x == 0) stamp(TR_PROLOGUE);
+    }
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer: the whole warp runs the loop, one
         // elected lane issues (see elect_one)
@@ -474,12 +541,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             const int total_units = s_tiles[p.num_local] * p.n_mtiles;
             const int sched_q = total_units / (int)gridDim.x;              // whole units per CTA
             const int sched_U0 = sched_q * (int)gridDim.x;                 // first chunked unit
-            int stage = 0; uint32_t phase = 0;
+            int stage = x.stage; uint32_t phase = x.phase;
             bool ok = true, issued = false;
-            bool waited = !early;               // early schedule: has this thread waited for the previous kernel yet
+            bool waited = !early || WHICH == SECOND;      // early schedule: has this thread waited for the previous kernel yet (GEMM2's
+                                                          // rows behind GEMM1 in the same launch come with a counter)
             int nk = 0;
             // the producer decides what this CTA does next and publishes it to the other roles
-            int n_item = 0, n_whole = 0;
+            int n_item = x.n_item, n_whole = 0;
             constexpr bool BOXED = C::BOXED && !G4;
             volatile int* const s_filled = s_flag + 12;  // 128-token tiles: boxes of each stage whose rows are not zero
             if (BOXED && lane < C::STAGES) s_filled[lane] = 128 / C::BOX_ROWS;
@@ -491,7 +559,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     int4* q = reinterpret_cast<int4*>(s_wq + slot * C::WQ_INTS);
                     q[0] = make_int4(w.u, w.gb, w.ge, w.ut);
                     q[1] = make_int4(w.piece, w.pieces, w.slot, w.un.e);
-                    q[2] = make_int4(w.un.mt, w.un.row0, w.un.nvalid, 0);
+                    q[2] = make_int4(w.un.mt, w.un.row0, w.un.nvalid, w.tile);
                     mbar_arrive(bar_wqfull + 8 * slot);      // release: the item is visible to whoever sees the phase flip
                 }
                 __syncwarp();
@@ -510,20 +578,38 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             // 400: 150 / 125.  The line is not sharp: 6 / 12 / 18 blocks with 128-token tiles 320 tokens 221 / 227 / 231, 600: 238 / 247 /
             // 248, 2048: 343 / 338 / 338; 4 / 8 / 12 / 20 blocks with narrow tiles differ by less than 1 us but for the shape of 64 blocks
             // (64 tokens 89.0 / 87.9 / 88.0 / 88.3) and 4 tokens of a 4096 x 4096 shape (40.0 / 40.0 / 40.0 / 44.4).
+            // With both GEMMs in one launch: GEMM1's left-over units stay whole while the CTA that runs one more unit than the others,
+            // and then one of GEMM2's, is done before all work is (F, in K blocks per CTA); else they are cut by the same cost at 4 blocks per
+            // piece (the piece that ends a unit stores nothing, and the stream goes on meanwhile), not counting the CTAs that start late
+            // because the front end runs on their SMs.  Pieces 1 / 2 / 3 / 4, us: 32 of 256 experts 2 tokens (32 units) 47 / 40 / 39 / 39, 4
+            // (96) 65 / 68 / 63 / 68, 16 (160, of which 12 are left over; 8 pieces 83) 95 / 89 / 87 / 87, 128 (320) 152 / 153 / 153 / 157, 257 (400) 195 / 201 / 208 / 210;
+            // 16 of the 4096-wide shape 1 (24) 33.9 / 30.3 / 29.6 / 28.7, 4 (72) 37.0 / 38.0 / 44.9 / 43.4.  GEMM2's are cut into pieces of 16 blocks
+            // at most: with K of 16 blocks they stay whole, K of 32 (8 of a 4096 x 4096 shape, 64 tokens) 79.4 / 78.2, K of 64 (4 of
+            // 5120 x 8192, 30 tokens) 117 with two launches, 106 with four pieces.
             // (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
             volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, [1] pieces
             bool sized = false;
             auto size_chunks = [&]() {
-                constexpr int PIECE_COST = C::TOK_ON_M ? (PART ? 6 : 12) : 8, MOST = 8;
+                constexpr int PIECE_COST = C::TOK_ON_M ? (PART ? 6 : 12) : WHICH == FIRST ? 4 : 8, MOST = 8;
                 static_assert(MOST <= MAX_PIECES, "arrivals of a split unit");
                 const int tail_units = total_units - sched_U0;
-                const int slots = (int)gridDim.x * ((NG + C::CHUNK_GROUPS - 1) / C::CHUNK_GROUPS);           // what sk_partial holds
+                const int slots = (int)gridDim.x * (BOTH ? p.slots : (NG + C::CHUNK_GROUPS - 1) / C::CHUNK_GROUPS);           // what sk_partial holds
+                const int late = WHICH == FIRST && sched_q == 0 && p.routed ? p.copied_want : 0;
                 int best = NG * C::KPB, chunk_groups = NG;
+                if (WHICH == FIRST && sched_q > 0 &&
+                           (sched_q + 1) * p.KB + p.next_KB <= (total_units * p.KB + s_tiles[p.num_local] * p.next_mtiles * p.next_KB) / (int)gridDim.x) {
+                    best = 0;
+                }
 #pragma unroll 1
                 for (int n = 2; n <= MOST && tail_units * n <= slots; ++n) {
                     const int len = (NG + n - 1) / n;
-                    const int cost = (tail_units * n + (int)gridDim.x - 1) / (int)gridDim.x * (len * C::KPB + PIECE_COST + n);
+                    const int cost = (tail_units * n + late + (int)gridDim.x - 1) / (int)gridDim.x * (len * C::KPB + PIECE_COST + n);
                     if (cost < best) { best = cost; chunk_groups = len; }
+                }
+                if (WHICH == SECOND) {
+                    int n = min(max((p.KB + 8) / 16, 1), MOST);
+                    while (n > 1 && tail_units * n > slots) --n;
+                    chunk_groups = min(chunk_groups, (NG + n - 1) / n);
                 }
                 if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = (NG + chunk_groups - 1) / chunk_groups; }
                 __syncwarp();
@@ -531,9 +617,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             };
             // A claim is an atomic round trip (~1 us under load): it is sent while the piece before it is still being loaded.
             // Without whole units the first chunk is the CTA's own number, so that the start does not wait for one.
-            int ahead = (int)blockIdx.x;                                   // lane 0's is the one that counts
-            bool have_ahead = sched_q == 0;
-            const int claim0 = sched_q == 0 ? (int)gridDim.x : 0;
+            // With both GEMMs in one launch everything is claimed, in the order GEMM1's whole units, its pieces, GEMM2's: a unit of
+            // GEMM2 then waits only for work that CTAs that run have taken up, whatever other streams keep from running.
+            int ahead = BOTH ? x.claimed : (int)blockIdx.x;                // lane 0's is the one that counts
+            bool have_ahead = BOTH || sched_q == 0;
+            const int claim0 = BOTH ? -x.claim_base : sched_q == 0 ? (int)gridDim.x : 0;
             auto claim_ahead = [&]() {
                 if (!have_ahead && lane == 0) ahead = claim0 + atomicAdd(claim, 1);
                 have_ahead = true;
@@ -558,7 +646,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
 #pragma unroll 1
             while (ok) {
                 WorkItem wi;
-                wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0};
+                wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0}; wi.tile = 0;
                 const int u_end = (t_unit + 1) * NG;
                 const bool ends_unit = t_lo > t_unit * NG && t_hi == u_end;         // the rest of the range is such a piece
                 if (C::STATIC_TAIL && t_lo < t_hi && !(ends_unit && n_whole < sched_q)) {
@@ -576,6 +664,27 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                         wi.slot = range_owner(wi.ut * NG, flat, parts);        // CTA of the unit's first piece
                         wi.piece = (int)blockIdx.x - wi.slot; wi.pieces = wi.piece + 1;
                     }
+                } else if (BOTH) {
+                    claim_ahead();
+                    int c = __shfl_sync(0xFFFFFFFFu, ahead, 0);
+                    if (c < sched_U0) {
+                        wi.u = c; wi.gb = 0; wi.ge = NG;
+                    } else {
+                        if (!sized) size_chunks();
+                        const int chunk_groups = s_sched[0], pieces = s_sched[1], items = sched_U0 + (total_units - sched_U0) * pieces;
+                        if (c >= items) {                     // the claim carries over into GEMM2's list
+                            x.claimed = ahead - items; x.claim_base += items; x.claim = claim;
+                            // (every CTA ends with one claim too many: behind the last of them nobody watches the routing any more)
+                            if (FUSE && p.met && c == items + (int)gridDim.x - 1 && lane < 2) p.met[lane] = 0;
+                            wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break;
+                        }
+                        c -= sched_U0;
+                        wi.ut = c / pieces; wi.piece = c - wi.ut * pieces; wi.pieces = pieces;
+                        wi.slot = wi.ut * pieces;
+                        wi.u = sched_U0 + wi.ut;
+                        wi.gb = wi.piece * chunk_groups; wi.ge = min(NG, wi.gb + chunk_groups);
+                    }
+                    have_ahead = false;
                 } else if (n_whole < sched_q) {
                     wi.u = n_whole * (int)gridDim.x + (int)blockIdx.x; wi.gb = 0; wi.ge = NG;
                     ++n_whole;
@@ -596,6 +705,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (lane == 0) atomicCAS(p.status, 0, ERR_BAD_SCHEDULE);
                     ok = false; break;
                 }
+                if (BOTH) wi.tile = s_tiles[wi.un.e] + (wi.un.row0 - s_row0[wi.un.e]) / NTOK;
+                // Are GEMM1's rows of the token tile there?
+                const int* const done = WHICH == SECOND ? p.tile_done + wi.tile : nullptr;
+                auto rows_done = [&]() -> bool {
+                    int n = 0;
+                    if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(done) : "memory");
+                    n = __shfl_sync(0xFFFFFFFFu, n, 0);
+                    __syncwarp();        // lane 0's acquire orders the loads of whichever lane issues them
+                    return merged(n >= p.tile_want);
+                };
+                bool there = WHICH == SECOND && rows_done();
+                if (there) wi.tile = -1;                          // (others need not look)
                 if (!publish(wi)) { ok = false; break; }
                 const int gb = wi.gb, ge = wi.ge;
                 const Unit un = wi.un;
@@ -673,6 +794,41 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 const int kb_clear = clears ? kb_first + C::STAGES : kb_first;
                 if (BOXED && !clears && lane < C::STAGES) s_filled[lane] = 128 / C::BOX_ROWS;
                 __syncwarp();
+                if constexpr (WHICH == SECOND) {
+                    // where they are not, the stages take the weights first
+                    if (!there) {
+                        const int npre = min(C::STAGES, kb_end - kb_first);
+                        int st_ = stage; uint32_t ph_ = phase;
+#pragma unroll 1
+                        for (int i = 0; i < npre; ++i) {
+                            if (!mbar_wait_warp(bar_empty + 8 * st_, ph_ ^ 1, p.status, ERR_WAIT_SMEM_EMPTY)) { ok = false; break; }
+                            if (elect_one()) load_weights(st_, kb_first + i);
+                            __syncwarp();
+                            if (++st_ == C::STAGES) { st_ = 0; ph_ ^= 1; }
+                        }
+                        if (!issued) { if (lane == 0) stamp(TR_TMA_FIRST); issued = true; }
+                        const unsigned long long t0 = globaltimer_ns();
+#pragma unroll 1
+                        for (uint32_t it = 1; ok && !there; ++it) {
+                            there = rows_done();
+                            if (!there && (it & 0xFFu) == 0 && __any_sync(0xFFFFFFFFu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) {
+                                if (lane == 0) atomicCAS(p.status, 0, ERR_WAIT_CHUNKS);
+                                ok = false;
+                            }
+                        }
+                        if (!ok) break;
+                        asm volatile("fence.proxy.async.global;" ::: "memory");       // the rows were stored through the generic proxy
+#pragma unroll 1
+                        for (int i = 0; i < npre; ++i) {
+                            if (elect_one()) load_tokens(stage, kb_first + i);
+                            __syncwarp();
+                            if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
+                        }
+                        kb_first += npre;
+                    } else {
+                        asm volatile("fence.proxy.async.global;" ::: "memory");
+                    }
+                }
                 if (!waited) {
                     // early schedule, first item: the (empty) stage ring takes weight tiles while the kernel before this one
                     // still runs, then the wait for it, then the token side of the same stages
@@ -723,14 +879,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (lane == 0) klog_put(0, nk);
                     ++nk;
                     if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
-                    if (!C::STATIC_TAIL && kb + 3 == kb_end && n_whole == sched_q && total_units > sched_U0) claim_ahead();
+                    if (BOTH ? kb + 3 == kb_end : !C::STATIC_TAIL && kb + 3 == kb_end && n_whole == sched_q && total_units > sched_U0) claim_ahead();
                 }
             }
             if (lane == 0) stamp(TR_TMA_LAST);
+            x.stage = stage; x.phase = phase; x.n_item = n_item; x.ok = ok;
             if (!ok) {
                 // gave up: end the list for the other roles (if the queue still moves), then give copies that are
                 // still in flight time to land before the CTA's shared memory goes away
-                WorkItem end_; end_.u = -1; end_.gb = end_.ge = end_.ut = end_.piece = end_.slot = 0; end_.pieces = 1; end_.un = Unit{0, 0, 0, 0};
+                WorkItem end_; end_.u = BOTH ? GAVE_UP : -1; end_.gb = end_.ge = end_.ut = end_.piece = end_.slot = 0; end_.pieces = 1; end_.un = Unit{0, 0, 0, 0}; end_.tile = 0;
                 publish(end_);
                 for (int i = 0; i < 64; ++i) __nanosleep(10000);
             }
@@ -740,11 +897,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         // ------------------------------------------------------------ MMA issuer (whole warp, one elected lane issues)
         {
             constexpr uint32_t idesc = make_idesc_f8(128, NTOK);
-            int stage = 0; uint32_t phase = 0;
-            int ab = 0; uint32_t aphase = 0;
+            int stage = x.stage; uint32_t phase = x.phase;
+            int ab = x.ab; uint32_t aphase = x.aphase;
             bool ok = true, seen = false;
             int nk = 0;
-            int n_item = 0;
+            int n_item = x.n_item;
             WorkItem wi;
 #pragma unroll 1
             while (ok && wq_fetch(n_item++, wi, ok)) {
@@ -832,6 +989,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                 }
             }
             if (lane == 0) stamp(TR_MMA_LAST);
+            x.stage = stage; x.phase = phase; x.ab = ab; x.aphase = aphase; x.n_item = n_item; x.ok = ok;
         }
         __syncwarp();
     } else if constexpr (C::TOK_ON_M) {
@@ -922,10 +1080,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
         const uint32_t tlane = (uint32_t)(quarter * 32) << 16;
         volatile int* const s_last = s_flag + 8;
         const uint32_t my_red = bar_red + 8 * (C::TOK_ON_M ? quarter : grp_id);
-        int stage = 0; uint32_t phase = 0;
-        int ab = 0; uint32_t aphase = 0;
-        uint32_t rphase = 0;
-        int rbuf = 0;                                  // half of s_red the next epilogue uses
+        int stage = x.stage; uint32_t phase = x.phase;
+        int ab = x.ab; uint32_t aphase = x.aphase;
+        uint32_t rphase = x.rphase;
+        int rbuf = x.rbuf;                             // half of s_red the next epilogue uses
         bool ok = true, seen = false;
         int ng = 0, nu = 0;
         int blk = 0;                                   // tokens on M: K blocks folded so far
@@ -940,10 +1098,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
             return r;
         };
 
-        int n_item = 0;
+        int n_item = x.n_item;
         WorkItem wi;
-        if (!(!C::TOK_ON_M && G1 && p.copied)) { pdl_wait(); pdl_launch(); }
-        if (FUSE && p.met && blockIdx.x == 0 && ptid < 2) p.met[ptid] = 0;
+        if ((WHICH != SECOND || x.fresh) && !(!C::TOK_ON_M && G1 && p.copied)) { pdl_wait(); pdl_launch(); }
+        if (FUSE && !BOTH && p.met && blockIdx.x == 0 && ptid < 2) p.met[ptid] = 0;
 #pragma unroll 1
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;
@@ -1181,7 +1339,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     for (int k = 0; k < ACC_VECS; ++k) __stcg(slot + k * C::NPT, make_float4(acc4(k)[0], acc4(k)[1], acc4(k)[2], acc4(k)[3]));
                 };
                 int* const arrived = p.sk_count + 4 * wi.ut;
-                if constexpr (C::STATIC_TAIL) {
+                constexpr bool ENDS = C::STATIC_TAIL || WHICH == FIRST;          // the piece that ends a unit finishes it
+                if constexpr (ENDS) {
                     // ---- piece of a split unit, static ranges: the piece that ends the unit finishes it.  The others store
                     // their partial sums and count their warps in with a release - no meeting of the warps, no answer to
                     // wait for; the finisher waits (bounded) for that count.
@@ -1239,7 +1398,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     if (seen_pieces != wi.pieces - 1) continue;
                     __threadfence();
                 }
-                if (!C::STATIC_TAIL && wi.piece != wi.pieces - 1) {
+                if (!ENDS && wi.piece != wi.pieces - 1) {
                     const float4* src = slot_of(wi.pieces - 1);
 #pragma unroll
                     for (int k = 0; k < ACC_VECS; ++k) {
@@ -1441,15 +1600,63 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CU
                     }
                 }
             }
+            if (WHICH == FIRST) {
+                // this warp's part of the unit's rows is stored: other CTAs load them by TMA once every warp has counted in
+                asm volatile("fence.proxy.async.global;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(p.tile_done + wi.tile) : "memory");
+            }
             if (ptid == 0) klog_put(5, nu++);
         }
+        x.stage = stage; x.phase = phase; x.ab = ab; x.aphase = aphase; x.rphase = rphase; x.rbuf = rbuf; x.n_item = n_item; x.ok = ok;
     }
 
     if (warp >= 4 && threadIdx.x == 128) stamp(TR_EPILOGUE);
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, C::TMEM_COLS); }
-    if (threadIdx.x == 0) stamp(TR_EXIT);
+}
+
+template <int NTOK, bool G1, bool G4 = false, bool PART = false, bool FUSE = false>
+__global__ void __launch_bounds__(GemmCfg<NTOK, G1>::NTHREADS, 1)
+gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_b0,
+            const __grid_constant__ CUtensorMap tm_b1, const __grid_constant__ CUtensorMap tm_s0,
+            const __grid_constant__ CUtensorMap tm_s1, const GemmParams p) {
+    using C = GemmCfg<NTOK, G1>;
+    extern __shared__ uint8_t smem_raw[];
+    GemmCta x;
+    gemm_setup<C>(x, smem_raw);
+    if (p.trace && threadIdx.x == 0) p.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = (long long)globaltimer_ns();
+    gemm_init<C, helper_warps<C::TOK_ON_M, G4>()>(x, tm_w, tm_b0, G1 ? tm_b0 : tm_b1);
+    gemm_roles<NTOK, G1, G4, PART, FUSE, SOLE>(x, tm_w, tm_b0, tm_b1, tm_s0, tm_s1, p);
+    gemm_teardown<C>(x);
+    if (p.trace && threadIdx.x == 0) p.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = clock64() - x.t_entry;
+}
+
+// parts: 1 GEMM1, 2 GEMM2, 3 both - in two launches for the stage times of the profile, with the same pieces and the same bits.
+template <int NTOK, bool FUSE>
+__global__ void __launch_bounds__(GemmCfg<NTOK, true, true>::NTHREADS, 1)
+gemm_both_kernel(const __grid_constant__ CUtensorMap tm_w13, const __grid_constant__ CUtensorMap tm_a,
+                 const __grid_constant__ CUtensorMap tm_w2, const __grid_constant__ CUtensorMap tm_hi,
+                 const __grid_constant__ CUtensorMap tm_lo, const GemmParams p1, const GemmParams p2, const int parts) {
+    using C = GemmCfg<NTOK, true, true>;
+    using C2 = GemmCfg<NTOK, false, true>;
+    static_assert(C::STAGE_BYTES == C2::STAGE_BYTES && C::SC_OFF == C2::SC_OFF && C::STAGES == C2::STAGES && C::SMEM_BYTES == C2::SMEM_BYTES &&
+                  C::BUFCOLS == C2::BUFCOLS && C::NACC == C2::NACC && C::KPB == C2::KPB && C::NTHREADS == C2::NTHREADS &&
+                  C::EMPTY_COUNT == C2::EMPTY_COUNT && C::RED_BYTES == C2::RED_BYTES, "the rings are carried over");
+    extern __shared__ uint8_t smem_raw[];
+    GemmCta x;
+    gemm_setup<C>(x, smem_raw);
+    if (p1.trace && threadIdx.x == 0) {
+        const long long now = (long long)globaltimer_ns();
+        p1.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
+        p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
+    }
+    gemm_init<C, 0>(x, tm_w13, tm_a, tm_w2);
+    if (parts & 1) {
+        gemm_roles<NTOK, true, false, false, false, FIRST>(x, tm_w13, tm_a, tm_a, tm_a, tm_a, p1);
+        x.fresh = false;
+    }
+    if (x.ok && (parts & 2)) gemm_roles<NTOK, false, false, false, FUSE, SECOND>(x, tm_w2, tm_hi, tm_lo, tm_hi, tm_lo, p2);
+    gemm_teardown<C>(x);
+    if (p2.trace && threadIdx.x == 0) p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = clock64() - x.t_entry;
 }
 
 }  // namespace b200moe

@@ -196,6 +196,60 @@ torch.save(outs, sys.argv[1])
         assert float((a != b).float().mean()) < 0.05
 
 
+@pytest.mark.parametrize("T,tile", [(1, 0), (5, 0), (40, 0), (129, 0), (288, 0), (700, 16), (500, 32)])
+def test_both_gemms_in_one_launch(ds_weights, T, tile):
+    """Narrow tiles over weights that L2 cannot hold run both GEMMs in one kernel: few units that are all cut (1 and 5 tokens), whole
+    ones behind both front ends, several token tiles per expert (forced tiles).  Against the two launches of the 128-token
+    family: the sums agree to the order of fp32 additions, so an output differs by a unit in the last place of bf16 (2^-8) where a
+    value between the GEMMs falls to the other side of an e4m3 rounding (a few in 10000; the 2-norm measured is 4e-4 at most).
+    The same bits from a poisoned workspace, with stage times (two launches), with the combine fused and from a replayed graph."""
+    import test_gpu_edges as edges
+    from justgoal_b200 import MoELayer
+    d = _inputs(T, ds_weights, seed=40 + T)
+    args = util.op_args(d)
+    layer = MoELayer(I.DEEPSEEK_V3)
+    layer.set_token_tile(tile)
+    assert int(layer.layout(T).token_tile) <= 32
+    n = 3 if T <= 128 else 5
+    assert layer.launches_per_forward(T) == n == edges._kernels_launched(lambda: layer.forward(*args))
+    out = layer.forward(*args).clone()
+    torch.cuda.synchronize()
+    assert layer.status(T) == 0
+    wide = MoELayer(I.DEEPSEEK_V3)
+    wide.set_token_tile(128)
+    assert wide.launches_per_forward(T) == n + 1
+    ref = wide.forward(*args)
+    rep = O.compare_output(out, ref, util.ATOL, util.RTOL)
+    assert rep["finite"] and rep["fail_frac"] == 0.0, rep
+    assert float((out.float() - ref.float()).norm()) <= 2e-3 * float(ref.float().norm())
+
+    def same(other):
+        torch.cuda.synchronize()
+        assert layer.status(T) == 0
+        assert torch.equal(out.view(torch.int16), other.view(torch.int16))
+
+    layer.workspace(T).fill_(0xFF)
+    same(layer.forward(*args))
+    layer.profile_enable(2)
+    same(layer.forward(*args))
+    assert all(v >= 0 for v in layer.profile_read(0).values())
+    layer.profile_enable(0)
+    layer.set_fused_combine(True)
+    assert layer.launches_per_forward(T) == n - 1 == edges._kernels_launched(lambda: layer.forward(*args))
+    layer.workspace(T).fill_(0xFF)
+    for _ in range(3):
+        fused = layer.forward(*args)
+    same(fused)
+    layer.set_fused_combine(False)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        replayed = layer.forward(*args)
+    for _ in range(3):
+        replayed.fill_(7.0)
+        g.replay()
+    same(replayed)
+
+
 @pytest.mark.parametrize("T,tile", [(901, 16), (901, 32), (901, 64), (901, 128), (64, 0), (3, 0), (4096, 0)])
 def test_forwards_repeat_their_bits(ds_weights, T, tile):
     """Sixty forwards of every tile family give the bits of the first: a read of a stage's scales that the stage's release does
