@@ -82,11 +82,11 @@ EncodeTiledFn get_encode() {
 // B200MOE_PDL=0): the next kernel's prologue overlaps the tail of the one before, and each
 // kernel calls griddepcontrol.wait before it touches anything an earlier kernel wrote.
 // B200MOE_PDL is a bit mask over the launch sites (1 route/count, 2 permute, 4 gather, 8 GEMM1,
-// 16 GEMM2, 32 combine); default: all.
-enum : int { PDL_ROUTE = 1, PDL_PERMUTE = 2, PDL_GATHER = 4, PDL_GEMM1 = 8, PDL_GEMM2 = 16, PDL_COMBINE = 32 };
+// 16 GEMM2, 32 combine, 64 the activation quantiser); default: all.
+enum : int { PDL_ROUTE = 1, PDL_PERMUTE = 2, PDL_GATHER = 4, PDL_GEMM1 = 8, PDL_GEMM2 = 16, PDL_COMBINE = 32, PDL_QUANT = 64 };
 int pdl_mask() {
     static int v = -1;
-    if (v < 0) { const char* e = getenv("B200MOE_PDL"); v = e ? atoi(e) : 63; }
+    if (v < 0) { const char* e = getenv("B200MOE_PDL"); v = e ? atoi(e) : 127; }
     return v;
 }
 
@@ -1188,15 +1188,18 @@ int b200moe_quantize_1x128(const void* x_bf16, int T, int H, void* q_e4m3, float
     // rows of few groups: more tokens, until all threads of a CTA have groups to work on (40000 x 128: eight tokens 25.1 us,
     // 64 tokens 4.7 us; 40000 x 512: 17.3 us with eight, 12.0 with 16)
     while (tpc * gpc < QUANT_TURN) tpc *= 2;
+    // Four tokens while eight leave fewer than eight CTAs per SM: the last CTAs of an SM are a smaller part of its work.  Eight / four, us: 3000 x
+    // 7168 14.0 / 13.0, 4096: 17.7 / 17.6, 6000: 26.9 / 24.8, 8192: 33.5 / 33.6, 14107: 53.3 / 55.8; 3000 x 4096 10.2 / 8.5, 6000: 15.2 / 13.6, 14107: 31.3 / 31.7.
+    if (tpc == QUANT_TOKENS && tpc / 2 * gpc >= QUANT_TURN && ctas(tpc, parts) < 8ll * sms) tpc /= 2;
     while (ctas(tpc, parts) < 2ll * sms && tpc > 1) tpc /= 2;
     int tsh = 0;
     while (1 << tsh < tpc) ++tsh;
     const dim3 grid((T + tpc - 1) / tpc, (groups + gpc - 1) / gpc);
     const bool wide = !((reinterpret_cast<uintptr_t>(x_bf16) & 31) || (reinterpret_cast<uintptr_t>(q_e4m3) & 15));
     auto* kern = wide ? quantize_1x128_kernel<true> : quantize_1x128_kernel<false>;
-    kern<<<grid, QUANT_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x_bf16), T, H, tsh, gpc, static_cast<uint8_t*>(q_e4m3), scale);
-    CU_TRY(cudaGetLastError());
+    g_call_pdl = pdl_mask() & PDL_QUANT;
+    CU_TRY(launch_k(PDL_QUANT, kern, grid, dim3(QUANT_THREADS), 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x_bf16), T, H,
+                    tsh, gpc, static_cast<uint8_t*>(q_e4m3), scale));
     return 0;
 }
 

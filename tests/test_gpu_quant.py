@@ -96,6 +96,50 @@ def test_quantiser_blocks_and_alignment(T, H, off):
     assert rc == 0 and torch.equal(qb[8:].cpu().view(T, H), q_ref.view(torch.uint8))
 
 
+@pytest.mark.parametrize("T,H", [(9471, 2048), (9473, 2048), (2369, 2048), (9472, 1024), (1187, 7168)])
+def test_quantiser_tokens_of_a_cta(T, H):
+    """Both sides of the lines between two, four and eight tokens per CTA (eight CTAs per SM of eight tokens, two of four), and rows of
+    few groups, whose CTAs keep eight."""
+    from justgoal_b200 import quantize_1x128
+    x = _case(T, H, seed=T)
+    q_ref, s_ref = I.quantize_rows_1x128(x)
+    q, s = quantize_1x128(x.cuda())
+    torch.cuda.synchronize()
+    assert torch.equal(s.cpu().view(torch.int32), s_ref.view(torch.int32))
+    assert torch.equal(q.cpu().view(torch.uint8), q_ref.view(torch.uint8))
+
+
+def test_quantiser_between_its_neighbours():
+    """The quantiser may start under the kernel that writes its input and lets the layer start under itself: a chain of copy,
+    quantiser, quantiser into the same input's other half and forward, queued without a host wait, gives the bytes of each call made
+    alone."""
+    from justgoal_b200 import MoELayer, quantize_1x128
+    shape, T = I.TINY_DS, 128
+    d = util.to_cuda(I.make_inputs(shape, T, seed=12))
+    layer = MoELayer(shape)
+    rest = [d[n] for n in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale", "local_expert_offset",
+                           "routed_scaling_factor")]
+    src = [_case(T, shape.hidden, seed=k).cuda() for k in range(3)]
+    want = []
+    for x in src:
+        q, s = quantize_1x128(x)
+        torch.cuda.synchronize()
+        out = layer.forward(d["routing_logits"], d["routing_bias"], q, s, *rest).clone()
+        torch.cuda.synchronize()
+        want.append((q.view(torch.uint8).clone(), s.clone(), out))
+    x, got = torch.empty_like(src[0]), []
+    for k in range(12):
+        x.copy_(src[k % 3])
+        q, s = quantize_1x128(x)
+        x.fill_(100.0)
+        quantize_1x128(x)
+        got.append((q.view(torch.uint8), s, layer.forward(d["routing_logits"], d["routing_bias"], q, s, *rest)))
+    torch.cuda.synchronize()
+    for k, (q, s, out) in enumerate(got):
+        assert torch.equal(q, want[k % 3][0]) and torch.equal(s, want[k % 3][1])
+        assert torch.equal(out.view(torch.int16), want[k % 3][2].view(torch.int16))
+
+
 def test_quantiser_feeds_the_operator():
     """bf16 activations -> quantiser kernel -> layer: same output as with host-quantised inputs."""
     from justgoal_b200 import MoELayer, quantize_1x128
