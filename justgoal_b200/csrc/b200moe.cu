@@ -133,37 +133,64 @@ int make_map(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uin
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Tokens per GEMM tile, from shapes only (never from data): the expected number of rows per
-// expert under uniform routing.
 // slices of SLICE_PAIRS (token, expert) pairs = CTAs of the permutation kernel (at least one)
 int num_slices(const b200moe_config& c, int T) {
     const long long n = (long long)T * c.top_k;
     return n <= 0 ? 1 : (int)((n + SLICE_PAIRS - 1) / SLICE_PAIRS);
 }
 
-// The 16-token tile wins while an expert sees fewer rows than the tile holds; above that the 128-token tile (tokens on M, one
-// N = 256 MMA per K step) is ahead of every narrower one although most of its rows are padding - the step is bound by the
-// weight stream, and the narrow tiles' weights-on-M MMAs are short of shared-memory bandwidth from 64 columns on.  The 64-token
-// tile is never the best choice; it stays available through b200moe_set_token_tile.
-// us per forward with the present kernels, tile 16 / 32 / 64 / 128, by expected rows per expert (r); one routing per count:
-//   32 of 256 experts       r=4 159/163/198/164, 6 160/176/201/180, 7 172/177/209/181, 8 180/174/211/185, 9 177/170/203/183, 10 188/197/219/194,
-//                           12 201/204/248/207, 16 233/227/253/217, 32 359/307/309/229, 56 500/399/357/278
-//   128 of 256 experts      r=6 665/728/880/632, 7 709/764/913/681, 8 774/753/947/681, 10 863/868/971/701
-//   16 of the 4096-wide     r=4 65/71/82/80, 7 67/72/84/81, 9 69/75/87/86, 10 69/75/88/85, 16 78/77/89/86
-//   8 of a 4096 x 4096      r=4 75/82/102/90, 8 76/83/101/90, 9 78/82/103/91, 12 95/90/107/96, 16 99/90/110/96
-// The lines at 7 and 9 rows were drawn with earlier kernels on the first of these shapes and are a compromise now: the best change
-// from narrow to 128 comes at about 14 rows there, at about 5 with many units (128 experts; the narrow tiles lose 12 to 18 % at 6 to
-// 9) and above 16 with few (where the 128-token tile is 20 % behind at 10).  The number of units should enter; it does not yet.
-// The estimate is that of a forward that routes itself.  Every token of forward_routed has a local expert, so an expert sees
-// more rows than estimated (DeepSeek-V3 routing, 32 local experts: twice as many), and calls of 150 to 290 tokens run a slower
-// tile than they could (32 local, tile 16 / 32 / 128: 150 tokens 229 / 215 / 212 us, 200: 250 / 245 / 217, 288: 287 / 274 / 222).
-int pick_token_tile(const b200moe_ctx* h, int T) {
-    if (h->token_tile) return h->token_tile;
+// Weights that L2 (126 MB) cannot hold: a call with few rows per expert is bound by streaming them from HBM.
+bool weights_stream(const b200moe_config& c) {
+    return (size_t)c.num_local_experts * 3 * c.hidden * c.intermediate >= ((size_t)128 << 20);
+}
+
+// Tokens per GEMM tile, from shapes only (never from data): by the expected number of rows per expert under uniform routing, 16 up
+// to `to32`, 32 up to `to128`, then 128.  A narrow tile reads its weights once as long as an expert's rows fit it, and runs both
+// GEMMs in one launch; above that the 128-token tile (tokens on M, one N = 256 MMA per K step) is ahead of every narrower one although
+// most of its rows are padding: the narrow tiles' weights-on-M MMAs are short of shared-memory bandwidth from 64 columns on.  The
+// 64-token tile is never the best choice; it stays available through b200moe_set_token_tile.
+// How far the narrow tiles reach depends on how even the loads are.  DeepSeek routing (biased, by groups) gives some experts three to
+// four times the mean, softmax routing seldom twice; and on how many units (experts x weight tiles) a CTA has: with many, the few
+// experts that need a second tile cost little else.  us per forward, tile 16 / 32 / 128, by expected rows per expert (r):
+//   32 of 256 experts (3.5 units per SM)    r=7 199/202/220, 8 203/207/224, 9 211/213/221, 9.7 220/228/220, 10.6 222/228/221
+//   64 of 256 (6.9)                         r=6 324/353/339, 7 362/392/359, 8 370/364/342, 9 404/404/365
+//   128 of 256 (14)                         r=6 644/678/645, 7 637/670/643, 8 729/723/657, 9 738/759/693
+//   256 of 256 (28)                         r=4 1122/1253/1145, 6 1276/1362/1250, 7 1309/1359/1259, 9 1509/1534/1311
+//   softmax routing, 8 of the 4096-wide (0.6)   r=14 49/53/60, 20 54/53/60, 25 57/53/59, 32 64/62/60
+//   16 of the 4096-wide (1.3)               r=9 68/72/85, 14 70/72/86, 18 80/72/86, 25 88/76/88, 32 93/79/88, 40 113/108/89
+//   32 (2.6)                                r=14 116/125/139, 20 152/128/142, 25 172/136/143, 32 204/178/144
+//   64 (5.2)                                r=9 208/238/247, 14 224/229/247, 20 295/246/252, 25 322/248/253, 32 362/320/257
+//   128 (10.4)                              r=6 388/471/455, 10 402/470/460, 14 471/497/467, 20 591/492/471
+// Layers whose weights L2 holds keep the lines at 7 and 9 rows, drawn with two launches.
+struct TileLines { double to32, to128; };
+TileLines tile_lines(const b200moe_ctx* h) {
     const b200moe_config& c = h->cfg;
-    const double avg = (double)T * c.top_k / c.num_experts;
-    if (avg <= 7.0) return 16;
-    if (avg <= 9.0) return 32;
-    return 128;
+    const double units = (double)c.num_local_experts * (c.intermediate / 128) / h->num_sms;
+    if (!weights_stream(c)) return {7.0, 9.0};
+    if (c.routing_mode == B200MOE_ROUTING_DEEPSEEK) return units > 5.0 ? TileLines{7.0, 7.0} : TileLines{7.0, 9.0};
+    return units > 8.0 ? TileLines{12.0, 12.0} : TileLines{14.0, 25.0};
+}
+// Every token of a routed call has a local expert: its experts see more rows than those of a forward that routes itself, by one over
+// the share of all tokens that have one (by groups: that one of the `local` groups is among the topk_group kept ones).
+// us, routed, tile 16 / 32 / 128 (the rule's estimate of r behind the token count): 32 of 256 experts 112 (7) 184/186/202, 144 (9) 199/200/211, 160
+// (10) 216/220/216, 250 (16) 276/253/223; 64 of 256: 160 (6) 323/338/332, 200 (8) 363/367/347; softmax, 16 of the 4096-wide: 147 (14) 69/70/85, 262 (25)
+// 85/72/87, 300 (29) 91/78/89, 400 (38) 111/107/89; 64: 224 (14) 229/233/246, 300 (19) 280/246/255.
+double routed_share(const b200moe_config& c) {
+    double none = 1.0;
+    if (c.routing_mode == B200MOE_ROUTING_DEEPSEEK) {
+        const int local = (c.num_local_experts * c.n_group + c.num_experts - 1) / c.num_experts;
+        for (int i = 0; i < c.topk_group; ++i) none *= c.n_group - local - i > 0 ? (double)(c.n_group - local - i) / (c.n_group - i) : 0.0;
+    } else {
+        for (int i = 0; i < c.top_k; ++i) none *= 1.0 - (double)c.num_local_experts / c.num_experts;
+    }
+    return 1.0 - none;
+}
+int pick_token_tile(const b200moe_ctx* h, int T, bool routed = false) {
+    if (h->token_tile) return h->token_tile;
+    const TileLines lines = tile_lines(h);
+    double avg = (double)T * h->cfg.top_k / h->cfg.num_experts;
+    if (routed && weights_stream(h->cfg)) avg /= routed_share(h->cfg);
+    return avg <= lines.to32 ? 16 : avg <= lines.to128 ? 32 : 128;
 }
 
 // 128-token tiles: do most tiles hold fewer than 128 rows?  Below one tile's worth of expected rows per expert they do, and
@@ -180,8 +207,8 @@ bool tiles_mostly_part_full(const b200moe_config& c, int T) {
 // GEMM1 reads its token rows by TMA gather (b200moe_set_tma_gather); behind a separate permutation there is then no
 // gather launch (the one-launch front ends copy the rows all the same).
 bool use_pairs(const b200moe_ctx* h, int ntok);
-bool gathers_by_tma(const b200moe_ctx* h, int T) {
-    const int ntok = pick_token_tile(h, T);
+bool gathers_by_tma(const b200moe_ctx* h, int T, bool routed = false) {
+    const int ntok = pick_token_tile(h, T, routed);
     return ntok == 128 && !use_pairs(h, ntok) && h->tma_gather;
 }
 
@@ -207,7 +234,7 @@ int narrow_slots(const b200moe_config& c, int ntok) {
 // pieces that a small layer makes is what this library has always stated, and the fused combine's bits go with them.
 bool use_both(const b200moe_ctx* h, int ntok) {
     const b200moe_config& c = h->cfg;
-    return ntok <= 32 && (size_t)c.num_local_experts * 3 * c.hidden * c.intermediate >= ((size_t)128 << 20) && narrow_slots(c, ntok) >= 2;
+    return ntok <= 32 && weights_stream(c) && narrow_slots(c, ntok) >= 2;
 }
 
 size_t sk_partial_bytes(const b200moe_config& c, int grid, int ntok) {
@@ -228,8 +255,7 @@ int rows_capacity_for(const b200moe_config& c, int T) {
 
 // Token tiles of a call with narrow tiles, at most: full ones and a part-full one per expert.
 size_t max_narrow_tiles(const b200moe_ctx* h, int T) {
-    const int ntok = pick_token_tile(h, T);
-    return ntok > 32 ? 0 : (size_t)(rows_capacity_for(h->cfg, T) / ntok + h->cfg.num_local_experts);
+    return pick_token_tile(h, T) > 32 ? 0 : (size_t)(rows_capacity_for(h->cfg, T) / 16 + h->cfg.num_local_experts);
 }
 
 void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
@@ -259,12 +285,15 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     L->act_lo = take(rows * c.intermediate);
     L->act_scale = take((size_t)(c.intermediate / 128) * rows * 4);
     L->y = take(rows * c.hidden * 2);
-    L->sk_partial = take(sk_partial_bytes(c, h->num_sms, (int)pick_token_tile(h, T)));
+    // (room for a routed call, which may take a wider tile than this one)
+    size_t partial = sk_partial_bytes(c, h->num_sms, pick_token_tile(h, T));
+    const size_t partial_routed = sk_partial_bytes(c, h->num_sms, pick_token_tile(h, T, true));
+    L->sk_partial = take(partial > partial_routed ? partial : partial_routed);
     L->trace = take((size_t)2 * h->num_sms * TRACE_SLOTS * 8 + 2 * 8 * KLOG_N * 8);   // [GEMM1 | GEMM2][CTA][slot], then K-block logs
     // A workspace serves every smaller call, and the counters above exist with narrow tiles only: as much room as the largest
     // call with them takes.
     if (pick_token_tile(h, T) == 128) {
-        const int narrow_T = (int)(9ll * c.num_experts / c.top_k);
+        const int narrow_T = (int)(tile_lines(h).to128 * c.num_experts / c.top_k);
         take((size_t)narrow_T * ((c.hidden + 255) / 256) * 4 + ((size_t)rows_capacity_for(c, narrow_T) / 16 + El) * 4 + 512);
     }
     L->rows_cap = rows;
@@ -860,7 +889,7 @@ int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
     // [count, permute, gather | all in one launch for small T], gemm1, gemm2, combine
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (use_both(h, pick_token_tile(h, num_tokens)) ? 1 : 0);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens, true) ? 1 : 0)) - (use_both(h, pick_token_tile(h, num_tokens, true)) ? 1 : 0);
     return 0;
 }
 
@@ -933,6 +962,7 @@ int b200moe_forward_routed(b200moe_handle h, const int32_t* topk_idx, const floa
     b200moe_ws_layout L;
     int rc = check_ws(h, T, workspace, workspace_bytes, &L);
     if (rc) return rc;
+    L.token_tile = (size_t)pick_token_tile(h, T, true);
     const b200moe_config& c = h->cfg;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* ws = static_cast<uint8_t*>(workspace);

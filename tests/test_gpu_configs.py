@@ -261,3 +261,47 @@ def test_forwards_repeat_their_bits(ds_weights, T, tile):
     first = layer.forward(*args).clone()
     outs = [torch.equal(first.view(torch.int16), layer.forward(*args).view(torch.int16)) for _ in range(60)]
     assert layer.status(T) == 0 and all(outs)
+
+
+@pytest.mark.parametrize("shape,tiles", [
+    (I.DEEPSEEK_V3, {224: 16, 225: 32, 288: 32, 289: 128}),
+    (I.DEEPSEEK_V3.with_local(64), {224: 16, 225: 128}),
+    (I.QWEN3_MOE, {224: 16, 225: 32, 400: 32, 401: 128}),
+    (I.QWEN3_MOE.with_local(128), {192: 16, 193: 128}),
+    (I.TINY_DS, {56: 16, 57: 32, 72: 32, 73: 128}),                # its weights fit into L2
+])
+def test_token_tile_lines(shape, tiles):
+    """Both sides of every line, and a workspace that serves every smaller call whatever tile that picks."""
+    from justgoal_b200 import MoELayer
+    layer = MoELayer(shape)
+    assert {T: int(layer.layout(T).token_tile) for T in tiles} == tiles
+    sizes = [int(layer.layout(T).total_bytes) for T in range(1, 520)]
+    for bucket in (64, 128, 256, 512):
+        assert max(sizes[:bucket]) == sizes[bucket - 1]
+
+
+@pytest.mark.parametrize("T", [100, 224, 225, 400])
+def test_qwen3_share_with_narrow_tiles(T):
+    """One rank's share of the softmax-routed shape on both sides of the line between its narrow tiles, against the oracle."""
+    _share_check(I.QWEN3_MOE, T, 48, 1.0, seed=20 + T)
+
+
+@pytest.mark.parametrize("T", [112, 113, 145])
+def test_routed_calls_take_the_tile_of_their_rows(ds_weights, T):
+    """A routed call's experts see about twice the rows (32 of 256 experts), so it leaves the narrow tiles earlier than a forward that
+    routes itself: the bits are those of the tile that its rows ask for, the launches those of a captured call."""
+    import test_gpu_edges as edges
+    from justgoal_b200 import MoELayer
+    d = _inputs(T, ds_weights, seed=60 + T)
+    layer, forced = MoELayer(I.DEEPSEEK_V3), MoELayer(I.DEEPSEEK_V3)
+    tile = {112: 16, 113: 32, 145: 128}[T]
+    forced.set_token_tile(tile)
+    assert int(layer.layout(T).token_tile) == 16
+    idx, w = layer.route(d["routing_logits"], d["routing_bias"], 2.5)
+    args = (idx, w, d["hidden_states"], d["hidden_states_scale"], *[d[n] for n in (
+        "gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")], 0)
+    layer.workspace(T).fill_(0xFF)
+    got, want = layer.forward_routed(*args).clone(), forced.forward_routed(*args)
+    torch.cuda.synchronize()
+    assert layer.status(T) == 0 and torch.equal(got, want)
+    assert layer.launches_routed(T) == edges._kernels_launched(lambda: layer.forward_routed(*args)) == (3 if T <= 128 else 6 if tile == 128 else 5)
