@@ -92,7 +92,7 @@ typedef struct b200moe_ws_layout {
                              delivered for output columns 256 j + {0, 128} + [32 q, 32 q + 32) - the combine
                              fused into the GEMM2 epilogue                                    */
     size_t rows_cap;      /* number of rows the row-indexed buffers hold                   */
-    size_t token_tile;    /* tokens per GEMM tile chosen for this T                        */
+    size_t token_tile;    /* tokens per GEMM tile of a b200moe_forward over T tokens       */
     size_t total_bytes;
 } b200moe_ws_layout;
 
@@ -282,11 +282,12 @@ int b200moe_status(b200moe_handle h, const void* workspace, void* cuda_stream, i
  * Measured slower than the separate kernel at 64 tokens; kept for hosts that count launches. */
 int b200moe_set_fused_combine(b200moe_handle h, int on);
 
-/* Token tile of the GEMMs.  0 (default): chosen from the token count - 16 tokens while an expert
- * expects about seven rows or fewer, 128 from about nine (measured crossovers on the DeepSeek-V3
- * shape), 32 in between.  16 / 32 / 64 / 128 force one kernel family for every token count (tuning
- * and tests; every size gives the same results within the operator's tolerance).  The workspace
- * size depends on the tile: query b200moe_workspace_bytes again after changing it. */
+/* Token tile of the GEMMs.  0 (default): chosen from the shape and the token count by the rows an
+ * expert expects - 16, then 32, then 128 (lines from measurements; a routed call's tokens all have a
+ * local expert, and b200moe_forward_routed counts them accordingly).  16 / 32 / 64 / 128 force one
+ * kernel family for every token count (tuning and tests; every size gives the same results within the
+ * operator's tolerance).  The workspace size depends on the tile: query b200moe_workspace_bytes again
+ * after changing it. */
 int b200moe_set_token_tile(b200moe_handle h, int tokens);
 
 /* TMA-gathered token rows (off by default).  on != 0: with 128-token tiles GEMM1 reads its token

@@ -92,10 +92,9 @@ int pdl_mask() {
 
 // Up to 2048 tokens all launches overlap, beyond that GEMM2 and the combine only: with GEMM1 behind a gather that it could not
 // stream weights under, early-resident dependents slowed calls of many thousands of tokens down by 2 to 5 %.  A shape-only decision.
-// With the present kernels (GEMM1 streams its first weights there too) that is no longer so, and the line costs 1 to 5 % beyond it.
-// Overlap of GEMM2 and the combine alone / of all launches, us: 16 experts of the 4096-wide shape 513 tokens 102 / 90, 2048
-// 135 / 121, 3000 170 / 162, 4096 204 / 201, 8192 322 / 308; 32 of 256 experts 513 tokens 240 / 222, 2048 314 / 294, 4096 408 / 387, 6000
-// 492 / 478, 12000 768 / 748; 128 of 256 experts 2048 tokens 1330 / 1299, 4000 1704 / 1699, 6000 2324 / 2289.
+// With the present kernels (GEMM1 streams its first weights there too) the two forms are level under the power limit: GEMM2 and the
+// combine alone / all launches, us, passes back to back: 32 of 256 experts 3000 tokens 426 / 429, 4096: 525 / 518, 14107: 1172 / 1186; 16 experts of the
+// 4096-wide shape 4096: 194 / 195; 64 of them 4000: 598 / 598.  Up to 2048 the overlap pays: 513 tokens of these shapes 240 / 222 and 102 / 90.
 thread_local int g_call_pdl = 0;
 inline void set_call_pdl(int num_tokens) { g_call_pdl = num_tokens <= 2048 ? pdl_mask() : pdl_mask() & (PDL_GEMM2 | PDL_COMBINE); }
 
