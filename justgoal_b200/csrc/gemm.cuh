@@ -590,7 +590,8 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
             volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, [1] pieces
             bool sized = false;
             auto size_chunks = [&]() {
-                constexpr int PIECE_COST = C::TOK_ON_M ? (PART ? 6 : 12) : WHICH == FIRST ? 4 : 8, MOST = 8;
+                constexpr int MOST = 8;
+                const int PIECE_COST = C::TOK_ON_M ? (PART ? 6 : 12) : WHICH == FIRST ? 4 : WHICH == SECOND && sched_q == 0 ? 5 : 8;
                 static_assert(MOST <= MAX_PIECES, "arrivals of a split unit");
                 const int tail_units = total_units - sched_U0;
                 const int slots = (int)gridDim.x * (BOTH ? p.slots : (NG + C::CHUNK_GROUPS - 1) / C::CHUNK_GROUPS);           // what sk_partial holds
