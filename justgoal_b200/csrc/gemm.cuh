@@ -612,7 +612,17 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                     while (n > 1 && tail_units * n > slots) --n;
                     chunk_groups = min(chunk_groups, (NG + n - 1) / n);
                 }
-                if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = (NG + chunk_groups - 1) / chunk_groups; }
+                // Units between half of the CTAs that can start at once and 5/8 of all are dealt out as one range per claim, which may
+                // end one unit and start the next: pieces of half a unit would be more than there are CTAs, and whole units leave a
+                // third of them without loads.  Pieces or whole / ranges, DeepSeek-V3 shape, median us: 4 experts (64 units, 116
+                // CTAs start at once) 48.9 / 44.3, 5 (80 units) 57.7 / 49.1; above the line 6 (96 units) 60.1 / 63.9, 7 (112)
+                // 67.9 / 68.7: GEMM2's loads fill what whole units leave.  Ranges from a third up were level (48 units 39.2 / 39.6).
+                int pieces = (NG + chunk_groups - 1) / chunk_groups;
+                const int parts = (int)gridDim.x - late;
+                if (WHICH == FIRST && sched_q == 0 && 2 * tail_units > parts && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= parts) {
+                    chunk_groups = parts; pieces = 0;
+                }
+                if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = pieces; }
                 __syncwarp();
                 sized = true;
             };
@@ -630,7 +640,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
             // Static tail: this CTA's range [t_lo, t_hi) of the flat (left-over unit, K group) space: the end of one unit
             // and perhaps the start of the next.  What others wait for comes first, then the whole units, then the piece
             // that ends a unit and waits itself (T=257: 214 -> 209 us against running it before the whole units).
-            int t_lo = 0, t_hi = 0, t_unit = 0;
+            int t_lo = 0, t_hi = 0, t_unit = 0, t_part = 0;
             const int flat = (total_units - sched_U0) * NG;
             // Up to half as many units as CTAs are cut into the same number of pieces each, more into one range per CTA.  (A range
             // that crosses a unit's end leaves its CTA two pieces.  One range per CTA / equal pieces / equal pieces or whole units
@@ -665,6 +675,26 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         wi.slot = range_owner(wi.ut * NG, flat, parts);        // CTA of the unit's first piece
                         wi.piece = (int)blockIdx.x - wi.slot; wi.pieces = wi.piece + 1;
                     }
+                } else if (WHICH == FIRST && t_lo < t_hi) {
+                    // A claim of GEMM1 that is a range of the flat (unit, K group) space: what others wait for, the start of the next
+                    // unit, comes first, then the piece that ends a unit and waits itself, for claims before this one.
+                    const int parts = s_sched[0];
+                    t_unit = t_lo / NG;
+                    const int end = (t_unit + 1) * NG;
+                    if (t_hi > end) {
+                        wi.ut = t_unit + 1; wi.gb = 0; wi.ge = t_hi - end;
+                        t_hi = end;
+                    } else {
+                        wi.ut = t_unit; wi.gb = t_lo - t_unit * NG; wi.ge = t_hi - t_unit * NG;
+                        t_lo = t_hi;
+                    }
+                    wi.u = sched_U0 + wi.ut;
+                    if (wi.ge < NG) {                         // leaves its partial sum in the range's slot
+                        wi.slot = t_part; wi.pieces = 2;
+                    } else if (wi.gb > 0) {
+                        wi.slot = range_owner(wi.ut * NG, flat, parts);
+                        wi.piece = t_part - wi.slot; wi.pieces = wi.piece + 1;
+                    }
                 } else if (BOTH) {
                     claim_ahead();
                     int c = __shfl_sync(0xFFFFFFFFu, ahead, 0);
@@ -672,7 +702,8 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         wi.u = c; wi.gb = 0; wi.ge = NG;
                     } else {
                         if (!sized) size_chunks();
-                        const int chunk_groups = s_sched[0], pieces = s_sched[1], items = sched_U0 + (total_units - sched_U0) * pieces;
+                        const int chunk_groups = s_sched[0], pieces = s_sched[1];
+                        const int items = sched_U0 + (WHICH == FIRST && pieces == 0 ? chunk_groups : (total_units - sched_U0) * pieces);
                         if (c >= items) {                     // the claim carries over into GEMM2's list
                             x.claimed = ahead - items; x.claim_base += items; x.claim = claim;
                             // (every CTA ends with one claim too many: behind the last of them nobody watches the routing any more)
@@ -680,6 +711,11 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                             wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break;
                         }
                         c -= sched_U0;
+                        if (WHICH == FIRST && pieces == 0) {
+                            t_part = c; t_lo = range_start(c, flat, chunk_groups); t_hi = range_start(c + 1, flat, chunk_groups);
+                            have_ahead = false;
+                            continue;
+                        }
                         wi.ut = c / pieces; wi.piece = c - wi.ut * pieces; wi.pieces = pieces;
                         wi.slot = wi.ut * pieces;
                         wi.u = sched_U0 + wi.ut;

@@ -305,3 +305,32 @@ def test_routed_calls_take_the_tile_of_their_rows(ds_weights, T):
     torch.cuda.synchronize()
     assert layer.status(T) == 0 and torch.equal(got, want)
     assert layer.launches_routed(T) == edges._kernels_launched(lambda: layer.forward_routed(*args)) == (3 if T <= 128 else 6 if tile == 128 else 5)
+
+
+@pytest.mark.parametrize("experts", [1, 4, 5, 6, 8, 9])
+def test_few_units_in_one_launch(ds_weights, experts):
+    """16 to 144 units of GEMM1 for 148 CTAs: cut into equal pieces up to half as many units as CTAs, dealt out as ranges that may end
+    one unit and start the next up to 5/8 (four and five experts), whole above.  Against the two launches of the 128-token family,
+    and the same bits twenty times on a poisoned workspace."""
+    from justgoal_b200 import MoELayer
+    T, K, E = 6, 8, I.DEEPSEEK_V3.num_experts
+    d = _inputs(T, ds_weights, seed=80)
+    idx = torch.arange(E - K, E, dtype=torch.int32).repeat(T, 1)                  # not on this rank
+    for t in range(T):
+        mine = [(t + k) % experts for k in range(min(K, experts))]
+        idx[t, :len(mine)] = torch.tensor(mine, dtype=torch.int32)
+    w = torch.rand(T, K, generator=torch.Generator().manual_seed(3)) + 0.1
+    args = (idx.cuda(), w.cuda(), d["hidden_states"], d["hidden_states_scale"], *[d[n] for n in (
+        "gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")], 0)
+    layer, wide = MoELayer(I.DEEPSEEK_V3), MoELayer(I.DEEPSEEK_V3)
+    wide.set_token_tile(128)
+    ref = wide.forward_routed(*args)
+    layer.workspace(T).fill_(0xFF)
+    first = layer.forward_routed(*args).clone()
+    assert int(layer.view(T, "status", torch.int32, (8,))[4]) == experts
+    assert float((first - ref).norm()) <= 2e-3 * float(ref.norm())
+    for k in range(20):
+        if k % 5 == 0:
+            layer.workspace(T).fill_(0xFF)
+        assert torch.equal(first, layer.forward_routed(*args))
+    assert layer.status(T) == 0 and wide.status(T) == 0
