@@ -62,10 +62,12 @@ typedef struct b200moe_ctx* b200moe_handle;
  * for tests and debugging only. */
 typedef struct b200moe_ws_layout {
     size_t status;        /* int32[8]: [0] device error word, [1] pairs P, [2] padded rows,
-                             [3] token tiles, [4] active experts                           */
+                             [3] token tiles, [4] active experts; [5], [6]: flag and count of the
+                             one-launch front ends                                         */
     size_t counts;        /* int32[E_local] tokens per local expert (sum of the slices)    */
     size_t expert_row0;   /* int32[E_local+1] first (padded) row of each expert            */
-    size_t tile_prefix;   /* int32[E_local+1] exclusive prefix of token tiles              */
+    size_t tile_prefix;   /* int32[E_local+1] exclusive prefix of token tiles; from the next multiple of 16 bytes on
+                             uint8[64]: CTA of a routed call's front end has copied its share of the rows  */
     size_t topk_idx;      /* int32[T, top_k] global expert ids                             */
     size_t topk_w;        /* float[T, top_k]                                               */
     size_t pair_row;      /* int32[T, top_k] row of a local pair (undefined if not local;
@@ -97,11 +99,12 @@ typedef struct b200moe_ws_layout {
 } b200moe_ws_layout;
 
 /* Create / destroy a layer handle on the CURRENT device.  Does one-time kernel attribute
- * setup and allocates 64 bytes of device memory (the counts of the one-launch front ends; no
+ * setup and allocates 64 bytes of device memory (the count at which the CTAs of the fused front end meet; no
  * later call allocates).  Replaces the one-time setup block of the reference
  * launcher (KF94/kernel.cu:5355-5402) and `moe_init` (SF1/kernel.py:40-44).
  * Calls that use one handle must be ordered with respect to each other on the GPU (one stream,
- * or events between streams): b200moe_forward calls for up to 128 tokens share those two words.
+ * or events between streams): b200moe_forward calls for up to 128 tokens share that count, from their first kernel to their
+ * last.  (b200moe_forward_routed keeps all of its state in the workspace.)
  * Use one handle per stream for forwards that may overlap. */
 int b200moe_create(const b200moe_config* cfg, b200moe_handle* out);
 int b200moe_destroy(b200moe_handle h);

@@ -52,8 +52,8 @@ struct b200moe_ctx {
     int token_tile;            // b200moe_set_token_tile: 0 = chosen from the token count, else 16 / 32 / 64 / 128
     int tma_gather;            // b200moe_set_tma_gather: GEMM1 (128-token tiles) gathers its token rows by TMA; default off
     int fuse_combine;          // b200moe_set_fused_combine: GEMM2 epilogue adds a token's rows up (narrow tiles); default off
-    int* d_sync;               // device, 64 bytes, zero between calls: the counts of the one-launch front ends
-                               // (front.cuh).  One forward per handle may be in flight at a time.
+    int* d_sync;               // device, 64 bytes, zero between calls: the count of the routing front end's meeting (front.cuh).
+                               // One b200moe_forward per handle may be in flight at a time.
     std::mutex map_mutex;
     MapKey map_key[MAP_SETS];
     MapSet map_set[MAP_SETS];
@@ -272,7 +272,7 @@ void layout(const b200moe_ctx* h, int T, b200moe_ws_layout* L) {
     // narrow token tiles: the combine is fused into GEMM2 and counts row deliveries per (token, 256 output columns)
     L->tok_count = take(pick_token_tile(h, T) < 128 ? (size_t)T * ((c.hidden + 255) / 256) * 4 : 0);   // zeroed with the head
     L->expert_row0 = take((size_t)(El + 1) * 4);
-    L->tile_prefix = take((size_t)(El + 1) * 4);
+    L->tile_prefix = take(align_up((size_t)(El + 1) * 4, 16) + FRONT_MAX_CTAS);       // then the bytes of a routed call's front end (front_copied)
     L->topk_idx = take((size_t)T * K * 4);
     L->topk_w = take((size_t)T * K * 4);
     L->pair_row = take((size_t)T * K * 4);
@@ -535,6 +535,11 @@ int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
     return 0;
 }
 
+// FrontParams::copied
+int* front_copied(const b200moe_ctx* h, uint8_t* ws, const b200moe_ws_layout& L, bool routed) {
+    return reinterpret_cast<int*>(routed ? ws + L.tile_prefix + align_up((size_t)(h->cfg.num_local_experts + 1) * 4, 16) : ws + L.status + ST_COPIED * 4);
+}
+
 // CTAs of the one-launch front ends: enough warps to route 128 tokens at once and to copy the rows in one pass, few enough that
 // GEMM1 can start on most SMs while the front end runs.  32 / 64 CTAs, us: 1 token 18.6 / 18.7 (no local expert), 8 tokens 99.1 / 99.1, 16
 // tokens 112.8 / 112.5, 32 tokens 125.0 / 124.3, 33 tokens 124.2 / 123.9, 64 tokens 144.9 / 144.0, 128 tokens 180 / 179; 96 CTAs gained
@@ -544,7 +549,7 @@ int maps_for(b200moe_ctx* h, const MapKey& k, MapSet* out) {
 int front_grid(const b200moe_ctx* h, int T, bool routed) {
     const b200moe_config& c = h->cfg;
     const double rows = (double)T * c.top_k * c.num_local_experts / c.num_experts * (routed ? 2 : 1);
-    const int want = rows <= 8.0 ? 8 : T <= 32 ? 32 : 64;
+    const int want = rows <= 8.0 ? 8 : T <= 32 ? 32 : FRONT_MAX_CTAS;
     return h->num_sms < want ? h->num_sms : want;
 }
 
@@ -582,6 +587,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     // per 128-K block from one producer warp), so the copy stays the default.
     const bool g4 = ntok == 128 && !pairs && h->tma_gather;
     const bool part = ntok == 128 && !pairs && !g4 && tiles_mostly_part_full(c, T);
+    const bool gemm1_watches = fused_front && !pairs && wire_pitch == 0 && !g4;      // GEMM1 starts from the routing of the front end
     if ((rc = maps_for(h, MapKey{w13, w2, a_perm, act_hi, act_lo, rows_cap, ntok}, &maps))) return rc;
     if (g4 && (rc = make_map(&maps.a, hidden, (uint64_t)T, H, 1, wire_pitch > 0 ? (uint64_t)wire_pitch : 0))) return rc;
     const CUtensorMap &m_w13 = maps.w13, &m_w2 = maps.w2, &m_a = maps.a, &m_hi = maps.hi, &m_lo = maps.lo;
@@ -599,7 +605,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         fp.plan = pp;
         fp.hidden = static_cast<const uint8_t*>(hidden); fp.hscale = static_cast<const float*>(hidden_scale);
         fp.a_perm = a_perm; fp.a_scale_perm = a_scale; fp.H = H;
-        fp.sync = h->d_sync; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = (int)(L.expert_row0 / 16);
+        fp.sync = h->d_sync; fp.copied = gemm1_watches && ntok < 128 ? front_copied(h, ws, L, !route_in_front) : nullptr; fp.head = reinterpret_cast<uint4*>(ws); fp.head_vec = (int)(L.expert_row0 / 16);
         const int fgrid = front_grid(h, T, !route_in_front);
         if (route_in_front) CU_TRY(launch_front_route(c, fgrid, fp, *route_in_front, st));
         else CU_TRY(launch_k(PDL_PERMUTE, front_small_kernel, dim3(fgrid), dim3(FRONT_THREADS), 0, st, fp));
@@ -641,12 +647,14 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
             g1.g4_scale = static_cast<const float*>(hidden_scale); g1.g4_tok_stride = 1; g1.ts_stride = T;
         }
     }
-    if (fused_front && !pairs && wire_pitch == 0 && !g4) {
+    if (gemm1_watches) {
         // the fused front end announces the routing result; GEMM1 schedules itself from it (gemm.cuh).  Not with gathered
         // rows: the producer reads row_token for its first loads, which the front end writes after the announcement.
         if (route_in_front) { g1.routed = h->d_sync; g1.routed_want = front_grid(h, T, !route_in_front); }
         else { g1.routed = status + ST_ROUTED; g1.routed_want = 1; }
-        g1.copied = h->d_sync + 1; g1.copied_want = front_grid(h, T, !route_in_front);
+        g1.front_ctas = front_grid(h, T, !route_in_front);
+        g1.copied = ntok < 128 ? front_copied(h, ws, L, !route_in_front) : nullptr;
+        g1.copied_bytes = !route_in_front;
         g1.topk_idx = topk_idx; g1.n_pairs = T * c.top_k; g1.local_offset = local_offset;
     }
     g1.tables_done = !fused_front && !pairs && !g4;      // the gather lets GEMM1 start only after the permutation has completed
@@ -687,7 +695,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.tok_count = reinterpret_cast<int*>(ws + L.tok_count);
         g2.row_token = row_token; g2.pair_row = pair_row; g2.c_topk = topk_idx; g2.c_stride = pp.pair_stride;
         g2.top_k = c.top_k; g2.T = T; g2.c_local_offset = local_offset;
-        g2.met = fused_front ? h->d_sync : nullptr;
+        g2.met = route_in_front ? h->d_sync : nullptr;
     }
     // (With stage times the two parts of the kernel that does both run as two launches: the same pieces, the same bits.)
     if (both) { if (h->prof_slots) CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, g2)); }
@@ -716,7 +724,7 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     SlotOut so;
     memset(&so, 0, sizeof(so));            // cap == 0: rows go to `out`
     if (slot_out) so = *slot_out;
-    int* const met = fused_front ? h->d_sync : nullptr;
+    int* const met = route_in_front ? h->d_sync : nullptr;
     const bool wide = combine_is_wide(T, H);
     auto combine = [&](auto kernel) {
         return launch_k(PDL_COMBINE, kernel, cgrid, dim3(256), 0, st, (const __half*)y, topk_idx, (const int32_t*)pair_row,
@@ -946,7 +954,7 @@ int b200moe_forward(b200moe_handle h, const void* logits, const void* bias, cons
     CU_TRY(prof_mark(h, 1, st));
     rc = run_experts(h, rp.topk_idx, rp.topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
                      OUT_BF16, ws, L, st, fused, nullptr, 0, fused ? &rp : nullptr, true);
-    if (rc && fused) cudaMemsetAsync(h->d_sync, 0, 64, st);       // the kernel that clears the front end's counts may not have been launched
+    if (rc && fused) cudaMemsetAsync(h->d_sync, 0, 64, st);       // the kernel that clears the meeting's count may not have been launched
     return rc;
 }
 
@@ -981,10 +989,8 @@ int b200moe_forward_routed(b200moe_handle h, const int32_t* topk_idx, const floa
         CU_TRY(cudaGetLastError());
     }
     CU_TRY(prof_mark(h, 1, st));
-    rc = run_experts(h, topk_idx, topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
-                     output_kind, ws, L, st, fused);
-    if (rc && fused) cudaMemsetAsync(h->d_sync, 0, 64, st);       // as in b200moe_forward
-    return rc;
+    return run_experts(h, topk_idx, topk_w, hidden, hidden_scale, w13, s13, w2, s2, T, local_offset, output,
+                       output_kind, ws, L, st, fused);
 }
 
 int b200moe_ep_row_bytes(b200moe_handle h, int* bytes) {
@@ -1237,7 +1243,7 @@ int b200moe_status(b200moe_handle h, const void* workspace, void* stream, int* w
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CU_TRY(cudaMemcpyAsync(word, workspace, sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    if (*word) CU_TRY(cudaMemset(h->d_sync, 0, 64));      // a front end that gave up at its meeting leaves the words dirty
+    if (*word) CU_TRY(cudaMemset(h->d_sync, 0, 64));      // a front end that gave up at its meeting
     return *word ? B200MOE_E_KERNEL : 0;
 }
 

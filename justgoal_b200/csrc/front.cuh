@@ -9,8 +9,8 @@
 // among the same-expert pairs of its warp (match.any) plus the counts of the warps before it, which keeps the rows of
 // an expert in token order.  CTA 0 alone writes the tables that later kernels read (counts, row maps); all CTAs
 // derive identical values.  Same results as count_kernel + permute_kernel + gather_kernel (permute.cuh).
-// The next kernel (GEMM1) does not wait for this one to finish before it starts to work: it watches the two counts of
-// FrontParams::sync (behind front_small_kernel a flag, ST_ROUTED, and the second count), see GemmParams::routed.  The reference fuses the same stages for small batches
+// The next kernel (GEMM1) does not wait for this one to finish before it starts to work: it watches the count of the meeting
+// (behind front_small_kernel a flag, ST_ROUTED) and FrontParams::copied, see GemmParams::routed.  The reference fuses the same stages for small batches
 // (kda05_reproduction_full_shape/fable-5.1/moe_fp8_fwd/<def>/fable51_moe_v94/kernel.cu:724-806) and issues its first
 // weight stages during the table build (its MOE_EARLY_W switch, same directory, main.py:50).
 #pragma once
@@ -30,10 +30,14 @@ struct FrontParams {
     uint8_t* a_perm;              // [rows_cap, H]
     float* a_scale_perm;          // [H/128, rows_cap]
     int H;
-    // `sync` is two words owned by the handle, zero between calls (the last kernel of the forward clears them): [0] CTAs that
-    // have arrived at the meeting (front_route_kernel only), [1] CTAs that have copied their share of the rows.  `head` is the part of the workspace that must be zero before the GEMMs run (status, split-unit counters), in 16-byte units: CTA 0
-    // clears it, so the forward needs no memset in front of the kernel.
+    // `sync` (front_route_kernel only) is a word owned by the handle, zero between calls (the last kernel of the forward clears
+    // it): CTAs that have arrived at the meeting.  `copied` lies in the workspace, whatever that held before, so that a routed
+    // call keeps nothing in the handle: CTAs that have copied their share of the rows.  Behind a meeting it is one count, in the
+    // head; without one (front_small_kernel) nobody could tell a CTA that the count is clear, so each has a byte, which it
+    // clears itself before the next kernel can look.  Null: the next kernel waits for this one.  `head` is the part of the workspace that must be zero before the GEMMs
+    // run (status, split-unit counters), in 16-byte units: CTA 0 clears it, so the forward needs no memset in front of the kernel.
     int* sync;
+    int* copied;
     uint4* head;
     int head_vec;
 };
@@ -156,8 +160,12 @@ __device__ __forceinline__ void front_body(const FrontParams& fp, FrontShared& s
         }
     }
     // this CTA's rows are there for the GEMM that follows (GemmParams::copied)
+    if (!fp.copied) return;
     __syncthreads();
-    if (tid == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(fp.sync + 1) : "memory");
+    if (tid == 0) {
+        if (FRESH) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(fp.copied) : "memory");
+        else asm volatile("st.release.gpu.global.u8 [%0], %1;" ::"l"(reinterpret_cast<uint8_t*>(fp.copied) + blockIdx.x), "h"((uint16_t)1) : "memory");
+    }
 }
 
 
@@ -170,6 +178,8 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const Fro
     front_clear(s);
     __syncthreads();
     pdl_wait();
+    const int clears = FRONT_THREADS - 1;                      // its warp is the least likely to have a pair
+    if (fp.copied && threadIdx.x == clears) reinterpret_cast<uint8_t*>(fp.copied)[blockIdx.x] = 0;
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < fp.head_vec; i += FRONT_THREADS) fp.head[i] = make_uint4(0u, 0u, 0u, 0u);
         __threadfence();
@@ -177,8 +187,18 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_small_kernel(const Fro
         if (threadIdx.x == 0)
             asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(fp.plan.status + ST_ROUTED), "r"(1) : "memory");
         __syncthreads();
+        pdl_launch();
+    } else if (!fp.copied) {
+        pdl_launch();
+    } else if (threadIdx.x >= clears - 31) {
+        // GEMM1 may start once every CTA has said so, and looks at this byte: one warp says it, behind a fence.  Kept in the
+        // handle as a count, for which no CTA had to fence, us: 64 experts of 1024 x 512 64 tokens 38.5 / 39.0, 8 softmax experts of the
+        // 4096-wide shape 128: 42.8 / 43.8, 16 of them 10: 39.4 / 40.6, 40: 57.7 / 58.0; 32 of 256 experts 2 tokens 55.5 / 55.7, 64: 134.4 /
+        // 135.1 (the whole CTA behind a barrier: 42.1, 45.6, 39.8, 59.4; 55.3, 135.5).
+        if (threadIdx.x == clears) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        __syncwarp();
+        pdl_launch();
     }
-    pdl_launch();
     front_body<false>(fp, s);
 }
 

@@ -98,13 +98,14 @@ struct GemmParams {
     // GEMM1 after a one-launch front end (small token counts), else null: the routing result of all tokens is visible when
     // *routed has reached routed_want (the CTAs that have routed their share, or a flag).  The CTAs then build the expert tables
     // themselves from topk_idx (the same histogram and scan as the front end) and the producer streams the first weight tiles
-    // while the front end still permutes and gathers.  The token rows: with narrow tiles they are there when *copied has reached
-    // copied_want, the CTAs that have copied their share - earlier than the front end's last CTA has left and a waiting kernel
-    // has learned of it -, otherwise after the wait for the front end.
+    // while the front end still permutes and gathers.  The token rows: with narrow tiles they are there when all
+    // front_ctas CTAs of the front end have copied their share, by the count at `copied` or, with copied_bytes, a byte each -
+    // earlier than the last of them has left and a waiting kernel has learned of it -, otherwise after the wait for the front end.
     const int* routed;
     const int* copied;
-    int routed_want, copied_want;
-    int* met;             // fused combine: the front end's two counts (FrontParams::sync), which the last kernel of a forward clears
+    int routed_want, front_ctas;
+    bool copied_bytes;
+    int* met;             // fused combine: the count of the front end's meeting, which the last kernel of a forward clears
     // Both GEMMs in one launch: counter of every token tile, zero at launch; a warp that has stored its part of a GEMM1 unit's
     // rows counts in, and a unit of GEMM2 may read the tile when tile_want have.
     int* tile_done;
@@ -595,7 +596,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                 static_assert(MOST <= MAX_PIECES, "arrivals of a split unit");
                 const int tail_units = total_units - sched_U0;
                 const int slots = (int)gridDim.x * (BOTH ? p.slots : (NG + C::CHUNK_GROUPS - 1) / C::CHUNK_GROUPS);           // what sk_partial holds
-                const int late = WHICH == FIRST && sched_q == 0 && p.routed ? p.copied_want : 0;
+                const int late = WHICH == FIRST && sched_q == 0 && p.routed ? p.front_ctas : 0;
                 int best = NG * C::KPB, chunk_groups = NG;
                 if (WHICH == FIRST && sched_q > 0 &&
                            (sched_q + 1) * p.KB + p.next_KB <= (total_units * p.KB + s_tiles[p.num_local] * p.next_mtiles * p.next_KB) / (int)gridDim.x) {
@@ -707,7 +708,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         if (c >= items) {                     // the claim carries over into GEMM2's list
                             x.claimed = ahead - items; x.claim_base += items; x.claim = claim;
                             // (every CTA ends with one claim too many: behind the last of them nobody watches the routing any more)
-                            if (FUSE && p.met && c == items + (int)gridDim.x - 1 && lane < 2) p.met[lane] = 0;
+                            if (FUSE && p.met && c == items + (int)gridDim.x - 1 && lane == 0) *p.met = 0;
                             wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break;
                         }
                         c -= sched_U0;
@@ -882,11 +883,26 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         const unsigned long long t0 = globaltimer_ns();
 #pragma unroll 1
                         for (uint32_t it = 1;; ++it) {
-                            int n = 0;
-                            if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(p.copied) : "memory");
-                            n = __shfl_sync(0xFFFFFFFFu, n, 0);
-                            __syncwarp();
-                            if (merged(n >= p.copied_want)) break;
+                            // (as few requests as possible: every CTA polls the same few bytes)
+                            bool mine = true;
+                            if (!p.copied_bytes) {
+                                int n = p.front_ctas;
+                                if (lane == 0) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(p.copied) : "memory");
+                                mine = n >= p.front_ctas;
+                            } else if (16 * lane < p.front_ctas) {
+                                uint32_t v[4];
+                                asm volatile("ld.acquire.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+                                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(p.copied + 4 * lane) : "memory");
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const int left = p.front_ctas - 16 * lane - 4 * j;           // bytes of this word that count
+                                    const uint32_t set = left >= 4 ? 0x01010101u : left > 0 ? 0x01010101u >> (8 * (4 - left)) : 0u;
+                                    mine = mine && (v[j] & (set * 255u)) == set;
+                                }
+                            }
+                            mine = __all_sync(0xFFFFFFFFu, mine);
+                            __syncwarp();        // the lanes' acquires order the loads of whichever lane issues them
+                            if (merged(mine)) break;
                             if ((it & 0xFFu) == 0 && __any_sync(0xFFFFFFFFu, globaltimer_ns() - t0 > WAIT_LIMIT_NS)) { ok = false; break; }
                         }
                         if (!ok && lane == 0) atomicCAS(p.status, 0, ERR_WAIT_GROUP);
@@ -1138,7 +1154,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
         int n_item = x.n_item;
         WorkItem wi;
         if ((WHICH != SECOND || x.fresh) && !(!C::TOK_ON_M && G1 && p.copied)) { pdl_wait(); pdl_launch(); }
-        if (FUSE && !BOTH && p.met && blockIdx.x == 0 && ptid < 2) p.met[ptid] = 0;
+        if (FUSE && !BOTH && p.met && blockIdx.x == 0 && ptid == 0) *p.met = 0;
 #pragma unroll 1
         while (ok && wq_fetch(n_item++, wi, ok)) {
             const int gb = wi.gb, ge = wi.ge;

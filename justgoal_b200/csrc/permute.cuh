@@ -16,12 +16,14 @@ namespace b200moe {
 
 constexpr int ROW_ALIGN = 16;
 constexpr int MAX_LOCAL = 256;
+constexpr int FRONT_MAX_CTAS = 64;     // CTAs of a one-launch front end (front.cuh)
 static_assert((ROW_ALIGN & (ROW_ALIGN - 1)) == 0, "row alignment is a power of two");
 constexpr int NO_ROW = 0x7FFFFFFF;      // pair_row of a local pair that got no row (the call was refused, see scan_counts)
 
 // status word layout (int32[8]) at the head of the workspace
 enum : int { ST_ERR = 0, ST_PAIRS = 1, ST_ROWS = 2, ST_TILES = 3, ST_ACTIVE = 4,
-              ST_ROUTED = 5 /* fused front end: 1 once the routing result of every token is visible */ };
+              ST_ROUTED = 5 /* front_small_kernel: 1 once the head is clear and the routing may be read */,
+              ST_COPIED = 6 /* front_route_kernel: CTAs that have copied their share of the rows */ };
 
 struct PlanParams {
     int T, top_k, num_local, local_offset, token_tile;
@@ -392,8 +394,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const __half* __restrict__
         }
         if (t0 == t_first) {
             pdl_wait(); pdl_launch();
-            // the front end's counts: all that watch them are done, and the next call counts behind this kernel
-            if (met && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) met[threadIdx.x] = 0;
+            // the count of the front end's meeting: all that watch it are done, and the next call counts behind this kernel
+            if (met && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *met = 0;
         }
         __syncthreads();
         const int nt = min(batch, T - t0);

@@ -334,3 +334,41 @@ def test_few_units_in_one_launch(ds_weights, experts):
             layer.workspace(T).fill_(0xFF)
         assert torch.equal(first, layer.forward_routed(*args))
     assert layer.status(T) == 0 and wide.status(T) == 0
+
+
+@pytest.mark.parametrize("T", [8, 30, 128])
+def test_routed_calls_of_one_handle_on_two_streams(ds_weights, T):
+    """Routed calls of up to 128 tokens share nothing but the handle: on two streams, a workspace each (full of other bytes), they give
+    the bits that the same calls give one after the other."""
+    import ctypes as C
+    from justgoal_b200 import MoELayer, _lib
+    layer = MoELayer(I.DEEPSEEK_V3)
+    n = int(layer.layout(T).total_bytes)
+    sides = []
+    for k in range(2):
+        d = _inputs(T, ds_weights, seed=90 + 2 * T + k)
+        idx, w = layer.route(d["routing_logits"], d["routing_bias"], 2.5)
+        sides.append((torch.cuda.Stream(), torch.full((n,), 0xFF, dtype=torch.uint8, device="cuda"),
+                      (idx, w, d["hidden_states"], d["hidden_states_scale"],
+                       *[d[m] for m in ("gemm1_weights", "gemm1_weights_scale", "gemm2_weights", "gemm2_weights_scale")])))
+
+    def call(side, out):
+        st, ws, tensors = side
+        rc = _lib.lib.b200moe_forward_routed(layer._h, *[C.c_void_p(t.data_ptr()) for t in tensors], T, 0, C.c_void_p(out.data_ptr()), 0,
+                                             C.c_void_p(ws.data_ptr()), n, C.c_void_p(st.cuda_stream))
+        _lib.check(rc, "b200moe_forward_routed")
+
+    want = [torch.empty(T, I.DEEPSEEK_V3.hidden, device="cuda") for _ in sides]
+    torch.cuda.synchronize()
+    for side, out in zip(sides, want):
+        call(side, out)
+        torch.cuda.synchronize()
+    outs = [[torch.full_like(want[0], 7.0) for _ in range(40)] for _ in sides]
+    torch.cuda.synchronize()
+    for k in range(40):
+        for side, o in zip(sides, outs):
+            call(side, o[k])
+    torch.cuda.synchronize()
+    for (st, ws, _), o, ref in zip(sides, outs, want):
+        assert int(ws[:4].view(torch.int32)[0]) == 0 and bool(torch.isfinite(ref).all())
+        assert all(torch.equal(x, ref) for x in o)

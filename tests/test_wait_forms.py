@@ -84,3 +84,19 @@ def test_what_one_lane_learns_about_other_ctas_orders_the_whole_warp():
         assert code.count(answer) == 1
         after = code[code.index(answer) + len(answer):].lstrip()
         assert after.startswith("__syncwarp();"), answer
+
+
+def test_routed_front_end_keeps_nothing_in_the_handle():
+    """Calls of b200moe_forward_routed on two streams share a handle and nothing else: what GEMM1 watches of their front end lies in the
+    workspace.  The handle's count belongs to the routing front end's meeting; every CTA clears its own word before GEMM1 can look."""
+    front, host = _code("front.cuh"), _code("b200moe.cu")
+    body = front[front.index("void front_body("):front.index("front_route_kernel(")]
+    assert "fp.sync" not in body
+    small = front[front.index("front_small_kernel("):front.index("template <int VPT")]
+    clear = small.index("(fp.copied)[blockIdx.x] = 0;")
+    assert "pdl_launch" not in small[:clear]
+    zero, nobody_looks, rest = small[clear:].split("pdl_launch();")[:3]
+    assert "__threadfence();" in zero and nobody_looks.endswith("else if (!fp.copied) {\n        ")
+    assert rest.index("threadIdx.x >= clears - 31") < rest.index("fence.acq_rel.gpu;") < rest.index("__syncwarp();")
+    assert "g1.copied = ntok < 128 ? front_copied(" in host and "d_sync" not in host[host.index("int* front_copied("):host.index("int front_grid(")]
+    assert re.findall(r"met = (\w+) \? h->d_sync", host) == ["route_in_front"] * 2
