@@ -698,7 +698,13 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
         g2.met = route_in_front ? h->d_sync : nullptr;
     }
     // (With stage times the two parts of the kernel that does both run as two launches: the same pieces, the same bits.)
-    if (both) { if (h->prof_slots) CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, g2)); }
+    if (both) {
+        if (h->prof_slots) {
+            GemmParams not_last = g2;
+            not_last.met = nullptr;
+            CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, not_last));
+        }
+    }
     else if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));
     else if (g4) CU_TRY(launch_gemm_g4(h->num_sms, st, m_w13, m_a, m_a, m_a, m_a, g1));
     else if (part) CU_TRY(launch_gemm_part<true>(h->num_sms, st, m_w13, m_a, m_a, maps.a_box, maps.a_box, g1));
@@ -1243,7 +1249,7 @@ int b200moe_status(b200moe_handle h, const void* workspace, void* stream, int* w
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     CU_TRY(cudaMemcpyAsync(word, workspace, sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    if (*word) CU_TRY(cudaMemset(h->d_sync, 0, 64));      // a front end that gave up at its meeting
+    if (*word) CU_TRY(cudaMemset(h->d_sync, 0, 64));      // (after an error, whatever came between)
     return *word ? B200MOE_E_KERNEL : 0;
 }
 

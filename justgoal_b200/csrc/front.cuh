@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(FRONT_THREADS, 1) front_route_kernel(const Fro
     if (threadIdx.x == 0) {
         // The meeting: one count, which GEMM1 watches too.  It builds its schedule from the routing and starts to stream weights
         // while this kernel still permutes and gathers.  Nobody clears the count before all that watch it are done: the last
-        // kernel of the forward does.  (A call that gave up leaves it dirty; b200moe_status() clears it when it reports the error.)
+        // kernel of the forward does, also of one that gave up.
         // An earlier form counted those that left as well, so that the last of them could clear both counts, and CTA 0 announced
         // the routing in a word of its own: two more round trips to L2 in front of GEMM1's first load.  With this one, `copied` and
         // eight CTAs up to eight tokens, start / now, us: 512-wide shape 1 token 20.6 / 19.1, 40: 22.4 / 21.6; 64 experts of

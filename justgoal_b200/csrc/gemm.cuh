@@ -105,7 +105,8 @@ struct GemmParams {
     const int* copied;
     int routed_want, front_ctas;
     bool copied_bytes;
-    int* met;             // fused combine: the count of the front end's meeting, which the last kernel of a forward clears
+    int* met;             // fused combine: the count of the front end's meeting, which the last kernel of a forward clears, and
+                          // behind it, with both GEMMs in one launch, a count of the CTAs that are done
     // Both GEMMs in one launch: counter of every token tile, zero at launch; a warp that has stored its part of a GEMM1 unit's
     // rows counts in, and a unit of GEMM2 may read the tile when tile_want have.
     int* tile_done;
@@ -707,8 +708,6 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         const int items = sched_U0 + (WHICH == FIRST && pieces == 0 ? chunk_groups : (total_units - sched_U0) * pieces);
                         if (c >= items) {                     // the claim carries over into GEMM2's list
                             x.claimed = ahead - items; x.claim_base += items; x.claim = claim;
-                            // (every CTA ends with one claim too many: behind the last of them nobody watches the routing any more)
-                            if (FUSE && p.met && c == items + (int)gridDim.x - 1 && lane == 0) *p.met = 0;
                             wi.u = -1; wi.gb = wi.ge = 0; publish(wi); break;
                         }
                         c -= sched_U0;
@@ -1709,6 +1708,12 @@ gemm_both_kernel(const __grid_constant__ CUtensorMap tm_w13, const __grid_consta
     }
     if (x.ok && (parts & 2)) gemm_roles<NTOK, false, false, false, FUSE, SECOND>(x, tm_w2, tm_hi, tm_lo, tm_hi, tm_lo, p2);
     gemm_teardown<C>(x);
+    if (FUSE && p2.met && threadIdx.x == 0) {
+        // The last kernel of the forward (met is null in the first of two launches) clears the count of the front end's meeting.  Every CTA comes by here, also one that gave up,
+        // after its warps 2-3 have waited for the front end: behind the last of them nobody watches the count any more.
+        __threadfence();
+        if (atomicAdd(p2.met + 1, 1) == (int)gridDim.x - 1) { p2.met[0] = 0; p2.met[1] = 0; }
+    }
     if (p2.trace && threadIdx.x == 0) p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = clock64() - x.t_entry;
 }
 

@@ -372,3 +372,41 @@ def test_routed_calls_of_one_handle_on_two_streams(ds_weights, T):
     for (st, ws, _), o, ref in zip(sides, outs, want):
         assert int(ws[:4].view(torch.int32)[0]) == 0 and bool(torch.isfinite(ref).all())
         assert all(torch.equal(x, ref) for x in o)
+
+
+@pytest.mark.parametrize("T", [1, 40, 128])
+def test_one_fused_launch_without_rows(ds_weights, T):
+    """Both GEMMs and the combine in one launch where no token has an expert on this rank: nothing in it waits for rows, and the next
+    call, which has some, still finds the front end's count at zero.  Queued in turn without a host wait, also from a graph."""
+    from justgoal_b200 import MoELayer
+    d = _inputs(T, ds_weights, seed=50 + T)
+    args = util.op_args(d)
+    none = list(args)
+    none[1] = args[1].clone()
+    none[1][:I.DEEPSEEK_V3.num_local_experts] = -100.0            # the selection bias of the local experts: never chosen
+    layer = MoELayer(I.DEEPSEEK_V3)
+    want = layer.forward(*args).clone()
+    layer.set_fused_combine(True)
+    assert layer.launches_per_forward(T) == 2
+
+    def turns():
+        return [(layer.forward(*none), layer.forward(*none), layer.forward(*args)) for _ in range(10)]
+
+    def check(outs):
+        torch.cuda.synchronize()
+        assert layer.status(T) == 0
+        for a, b, c in outs:
+            assert float(a.float().abs().max()) == float(b.float().abs().max()) == 0.0
+            assert torch.equal(c.view(torch.int16), want.view(torch.int16))
+
+    layer.workspace(T).fill_(0xFF)
+    check(turns())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        outs = turns()
+    for _ in range(3):
+        for o in outs:
+            for x in o:
+                x.fill_(7.0)
+        g.replay()
+    check(outs)

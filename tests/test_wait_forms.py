@@ -100,3 +100,19 @@ def test_routed_front_end_keeps_nothing_in_the_handle():
     assert rest.index("threadIdx.x >= clears - 31") < rest.index("fence.acq_rel.gpu;") < rest.index("__syncwarp();")
     assert "g1.copied = ntok < 128 ? front_copied(" in host and "d_sync" not in host[host.index("int* front_copied("):host.index("int front_grid(")]
     assert re.findall(r"met = (\w+) \? h->d_sync", host) == ["route_in_front"] * 2
+
+
+def test_meeting_count_is_cleared_whatever_happened():
+    """The count of the front end's meeting is cleared by the last kernel of a forward, also after a wait that ran out (the next call
+    would not wait for its routing otherwise), and only when nobody watches it any more.  Where one launch does both GEMMs and the
+    combine, that is behind the last CTA of the launch, whose warps have all come back; never at a claim, which a CTA that gave up does
+    not take and which, in a call without rows, need not wait for the front end."""
+    code = _code("gemm.cuh")
+    roles = code[code.index("void gemm_roles("):code.index("gemm_kernel(const __grid_constant__")]
+    assert re.findall(r"\*p\.met = |p\.met\[", roles) == ["*p.met = "]
+    line = next(s for s in roles.splitlines() if "*p.met = 0;" in s)
+    assert "FUSE && !BOTH" in line and "pdl_wait();" in roles[:roles.index(line)].splitlines()[-1]
+    both = code[code.index("gemm_both_kernel(const __grid_constant__"):]
+    tail = both[both.index("gemm_teardown<C>(x);"):]
+    assert "p2.met" not in both[:both.index("gemm_teardown<C>(x);")] and "x.ok" not in tail
+    assert tail.index("__threadfence();") < tail.index("atomicAdd(p2.met + 1, 1) == (int)gridDim.x - 1") < tail.index("p2.met[0] = 0; p2.met[1] = 0;")
