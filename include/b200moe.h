@@ -309,7 +309,7 @@ int b200moe_set_tma_gather(b200moe_handle h, int on);
 int b200moe_set_wait_limit_ns(b200moe_handle h, unsigned long long nanoseconds);
 
 /* Number of this library's kernels one forward over T tokens launches (a count of
- * launches, not of kernels that do useful work). */
+ * launches, not of kernels that do useful work), with stage timing on or off as it is. */
 int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches);
 /* The same count for b200moe_forward_routed over num_tokens tokens, and for b200moe_forward_routed_slots over
  * num_slots = world * cap slots (at least one). */

@@ -236,6 +236,9 @@ bool use_both(const b200moe_ctx* h, int ntok) {
     return ntok <= 32 && weights_stream(c) && narrow_slots(c, ntok) >= 2;
 }
 
+// ... and is that one launch made?  With stage times its two parts are launched one after the other.
+bool one_gemm_launch(const b200moe_ctx* h, int ntok) { return use_both(h, ntok) && !h->prof_slots; }
+
 size_t sk_partial_bytes(const b200moe_config& c, int grid, int ntok) {
     switch (ntok) {
         case 16: return sk_partial_bytes_ntok<16>(c, grid);
@@ -895,21 +898,21 @@ int b200moe_launches_per_forward(b200moe_handle h, int num_tokens, int* launches
     // [route, permute, gather | fused route+permute+gather for small T], gemm1, gemm2, [combine unless fused into gemm2]
     const int ntok = pick_token_tile(h, num_tokens);
     const bool fuse = h->fuse_combine && ntok < 128 && !use_pairs(h, ntok);
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (fuse ? 1 : 0) - (use_both(h, ntok) ? 1 : 0);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens) ? 1 : 0)) - (fuse ? 1 : 0) - (one_gemm_launch(h, ntok) ? 1 : 0);
     return 0;
 }
 
 int b200moe_launches_routed(b200moe_handle h, int num_tokens, int* launches) {
     if (!h || !launches || num_tokens < 0) return B200MOE_E_BADARG;
     // [count, permute, gather | all in one launch for small T], gemm1, gemm2, combine
-    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens, true) ? 1 : 0)) - (use_both(h, pick_token_tile(h, num_tokens, true)) ? 1 : 0);
+    *launches = num_tokens == 0 ? 0 : (num_tokens <= FRONT_MAX_T ? 4 : 6 - (gathers_by_tma(h, num_tokens, true) ? 1 : 0)) - (one_gemm_launch(h, pick_token_tile(h, num_tokens, true)) ? 1 : 0);
     return 0;
 }
 
 int b200moe_launches_routed_slots(b200moe_handle h, int num_slots, int* launches) {
     if (!h || !launches || num_slots < 1) return B200MOE_E_BADARG;
     // count, permute, gather, gemm1, gemm2, combine whatever the number of slots
-    *launches = 6 - (gathers_by_tma(h, num_slots) ? 1 : 0) - (use_both(h, pick_token_tile(h, num_slots)) ? 1 : 0);
+    *launches = 6 - (gathers_by_tma(h, num_slots) ? 1 : 0) - (one_gemm_launch(h, pick_token_tile(h, num_slots)) ? 1 : 0);
     return 0;
 }
 

@@ -231,6 +231,7 @@ def test_both_gemms_in_one_launch(ds_weights, T, tile):
     layer.workspace(T).fill_(0xFF)
     same(layer.forward(*args))
     layer.profile_enable(2)
+    assert layer.launches_per_forward(T) == n + 1 == edges._kernels_launched(lambda: layer.forward(*args))
     same(layer.forward(*args))
     assert all(v >= 0 for v in layer.profile_read(0).values())
     layer.profile_enable(0)
@@ -305,6 +306,11 @@ def test_routed_calls_take_the_tile_of_their_rows(ds_weights, T):
     torch.cuda.synchronize()
     assert layer.status(T) == 0 and torch.equal(got, want)
     assert layer.launches_routed(T) == edges._kernels_launched(lambda: layer.forward_routed(*args)) == (3 if T <= 128 else 6 if tile == 128 else 5)
+    layer.profile_enable(1)
+    assert layer.launches_routed(T) == edges._kernels_launched(lambda: layer.forward_routed(*args)) == (4 if T <= 128 else 6)
+    assert layer.launches_routed_slots(8) == 6
+    layer.profile_enable(0)
+    assert layer.launches_routed_slots(8) == 5
 
 
 @pytest.mark.parametrize("experts", [1, 4, 5, 6, 8, 9])
