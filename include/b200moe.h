@@ -89,7 +89,8 @@ typedef struct b200moe_ws_layout {
     size_t trace;         /* int64[2][SMs][16] per-CTA time lines of GEMM1 and GEMM2: slot 0 =
                              %globaltimer at entry, slots 1..11 = SM clocks since entry at:
                              prologue done, first/last TMA issue, first/last MMA, first/last
-                             promotion, partial published, partials added, epilogue, exit     */
+                             promotion, partial published, partials added, epilogue, exit
+                             (of the launch; one launch that does both GEMMs stamps it twice) */
     size_t tok_count;     /* int32[T][ceil(H/256)] (narrow token tiles only, else empty): byte q = rows of token t
                              delivered for output columns 256 j + {0, 128} + [32 q, 32 q + 32) - the combine
                              fused into the GEMM2 epilogue                                    */

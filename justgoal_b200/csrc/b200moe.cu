@@ -703,9 +703,10 @@ int run_experts(b200moe_ctx* h, const int32_t* topk_idx, const float* topk_w, co
     // (With stage times the two parts of the kernel that does both run as two launches: the same pieces, the same bits.)
     if (both) {
         if (h->prof_slots) {
-            GemmParams not_last = g2;
-            not_last.met = nullptr;
-            CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, not_last));
+            GemmParams later = g2;
+            later.met = nullptr; later.trace = nullptr;
+            CU_TRY(launch_gemm_both(ntok, fuse, 1, h->num_sms, st, maps, g1, later));
+            g1.trace = nullptr;
         }
     }
     else if (pairs) CU_TRY(launch_gemm_pair<true>(h->pair_grid[0], st, m_w13, m_a, m_a, g1));

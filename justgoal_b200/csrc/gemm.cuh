@@ -1696,10 +1696,10 @@ gemm_both_kernel(const __grid_constant__ CUtensorMap tm_w13, const __grid_consta
     extern __shared__ uint8_t smem_raw[];
     GemmCta x;
     gemm_setup<C>(x, smem_raw);
-    if (p1.trace && threadIdx.x == 0) {
+    if (threadIdx.x == 0) {                     // (trace is null for the GEMM that this launch does not do)
         const long long now = (long long)globaltimer_ns();
-        p1.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
-        p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
+        if (p1.trace) p1.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
+        if (p2.trace) p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_ENTRY] = now;
     }
     gemm_init<C, 0>(x, tm_w13, tm_a, tm_w2);
     if (parts & 1) {
@@ -1709,12 +1709,16 @@ gemm_both_kernel(const __grid_constant__ CUtensorMap tm_w13, const __grid_consta
     if (x.ok && (parts & 2)) gemm_roles<NTOK, false, false, false, FUSE, SECOND>(x, tm_w2, tm_hi, tm_lo, tm_hi, tm_lo, p2);
     gemm_teardown<C>(x);
     if (FUSE && p2.met && threadIdx.x == 0) {
-        // The last kernel of the forward (met is null in the first of two launches) clears the count of the front end's meeting.  Every CTA comes by here, also one that gave up,
+        // The last kernel of the forward (met is null in another one) clears the count of the front end's meeting.  Every CTA comes by here, also one that gave up,
         // after its warps 2-3 have waited for the front end: behind the last of them nobody watches the count any more.
         __threadfence();
         if (atomicAdd(p2.met + 1, 1) == (int)gridDim.x - 1) { p2.met[0] = 0; p2.met[1] = 0; }
     }
-    if (p2.trace && threadIdx.x == 0) p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = clock64() - x.t_entry;
+    if (threadIdx.x == 0) {
+        const long long cycles = clock64() - x.t_entry;
+        if (p1.trace) p1.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = cycles;
+        if (p2.trace) p2.trace[(size_t)blockIdx.x * TRACE_SLOTS + TR_EXIT] = cycles;
+    }
 }
 
 }  // namespace b200moe

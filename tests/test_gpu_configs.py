@@ -416,3 +416,28 @@ def test_one_fused_launch_without_rows(ds_weights, T):
                 x.fill_(7.0)
         g.replay()
     check(outs)
+
+
+@pytest.mark.parametrize("T", [40, 200])
+def test_time_lines_of_one_launch_and_of_its_parts(ds_weights, T):
+    """Entry and exit of GEMM1's and GEMM2's time lines: the same where one launch does both, each launch's own where stage times split it
+    (GEMM2's CTAs enter after GEMM1's)."""
+    from justgoal_b200 import MoELayer
+    args = util.op_args(_inputs(T, ds_weights, seed=30 + T))
+    layer = MoELayer(I.DEEPSEEK_V3)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def lines():
+        layer.workspace(T).fill_(0xFF)
+        layer.forward(*args)
+        torch.cuda.synchronize()
+        assert layer.status(T) == 0
+        t = layer.view(T, "trace", torch.int64, (2, sms, 16)).cpu()
+        return t[:, :, 0], t[:, :, 11]
+
+    entry, cycles = lines()
+    assert torch.equal(entry[0], entry[1]) and torch.equal(cycles[0], cycles[1]) and int(cycles.min()) > 0
+    layer.profile_enable(1)
+    entry, cycles = lines()
+    assert int(entry.min()) > 0 and int(cycles.min()) > 0
+    assert int(entry[0].min()) < int(entry[1].min()) and not torch.equal(cycles[0], cycles[1])
