@@ -614,14 +614,17 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                     while (n > 1 && tail_units * n > slots) --n;
                     chunk_groups = min(chunk_groups, (NG + n - 1) / n);
                 }
-                // Units between half of the CTAs that can start at once and 5/8 of all are dealt out as one range per claim, which may
-                // end one unit and start the next: pieces of half a unit would be more than there are CTAs, and whole units leave a
-                // third of them without loads.  Pieces or whole / ranges, DeepSeek-V3 shape, median us: 4 experts (64 units, 116
-                // CTAs start at once) 48.9 / 44.3, 5 (80 units) 57.7 / 49.1; above the line 6 (96 units) 60.1 / 63.9, 7 (112)
-                // 67.9 / 68.7: GEMM2's loads fill what whole units leave.  Ranges from a third up were level (48 units 39.2 / 39.6).
+                // Units between a third of the CTAs that can start at once and 5/8 of all are dealt out as one range per claim, which
+                // may end one unit and start the next: equal pieces come out as half a unit each, or whole units, and leave a third of
+                // the CTAs without loads.  Two launches / one with equal pieces or whole units / one with ranges, median us: DeepSeek-V3
+                // shape, routed, 3 experts (48 units, 140 CTAs start at once) 38.0 / 39.6 / 38.8, 4 (64 units, 116 CTAs) 44.7 / 48.9 / 44.3,
+                // 5 (80 units) 49.9 / 57.7 / 49.2; forward, 3 experts 43.1 / 42.4 / 41.0; 4 experts of the 4096-wide shape (48 units) routed
+                // 30.8 / 32.3 / 31.8, forward 32.3 / 33.1 / 32.0.  Above the line 6 (96 units) 58.9 / 60.1 / 63.9, 7 (112) 64.1 / 63.8 / 68.7: GEMM2's loads
+                // fill what whole units leave.  Below it 2 (32 units) 32.7 / 33.3 / 33.4: what is left there is the claim that the
+                // start waits for.
                 int pieces = (NG + chunk_groups - 1) / chunk_groups;
                 const int parts = (int)gridDim.x - late;
-                if (WHICH == FIRST && sched_q == 0 && 2 * tail_units > parts && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= parts) {
+                if (WHICH == FIRST && sched_q == 0 && 3 * tail_units > parts && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= parts) {
                     chunk_groups = parts; pieces = 0;
                 }
                 if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = pieces; }

@@ -313,10 +313,10 @@ def test_routed_calls_take_the_tile_of_their_rows(ds_weights, T):
     assert layer.launches_routed_slots(8) == 5
 
 
-@pytest.mark.parametrize("experts", [1, 4, 5, 6, 8, 9])
+@pytest.mark.parametrize("experts", [1, 2, 3, 4, 5, 6, 8, 9])
 def test_few_units_in_one_launch(ds_weights, experts):
-    """16 to 144 units of GEMM1 for 148 CTAs: cut into equal pieces up to half as many units as CTAs, dealt out as ranges that may end
-    one unit and start the next up to 5/8 (four and five experts), whole above.  Against the two launches of the 128-token family,
+    """16 to 144 units of GEMM1 for 148 CTAs: cut into equal pieces up to a third as many units as CTAs that start at once, dealt out
+    as ranges that may end one unit and start the next up to 5/8 of all (three to five experts), whole above.  Against the two launches of the 128-token family,
     and the same bits twenty times on a poisoned workspace."""
     from justgoal_b200 import MoELayer
     T, K, E = 6, 8, I.DEEPSEEK_V3.num_experts
