@@ -589,7 +589,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
             // at most: with K of 16 blocks they stay whole, K of 32 (8 of a 4096 x 4096 shape, 64 tokens) 79.4 / 78.2, K of 64 (4 of
             // 5120 x 8192, 30 tokens) 117 with two launches, 106 with four pieces.
             // (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
-            volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, [1] pieces
+            volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, or the number of ranges, [1] pieces, or 0
             bool sized = false;
             auto size_chunks = [&]() {
                 constexpr int MOST = 8;
@@ -623,11 +623,11 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                 // fill what whole units leave.  Below it 2 (32 units) 32.7 / 33.3 / 33.4: what is left there is the claim that the
                 // start waits for.
                 int pieces = (NG + chunk_groups - 1) / chunk_groups;
-                const int parts = (int)gridDim.x - late;
-                if (WHICH == FIRST && sched_q == 0 && 3 * tail_units > parts && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= parts) {
-                    chunk_groups = parts; pieces = 0;
+                const int ranges = (int)gridDim.x - late;
+                if (WHICH == FIRST && sched_q == 0 && 3 * tail_units > ranges && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= ranges) {
+                    chunk_groups = ranges; pieces = 0;
                 }
-                if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = pieces; }
+                if (lane == 0) { s_sched[0] = chunk_groups; s_sched[1] = pieces; }       // no pieces: s_sched[0] ranges
                 __syncwarp();
                 sized = true;
             };
@@ -642,30 +642,34 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                 if (!have_ahead && lane == 0) ahead = claim0 + atomicAdd(claim, 1);
                 have_ahead = true;
             };
-            // Static tail: this CTA's range [t_lo, t_hi) of the flat (left-over unit, K group) space: the end of one unit
-            // and perhaps the start of the next.  What others wait for comes first, then the whole units, then the piece
-            // that ends a unit and waits itself (T=257: 214 -> 209 us against running it before the whole units).
-            int t_lo = 0, t_hi = 0, t_unit = 0, t_part = 0;
+            // A range [t_lo, t_hi) of the flat (left-over unit, K group) space, number t_part of `ranges` equal ones: the end of one unit
+            // and perhaps the start of the next.  What others wait for comes first, then the piece that ends a unit and waits itself.
+            // A static tail has one range per CTA, numbered like the CTAs, and its whole units between the two (T=257: 214 ->
+            // 209 us against running the waiting piece before the whole units); with both GEMMs in one launch a range is a claim of
+            // GEMM1's, and what it waits for are claims before it.
+            int t_lo = 0, t_hi = 0, t_unit = 0, t_part = (int)blockIdx.x;
             const int flat = (total_units - sched_U0) * NG;
             // Up to half as many units as CTAs are cut into the same number of pieces each, more into one range per CTA.  (A range
             // that crosses a unit's end leaves its CTA two pieces.  One range per CTA / equal pieces / equal pieces or whole units
             // whatever their number, us: 2 tokens 39.8 / 38.9 / 38.9, 16: 89.8 / 88.0 / 88.0, 24: 100.4 / 99.3 / 99.8, 128: 161.4 / 160.4 /
             // 160.0, 200: 185.1 / 186.1 / 182.2; 16 experts of the 4096-wide shape 64: 66.2 / 63.6 / 63.6; 8 of a 4096 x 4096 shape 128:
             // 83.5 / 83.7 / 85.7.)
-            const int parts = 2 * (total_units - sched_U0) > (int)gridDim.x || flat == 0
-                                  ? min(flat, (int)gridDim.x)
-                                  : (total_units - sched_U0) * min(NG, (int)gridDim.x / (total_units - sched_U0));
-            if (C::STATIC_TAIL && (int)blockIdx.x < parts) {
-                t_lo = range_start((int)blockIdx.x, flat, parts); t_hi = range_start((int)blockIdx.x + 1, flat, parts);
+            const int static_ranges = 2 * (total_units - sched_U0) > (int)gridDim.x || flat == 0
+                                          ? min(flat, (int)gridDim.x)
+                                          : (total_units - sched_U0) * min(NG, (int)gridDim.x / (total_units - sched_U0));
+            auto take_range = [&](int part, int ranges) {
+                t_part = part; t_lo = range_start(part, flat, ranges); t_hi = range_start(part + 1, flat, ranges);
                 t_unit = t_lo / NG;
-            }
+            };
+            if (C::STATIC_TAIL && (int)blockIdx.x < static_ranges) take_range((int)blockIdx.x, static_ranges);
 #pragma unroll 1
             while (ok) {
                 WorkItem wi;
                 wi.ut = wi.piece = wi.slot = 0; wi.pieces = 1; wi.un = Unit{0, 0, 0, 0}; wi.tile = 0;
                 const int u_end = (t_unit + 1) * NG;
                 const bool ends_unit = t_lo > t_unit * NG && t_hi == u_end;         // the rest of the range is such a piece
-                if (C::STATIC_TAIL && t_lo < t_hi && !(ends_unit && n_whole < sched_q)) {
+                if ((C::STATIC_TAIL || WHICH == FIRST) && t_lo < t_hi && !(C::STATIC_TAIL && ends_unit && n_whole < sched_q)) {
+                    const int ranges = C::STATIC_TAIL ? static_ranges : s_sched[0];
                     if (t_hi > u_end) {                       // the start of the next unit
                         wi.ut = t_unit + 1; wi.gb = 0; wi.ge = t_hi - u_end;
                         t_hi = u_end;
@@ -674,30 +678,10 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         t_lo = t_hi;
                     }
                     wi.u = sched_U0 + wi.ut;
-                    if (wi.ge < NG) {                         // does not end its unit: leaves its partial sum in its own slot
-                        wi.slot = (int)blockIdx.x; wi.pieces = 2;
-                    } else if (wi.gb > 0) {
-                        wi.slot = range_owner(wi.ut * NG, flat, parts);        // CTA of the unit's first piece
-                        wi.piece = (int)blockIdx.x - wi.slot; wi.pieces = wi.piece + 1;
-                    }
-                } else if (WHICH == FIRST && t_lo < t_hi) {
-                    // A claim of GEMM1 that is a range of the flat (unit, K group) space: what others wait for, the start of the next
-                    // unit, comes first, then the piece that ends a unit and waits itself, for claims before this one.
-                    const int parts = s_sched[0];
-                    t_unit = t_lo / NG;
-                    const int end = (t_unit + 1) * NG;
-                    if (t_hi > end) {
-                        wi.ut = t_unit + 1; wi.gb = 0; wi.ge = t_hi - end;
-                        t_hi = end;
-                    } else {
-                        wi.ut = t_unit; wi.gb = t_lo - t_unit * NG; wi.ge = t_hi - t_unit * NG;
-                        t_lo = t_hi;
-                    }
-                    wi.u = sched_U0 + wi.ut;
-                    if (wi.ge < NG) {                         // leaves its partial sum in the range's slot
+                    if (wi.ge < NG) {                         // does not end its unit: leaves its partial sum in the range's slot
                         wi.slot = t_part; wi.pieces = 2;
                     } else if (wi.gb > 0) {
-                        wi.slot = range_owner(wi.ut * NG, flat, parts);
+                        wi.slot = range_owner(wi.ut * NG, flat, ranges);       // range of the unit's first piece
                         wi.piece = t_part - wi.slot; wi.pieces = wi.piece + 1;
                     }
                 } else if (BOTH) {
@@ -715,7 +699,7 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                         }
                         c -= sched_U0;
                         if (WHICH == FIRST && pieces == 0) {
-                            t_part = c; t_lo = range_start(c, flat, chunk_groups); t_hi = range_start(c + 1, flat, chunk_groups);
+                            take_range(c, chunk_groups);
                             have_ahead = false;
                             continue;
                         }
@@ -756,7 +740,6 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                     return merged(n >= p.tile_want);
                 };
                 bool there = WHICH == SECOND && rows_done();
-                if (there) wi.tile = -1;                          // (others need not look)
                 if (!publish(wi)) { ok = false; break; }
                 const int gb = wi.gb, ge = wi.ge;
                 const Unit un = wi.un;
