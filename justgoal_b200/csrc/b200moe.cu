@@ -160,6 +160,8 @@ bool weights_stream(const b200moe_config& c) {
 //   32 (2.6)                                r=14 116/125/139, 20 152/128/142, 25 172/136/143, 32 204/178/144
 //   64 (5.2)                                r=9 208/238/247, 14 224/229/247, 20 295/246/252, 25 322/248/253, 32 362/320/257
 //   128 (10.4)                              r=6 388/471/455, 10 402/470/460, 14 471/497/467, 20 591/492/471
+// Two steps of units per SM stand for curves that move with every shape, so some sides of the lines are known to be the slower ones: 16
+// softmax experts at 26 to 34 rows (300 routed tokens 89 us with 128-token tiles, 78 with 32), 256 of 256 at 5 to 7 rows (2 to 4 %).
 // Layers whose weights L2 holds keep the lines at 7 and 9 rows, drawn with two launches.
 struct TileLines { double to32, to128; };
 TileLines tile_lines(const b200moe_ctx* h) {
@@ -228,9 +230,9 @@ int narrow_slots(const b200moe_config& c, int ntok) {
 }
 
 // Both GEMMs in one launch?  With narrow tiles and weights that L2 (126 MB) cannot hold, where the call is two streams from HBM
-// (both sides: head of gemm.cuh).  Smaller layers keep the two launches: they are ahead by up to 12 % in one launch as well where
-// they have many units (64 experts of 1024 x 512, 64 tokens 42.1 / 36.4 us; 512-wide 21.5 / 20.3), but the number of launches and of
-// pieces that a small layer makes is what this library has always stated, and the fused combine's bits go with them.
+// (both sides: head of gemm.cuh).  Smaller layers keep the two launches, although one was ahead by up to 12 % where it was tried (64
+// experts of 1024 x 512, 64 tokens, two / one 42.1 / 36.4 us; 512-wide 21.5 / 20.3): this line is one of compatibility (launch counts and
+// last bits of small layers as they were), not of speed.
 bool use_both(const b200moe_ctx* h, int ntok) {
     const b200moe_config& c = h->cfg;
     return ntok <= 32 && weights_stream(c) && narrow_slots(c, ntok) >= 2;
@@ -1233,7 +1235,8 @@ int b200moe_quantize_1x128(const void* x_bf16, int T, int H, void* q_e4m3, float
     // rows of few groups: more tokens, until all threads of a CTA have groups to work on (40000 x 128: eight tokens 25.1 us,
     // 64 tokens 4.7 us; 40000 x 512: 17.3 us with eight, 12.0 with 16)
     while (tpc * gpc < QUANT_TURN) tpc *= 2;
-    // Four tokens while eight leave fewer than eight CTAs per SM: the last CTAs of an SM are a smaller part of its work.  Eight / four, us: 3000 x
+    // Four tokens while eight leave fewer than eight CTAs per SM: the last CTAs of an SM are a smaller part of its work.  Eight / four, us in
+    // a row of quantiser calls: 3000 x
     // 7168 14.0 / 13.0, 4096: 17.7 / 17.6, 6000: 26.9 / 24.8, 8192: 33.5 / 33.6, 14107: 53.3 / 55.8; 3000 x 4096 10.2 / 8.5, 6000: 15.2 / 13.6, 14107: 31.3 / 31.7.
     if (tpc == QUANT_TOKENS && tpc / 2 * gpc >= QUANT_TURN && ctas(tpc, parts) < 8ll * sms) tpc /= 2;
     while (ctas(tpc, parts) < 2ll * sms && tpc > 1) tpc /= 2;

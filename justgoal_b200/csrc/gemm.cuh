@@ -47,8 +47,8 @@
 // has to be resident, whatever other streams run.  GEMM1's left-over units mostly stay whole, because the CTAs without one take up
 // GEMM2's units of the experts that are done.  A token tile's rows are handed over by a counter (tile_done).  us, two launches / one:
 // 32 of 256 experts 12 tokens 90 / 82, 64: 132 / 122, 128: 161 / 150, 200: 190 / 182; 128 of 256 experts 4: 136 / 127, 64: 450 / 440; 16
-// experts of the 4096-wide shape 16: 62.5 / 54.5, 128: 70.5 / 67.5; 4 of 5120 x 8192 30: 117 / 106.  It does not pay with one or two experts and
-// many CTAs to share them (routed, 1 token 32.7 / 34.0), nor with more units than a few per CTA (128 experts, 200 tokens 630 / 635).
+// experts of the 4096-wide shape 16: 62.5 / 54.5, 128: 70.5 / 67.5; 4 of 5120 x 8192 30: 117 / 106.  It is level with more units than a few per
+// CTA (128 experts, 200 tokens 609 / 610) and with two to five experts in use (both sides at size_chunks).
 //
 // Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer + TMEM owner (whole warps, one elected lane issues),
 // warps 2-3: scales of 128-token tiles on their way into shared memory, otherwise idle (they complete the first warpgroup so register
@@ -586,8 +586,10 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
             // because the front end runs on their SMs.  Pieces 1 / 2 / 3 / 4, us: 32 of 256 experts 2 tokens (32 units) 47 / 40 / 39 / 39, 4
             // (96) 65 / 68 / 63 / 68, 16 (160, of which 12 are left over; 8 pieces 83) 95 / 89 / 87 / 87, 128 (320) 152 / 153 / 153 / 157, 257 (400) 195 / 201 / 208 / 210;
             // 16 of the 4096-wide shape 1 (24) 33.9 / 30.3 / 29.6 / 28.7, 4 (72) 37.0 / 38.0 / 44.9 / 43.4.  GEMM2's are cut into pieces of 16 blocks
-            // at most: with K of 16 blocks they stay whole, K of 32 (8 of a 4096 x 4096 shape, 64 tokens) 79.4 / 78.2, K of 64 (4 of
-            // 5120 x 8192, 30 tokens) 117 with two launches, 106 with four pieces.
+            // at most (K of 32, 8 of a 4096 x 4096 shape, 64 tokens, whole / cut 79.4 / 78.2; K of 64, 4 of 5120 x 8192, 30 tokens, two launches /
+            // four pieces 117 / 106), and by the cost into smaller ones: 8 blocks a piece, but 5 where the whole launch has less than one of
+            // its units per CTA and the CTAs without one would idle (1 expert of the DeepSeek-V3 shape, 28 units of 16 blocks, whole /
+            // four pieces 32.4 / 30.3; 2 experts, 56 units, whole, which is what 7 blocks would do, / two pieces 35.9 / 34.5).
             // (Kept in shared memory between the rare claims rather than in registers for the whole loop.)
             volatile int* const s_sched = s_flag + 4;                      // [0] chunk_groups, or the number of ranges, [1] pieces, or 0
             bool sized = false;
@@ -620,8 +622,8 @@ __device__ __forceinline__ void gemm_roles(GemmCta& x, const CUtensorMap& tm_w, 
                 // shape, routed, 3 experts (48 units, 140 CTAs start at once) 38.0 / 39.6 / 38.8, 4 (64 units, 116 CTAs) 44.7 / 48.9 / 44.3,
                 // 5 (80 units) 49.9 / 57.7 / 49.2; forward, 3 experts 43.1 / 42.4 / 41.0; 4 experts of the 4096-wide shape (48 units) routed
                 // 30.8 / 32.3 / 31.8, forward 32.3 / 33.1 / 32.0.  Above the line 6 (96 units) 58.9 / 60.1 / 63.9, 7 (112) 64.1 / 63.8 / 68.7: GEMM2's loads
-                // fill what whole units leave.  Below it 2 (32 units) 32.7 / 33.3 / 33.4: what is left there is the claim that the
-                // start waits for.
+                // fill what whole units leave.  Below it 1 (16 units) 29.4 / 27.5 with pieces, 2 (32 units) 32.7 / 33.5 / 33.4: what is left
+                // there is the claim that the start waits for.
                 int pieces = (NG + chunk_groups - 1) / chunk_groups;
                 const int ranges = (int)gridDim.x - late;
                 if (WHICH == FIRST && sched_q == 0 && 3 * tail_units > ranges && 8 * tail_units <= 5 * (int)gridDim.x && tail_units <= ranges) {

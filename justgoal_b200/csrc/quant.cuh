@@ -13,8 +13,10 @@
 // store (one 4-byte store per group into the [H/128, T] layout touched a sector each).
 //
 // Launched with programmatic stream serialization: the kernel's start hides under the tail of the one before it (often the one
-// that writes x: nothing is read or written before the wait), and the layer that follows starts under this one.  4096 x 7168 20.4 ->
-// 17.6 us (5.0 TB/s), 2048: 12.3 -> 10.0, 14107: 55.3 -> 52.9.
+// that writes x: nothing is read or written before the wait), and the layer that follows starts under this one.  With four tokens per CTA
+// (the host's rule) in a row of calls of this kernel alone, where each starts under the one before it: 4096 x 7168 20.4 -> 17.6 us
+// (5.0 TB/s), 2048: 12.3 -> 10.0, 14107: 55.3 -> 52.9; through the public entry point, with the copies of other work around it,
+// 4096: 20.5 -> 19.0.
 //
 // The divisions.  Eight IEEE divisions per lane and 128 columns made the kernel instruction-bound (4096 x 7168: 30.8 us,
 // 2.9 TB/s).  With y = fl(1/s) a quotient needs three operations (Markstein, "IA-64 and Elementary Functions", ch. 8):
